@@ -90,27 +90,65 @@ __device__ __forceinline__ bool box_hit(float4 lo, float4 hi, F3 o, F3 inv, floa
     return true;
 }
 
+// The traversal's constants of a ray, in the form the box test reads them: (x, y) pairs
+// for the packed two-lane FP32 instructions.
+struct RayBox {
+    unsigned long long noxy, ixy;   // (-o.x, -o.y), (1/d.x, 1/d.y)
+    float noz, iz;
+    bool sx, sy, sz;                // 1/d < 0: the high plane is the near one
+};
+
+__device__ __forceinline__ unsigned long long pack2(float a, float b) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+// (a - o) * inv of two coordinates at once, each lane rounded as the scalar operations
+// round (a + (-o) is a - o)
+__device__ __forceinline__ void slab2(float ax, float ay, unsigned long long no, unsigned long long inv, float& tx,
+                                      float& ty) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pack2(ax, ay)), "l"(no));
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(r), "l"(inv));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(tx), "=f"(ty) : "l"(r));
+}
+__device__ __forceinline__ float max3f(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ float min3f(float a, float b, float c) {
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
+__device__ __forceinline__ RayBox ray_box(F3 o, F3 inv) {
+    return {pack2(-o.x, -o.y), pack2(inv.x, inv.y), -o.z, inv.z, inv.x < 0, inv.y < 0, inv.z < 0};
+}
+
 // box_hit in two parts: the same slab arithmetic, with the box's entry distance n
 // (tmin and the three near-slab distances, NaNs skipped, as box_hit folds them) kept.
 // box_hit's early exits never change its answer (the interval only narrows), so it
 // equals !(far < near) over all three slabs: box_entry returns exactly box_hit(tmax),
 // and for any tmax' <= tmax, box_hit(tmax') == box_entry(tmax) && !(tmax' < n).
-__device__ __forceinline__ bool box_entry(float4 lo, float4 hi, F3 o, F3 inv, float tmin, float tmax, float& n) {
-    float a = tmin, b = tmax;
-    float t0 = (lo.x - o.x) * inv.x, t1 = (hi.x - o.x) * inv.x;
-    if (inv.x < 0) { float s = t0; t0 = t1; t1 = s; }
-    a = t0 > a ? t0 : a;
-    b = t1 < b ? t1 : b;
-    t0 = (lo.y - o.y) * inv.y; t1 = (hi.y - o.y) * inv.y;
-    if (inv.y < 0) { float s = t0; t0 = t1; t1 = s; }
-    a = t0 > a ? t0 : a;
-    b = t1 < b ? t1 : b;
-    t0 = (lo.z - o.z) * inv.z; t1 = (hi.z - o.z) * inv.z;
-    if (inv.z < 0) { float s = t0; t0 = t1; t1 = s; }
-    a = t0 > a ? t0 : a;
-    b = t1 < b ? t1 : b;
-    n = a;
-    return !(b < a);
+// box_hit's folds `t > a ? t : a` and `t < b ? t : b` skip a NaN t, as the max and min
+// instructions do (a and b are never NaN), and the order of the folds does not matter;
+// the two differ only in the sign of a zero, which no comparison sees.
+// The traversal is issue- and latency-bound, and compares and selects run at half the
+// FP32 rate, so the test is kept to 8 packed or scalar FP32 operations, 6 selects, 6
+// (three-input) maxima and minima and one compare per box, against 12 + 6 + 12 + 3 with
+// the folds written as compare-and-select: light pass 12.97 -> 12.02 ms (water pool,
+// 16.7M paths), 40.9 -> 36.5 ms (2,000 gems, 4.2M paths).
+__device__ __forceinline__ bool box_entry(float4 lo, float4 hi, const RayBox& r, float tmin, float tmax, float& n) {
+    float lx, ly, hx, hy;
+    slab2(lo.x, lo.y, r.noxy, r.ixy, lx, ly);
+    slab2(hi.x, hi.y, r.noxy, r.ixy, hx, hy);
+    const float lz = (lo.z + r.noz) * r.iz, hz = (hi.z + r.noz) * r.iz;
+    const float near = max3f(r.sx ? hx : lx, r.sy ? hy : ly, r.sz ? hz : lz);
+    const float far = min3f(r.sx ? lx : hx, r.sy ? ly : hy, r.sz ? lz : hz);
+    n = fmaxf(near, tmin);
+    return !(fminf(far, tmax) < n);
 }
 
 // Möller-Trumbore as src/Triangle.cpp:44-66 computes it.
@@ -189,8 +227,9 @@ __device__ __forceinline__ bool mesh_traverse_children(const SceneView& s, int m
     const int root = __ldg(&s.mesh_root[mesh]);
     float4 lo = __ldg(&s.nodes[2 * root]);
     float4 hi = __ldg(&s.nodes[2 * root + 1]);
+    const RayBox rb = ray_box(o, inv);
     float n;
-    bool active = box_entry(lo, hi, o, inv, tmin, rec.t, n);
+    bool active = box_entry(lo, hi, rb, tmin, rec.t, n);
     int sp = 0;
     while (active) {
         const uint32_t w0 = __float_as_uint(lo.w), w1 = __float_as_uint(hi.w);
@@ -202,8 +241,8 @@ __device__ __forceinline__ bool mesh_traverse_children(const SceneView& s, int m
             const float4 llo = __ldg(&s.nodes[2 * w0]), lhi = __ldg(&s.nodes[2 * w0 + 1]);
             const float4 rlo = __ldg(&s.nodes[2 * w1]), rhi = __ldg(&s.nodes[2 * w1 + 1]);
             float nl, nr;
-            const bool hl = box_entry(llo, lhi, o, inv, tmin, rec.t, nl);
-            const bool hr = box_entry(rlo, rhi, o, inv, tmin, rec.t, nr);
+            const bool hl = box_entry(llo, lhi, rb, tmin, rec.t, nl);
+            const bool hr = box_entry(rlo, rhi, rb, tmin, rec.t, nr);
             if (hl && hr) {
                 if (sp >= kStackSize) { *overflow = 1; return false; }
                 stack[sp++] = make_int2((int)w1, __float_as_int(nr));
@@ -255,8 +294,9 @@ __device__ __forceinline__ bool mesh_traverse_steps(const SceneView& s, int mesh
     const int root = __ldg(&s.mesh_root[mesh]);
     float4 lo = __ldg(&s.nodes[2 * root]);
     float4 hi = __ldg(&s.nodes[2 * root + 1]);
+    const RayBox rb = ray_box(o, inv);
     float n;
-    bool active = box_entry(lo, hi, o, inv, tmin, rec.t, n);
+    bool active = box_entry(lo, hi, rb, tmin, rec.t, n);
     int sp = 0;
     bool ok = true;
     while (__any_sync(lanes, active)) {
@@ -267,8 +307,8 @@ __device__ __forceinline__ bool mesh_traverse_steps(const SceneView& s, int mesh
             const float4 llo = __ldg(&s.nodes[2 * w0]), lhi = __ldg(&s.nodes[2 * w0 + 1]);
             const float4 rlo = __ldg(&s.nodes[2 * w1]), rhi = __ldg(&s.nodes[2 * w1 + 1]);
             float nl, nr;
-            const bool hl = box_entry(llo, lhi, o, inv, tmin, rec.t, nl);
-            const bool hr = box_entry(rlo, rhi, o, inv, tmin, rec.t, nr);
+            const bool hl = box_entry(llo, lhi, rb, tmin, rec.t, nl);
+            const bool hr = box_entry(rlo, rhi, rb, tmin, rec.t, nr);
             if (hl && hr) {
                 if (sp < kStackSize) stack[sp++] = make_int2((int)w1, __float_as_int(nr));
                 else { *overflow = 1; ok = false; active = false; continue; }
