@@ -237,8 +237,7 @@ const char* rc_last_error(void);
  * [11] scene radius, [12] current merge radius, [13] kernel launches,
  * [14] photon-query distance tests in the gather, [15] photon chunks (of at most 32)
  * tested by the gather's query groups, [16] closest-hit queries (rays) the light pass
- * traced (persistent launch shapes; 0 for the wavefront pass, the Metropolis samplers
- * and a batch render).
+ * traced (0 for the Metropolis samplers and a batch render).
  * With the learned proposal, [8] is the proposal inference + training time.
  * With uniformly sampled light paths the camera pass runs on
  * a second stream beside the light pass and the KD build: its window [6] opens with the
@@ -288,10 +287,9 @@ int rc_trace_rays(int n, const float* origins, const float* directions, float tm
  * oracle): [hit, t, u, v, Ng xyz, Ns xyz, position xyz, front_face, material, tri]. */
 int rc_trace_rays_full(int n, const float* origins, const float* directions, float tmin, float* out);
 
-/* rc_trace_rays_full through a chosen traversal: 0 the persistent passes' (one lane per
- * ray, both children's boxes tested at the parent), 1 the wavefront pass's (the same
- * tests, a warp's lanes stepping one node at a time together), 2 the reference's own
- * form (pop a node, test its box).  All visit the reference's nodes in its order and
+/* rc_trace_rays_full through a chosen traversal: 0 the staged passes' (a warp's lanes in
+ * phases, both children's boxes tested at the parent), 1 the persistent passes' (the same
+ * tests, each lane on its own), 2 the reference's own form (pop a node, test its box).  All visit the reference's nodes in its order and
  * return its hits.  RC_E_INVALID for any other shape. */
 int rc_trace_rays_shape(int n, const float* origins, const float* directions, float tmin, float* out, int shape);
 
@@ -310,8 +308,8 @@ int rc_light_photons(int iteration, float* out, long long cap, long long* count)
 int rc_mlt_photons(int variant, int iteration, float* out, long long cap, long long* count,
                    unsigned long long* large_steps);
 
-/* rc_light_photons with the light pass in launch shape `shape` (0 .. 5: the persistent
- * pass's block/register shapes, 6 = the wavefront pass), for comparing them; the
+/* rc_light_photons with the light pass in launch shape `shape` (0 .. 3: the persistent
+ * pass's block/register shapes, 4 .. 6: the staged pass's), for comparing them; the
  * photons of every shape are the same, only their storage order differs. */
 int rc_light_photons_shape(int shape, int iteration, float* out, long long cap, long long* count);
 

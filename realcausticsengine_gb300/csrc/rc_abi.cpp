@@ -88,7 +88,7 @@ struct DeviceState {
     // light-path processing order (launch_light_order) and its scratch
     DevBuf<uint32_t> path_order;
     DevBuf<unsigned char> order_scratch;
-    DevBuf<unsigned char> wf_scratch;   // wavefront light pass: path state and queues
+    DevBuf<unsigned char> light_park, camera_park;   // parked paths of the staged passes
     // learned emission proposal
     std::unique_ptr<MlpStore> mlp;
     DevBuf<float4> prop, train_pos, train_dir;
@@ -127,7 +127,8 @@ struct DeviceState {
         box_lo.release(); box_hi.release();
         accum.release();
         image.release();
-        path_order.release(); order_scratch.release(); wf_scratch.release();
+        path_order.release(); order_scratch.release();
+        light_park.release(); camera_park.release();
         mlp.reset();
         prop.release(); train_pos.release(); train_dir.release(); contrib.release(); train_wsum.release();
         prop_table.release();
@@ -152,13 +153,19 @@ struct DeviceState {
     }
 };
 
-// Autotuner choices: launch variant per size class (log2 of light paths, pixels or
-// queries), -1 = untuned.  Kept for the process and shared by every context (a new
-// scene, or a scene in another context, reuses them).
+// Autotuner choices: launch variant per size class (log2 of light paths or pixels, and of
+// the scene's triangles; log2 of queries), -1 = untuned.  Kept for the process and shared
+// by every context (a new scene, or a scene in another context, reuses them).  The
+// triangles are in the key because the light and camera passes' best shape depends on how
+// long a search is: at 4.2M light paths 2,000 gems (261k triangles) run 20.7 ms staged
+// against 35.4, at 1M a glass sphere (20k) 0.53 ms staged against 0.38.
 struct TuneTables {
-    std::atomic<int> light[64], camera[64], gather[64];
+    std::atomic<int> light[64][32], camera[64][32], gather[64];
     TuneTables() {
-        for (int i = 0; i < 64; ++i) { light[i] = -1; camera[i] = -1; gather[i] = -1; }
+        for (int i = 0; i < 64; ++i) {
+            gather[i] = -1;
+            for (int j = 0; j < 32; ++j) { light[i][j] = -1; camera[i][j] = -1; }
+        }
     }
 };
 TuneTables g_tune;
@@ -605,24 +612,43 @@ int autotune_variants(int nvariants, Run&& run, const char* what, long long size
 }
 
 int size_class(long long n) { return n > 0 ? 63 - __builtin_clzll((unsigned long long)n) : 0; }
+std::atomic<int>& light_slot(long long paths) {
+    return g_tune.light[size_class(paths)][std::min(size_class(ctx().dev.num_tris), 31)];
+}
+std::atomic<int>& camera_slot(long long pixels) {
+    return g_tune.camera[size_class(pixels)][std::min(size_class(ctx().dev.num_tris), 31)];
+}
+constexpr int kUntunedPass = 2;   // the light and camera passes' shape where nothing was timed
 
-// The light pass in launch shape v: the persistent pass's shapes, or (v ==
-// pass_variants()) the wavefront pass with its path state in the context's scratch.
-// `tail`, if given, is recorded where work forked from it can fill the slots the pass
-// stops using: before the wavefront pass's last launch, before a persistent pass.
+// The scratch of a staged pass over n paths (nullptr for a persistent shape); a capturing
+// stream needs it reserved before (async_setup).
+int reserve_park(DevBuf<unsigned char>& b, int v, long long n, void** park) {
+    *park = nullptr;
+    if (!pass_is_staged(v)) return RC_OK;
+    RC_CUDA(b.reserve(pass_park_bytes(n)));
+    *park = b.p;
+    return RC_OK;
+}
+
+// The light pass in launch shape v.  `tail`, if given, is recorded first: work forked from
+// it takes the block slots that the pass's tail frees (measured 20.62 -> 20.53 ms per
+// water-pool iteration against forking after it).
 int light_pass(const VMParams& p, PhotonBuf ph, cudaStream_t s, int v, cudaEvent_t tail = nullptr) {
     DeviceState& d = ctx().dev;
-    if (v == pass_variants()) {
-        RC_CUDA(d.wf_scratch.reserve(light_wavefront_scratch_bytes(p.num_light_paths)));
-        RC_CUDA(cudaMemsetAsync(d.counters.p + 8, 0, sizeof(unsigned long long), s));   // (not counted)
-        launch_light_wavefront(p, ph, d.wf_scratch.p, s, tail);
-        return RC_OK;
-    }
-    // (the persistent pass holds every block slot until its pool drains: work forked
-    // before it takes the slots its tail frees; measured 20.62 -> 20.53 ms per water-pool
-    // iteration against forking after it)
+    void* park = nullptr;
+    const int r = reserve_park(d.light_park, v, p.num_light_paths, &park);
+    if (r) return r;
     if (tail) RC_CUDA(cudaEventRecord(tail, s));
-    launch_light_pass(p, ph, d.counters.p + 6, s, v, d.counters.p + 8);
+    launch_light_pass(p, ph, d.counters.p + 6, s, v, d.counters.p + 8, park);
+    return RC_OK;
+}
+
+int camera_pass(const VMParams& p, QueryBuf qb, cudaStream_t s, int v) {
+    DeviceState& d = ctx().dev;
+    void* park = nullptr;
+    const int r = reserve_park(d.camera_park, v, (long long)p.camera.width * p.camera.height, &park);
+    if (r) return r;
+    launch_camera_pass(p, qb, d.counters.p + 7, s, v, park);
     return RC_OK;
 }
 
@@ -698,7 +724,9 @@ int debug_bvh_obj(HostScene& sc) {
 // One progressive iteration with host round trips (counts read back, buffers grown on
 // overflow).  redo_iteration >= 0 renders that iteration index again without counting
 // it (an iteration an asynchronous replay had to skip).
-int render_iteration(HostScene& sc, int redo_iteration = -1) {
+// tune_passes false: the light and camera passes are not timed (the first iterations of a
+// batch's scenes, whose further ones run the batch's own passes).
+int render_iteration(HostScene& sc, int redo_iteration = -1, bool tune_passes = true) {
     DeviceState& d = ctx().dev;
     cudaStream_t s = d.stream;
     int r0 = RC_OK;
@@ -754,8 +782,9 @@ int render_iteration(HostScene& sc, int redo_iteration = -1) {
     // hidden; 8 per chain at 960x540: 4.75 ms per iteration serial against 5.28 beside)
     const bool mlt_long = (long long)cfg().mlt_chains * 64 <= p.num_light_paths;
     const bool cam_side = (sampler == RC_SAMPLER_UNIFORM || mlt_long) &&
-                          (!cfg().autotune || g_tune.camera[size_class(npix)].load() >= 0);
-    const int cam_var = cfg().autotune ? std::max(g_tune.camera[size_class(npix)].load(), 0) : 0;
+                          (!cfg().autotune || !tune_passes || camera_slot(npix).load() >= 0);
+    const int cam_tuned = cfg().autotune ? camera_slot(npix).load() : 0;
+    const int cam_var = cam_tuned >= 0 ? cam_tuned : kUntunedPass;
     if (cam_side) {
         RC_CUDA(d.q0.reserve(qcap)); RC_CUDA(d.q1.reserve(qcap)); RC_CUDA(d.q2.reserve(qcap));
         RC_CUDA(d.q3.reserve(qcap)); RC_CUDA(d.q4.reserve(qcap));
@@ -792,13 +821,13 @@ int render_iteration(HostScene& sc, int redo_iteration = -1) {
         }
         int lvar = 0;
         if (sampler == RC_SAMPLER_UNIFORM && cfg().autotune) {
-            std::atomic<int>& slot = g_tune.light[size_class(p.num_light_paths)];
-            if (slot.load() < 0)
-                slot = autotune_variants(pass_variants() + 1, [&](int v) {
+            std::atomic<int>& slot = light_slot(p.num_light_paths);
+            if (slot.load() < 0 && tune_passes)
+                slot = autotune_variants(pass_variants(), [&](int v) {
                     cudaMemsetAsync(d.counters.p, 0, sizeof(unsigned long long), s);
                     light_pass(p, ph, s, v);
                 }, "light pass", p.num_light_paths);
-            lvar = slot.load();
+            lvar = slot.load() >= 0 ? slot.load() : kUntunedPass;
             RC_CUDA(cudaMemsetAsync(d.counters.p, 0, sizeof(unsigned long long), s));
         }
         // the camera pass forks where the light pass stops filling the GPU
@@ -820,7 +849,8 @@ int render_iteration(HostScene& sc, int redo_iteration = -1) {
             RC_CUDA(cudaMemsetAsync(d.counters.p + 1, 0, sizeof(unsigned long long), d.side));
             QueryBuf qb{d.q0.p, d.q1.p, d.q2.p, d.q3.p, d.q4.p, qcap, d.counters.p + 1};
             RC_CUDA(cudaEventRecord(d.ev[4], d.side));
-            launch_camera_pass(p, qb, d.counters.p + 7, d.side, cam_var);
+            r0 = camera_pass(p, qb, d.side, cam_var);
+            if (r0) return r0;
             RC_CUDA(cudaGetLastError());
             RC_CUDA(cudaEventRecord(d.ev[5], d.side));
             RC_CUDA(cudaEventRecord(d.join, d.side));
@@ -903,17 +933,18 @@ int render_iteration(HostScene& sc, int redo_iteration = -1) {
         QueryBuf qb{d.q0.p, d.q1.p, d.q2.p, d.q3.p, d.q4.p, qcap, d.counters.p + 1};
         int cvar = 0;
         if (cfg().autotune) {
-            std::atomic<int>& slot = g_tune.camera[size_class(npix)];
-            if (slot.load() < 0)
+            std::atomic<int>& slot = camera_slot(npix);
+            if (slot.load() < 0 && tune_passes)
                 slot = autotune_variants(pass_variants(), [&](int v) {
                     cudaMemsetAsync(d.counters.p + 1, 0, sizeof(unsigned long long), s);
-                    launch_camera_pass(p, qb, d.counters.p + 7, s, v);
+                    camera_pass(p, qb, s, v);
                 }, "camera pass", npix);
-            cvar = slot.load();
+            cvar = slot.load() >= 0 ? slot.load() : kUntunedPass;
             RC_CUDA(cudaMemsetAsync(d.counters.p + 1, 0, sizeof(unsigned long long), s));
         }
         RC_CUDA(cudaEventRecord(d.ev[4], s));
-        launch_camera_pass(p, qb, d.counters.p + 7, s, cvar);
+        r = camera_pass(p, qb, s, cvar);
+        if (r) return r;
         RC_CUDA(cudaGetLastError());
         RC_CUDA(cudaEventRecord(d.ev[5], s));
         RC_CUDA(cudaMemcpyAsync(&nq, d.counters.p + 1, sizeof(nq), cudaMemcpyDeviceToHost, s));
@@ -1064,14 +1095,16 @@ int async_setup(const HostScene& sc) {
     RC_CUDA(d.qscratch.reserve(query_order_scratch_bytes(d.async_qcap)));
     RC_CUDA(d.accum.reserve(3 * npix));
     auto var = [](int v, int dflt) { return v >= 0 ? v : dflt; };
-    d.async_lvar = var(g_tune.light[size_class(cfg().photons_per_iter > 0 ? cfg().photons_per_iter : npix)].load(), 0);
-    d.async_cvar = var(g_tune.camera[size_class(npix)].load(), 0);
+    d.async_lvar = var(light_slot(cfg().photons_per_iter > 0 ? cfg().photons_per_iter : npix).load(), kUntunedPass);
+    d.async_cvar = var(camera_slot(npix).load(), kUntunedPass);
     d.async_gvar = var(g_tune.gather[size_class((long long)d.last_queries)].load(), gather_default_variant());
     if (!cfg().autotune) d.async_lvar = d.async_cvar = 0, d.async_gvar = gather_default_variant();
-    if (d.async_lvar == pass_variants()) {   // the wavefront pass's state: reserved before any capture
-        const long long paths = cfg().photons_per_iter > 0 ? cfg().photons_per_iter : npix;
-        RC_CUDA(d.wf_scratch.reserve(light_wavefront_scratch_bytes(paths)));
-    }
+    // the staged passes' scratch: reserved before any capture
+    const long long paths = cfg().photons_per_iter > 0 ? cfg().photons_per_iter : npix;
+    void* park = nullptr;
+    int r = reserve_park(d.light_park, d.async_lvar, paths, &park);
+    if (!r) r = reserve_park(d.camera_park, d.async_cvar, npix, &park);
+    if (r) return r;
     return RC_OK;
 }
 
@@ -1149,7 +1182,8 @@ int enqueue_async_iteration(HostScene& sc, int it, int* flag) {
     RC_CUDA(record(d.ev[1], s));
     RC_CUDA(cudaStreamWaitEvent(d.side, d.fork, 0));
     RC_CUDA(record(d.ev[4], d.side));
-    launch_camera_pass(p, qb, d.counters.p + 7, d.side, d.async_cvar);
+    r = camera_pass(p, qb, d.side, d.async_cvar);
+    if (r) return r;
     RC_CUDA(record(d.ev[5], d.side));
     RC_CUDA(cudaEventRecord(d.join, d.side));
     return async_tail(sc, p, s, d.join, flag);
@@ -1316,10 +1350,12 @@ struct BatchRun {
     DevBuf<BatchScene> scenes;          // per graph iteration: its scenes' entries, end to end
     DevBuf<long long> prefix;           // per graph iteration: path prefix (m + 1), pixel prefix (m + 1)
     DevBuf<unsigned long long> next;    // [0] next light path, [1] next pixel
+    DevBuf<unsigned char> light_park, camera_park;   // parked paths of the staged passes
     cudaGraphExec_t exec = nullptr;
     ~BatchRun() {
         if (exec) cudaGraphExecDestroy(exec);
         scenes.release(); prefix.release(); next.release();
+        light_park.release(); camera_park.release();
         for (cudaEvent_t e : {start, light, camera, join, cam_fork, t0, t1, light_start, light_end, camera_start,
                               camera_end})
             if (e) cudaEventDestroy(e);
@@ -1374,7 +1410,7 @@ int batch_render(Context* const* cs, int n, int iterations, double* out) {
         pcap_was[i] = d.async_pcap < 0 ? -1 : 0;
         if (d.async_pcap <= 0) {
             if (d.iterations_done == 0 && remaining[i] > 0) {
-                r = render_iteration(sc);
+                r = render_iteration(sc, -1, false);
                 if (r) return scene_fail(i, r);
                 remaining[i]--;
             }
@@ -1434,6 +1470,11 @@ int batch_render(Context* const* cs, int n, int iterations, double* out) {
     RC_CUDA(B.scenes.reserve(entries.size()));
     RC_CUDA(B.prefix.reserve(prefix.size()));
     RC_CUDA(B.next.reserve(2));
+    const bool tuned = g_batch_light.load() >= 0 && g_batch_camera.load() >= 0;
+    if (!tuned || pass_is_staged(g_batch_light.load()))
+        RC_CUDA(B.light_park.reserve(pass_park_bytes(*std::max_element(total_paths.begin(), total_paths.end()))));
+    if (!tuned || pass_is_staged(g_batch_camera.load()))
+        RC_CUDA(B.camera_park.reserve(pass_park_bytes(*std::max_element(total_pixels.begin(), total_pixels.end()))));
     RC_CUDA(cudaMemcpy(B.scenes.p, entries.data(), entries.size() * sizeof(BatchScene), cudaMemcpyHostToDevice));
     RC_CUDA(cudaMemcpy(B.prefix.p, prefix.data(), prefix.size() * sizeof(long long), cudaMemcpyHostToDevice));
     RC_CUDA(cudaStreamCreateWithFlags(&B.main, cudaStreamNonBlocking));
@@ -1481,11 +1522,11 @@ int batch_render(Context* const* cs, int n, int iterations, double* out) {
         };
         g_batch_light = tune([&](int v) {
             reset(0);
-            launch_light_pass_batch(sc0, pp, m, total_paths[0], B.next.p, B.main, v);
+            launch_light_pass_batch(sc0, pp, m, total_paths[0], B.next.p, B.main, v, B.light_park.p);
         });
         g_batch_camera = tune([&](int v) {
             reset(1);
-            launch_camera_pass_batch(sc0, pp + m + 1, m, total_pixels[0], B.next.p + 1, B.main, v);
+            launch_camera_pass_batch(sc0, pp + m + 1, m, total_pixels[0], B.next.p + 1, B.main, v, B.camera_park.p);
         });
         RC_CUDA(cudaStreamSynchronize(B.main));
         RC_CUDA(cudaGetLastError());
@@ -1520,13 +1561,13 @@ int batch_render(Context* const* cs, int n, int iterations, double* out) {
             RC_CUDA(cudaEventRecord(B.cam_fork, B.main));
             RC_CUDA(record(B.light_start, B.main));
             launch_light_pass_batch(B.scenes.p + entry_at[j], B.prefix.p + prefix_at[j], m, total_paths[j], B.next.p,
-                                    B.main, lvar);
+                                    B.main, lvar, B.light_park.p);
             RC_CUDA(record(B.light_end, B.main));
             RC_CUDA(cudaEventRecord(B.light, B.main));
             RC_CUDA(cudaStreamWaitEvent(B.side, B.cam_fork, 0));
             RC_CUDA(record(B.camera_start, B.side));
             launch_camera_pass_batch(B.scenes.p + entry_at[j], B.prefix.p + prefix_at[j] + m + 1, m, total_pixels[j],
-                                     B.next.p + 1, B.side, cvar);
+                                     B.next.p + 1, B.side, cvar, B.camera_park.p);
             RC_CUDA(record(B.camera_end, B.side));
             RC_CUDA(cudaEventRecord(B.camera, B.side));
             for (int a = 0; a < m; ++a) {
@@ -2184,7 +2225,8 @@ int rc_camera_queries(int iteration, float* out, long long cap, long long* count
         RC_CUDA(d.counters.reserve(10));
         RC_CUDA(cudaMemsetAsync(d.counters.p + 1, 0, sizeof(unsigned long long), s));
         QueryBuf qb{d.q0.p, d.q1.p, d.q2.p, d.q3.p, d.q4.p, (long long)d.q0.n, d.counters.p + 1};
-        launch_camera_pass(p, qb, d.counters.p + 7, s);
+        r = camera_pass(p, qb, s, 0);
+        if (r) return r;
         RC_CUDA(cudaGetLastError());
         RC_CUDA(cudaMemcpyAsync(&nq, d.counters.p + 1, sizeof(nq), cudaMemcpyDeviceToHost, s));
         RC_CUDA(cudaStreamSynchronize(s));
@@ -2207,7 +2249,7 @@ int rc_light_photons_shape(int shape, int iteration, float* out, long long cap, 
     int r = prepare();
     if (r) return r;
     if (iteration < 0 || (cap > 0 && !out)) { ctx().err = "bad photon output"; return RC_E_INVALID; }
-    if (shape < 0 || shape > pass_variants()) { ctx().err = "light pass shape out of range"; return RC_E_INVALID; }
+    if (shape < 0 || shape >= pass_variants()) { ctx().err = "light pass shape out of range"; return RC_E_INVALID; }
     HostScene& sc = *ctx().scene;
     DeviceState& d = ctx().dev;
     cudaStream_t s = d.stream;
@@ -2311,14 +2353,16 @@ int rc_trace_rays(int n, const float* origins, const float* directions, float tm
     cudaStream_t s = ctx().dev.stream;
     DevBuf<float> o, d;
     DevBuf<unsigned> w;
+    DevBuf<HitRec> h;
     RC_CUDA(o.reserve(3 * (size_t)n)); RC_CUDA(d.reserve(3 * (size_t)n)); RC_CUDA(w.reserve(8 * (size_t)n));
+    RC_CUDA(h.reserve((size_t)n));
     RC_CUDA(cudaMemcpyAsync(o.p, origins, 12 * (size_t)n, cudaMemcpyHostToDevice, s));
     RC_CUDA(cudaMemcpyAsync(d.p, directions, 12 * (size_t)n, cudaMemcpyHostToDevice, s));
-    launch_trace_rays(ctx().dev.view, n, o.p, d.p, tmin, nullptr, w.p, ctx().dev.errors.p, s);
+    launch_trace_rays(ctx().dev.view, n, o.p, d.p, tmin, h.p, nullptr, w.p, ctx().dev.errors.p, s);
     RC_CUDA(cudaGetLastError());
     RC_CUDA(cudaMemcpyAsync(out, w.p, 32 * (size_t)n, cudaMemcpyDeviceToHost, s));
     RC_CUDA(cudaStreamSynchronize(s));
-    o.release(); d.release(); w.release();
+    o.release(); d.release(); w.release(); h.release();
     return check_errors();
 }
 
@@ -2334,14 +2378,16 @@ int rc_trace_rays_shape(int n, const float* origins, const float* directions, fl
     if (n == 0) return RC_OK;
     cudaStream_t s = ctx().dev.stream;
     DevBuf<float> o, d, f;
+    DevBuf<HitRec> h;
     RC_CUDA(o.reserve(3 * (size_t)n)); RC_CUDA(d.reserve(3 * (size_t)n)); RC_CUDA(f.reserve(16 * (size_t)n));
+    RC_CUDA(h.reserve((size_t)n));
     RC_CUDA(cudaMemcpyAsync(o.p, origins, 12 * (size_t)n, cudaMemcpyHostToDevice, s));
     RC_CUDA(cudaMemcpyAsync(d.p, directions, 12 * (size_t)n, cudaMemcpyHostToDevice, s));
-    launch_trace_rays(ctx().dev.view, n, o.p, d.p, tmin, f.p, nullptr, ctx().dev.errors.p, s, shape);
+    launch_trace_rays(ctx().dev.view, n, o.p, d.p, tmin, h.p, f.p, nullptr, ctx().dev.errors.p, s, shape);
     RC_CUDA(cudaGetLastError());
     RC_CUDA(cudaMemcpyAsync(out, f.p, 64 * (size_t)n, cudaMemcpyDeviceToHost, s));
     RC_CUDA(cudaStreamSynchronize(s));
-    o.release(); d.release(); f.release();
+    o.release(); d.release(); f.release(); h.release();
     return check_errors();
 }
 

@@ -6,9 +6,8 @@
 // aabb::hit (src/aabb.cpp:6-41) and Triangle::hit (src/Triangle.cpp:20-88):
 //  * stack DFS, right child pushed before left, so the left subtree is visited first;
 //  * every box is tested against the current closest distance of its own level (the
-//    warp-stepped mesh traversal tests both children's boxes at their parent and keeps
-//    the right one's entry distance on the stack: mesh_traverse_steps says why that is
-//    the same test);
+//    passes test both children's boxes at their parent and keep the right one's entry
+//    distance on the stack: mesh_traverse_children says why that is the same test);
 //  * a world leaf starts a fresh record (distance = inf) and, if any of its meshes is
 //    hit, OVERWRITES the running result - so the answer is the last hit world leaf's
 //    closest triangle, exactly as the reference returns it;
@@ -44,21 +43,17 @@ struct SceneView {
 constexpr int kStackSize = 64;   // BVH_STACK_SIZE in the reference
 
 // Traversal stacks.  LocalStack / LocalPairStack: per-thread arrays (local memory),
-// declared by each mesh traversal when the caller passes the CallStack or
-// WarpStepStack tag, so that their lifetime is the traversal.  (Stacks held for a
-// whole persistent kernel, or kept in shared memory as [kStackSize][block] columns,
-// measured 1.5-3.6x slower on the water workload.)  Any type with int& operator[] can
-// serve as the stack of mesh_traverse_impl.
+// declared by each mesh traversal when the caller passes the CallStack tag, so that
+// their lifetime is the traversal.  (Stacks kept in shared memory as
+// [kStackSize][block] columns measured 1.5-3.6x slower on the water workload.)  Any
+// type with int& operator[] can serve as the stack of mesh_traverse_impl.
 struct LocalStack {
     int s[kStackSize];
     __device__ __forceinline__ int& operator[](int i) { return s[i]; }
 };
 // CallStack: the tag of the persistent passes' traversal (mesh_traverse_children).
 struct CallStack {};
-// WarpStepStack: the tag of the warp-stepped traversal (mesh_traverse_steps), for
-// kernels whose lanes all trace at once; its per-traversal stack holds node index and
-// box entry distance (float bits) per entry.
-struct WarpStepStack {};
+// Its per-traversal stack: node index and box entry distance (float bits) per entry.
 struct LocalPairStack {
     int2 s[kStackSize];
     __device__ __forceinline__ int2& operator[](int i) { return s[i]; }
@@ -214,12 +209,17 @@ __device__ __forceinline__ bool mesh_traverse_impl(const SceneView& s, int mesh,
 
 // Mesh::hit (src/mesh.cpp:70-105) visits nodes in left-first DFS order and tests each
 // box when it is popped, against the running distance then.  mesh_traverse_children
-// (the persistent passes, one lane per ray) and mesh_traverse_steps (the wavefront
-// pass, a warp's lanes stepping together) test both children's boxes at their parent
-// instead, with the same outcome (below).  Measured on the water pool (light pass per
-// iteration): pop-and-test (mesh_traverse_impl) 13.3 ms, children tested at the parent
-// 11.9 ms, the same with a warp's lanes stepping together (mesh_traverse_steps) 13.3
-// ms, four-wide records of grandchildren tested at the grandparent 14.7 ms.
+// (the persistent passes, one lane per ray) and search_run (the staged passes, a warp's
+// lanes in phases) test both children's boxes at their parent instead, with the same
+// outcome: the left child is the node the reference pops next, with the same distance, so
+// its test is the reference's; the right child is popped only after the left subtree, when
+// the distance may have shrunk.  The distance never grows, so a right box that fails now
+// fails then too (box_hit is monotone in tmax) and is not pushed; one that passes is
+// pushed with its entry distance n, and at its pop the reference's test is
+// !(distance < n) (box_entry).  Same nodes, same triangles, same order.
+// Measured on the water pool (light pass per iteration): pop-and-test
+// (mesh_traverse_impl) 13.3 ms, children tested at the parent 11.9 ms, four-wide records
+// of grandchildren tested at the grandparent 14.7 ms.
 template <class Stack>
 __device__ __forceinline__ bool mesh_traverse_children(const SceneView& s, int mesh, F3 o, F3 d, F3 inv,
                                                        float tmin, HitRec& rec, bool& any, int* overflow,
@@ -278,72 +278,6 @@ __device__ __forceinline__ bool mesh_traverse_children(const SceneView& s, int m
     return true;
 }
 
-// Why testing the children at their parent gives the reference's result: the left
-// child is the node the reference pops next, with the same distance, so its test is
-// the reference's; the right child is popped only after the left subtree, when the
-// distance may have shrunk.  The distance never grows, so a right box that fails now
-// fails then too (box_hit is monotone in tmax) and is not pushed; one that passes is
-// pushed with its entry distance n, and at its pop the reference's test is
-// !(distance < n) (box_entry).  Same nodes, same triangles, same order.
-template <class Stack>
-__device__ __forceinline__ bool mesh_traverse_steps(const SceneView& s, int mesh, F3 o, F3 d, F3 inv, float tmin,
-                                                   HitRec& rec, bool& any, int* overflow, Stack& stack) {
-    // the lanes that arrive together step together: one node per lane per round, the
-    // round ending in a vote, so that a warp's lanes meet again after every node
-    const unsigned lanes = __activemask();
-    const int root = __ldg(&s.mesh_root[mesh]);
-    float4 lo = __ldg(&s.nodes[2 * root]);
-    float4 hi = __ldg(&s.nodes[2 * root + 1]);
-    const RayBox rb = ray_box(o, inv);
-    float n;
-    bool active = box_entry(lo, hi, rb, tmin, rec.t, n);
-    int sp = 0;
-    bool ok = true;
-    while (__any_sync(lanes, active)) {
-        if (!active) continue;
-        const uint32_t w0 = __float_as_uint(lo.w), w1 = __float_as_uint(hi.w);
-        bool descend = false;
-        if (!(w0 & 0x80000000u)) {
-            const float4 llo = __ldg(&s.nodes[2 * w0]), lhi = __ldg(&s.nodes[2 * w0 + 1]);
-            const float4 rlo = __ldg(&s.nodes[2 * w1]), rhi = __ldg(&s.nodes[2 * w1 + 1]);
-            float nl, nr;
-            const bool hl = box_entry(llo, lhi, rb, tmin, rec.t, nl);
-            const bool hr = box_entry(rlo, rhi, rb, tmin, rec.t, nr);
-            if (hl && hr) {
-                if (sp < kStackSize) stack[sp++] = make_int2((int)w1, __float_as_int(nr));
-                else { *overflow = 1; ok = false; active = false; continue; }
-            }
-            descend = hl || hr;
-            lo = hl ? llo : rlo;
-            hi = hl ? lhi : rhi;
-        } else {
-            const int cnt = (int)(w0 & 0x7fffffffu);
-            for (int k = 0; k < cnt; ++k) {
-                const int slot = (int)w1 + k;
-                float t, u, v;
-                if (tri_hit(s, slot, o, d, tmin, rec.t, t, u, v)) {
-                    rec.t = t; rec.u = u; rec.v = v; rec.slot = slot;
-                    any = true;
-                }
-            }
-        }
-        if (!descend) {
-            // pop pending right children until one whose box the current distance reaches
-            int next = -1;
-            while (sp > 0 && next < 0) {
-                const int2 e = stack[--sp];
-                if (!(rec.t < __int_as_float(e.y))) next = e.x;
-            }
-            active = next >= 0;
-            if (active) {
-                lo = __ldg(&s.nodes[2 * next]);
-                hi = __ldg(&s.nodes[2 * next + 1]);
-            }
-        }
-    }
-    return ok;
-}
-
 template <class Stack>
 __device__ __forceinline__ bool mesh_traverse(const SceneView& s, int mesh, F3 o, F3 d, F3 inv, float tmin,
                                               HitRec& rec, bool& any, int* overflow, Stack& stack) {
@@ -355,13 +289,6 @@ __device__ __forceinline__ bool mesh_traverse<CallStack>(const SceneView& s, int
                                                          CallStack&) {
     LocalPairStack st;
     return mesh_traverse_children(s, mesh, o, d, inv, tmin, rec, any, overflow, st);
-}
-template <>
-__device__ __forceinline__ bool mesh_traverse<WarpStepStack>(const SceneView& s, int mesh, F3 o, F3 d, F3 inv,
-                                                             float tmin, HitRec& rec, bool& any, int* overflow,
-                                                             WarpStepStack&) {
-    LocalPairStack st;
-    return mesh_traverse_steps(s, mesh, o, d, inv, tmin, rec, any, overflow, st);
 }
 
 // Scene::hit.  `out` is the reported record (t = inf when nothing was hit).  `stack`
@@ -417,6 +344,134 @@ __device__ __forceinline__ bool scene_hit(const SceneView& s, F3 o, F3 d, float 
         }
     }
     return hit;
+}
+
+// Scene::hit as a state machine: one lane's search, put down and taken up between nodes,
+// so that a warp can run its lanes' searches in phases (search_run) and lanes whose
+// search has ended can shade and start new rays while the others' searches wait.  Each
+// search visits the nodes and triangles that scene_hit visits, in the same order, with
+// the same tests.
+constexpr uint32_t kLeafFlag = 0x80000000u;     // as in the node words
+constexpr uint32_t kSearchIdle = 0xffffffffu;
+struct SearchStack {
+    int2 s[kStackSize];    // waiting right children: node, entry distance
+    int w[kStackSize];     // waiting world nodes
+};
+struct Search {
+    RayBox rb;             // the ray's (negated) origin and reciprocals
+    HitRec rec, out;       // the current world leaf's record; the reported hit so far
+    uint32_t w0, w1;       // current node: child indices, or kLeafFlag | triangles left, next slot;
+                           // kLeafFlag alone: between meshes; kSearchIdle: no search
+    int sp;                // waiting right children
+    int mesh, mesh_end;    // rest of the current leaf's mesh list
+    int wsp;               // waiting world nodes
+    __device__ __forceinline__ F3 origin() const {
+        float nx, ny;
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(nx), "=f"(ny) : "l"(rb.noxy));
+        return {-nx, -ny, -rb.noz};
+    }
+};
+
+__device__ __forceinline__ void search_begin(Search& q, SearchStack& st, F3 o, F3 d) {
+    q.rb = ray_box(o, F3{1.0f / d.x, 1.0f / d.y, 1.0f / d.z});
+    q.rec = q.out = HitRec{INFINITY, 0.0f, 0.0f, -1};
+    q.w0 = kLeafFlag;
+    q.sp = 0;
+    q.mesh = q.mesh_end = 0;
+    st.w[0] = 0;
+    q.wsp = 1;
+}
+
+// Between meshes: on to the next mesh whose root box the ray enters, or idle: the search has
+// ended and q.out is the reported hit.  A world leaf starts a fresh record and overwrites
+// the reported one if any of its meshes was hit.
+__device__ __forceinline__ void search_world(const SceneView& s, Search& q, SearchStack& st, float tmin,
+                                             int* overflow) {
+    for (;;) {
+        float n;
+        if (q.mesh < q.mesh_end) {
+            const int root = __ldg(&s.mesh_root[__ldg(&s.world_mesh[q.mesh++])]);
+            const float4 lo = __ldg(&s.nodes[2 * root]), hi = __ldg(&s.nodes[2 * root + 1]);
+            if (!box_entry(lo, hi, q.rb, tmin, q.rec.t, n)) continue;
+            q.w0 = __float_as_uint(lo.w);
+            q.w1 = __float_as_uint(hi.w);
+            return;
+        }
+        if (q.rec.slot >= 0) q.out = q.rec;
+        q.rec = HitRec{INFINITY, 0.0f, 0.0f, -1};
+        if (q.wsp == 0) { q.w0 = kSearchIdle; return; }
+        const int id = st.w[--q.wsp];
+        const float4 lo = __ldg(&s.wnode_lo[id]), hi = __ldg(&s.wnode_hi[id]);
+        if (!box_entry(lo, hi, q.rb, tmin, q.out.t, n)) continue;
+        const uint32_t w0 = __float_as_uint(lo.w), w1 = __float_as_uint(hi.w);
+        if (w0 & kLeafFlag) {
+            q.mesh = (int)w1;
+            q.mesh_end = (int)(w1 + (w0 & ~kLeafFlag));
+        } else {
+            if (q.wsp + 2 > kStackSize) { *overflow = 1; q.out.slot = -1; q.w0 = kSearchIdle; return; }
+            st.w[q.wsp++] = (int)w1;
+            st.w[q.wsp++] = (int)w0;
+        }
+    }
+}
+
+// The next waiting right child that the current distance reaches, or between meshes.
+__device__ __forceinline__ void search_pop(const SceneView& s, Search& q, SearchStack& st) {
+    q.w0 = kLeafFlag;
+    while (q.sp > 0) {
+        const int2 e = st.s[--q.sp];
+        if (q.rec.t < __int_as_float(e.y)) continue;
+        q.w0 = __float_as_uint(__ldg(&s.nodes[2 * e.x].w));
+        q.w1 = __float_as_uint(__ldg(&s.nodes[2 * e.x + 1].w));
+        break;
+    }
+}
+
+// A warp's searches (every lane of the warp calls it), until at most `keep` lanes still
+// search.  Per round, the lanes at inner nodes test their two children, or the lanes at
+// leaves test their next triangle, or the lanes between meshes go on to their next one,
+// whichever are the most; lanes that have nothing left below take their next waiting node.
+// (A lane per ray in a plain loop runs a warp's inner, leaf and between-mesh code in turn
+// for the few lanes that need each: 9.4 lanes active on average on the water pool, 15.4 in
+// phases.  Up to kInnerSteps node steps go between two votes: 1, 2, 3 steps 9.8, 9.8, 9.6
+// ms of light pass.)
+constexpr int kInnerSteps = 3;
+__device__ __forceinline__ void search_run(const SceneView& s, Search& q, SearchStack& st, F3 d, float tmin, int keep,
+                                           int* overflow) {
+    for (;;) {
+        const unsigned idle = __ballot_sync(0xffffffffu, q.w0 == kSearchIdle);
+        if (32 - __popc(idle) <= keep) break;
+        const unsigned inner = __ballot_sync(0xffffffffu, (int)q.w0 >= 0);
+        const unsigned between = __ballot_sync(0xffffffffu, q.w0 == kLeafFlag);
+        const int ni = __popc(inner), nb = __popc(between), nl = 32 - __popc(idle | inner | between);
+        if (ni >= nl && ni >= nb) {
+#pragma unroll 1
+            for (int k = 0; k < kInnerSteps; ++k)
+                if ((int)q.w0 >= 0) {
+                    const float4 llo = __ldg(&s.nodes[2 * q.w0]), lhi = __ldg(&s.nodes[2 * q.w0 + 1]);
+                    const float4 rlo = __ldg(&s.nodes[2 * q.w1]), rhi = __ldg(&s.nodes[2 * q.w1 + 1]);
+                    float el, er;
+                    const bool hl = box_entry(llo, lhi, q.rb, tmin, q.rec.t, el);
+                    const bool hr = box_entry(rlo, rhi, q.rb, tmin, q.rec.t, er);
+                    const bool push = hl && hr, full = q.sp >= kStackSize;
+                    if (push && !full) st.s[q.sp++] = make_int2((int)q.w1, __float_as_int(er));
+                    q.w0 = __float_as_uint(hl ? llo.w : rlo.w);
+                    q.w1 = __float_as_uint(hl ? lhi.w : rhi.w);
+                    if (!(hl || hr)) search_pop(s, q, st);
+                    if (push && full) { *overflow = 1; q.out.slot = -1; q.w0 = kSearchIdle; }
+                }
+        } else if (nl >= nb) {
+            if ((int)q.w0 < 0 && q.w0 != kLeafFlag && q.w0 != kSearchIdle) {
+                float t, u, v;
+                if (tri_hit(s, (int)q.w1, q.origin(), d, tmin, q.rec.t, t, u, v)) q.rec = HitRec{t, u, v, (int)q.w1};
+                --q.w0;
+                ++q.w1;
+                if (q.w0 == kLeafFlag) search_pop(s, q, st);
+            }
+        } else if (q.w0 == kLeafFlag) {
+            search_world(s, q, st, tmin, overflow);
+        }
+    }
 }
 
 // Scene::hit with per-traversal local-memory stacks.

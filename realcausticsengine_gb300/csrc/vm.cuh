@@ -113,20 +113,22 @@ void launch_light_order(const VMParams& p, void* scratch, uint32_t* order, cudaS
 // with tile_scratch (scan_scratch_words(m) words) for the tile totals.
 size_t scan_scratch_words(long long m);
 void launch_scan_counts(uint32_t* counts, long long m, uint32_t* tile_scratch, cudaStream_t s);
-// next_path: device counter for the persistent kernel (nullptr: one thread per path);
-// rays (optional): receives the number of closest-hit queries the pass traced.
+// next_path: device counter for the persistent shapes; rays (optional): receives the number
+// of closest-hit queries the pass traced; park: scratch of the staged shapes
+// (pass_park_bytes of the paths or pixels), without which a staged shape runs as shape 0.
 void launch_light_pass(const VMParams& p, PhotonBuf ph, unsigned long long* next_path, cudaStream_t s, int variant = 0,
-                       unsigned long long* rays = nullptr);
-void launch_camera_pass(const VMParams& p, QueryBuf qb, unsigned long long* next_pixel, cudaStream_t s, int variant = 0);
-// The persistent light and camera passes over n resident scenes in one launch each:
-// scenes[i] (device memory) holds scene i's parameters and buffers, path_prefix
-// (pixel_prefix) n + 1 device words with the first work index of each scene and the
-// total at [n].  A scene's photons (queries) are the ones its own pass stores, in
-// another order.  variant: the launch shapes of the single-scene passes (0-4).
+                       unsigned long long* rays = nullptr, void* park = nullptr);
+void launch_camera_pass(const VMParams& p, QueryBuf qb, unsigned long long* next_pixel, cudaStream_t s, int variant = 0,
+                        void* park = nullptr);
+// The light and camera passes over n resident scenes: scenes[i] (device memory) holds
+// scene i's parameters and buffers, path_prefix (pixel_prefix) n + 1 device words with the
+// first work index of each scene and the total at [n].  A scene's photons (queries) are
+// the ones its own pass stores, in another order.  variant: the launch shapes of the
+// single-scene passes.
 void launch_light_pass_batch(const BatchScene* scenes, const long long* path_prefix, int n, long long total_paths,
-                             unsigned long long* next_path, cudaStream_t s, int variant = 0);
+                             unsigned long long* next_path, cudaStream_t s, int variant = 0, void* park = nullptr);
 void launch_camera_pass_batch(const BatchScene* scenes, const long long* pixel_prefix, int n, long long total_pixels,
-                              unsigned long long* next_pixel, cudaStream_t s, int variant = 0);
+                              unsigned long long* next_pixel, cudaStream_t s, int variant = 0, void* park = nullptr);
 // Debug view `mode` (2 normals, 3 facing, 4 materials with IOR `ior`) added into the
 // FP64 image accumulation.
 void launch_debug_view(const VMParams& p, int mode, float ior, double* accum, cudaStream_t s);
@@ -140,10 +142,10 @@ void launch_pad_photons(float4* pos, const unsigned long long* count, long long 
                         cudaStream_t s);
 void launch_check_counts(const unsigned long long* photons, long long photon_cap, const unsigned long long* queries,
                          long long query_cap, int* flag, cudaStream_t s);
-// shape 0: the persistent passes' traversal; 1: the wavefront pass's warp-stepped one;
-// 2: pop-and-test (the reference's form).
-void launch_trace_rays(const SceneView& s, int n, const float* o, const float* d, float tmin, float* out_full,
-                       unsigned* out_words, int* err, cudaStream_t st, int shape = 0);
+// shape 0: the staged passes' search; 1: the persistent passes' traversal; 2: pop-and-test
+// (the reference's form).  found: n records of scratch.
+void launch_trace_rays(const SceneView& s, int n, const float* o, const float* d, float tmin, HitRec* found,
+                       float* out_full, unsigned* out_words, int* err, cudaStream_t st, int shape = 0);
 // Photon records in tree order (tp.t0/t1/t2 from ph.pos/dir/tp; only t0 when ph.dir is null).
 void launch_tree_records(PhotonBuf ph, const KdTree& tree, TreePhotons tp, cudaStream_t s);
 // Node bounding boxes used by the gather to prune exactly: the photons in tree order
@@ -186,18 +188,12 @@ void launch_gather_sets(const KdTree& tree, const float4* t0, const float* qpos,
                         int variant, unsigned long long* counters, int* err, cudaStream_t s);
 int gather_variants();
 int gather_default_variant();
-// Wavefront light pass: the same paths and photons as launch_light_pass, one bounce of
-// every live path per round, split into a closest-hit kernel and a shading kernel with
-// path state and queues in `scratch` (light_wavefront_scratch_bytes(num_light_paths)).
-// `tail`, if given, is recorded on s before the last launch (the few paths left after the
-// rounds, which leaves most SMs idle): work that waits on it fills them.
-size_t light_wavefront_scratch_bytes(long long n);
-void launch_light_wavefront(const VMParams& p, PhotonBuf ph, void* scratch, cudaStream_t s,
-                            cudaEvent_t tail = nullptr);
-// Launch shapes of the persistent light and camera passes (block size x traversal-stack
-// placement), chosen by the autotuner; 0 is the default.  The light pass has one more:
-// pass_variants() is the wavefront pass.
+// Launch shapes of the light and camera passes, chosen by the autotuner: the persistent
+// shapes (block size, registers; 0 is the default) and the staged ones (two launches, the
+// paths that go on parked in between; vm_kernels.cu).
 int pass_variants();
+bool pass_is_staged(int v);
+size_t pass_park_bytes(long long n);
 const char* pass_variant_name(int v);
 const char* gather_variant_name(int v);
 

@@ -1,4 +1,6 @@
 // Light pass, camera pass and the closest-hit parity kernel.
+#include <algorithm>
+
 #include "vm.cuh"
 #include "bsdf.cuh"
 #include "lights.cuh"
@@ -67,17 +69,10 @@ __device__ __forceinline__ bool light_path_start(const VMParams& P, long long pi
 // two halves: the closest hit of the path's next segment (false: the path ends), then
 // the shading at that hit - photon store, BSDF sample, Russian roulette, dVM update -
 // which returns false when the path ends.  The persistent pass runs both per bounce,
-// the wavefront pass runs them in separate kernels.
-template <class Stack>
-__device__ __forceinline__ bool light_path_trace(const VMParams& P, const LightPath& s, HitRec& h, Stack& stack) {
-    const F3 ro = s.o + s.d * kRayEps;
-    return scene_hit(P.scene, ro, s.d, kRayEps, h, P.error + ERR_STACK, stack);
-}
-
+// the staged pass searches for a whole warp at a time (search_run).  ro: the ray's origin.
 template <bool kGrouped = false>
 __device__ __forceinline__ bool light_path_shade(const VMParams& P, const PhotonBuf& ph, LightPath& s,
-                                                 const HitRec& h) {
-    const F3 ro = s.o + s.d * kRayEps;
+                                                 const HitRec& h, F3 ro) {
     Isect is;
     fill_isect(P.scene, h, ro, s.d, is);
     if ((unsigned)is.material >= (unsigned)P.num_materials) { atomicOr(P.error + ERR_MATERIAL, 1); return false; }
@@ -122,105 +117,10 @@ __device__ __forceinline__ bool light_path_shade(const VMParams& P, const Photon
 template <bool kGrouped = false, class Stack>
 __device__ __forceinline__ bool light_path_bounce(const VMParams& P, const PhotonBuf& ph, LightPath& s,
                                                   Stack& stack) {
+    const F3 ro = s.o + s.d * kRayEps;
     HitRec h;
-    if (!light_path_trace(P, s, h, stack)) return false;
-    return light_path_shade<kGrouped>(P, ph, s, h);
-}
-
-// Wavefront light pass: the same paths, bounces and photons as the persistent pass,
-// with each bounce split over two kernels that every queued path passes through: a
-// trace kernel (the closest hit only, so it keeps few registers and every lane holds a
-// live ray) and a shade kernel that appends the paths that continue to the next queue.
-// Path state between the kernels, per slot (slot = position in the light-path order):
-//   o4 = origin | dVM, d4 = direction | tp.r, t2 = tp.gb,
-//   m4 = path index, length, diffuse bounces, last event | (dispersion channel + 1) << 8,
-//   hit = t, u, v, triangle slot (-1: the path ends).
-struct WfState {
-    float4* o4; float4* d4; float2* t2; int4* m4; float4* hit;
-    uint32_t* queue[2];
-    unsigned long long* count;   // [2] queue lengths
-};
-
-__device__ __forceinline__ void wf_store(const WfState& W, uint32_t slot, const LightPath& s) {
-    W.o4[slot] = make_float4(s.o.x, s.o.y, s.o.z, s.dVM);
-    W.d4[slot] = make_float4(s.d.x, s.d.y, s.d.z, s.tp.x);
-    W.t2[slot] = make_float2(s.tp.y, s.tp.z);
-    W.m4[slot] = make_int4((int)(uint32_t)s.idx, s.len, s.diffuse, (s.last & 0xff) | ((s.channel + 1) << 8));
-}
-
-__device__ __forceinline__ void wf_load(const VMParams& P, const WfState& W, uint32_t slot, LightPath& s) {
-    const float4 o = W.o4[slot], d = W.d4[slot];
-    const float2 t = W.t2[slot];
-    const int4 m = W.m4[slot];
-    s.o = f3(o.x, o.y, o.z); s.dVM = o.w;
-    s.d = f3(d.x, d.y, d.z);
-    s.tp = f3(d.w, t.x, t.y);
-    s.idx = (long long)(uint32_t)m.x;
-    s.len = m.y; s.diffuse = m.z;
-    s.last = m.w & 0xff;
-    s.channel = (m.w >> 8) - 1;
-    s.rng.init(P.seed, (uint64_t)s.idx, P.iteration, STREAM_LIGHT);
-}
-
-__device__ __forceinline__ void wf_push(const WfState& W, int q, uint32_t slot) {
-    W.queue[q][warp_append(&W.count[q])] = slot;
-}
-
-__global__ void k_wf_start(const VMParams P, WfState W) {
-    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i >= P.num_light_paths) return;
-    const long long pidx = P.path_order ? (long long)__ldg(&P.path_order[i]) : i;
-    LightPath s;
-    if (!light_path_start(P, pidx, s)) return;
-    wf_store(W, (uint32_t)i, s);
-    wf_push(W, 0, (uint32_t)i);
-}
-
-template <int kMinBlocks>
-__global__ void __launch_bounds__(128, kMinBlocks) k_wf_trace(const VMParams P, WfState W, int q) {
-    const unsigned long long n = W.count[q];
-    WarpStepStack stk;   // the lanes of a warp trace together here: step them together
-    for (unsigned long long j = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; j < n;
-         j += (unsigned long long)gridDim.x * blockDim.x) {
-        const uint32_t slot = W.queue[q][j];
-        const float4 o = W.o4[slot], d = W.d4[slot];
-        LightPath s;
-        s.o = f3(o.x, o.y, o.z);
-        s.d = f3(d.x, d.y, d.z);
-        HitRec h;
-        if (!light_path_trace(P, s, h, stk)) h.slot = -1;
-        W.hit[slot] = make_float4(h.t, h.u, h.v, __int_as_float(h.slot));
-    }
-}
-
-// The paths still queued after the last wavefront round, each taken through all of its
-// remaining bounces by one thread (few paths remain; one launch instead of a round per
-// bounce, each of which waits for its longest traversal).
-__global__ void __launch_bounds__(128, 8) k_wf_finish(const VMParams P, PhotonBuf ph, WfState W, int q) {
-    const unsigned long long n = W.count[q];
-    CallStack stk;
-    for (unsigned long long j = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; j < n;
-         j += (unsigned long long)gridDim.x * blockDim.x) {
-        LightPath s;
-        wf_load(P, W, W.queue[q][j], s);
-        while (light_path_bounce(P, ph, s, stk)) {}
-    }
-}
-
-__global__ void __launch_bounds__(128) k_wf_shade(const VMParams P, PhotonBuf ph, WfState W, int q) {
-    const unsigned long long n = W.count[q];
-    for (unsigned long long j = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; j < n;
-         j += (unsigned long long)gridDim.x * blockDim.x) {
-        const uint32_t slot = W.queue[q][j];
-        const float4 hv = W.hit[slot];
-        HitRec h{hv.x, hv.y, hv.z, __float_as_int(hv.w)};
-        if (h.slot < 0) continue;
-        LightPath s;
-        wf_load(P, W, slot, s);
-        if (!light_path_shade(P, ph, s, h)) continue;
-        wf_store(W, slot, s);
-        wf_push(W, q ^ 1, slot);
-    }
+    if (!scene_hit(P.scene, ro, s.d, kRayEps, h, P.error + ERR_STACK, stack)) return false;
+    return light_path_shade<kGrouped>(P, ph, s, h, ro);
 }
 
 // Light-path order: 4D Morton key of a path's emission samples (the same Philox draws
@@ -321,9 +221,15 @@ struct CameraPath {
     float dVM;
     int len;
     int channel;      // dispersion channel, -1 until a dispersive material is met
-    int target;
+    int target;       // pixel the path adds to: the one its jittered sample falls in
+    uint32_t pix;     // the path's index
+    int step;         // 1: the sample falls one column on, 2: one row on
     PathRng rng;
 };
+
+__device__ __forceinline__ int camera_target(const VMParams& P, int X, int row) {
+    return (int)((long long)X + (long long)(P.camera.height - row) * P.camera.width);
+}
 
 // Generate_camera_sample + Image_Buffer::add_color's row mapping; false when the
 // sample falls outside the image buffer (camera row 0, src/Image_Buffer.h:28-31).
@@ -348,15 +254,14 @@ __device__ __forceinline__ bool camera_path_start(const VMParams& P, long long p
     s.len = 0;
     s.channel = -1;
     s.target = (int)target;
+    s.pix = (uint32_t)pix;
+    s.step = (X != (int)x ? 1 : 0) | ((int)sy != (int)y ? 2 : 0);
     return true;
 }
 
-template <bool kGrouped = false, class Stack>
-__device__ __forceinline__ bool camera_path_bounce(const VMParams& P, const QueryBuf& qb, CameraPath& s,
-                                                   Stack& stack) {
-    F3 ro = s.o + s.d * kRayEps;
-    HitRec h;
-    if (!scene_hit(P.scene, ro, s.d, kRayEps, h, P.error + ERR_STACK, stack)) return false;
+template <bool kGrouped = false>
+__device__ __forceinline__ bool camera_path_shade(const VMParams& P, const QueryBuf& qb, CameraPath& s,
+                                                  const HitRec& h, F3 ro) {
     Isect is;
     fill_isect(P.scene, h, ro, s.d, is);
     if ((unsigned)is.material >= (unsigned)P.num_materials) { atomicOr(P.error + ERR_MATERIAL, 1); return false; }
@@ -394,6 +299,15 @@ __device__ __forceinline__ bool camera_path_bounce(const VMParams& P, const Quer
     else s.dVM = (smp.cos_out / smp.fwd) * (1.0f + smp.rev * s.dVM);
     s.len++;
     return true;
+}
+
+template <bool kGrouped = false, class Stack>
+__device__ __forceinline__ bool camera_path_bounce(const VMParams& P, const QueryBuf& qb, CameraPath& s,
+                                                   Stack& stack) {
+    const F3 ro = s.o + s.d * kRayEps;
+    HitRec h;
+    if (!scene_hit(P.scene, ro, s.d, kRayEps, h, P.error + ERR_STACK, stack)) return false;
+    return camera_path_shade<kGrouped>(P, qb, s, h, ro);
 }
 
 template <int kBlock, int kMinBlocks>
@@ -507,19 +421,252 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) k_camera_pass_batch(const 
     }
 }
 
-// Stack: CallStack (the persistent passes' traversal: children tested at the parent),
-// WarpStepStack (the wavefront pass's warp-stepped one) or LocalStack (pop-and-test, the
-// reference's own form).
+// Staged passes: a pass in two launches.  k_pass_first takes fresh paths, 32 at a time per
+// warp, through their first kSegs segments, all lanes together: they start coherent (the
+// light-path order; the pixels of a row), and mixing them with paths further on costs more
+// than the idle lanes do.  The paths that go on are parked, packed (48 bytes each).
+// k_pass_rest takes the parked paths to their ends; these are incoherent, so lanes shade as
+// soon as at most kKeep lanes of the warp still search, and ended paths are replaced once
+// kFree lanes are free.  Paths, samples and stored records are the persistent passes'.
+//
+// What bounds the passes is the instruction issue of the closest-hit search (repeating the
+// search doubles k_pass_first's time); a step of 32 lanes at different places of the tree
+// had 9 to 10 of them active.  The search by phases (search_run) has 13 to 15.  Measured
+// against the best persistent shape: light pass of the 1080p water pool (16.7M paths)
+// 11.3 -> 9.6 ms, of 2,000 gems (4.2M paths) 35.9 -> 21.1 ms.  Tried and lost: one
+// kernel that holds the continuing paths back per warp in global memory and switches
+// between the two modes (11.4 ms on the pool); the state a search needs rarely in shared
+// memory (9.7 ms); four-wide nodes with 8-bit child boxes, conservative with an exact test
+// per leaf (10.2 ms; 17.7 ms on the gems).
+// Small passes end with a few long paths whatever the order; there the persistent shapes
+// stay ahead (518,400 paths: 0.59 against 0.79 ms), and the autotuner keeps one of them.
+struct Parked {
+    float4* a;   // origin | dVM
+    float4* b;   // direction | throughput.r
+    float4* c;   // throughput.gb | path index | meta, scene << 16
+    unsigned long long* count;   // [0] parked paths, [1], [2] next path of the two launches
+};
+constexpr long long kParkChunk = 1LL << 24;   // paths per pair of launches (800 MB parked at most)
+
+struct LightKind {
+    using Path = LightPath;
+    using Out = PhotonBuf;
+    static __device__ __forceinline__ bool start(const VMParams& P, uint32_t i, Path& s) {
+        return light_path_start(P, P.path_order ? (long long)__ldg(&P.path_order[i]) : (long long)i, s);
+    }
+    static __device__ __forceinline__ uint32_t index(const Path& s) { return (uint32_t)s.idx; }
+    static __device__ __forceinline__ uint32_t meta(const Path& s) {
+        return (uint32_t)s.last | ((uint32_t)s.len << 5) | ((uint32_t)s.diffuse << 11) | ((uint32_t)(s.channel + 1) << 14);
+    }
+    static __device__ __forceinline__ void restore(const VMParams& P, uint32_t idx, uint32_t m, Path& s) {
+        s.idx = (long long)idx;
+        s.last = (int)(m & 31u);
+        s.len = (int)((m >> 5) & 63u);
+        s.diffuse = (int)((m >> 11) & 7u);
+        s.channel = (int)((m >> 14) & 3u) - 1;
+        s.rng.init(P.seed, (uint64_t)idx, P.iteration, STREAM_LIGHT);
+    }
+    template <bool kGrouped>
+    static __device__ __forceinline__ bool shade(const VMParams& P, const Out& out, Path& s, const HitRec& h, F3 ro) {
+        return light_path_shade<kGrouped>(P, out, s, h, ro);
+    }
+};
+static_assert(2 * EV_SPECULAR - 1 == 31 && kMaxDiffuse + 1 <= 7, "LightKind::meta's fields");
+
+struct CameraKind {
+    using Path = CameraPath;
+    using Out = QueryBuf;
+    static __device__ __forceinline__ bool start(const VMParams& P, uint32_t i, Path& s) {
+        return camera_path_start(P, (long long)i, s);
+    }
+    static __device__ __forceinline__ uint32_t index(const Path& s) { return s.pix; }
+    static __device__ __forceinline__ uint32_t meta(const Path& s) {
+        return (uint32_t)s.len | ((uint32_t)(s.channel + 1) << 6) | ((uint32_t)s.step << 8);
+    }
+    static __device__ __forceinline__ void restore(const VMParams& P, uint32_t idx, uint32_t m, Path& s) {
+        s.pix = idx;
+        s.len = (int)(m & 63u);
+        s.channel = (int)((m >> 6) & 3u) - 1;
+        s.step = (int)((m >> 8) & 3u);
+        const int W = P.camera.width, y = (int)idx / W, x = (int)idx - y * W;
+        s.target = camera_target(P, x + (s.step & 1), y + (s.step >> 1));
+        s.rng.init(P.camera_seed, (uint64_t)idx, P.iteration, STREAM_CAMERA);
+    }
+    template <bool kGrouped>
+    static __device__ __forceinline__ bool shade(const VMParams& P, const Out& out, Path& s, const HitRec& h, F3 ro) {
+        return camera_path_shade<kGrouped>(P, out, s, h, ro);
+    }
+};
+
+// The scenes of a pass: one, its parameters in the kernel's, or the batch's.  Work indices
+// run from first to first + count.
+template <class Kind> struct OneScene {
+    static constexpr bool kMany = false;
+    VMParams p;
+    typename Kind::Out out;
+    unsigned long long first, count;
+    __device__ __forceinline__ const VMParams& params(int) const { return p; }
+    __device__ __forceinline__ const typename Kind::Out& buffers(int) const { return out; }
+    __device__ __forceinline__ int locate(unsigned long long g, uint32_t& local) const {
+        local = (uint32_t)g;
+        return 0;
+    }
+};
+__device__ __forceinline__ const PhotonBuf& batch_buffers(const BatchScene& b, const LightKind*) { return b.ph; }
+__device__ __forceinline__ const QueryBuf& batch_buffers(const BatchScene& b, const CameraKind*) { return b.qb; }
+template <class Kind> struct ManyScenes {
+    static constexpr bool kMany = true;
+    const BatchScene* b;
+    const long long* prefix;
+    int n;
+    unsigned long long first, count;
+    __device__ __forceinline__ const VMParams& params(int sid) const { return b[sid].p; }
+    __device__ __forceinline__ const typename Kind::Out& buffers(int sid) const {
+        return batch_buffers(b[sid], (const Kind*)nullptr);
+    }
+    __device__ __forceinline__ int locate(unsigned long long g, uint32_t& local) const {
+        const int sid = batch_scene_of(prefix, n, (long long)g);
+        local = (uint32_t)((long long)g - __ldg(&prefix[sid]));
+        return sid;
+    }
+};
+
+template <class Kind, class Scenes, int kMinBlocks, int kSegs>
+__global__ void __launch_bounds__(128, kMinBlocks) k_pass_first(const Scenes S, const Parked park,
+                                                                unsigned long long* __restrict__ rays) {
+    SearchStack st;
+    Search q;
+    const int lane = threadIdx.x & 31;
+    unsigned traced = 0;   // closest-hit queries of this lane
+    while (true) {
+        unsigned long long base = 0;
+        if (lane == 0) base = atomicAdd(park.count + 1, 32ull);
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (base >= S.count) break;
+        typename Kind::Path s;
+        bool alive = false;
+        int sid = 0;
+        if (base + lane < S.count) {
+            uint32_t local;
+            sid = S.locate(S.first + base + lane, local);
+            alive = Kind::start(S.params(sid), local, s);
+        }
+        const VMParams& P = S.params(sid);
+#pragma unroll 1
+        for (int k = 0; k < kSegs; ++k) {
+            q.w0 = kSearchIdle;
+            if (alive) {
+                search_begin(q, st, s.o + s.d * kRayEps, s.d);
+                ++traced;
+            }
+            __syncwarp();
+            search_run(P.scene, q, st, s.d, kRayEps, 0, P.error + ERR_STACK);
+            if (alive)
+                alive = q.out.slot >= 0 && Kind::template shade<Scenes::kMany>(P, S.buffers(sid), s, q.out, q.origin());
+            __syncwarp();
+        }
+        if (alive) {
+            const unsigned long long j = warp_append(park.count);
+            park.a[j] = make_float4(s.o.x, s.o.y, s.o.z, s.dVM);
+            park.b[j] = make_float4(s.d.x, s.d.y, s.d.z, s.tp.x);
+            park.c[j] = make_float4(s.tp.y, s.tp.z, __uint_as_float(Kind::index(s)),
+                                    __uint_as_float(Kind::meta(s) | ((uint32_t)sid << 16)));
+        }
+        __syncwarp();
+    }
+    const unsigned w = __reduce_add_sync(0xffffffffu, traced);
+    if (rays && lane == 0) atomicAdd(rays, (unsigned long long)w);
+}
+
+template <class Kind, class Scenes, int kMinBlocks, int kKeep, int kFree>
+__global__ void __launch_bounds__(128, kMinBlocks) k_pass_rest(const Scenes S, const Parked park,
+                                                               unsigned long long* __restrict__ rays) {
+    SearchStack st;
+    Search q;
+    q.w0 = kSearchIdle;
+    const int lane = threadIdx.x & 31;
+    const unsigned long long total = park.count[0];
+    typename Kind::Path s;
+    int sid = 0;
+    bool alive = false, left = true;
+    unsigned traced = 0;
+    while (true) {
+        const unsigned need = __ballot_sync(0xffffffffu, !alive);
+        if (left && (__popc(need) >= kFree || need == 0xffffffffu)) {
+            const int leader = __ffs(need) - 1;
+            unsigned long long base = 0;
+            if (lane == leader) base = atomicAdd(park.count + 2, (unsigned long long)__popc(need));
+            base = __shfl_sync(0xffffffffu, base, leader);
+            const unsigned long long mine = base + __popc(need & ((1u << lane) - 1u));
+            if (!alive && mine < total) {
+                const float4 a = park.a[mine], b = park.b[mine], c = park.c[mine];
+                const uint32_t m = __float_as_uint(c.w);
+                sid = Scenes::kMany ? (int)(m >> 16) : 0;
+                s.o = f3(a.x, a.y, a.z); s.dVM = a.w;
+                s.d = f3(b.x, b.y, b.z); s.tp = f3(b.w, c.x, c.y);
+                Kind::restore(S.params(sid), __float_as_uint(c.z), m & 0xffffu, s);
+                alive = true;
+            }
+            if (base + __popc(need) >= total) left = false;
+        }
+        const int n = __popc(__ballot_sync(0xffffffffu, alive));
+        if (n == 0) {
+            if (!left) break;
+            continue;
+        }
+        if (alive && q.w0 == kSearchIdle) {
+            search_begin(q, st, s.o + s.d * kRayEps, s.d);
+            ++traced;
+        }
+        __syncwarp();
+        const VMParams& P = S.params(sid);
+        search_run(P.scene, q, st, s.d, kRayEps, min(kKeep, n - 1), P.error + ERR_STACK);
+        if (alive && q.w0 == kSearchIdle)
+            alive = q.out.slot >= 0 && Kind::template shade<Scenes::kMany>(P, S.buffers(sid), s, q.out, q.origin());
+        __syncwarp();
+    }
+    const unsigned w = __reduce_add_sync(0xffffffffu, traced);
+    if (rays && lane == 0) atomicAdd(rays, (unsigned long long)w);
+}
+
+// Closest hits of given rays by the staged passes' search.
+__global__ void __launch_bounds__(128) k_trace_search(const SceneView S, int n, const float* __restrict__ o,
+                                                      const float* __restrict__ d, float tmin,
+                                                      HitRec* __restrict__ hits, int* err) {
+    SearchStack st;
+    Search q;
+    q.w0 = kSearchIdle;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    F3 rd = f3(0.0f);
+    if (i < n) {
+        rd = f3(d[3 * i], d[3 * i + 1], d[3 * i + 2]);
+        search_begin(q, st, f3(o[3 * i], o[3 * i + 1], o[3 * i + 2]), rd);
+    }
+    __syncwarp();
+    search_run(S, q, st, rd, tmin, 0, err);
+    if (i < n) hits[i] = q.out;
+}
+
+// The hit records of given rays: `found` (k_trace_search), or searched here with Stack:
+// CallStack (the persistent passes' traversal: children tested at the parent) or
+// LocalStack (pop-and-test, the reference's own form).
 template <class Stack>
 __global__ void k_trace_rays(const SceneView S, int n, const float* __restrict__ o, const float* __restrict__ d,
-                             float tmin, float* out_full, unsigned* out_words, int* err) {
+                             float tmin, const HitRec* __restrict__ found, float* out_full, unsigned* out_words,
+                             int* err) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     F3 ro = f3(o[3 * i], o[3 * i + 1], o[3 * i + 2]);
     F3 rd = f3(d[3 * i], d[3 * i + 1], d[3 * i + 2]);
     HitRec h;
-    Stack stk;
-    bool hit = scene_hit(S, ro, rd, tmin, h, err, stk);
+    bool hit;
+    if (found) {
+        h = found[i];
+        hit = h.slot >= 0;
+    } else {
+        Stack stk;
+        hit = scene_hit(S, ro, rd, tmin, h, err, stk);
+    }
     Isect is;
     if (hit) fill_isect(S, h, ro, rd, is);
     if (out_words) {
@@ -639,111 +786,123 @@ void launch_light_order(const VMParams& p, void* scratch, uint32_t* order, cudaS
     k_light_scatter<<<g, 256, 0, s>>>(keys, n, counts, order);
 }
 
-size_t light_wavefront_scratch_bytes(long long n) {
-    const size_t m = (size_t)(n > 0 ? n : 1);
-    auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
-    return al(16 * m) * 4 + al(8 * m) + al(16 * m) + 2 * al(4 * m) + 256;
-}
-
-void launch_light_wavefront(const VMParams& p, PhotonBuf ph, void* scratch, cudaStream_t s, cudaEvent_t tail) {
-    const long long n = p.num_light_paths;
-    if (n <= 0) return;
-    auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
-    char* c = static_cast<char*>(scratch);
-    WfState W;
-    W.o4 = (float4*)c; c += al(16 * (size_t)n);
-    W.d4 = (float4*)c; c += al(16 * (size_t)n);
-    W.m4 = (int4*)c; c += al(16 * (size_t)n);
-    W.hit = (float4*)c; c += al(16 * (size_t)n);
-    W.t2 = (float2*)c; c += al(8 * (size_t)n);
-    W.queue[0] = (uint32_t*)c; c += al(4 * (size_t)n);
-    W.queue[1] = (uint32_t*)c; c += al(4 * (size_t)n);
-    W.count = (unsigned long long*)c;
-    cudaMemsetAsync(W.count, 0, 2 * sizeof(unsigned long long), s);
-    k_wf_start<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(p, W);
-    static thread_local unsigned trace_grid = 0, shade_grid = 0, finish_grid = 0;
-    if (!trace_grid) {
-        trace_grid = persistent_grid(k_wf_trace<8>, 128, 0, 1LL << 40);
-        shade_grid = persistent_grid(k_wf_shade, 128, 0, 1LL << 40);
-        finish_grid = persistent_grid(k_wf_finish, 128, 0, 1LL << 40);
-    }
-    // a bounce per round for the first kWavefrontRounds bounces (most paths end by then),
-    // then one launch finishes the rest
-    constexpr int kWavefrontRounds = 4;
-    int q = 0;
-    for (int b = 0; b < kWavefrontRounds; ++b, q ^= 1) {
-        k_wf_trace<8><<<trace_grid, 128, 0, s>>>(p, W, q);
-        cudaMemsetAsync(W.count + (q ^ 1), 0, sizeof(unsigned long long), s);
-        k_wf_shade<<<shade_grid, 128, 0, s>>>(p, ph, W, q);
-    }
-    if (tail) cudaEventRecord(tail, s);
-    k_wf_finish<<<finish_grid, 128, 0, s>>>(p, ph, W, q);
-}
-
-int pass_variants() { return 6; }
+int pass_variants() { return 7; }
+bool pass_is_staged(int v) { return v >= 4 && v < 7; }
+size_t pass_park_bytes(long long n) { return 48 * (size_t)std::min(std::max(n, 1LL), kParkChunk) + 256; }
 
 const char* pass_variant_name(int v) {
-    static const char* names[6] = {"256 threads, >= 3 blocks/SM (<= 85 registers)",
+    static const char* names[7] = {"256 threads, >= 3 blocks/SM (<= 85 registers)",
                                    "128 threads, >= 7 blocks/SM (<= 73 registers)",
                                    "128 threads, >= 8 blocks/SM (<= 64 registers)",
-                                   "128 threads, >= 5 blocks/SM (<= 102 registers)",
-                                   "128 threads, >= 10 blocks/SM (<= 51 registers)",
-                                   "128 threads, >= 9 blocks/SM (<= 56 registers)"};
-    if (v == 6) return "wavefront: closest-hit and shading kernels per bounce";
-    return (v >= 0 && v < 6) ? names[v] : "?";
+                                   "128 threads, >= 9 blocks/SM (<= 56 registers)",
+                                   "staged: 2 segments, then 8 lanes kept, 8 freed",
+                                   "staged: 2 segments, then 12 lanes kept, 4 freed",
+                                   "staged: 1 segment, then 12 lanes kept, 4 freed"};
+    return (v >= 0 && v < 7) ? names[v] : "?";
 }
 
+namespace {
+
+template <class Kind, int kSegs, int kMinFirst, int kMinRest, int kKeep, int kFree, class Scenes>
+void launch_staged(Scenes S, long long n, void* scratch, unsigned long long* rays, cudaStream_t s) {
+    const long long chunk = std::min(n, kParkChunk);
+    float4* const m = static_cast<float4*>(scratch);
+    const Parked park{m, m + chunk, m + 2 * chunk, reinterpret_cast<unsigned long long*>(m + 3 * chunk)};
+    auto* const first = k_pass_first<Kind, Scenes, kMinFirst, kSegs>;
+    auto* const rest = k_pass_rest<Kind, Scenes, kMinRest, kKeep, kFree>;
+    // per host thread: contexts on different threads launch concurrently
+    static thread_local unsigned full_first = 0, full_rest = 0;
+    if (!full_first) {
+        full_first = persistent_grid(first, 128, 0, 1LL << 40);
+        full_rest = persistent_grid(rest, 128, 0, 1LL << 40);
+    }
+    if (rays) cudaMemsetAsync(rays, 0, sizeof(unsigned long long), s);
+    for (long long lo = 0; lo < n; lo += chunk) {
+        const long long c = std::min(chunk, n - lo);
+        const unsigned need = (unsigned)((c + 127) / 128);
+        S.first = (unsigned long long)lo;
+        S.count = (unsigned long long)c;
+        cudaMemsetAsync(park.count, 0, 3 * sizeof(unsigned long long), s);
+        first<<<std::min(need, full_first), 128, 0, s>>>(S, park, rays);
+        rest<<<std::min(need, full_rest), 128, 0, s>>>(S, park, rays);
+    }
+}
+
+template <class Kind, class Scenes>
+void launch_staged_variant(const Scenes& S, long long n, void* scratch, unsigned long long* rays, cudaStream_t s,
+                           int variant) {
+    switch (variant) {
+    case 5: launch_staged<Kind, 2, 9, 9, 12, 4>(S, n, scratch, rays, s); break;
+    case 6: launch_staged<Kind, 1, 10, 8, 12, 4>(S, n, scratch, rays, s); break;
+    default: launch_staged<Kind, 2, 8, 8, 8, 8>(S, n, scratch, rays, s); break;
+    }
+}
+
+}  // namespace
+
 void launch_light_pass(const VMParams& p, PhotonBuf ph, unsigned long long* next_path, cudaStream_t s, int variant,
-                       unsigned long long* rays) {
-    long long n = p.num_light_paths;
+                       unsigned long long* rays, void* park) {
+    const long long n = p.num_light_paths;
     if (n <= 0) return;
     if (!next_path) return;
+    if (pass_is_staged(variant) && park && n < (1LL << 32)) {
+        launch_staged_variant<LightKind>(OneScene<LightKind>{p, ph, 0, 0}, n, park, rays, s, variant);
+        return;
+    }
     switch (variant) {
     case 1: launch_light_t<128, 7>(p, ph, next_path, rays, s); break;
     case 2: launch_light_t<128, 8>(p, ph, next_path, rays, s); break;
-    case 3: launch_light_t<128, 5>(p, ph, next_path, rays, s); break;
-    case 4: launch_light_t<128, 10>(p, ph, next_path, rays, s); break;
-    case 5: launch_light_t<128, 9>(p, ph, next_path, rays, s); break;
+    case 3: launch_light_t<128, 9>(p, ph, next_path, rays, s); break;
     default: launch_light_t<256, 3>(p, ph, next_path, rays, s); break;
     }
 }
 
-void launch_camera_pass(const VMParams& p, QueryBuf qb, unsigned long long* next_pixel, cudaStream_t s, int variant) {
-    long long n = (long long)p.camera.width * p.camera.height;
+void launch_camera_pass(const VMParams& p, QueryBuf qb, unsigned long long* next_pixel, cudaStream_t s, int variant,
+                        void* park) {
+    const long long n = (long long)p.camera.width * p.camera.height;
     if (n <= 0) return;
     if (!next_pixel) return;
+    if (pass_is_staged(variant) && park && n < (1LL << 31)) {
+        launch_staged_variant<CameraKind>(OneScene<CameraKind>{p, qb, 0, 0}, n, park, nullptr, s, variant);
+        return;
+    }
     switch (variant) {
     case 1: launch_camera_t<128, 7>(p, qb, next_pixel, s); break;
     case 2: launch_camera_t<128, 8>(p, qb, next_pixel, s); break;
-    case 3: launch_camera_t<128, 5>(p, qb, next_pixel, s); break;
-    case 4: launch_camera_t<128, 10>(p, qb, next_pixel, s); break;
-    case 5: launch_camera_t<128, 9>(p, qb, next_pixel, s); break;
+    case 3: launch_camera_t<128, 9>(p, qb, next_pixel, s); break;
     default: launch_camera_t<256, 3>(p, qb, next_pixel, s); break;
     }
 }
 
+// (a parked path names its scene in 16 bits; a scene's own indices fit 32)
 void launch_light_pass_batch(const BatchScene* scenes, const long long* path_prefix, int n, long long total_paths,
-                             unsigned long long* next_path, cudaStream_t s, int variant) {
+                             unsigned long long* next_path, cudaStream_t s, int variant, void* park) {
     if (n <= 0 || total_paths <= 0 || !next_path) return;
+    if (pass_is_staged(variant) && park && n < (1 << 16)) {
+        launch_staged_variant<LightKind>(ManyScenes<LightKind>{scenes, path_prefix, n, 0, 0}, total_paths, park, nullptr,
+                                         s, variant);
+        return;
+    }
     switch (variant) {
     case 1: launch_light_batch_t<128, 7>(scenes, path_prefix, n, total_paths, next_path, s); break;
     case 2: launch_light_batch_t<128, 8>(scenes, path_prefix, n, total_paths, next_path, s); break;
-    case 3: launch_light_batch_t<128, 5>(scenes, path_prefix, n, total_paths, next_path, s); break;
-    case 4: launch_light_batch_t<128, 10>(scenes, path_prefix, n, total_paths, next_path, s); break;
-    case 5: launch_light_batch_t<128, 9>(scenes, path_prefix, n, total_paths, next_path, s); break;
+    case 3: launch_light_batch_t<128, 9>(scenes, path_prefix, n, total_paths, next_path, s); break;
     default: launch_light_batch_t<256, 3>(scenes, path_prefix, n, total_paths, next_path, s); break;
     }
 }
 
 void launch_camera_pass_batch(const BatchScene* scenes, const long long* pixel_prefix, int n, long long total_pixels,
-                              unsigned long long* next_pixel, cudaStream_t s, int variant) {
+                              unsigned long long* next_pixel, cudaStream_t s, int variant, void* park) {
     if (n <= 0 || total_pixels <= 0 || !next_pixel) return;
+    if (pass_is_staged(variant) && park && n < (1 << 16)) {
+        launch_staged_variant<CameraKind>(ManyScenes<CameraKind>{scenes, pixel_prefix, n, 0, 0}, total_pixels, park,
+                                          nullptr, s, variant);
+        return;
+    }
     switch (variant) {
     case 1: launch_camera_batch_t<128, 7>(scenes, pixel_prefix, n, total_pixels, next_pixel, s); break;
     case 2: launch_camera_batch_t<128, 8>(scenes, pixel_prefix, n, total_pixels, next_pixel, s); break;
-    case 3: launch_camera_batch_t<128, 5>(scenes, pixel_prefix, n, total_pixels, next_pixel, s); break;
-    case 4: launch_camera_batch_t<128, 10>(scenes, pixel_prefix, n, total_pixels, next_pixel, s); break;
-    case 5: launch_camera_batch_t<128, 9>(scenes, pixel_prefix, n, total_pixels, next_pixel, s); break;
+    case 3: launch_camera_batch_t<128, 9>(scenes, pixel_prefix, n, total_pixels, next_pixel, s); break;
     default: launch_camera_batch_t<256, 3>(scenes, pixel_prefix, n, total_pixels, next_pixel, s); break;
     }
 }
@@ -828,15 +987,16 @@ void launch_check_counts(const unsigned long long* photons, long long photon_cap
     k_check_counts<<<1, 1, 0, s>>>(photons, photon_cap, queries, query_cap, flag);
 }
 
-void launch_trace_rays(const SceneView& sv, int n, const float* o, const float* d, float tmin, float* out_full,
-                       unsigned* out_words, int* err, cudaStream_t st, int shape) {
+void launch_trace_rays(const SceneView& sv, int n, const float* o, const float* d, float tmin, HitRec* found,
+                       float* out_full, unsigned* out_words, int* err, cudaStream_t st, int shape) {
     if (n <= 0) return;
-    if (shape == 1)
-        k_trace_rays<WarpStepStack><<<(n + 127) / 128, 128, 0, st>>>(sv, n, o, d, tmin, out_full, out_words, err);
-    else if (shape == 2)
-        k_trace_rays<LocalStack><<<(n + 127) / 128, 128, 0, st>>>(sv, n, o, d, tmin, out_full, out_words, err);
+    const unsigned g = (unsigned)((n + 127) / 128);
+    if (shape == 0) k_trace_search<<<g, 128, 0, st>>>(sv, n, o, d, tmin, found, err);
+    if (shape == 2)
+        k_trace_rays<LocalStack><<<g, 128, 0, st>>>(sv, n, o, d, tmin, nullptr, out_full, out_words, err);
     else
-        k_trace_rays<CallStack><<<(n + 127) / 128, 128, 0, st>>>(sv, n, o, d, tmin, out_full, out_words, err);
+        k_trace_rays<CallStack><<<g, 128, 0, st>>>(sv, n, o, d, tmin, shape == 0 ? found : nullptr, out_full, out_words,
+                                                   err);
 }
 
 }  // namespace rc

@@ -131,8 +131,8 @@ class Renderer:
         return dict(zip(STAT_NAMES, a.tolist()))
 
     def trace(self, origins: np.ndarray, dirs: np.ndarray, tmin: float = 0.001, shape: int = 0) -> np.ndarray:
-        """Closest hits (n, 16) through traversal `shape`: 0 the persistent passes',
-        1 the wavefront pass's warp-stepped one, 2 pop-and-test (the reference's form)."""
+        """Closest hits (n, 16) through traversal `shape`: 0 the staged passes' search in
+        phases, 1 the persistent passes', 2 pop-and-test (the reference's form)."""
         o = np.ascontiguousarray(origins, np.float32)
         d = np.ascontiguousarray(dirs, np.float32)
         n = len(o)
@@ -150,7 +150,7 @@ class Renderer:
         return out[:n.value]
 
     def light_photons_shape(self, shape: int, iteration: int) -> np.ndarray:
-        """Photons of one light pass in launch shape `shape` (6: the wavefront pass)."""
+        """Photons of one light pass in launch shape `shape` (0-3 persistent, 4-6 staged)."""
         n = C.c_longlong()
         check(self.L.rc_light_photons_shape(shape, int(iteration), None, 0, C.byref(n)), "rc_light_photons_shape")
         out = np.zeros((max(n.value, 1), 12), np.float32)
