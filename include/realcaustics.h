@@ -232,7 +232,7 @@ const char* rc_last_error(void);
 
 /* Per-iteration statistics of the last rc_render call.
  * out[0] light paths, [1] stored photons, [2] merge queries, [3] photons merged,
- * [4] light-pass ms, [5] KD-build ms, [6] camera-pass ms, [7] gather ms,
+ * [4] light-pass ms, [5] photon-order ms (sort, boxes and records for the gather), [6] camera-pass ms, [7] gather ms,
  * [8] accumulate ms, [9] total device ms, [10] iterations rendered so far,
  * [11] scene radius, [12] current merge radius, [13] kernel launches,
  * [14] photon-query distance tests in the gather, [15] photon chunks (of at most 32)
@@ -240,7 +240,7 @@ const char* rc_last_error(void);
  * traced (0 for the Metropolis samplers and a batch render).
  * With the learned proposal, [8] is the proposal inference + training time.
  * With uniformly sampled light paths the camera pass runs on
- * a second stream beside the light pass and the KD build: its window [6] opens with the
+ * a second stream beside the light pass and the photon order: its window [6] opens with the
  * light pass, and [9] counts the overlapped span once. */
 int rc_get_stats(double* out, int n);
 
@@ -318,6 +318,10 @@ int rc_light_photons_shape(int shape, int iteration, float* out, long long cap, 
  * storage order, as 4 floats each: [position xyz, camera dVM].  *count receives the
  * number written (may exceed cap). */
 int rc_camera_queries(int iteration, float* out, long long cap, long long* count);
+
+/* rc_camera_queries with the camera pass in launch shape `shape` (as rc_light_photons_shape);
+ * the queries of every shape are the same, only their storage order differs. */
+int rc_camera_queries_shape(int shape, int iteration, float* out, long long cap, long long* count);
 
 /* Build the photon KD-tree on the GPU over n photon positions (3 floats each) and
  * answer q radius queries (squared radius r2): counts[j] = number of photons with

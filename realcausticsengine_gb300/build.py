@@ -30,6 +30,7 @@ SOURCES = [
     ("rc_abi.cpp", "nvcc"),
     ("vm_kernels.cu", "nvcc"),
     ("gather.cu", "nvcc"),
+    ("photon_order.cu", "nvcc"),
     ("kdtree.cu", "nvcc"),
     ("kd_noalloc.cu", "nvcc"),
     ("vm_mlt.cu", "nvcc"),

@@ -11,15 +11,13 @@
 // boxes that provably hold no accepted photon and tests every other photon with the
 // reference's predicate.
 //
-// Layout (launch_kd_boxes).  The photons in tree order are cut into 2^Lc chunks, Lc
-// being the shallowest level whose nodes hold at most 31 photons: chunk i is node
-// (2^Lc + i)'s contiguous range plus the gap before the next chunk's range, which holds
-// at most one inner node's median photon (that of the two nodes' lowest common
-// ancestor), so a chunk holds at most 32 photons.  Each chunk has its photons' bounding
-// box, with its first position and count in the spare .w words; every node above has
-// the union of its children's boxes.
+// Layout (launch_photon_order).  The photons, sorted along a Hilbert curve, are cut into
+// 2^Lc runs of at most 32 (chunks), Lc being the shallowest level whose runs hold at most
+// 31 where the cut is even.  Each chunk has its photons' bounding box, with its first
+// position and count in the spare .w words; every node above has the union of its
+// children's boxes.
 //
-// Work split (k_gather).  Queries are sorted by Morton code (launch_query_order) and a
+// Work split (k_gather).  Queries are sorted along the same curve (launch_query_order) and a
 // warp owns G consecutive ones (a group), one per lane.  The warp descends the box hierarchy
 // once for the whole group, E levels per step (lane j tests descendant j's box against
 // the group's bounding box grown by the radius), down to the candidate chunks.  At a
@@ -41,7 +39,6 @@ namespace rc {
 namespace {
 
 constexpr int kWarpsPerBlock = 8;
-constexpr long long kChunkNode = 31;   // photons per chunk-level node (the chunk adds at most one median)
 // DFS stack of subtree roots per warp.  Lc <= 24 for n < 2^28 photons, so a path from
 // the root crosses at most ceil(24 / E) expansion steps, the last of which reaches the
 // chunks (processed at once, never pushed): at most 4 x 31 + 1 = 125 (E = 5) or
@@ -52,7 +49,7 @@ constexpr unsigned kFull = 0xffffffffu;
 struct ChunkTree {
     const float4* __restrict__ lo;    // node boxes, heap order, levels [0, lc]; chunk level: .w = first position
     const float4* __restrict__ hi;    //                                          chunk level: .w = photon count
-    const float4* __restrict__ pos;   // photon positions in tree order (TreePhotons::t0)
+    const float4* __restrict__ pos;   // sorted photon positions (TreePhotons::t0)
     int lc;                           // chunk level (-1: no photons)
 };
 
@@ -480,257 +477,8 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, MinBlocks)
     }
 }
 
-// Exclusive scan of m counters in one CTA of 1024 threads (m up to a few million).
-__global__ void __launch_bounds__(1024) k_scan_counts(uint32_t* counts, long long m) {
-    __shared__ uint32_t warp_sums[32];
-    __shared__ uint32_t carry;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    for (long long base = 0; base < m; base += 1024 * 8) {
-        uint32_t v[8];
-        uint32_t sum = 0;
-        long long i0 = base + (long long)threadIdx.x * 8;
-        for (int k = 0; k < 8; ++k) { v[k] = (i0 + k < m) ? counts[i0 + k] : 0u; sum += v[k]; }
-        uint32_t incl = sum;
-        const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-        for (int o = 1; o < 32; o <<= 1) {
-            uint32_t y = __shfl_up_sync(kFull, incl, o);
-            if (lane >= o) incl += y;
-        }
-        if (lane == 31) warp_sums[wid] = incl;
-        __syncthreads();
-        if (wid == 0) {
-            uint32_t w = warp_sums[lane], wi = w;
-            for (int o = 1; o < 32; o <<= 1) {
-                uint32_t y = __shfl_up_sync(kFull, wi, o);
-                if (lane >= o) wi += y;
-            }
-            warp_sums[lane] = wi - w;
-        }
-        __syncthreads();
-        uint32_t run = carry + warp_sums[wid] + incl - sum;
-        for (int k = 0; k < 8; ++k) {
-            if (i0 + k < m) counts[i0 + k] = run;
-            run += v[k];
-        }
-        __syncthreads();
-        if (threadIdx.x == 1023) carry = run;
-        __syncthreads();
-    }
-}
-
-// Multi-block form of the same scan for large m: each block scans one 8192-counter tile
-// in place and writes its total, one block scans the totals, a third pass adds them.
-constexpr long long kScanTile = 1024 * 8;
-__global__ void __launch_bounds__(1024) k_scan_tile(uint32_t* counts, long long m, uint32_t* tile_sums) {
-    __shared__ uint32_t warp_sums[32];
-    const long long base = blockIdx.x * kScanTile;
-    uint32_t v[8];
-    uint32_t sum = 0;
-    const long long i0 = base + (long long)threadIdx.x * 8;
-    for (int k = 0; k < 8; ++k) { v[k] = (i0 + k < m) ? counts[i0 + k] : 0u; sum += v[k]; }
-    uint32_t incl = sum;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    for (int o = 1; o < 32; o <<= 1) {
-        uint32_t y = __shfl_up_sync(kFull, incl, o);
-        if (lane >= o) incl += y;
-    }
-    if (lane == 31) warp_sums[wid] = incl;
-    __syncthreads();
-    if (wid == 0) {
-        uint32_t w = warp_sums[lane], wi = w;
-        for (int o = 1; o < 32; o <<= 1) {
-            uint32_t y = __shfl_up_sync(kFull, wi, o);
-            if (lane >= o) wi += y;
-        }
-        warp_sums[lane] = wi - w;
-        if (lane == 31) tile_sums[blockIdx.x] = wi;
-    }
-    __syncthreads();
-    uint32_t run = warp_sums[wid] + incl - sum;
-    for (int k = 0; k < 8; ++k) {
-        if (i0 + k < m) counts[i0 + k] = run;
-        run += v[k];
-    }
-}
-
-__global__ void k_scan_tile_add(uint32_t* counts, long long m, const uint32_t* __restrict__ tile_offsets) {
-    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i < m) counts[i] += tile_offsets[i / kScanTile];
-}
-
-// Query order: a stable LSD radix sort of the queries' 30-bit Morton codes (10 bits per
-// axis over the queries' bounding box), three passes of 10-bit digits.  Consecutive
-// queries of the sorted order are then close in space whatever the photon density (an
-// order by KD cell is not: a cell of a sparsely lit region holds hundreds of queries).
-constexpr int kRsBits = 10, kRsBins = 1 << kRsBits, kRsThreads = 256, kRsWarps = kRsThreads / 32;
-constexpr int kRsPerWarp = 256;                        // keys a warp ranks per tile
-constexpr long long kRsTile = kRsWarps * kRsPerWarp;   // keys per block
-
-__device__ __forceinline__ uint32_t spread10(uint32_t v) {
-    v &= 0x3ffu;
-    v = (v | (v << 16)) & 0x030000FFu;
-    v = (v | (v << 8)) & 0x0300F00Fu;
-    v = (v | (v << 4)) & 0x030C30C3u;
-    v = (v | (v << 2)) & 0x09249249u;
-    return v;
-}
-
-__device__ __forceinline__ uint32_t cell10(float v) {
-    return v > 0.0f ? (v < 1023.0f ? (uint32_t)v : 1023u) : 0u;   // NaN -> 0
-}
-
-__global__ void k_query_keys(const float* __restrict__ qpos, int stride, long long nq,
-                             const unsigned long long* __restrict__ nq_dev, QueryFrame f, uint32_t* __restrict__ keys,
-                             uint32_t* __restrict__ vals) {
-    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (nq_dev) nq = (long long)min(*nq_dev, (unsigned long long)nq);
-    if (i >= nq) return;
-    const float* q = qpos + (long long)stride * i;
-    const uint32_t cx = cell10((q[0] - f.lo[0]) * f.scale[0]);
-    const uint32_t cy = cell10((q[1] - f.lo[1]) * f.scale[1]);
-    const uint32_t cz = cell10((q[2] - f.lo[2]) * f.scale[2]);
-    keys[i] = spread10(cx) | (spread10(cy) << 1) | (spread10(cz) << 2);
-    vals[i] = (uint32_t)i;
-}
-
-// Per-block digit counts, digit-major (hist[d * blocks + b]), so that one exclusive scan
-// of the whole array gives every (digit, block) its first output position.
-__global__ void __launch_bounds__(kRsThreads) k_rs_hist(const uint32_t* __restrict__ keys, long long nq,
-                                                        const unsigned long long* __restrict__ nq_dev, int shift,
-                                                        uint32_t* __restrict__ hist) {
-    __shared__ uint32_t cnt[kRsBins];
-    for (int d = threadIdx.x; d < kRsBins; d += kRsThreads) cnt[d] = 0;
-    __syncthreads();
-    if (nq_dev) nq = (long long)min(*nq_dev, (unsigned long long)nq);
-    const long long base = (long long)blockIdx.x * kRsTile;
-    for (int k = threadIdx.x; k < kRsTile; k += kRsThreads) {
-        const long long i = base + k;
-        if (i < nq) atomicAdd(&cnt[(keys[i] >> shift) & (kRsBins - 1)], 1u);
-    }
-    __syncthreads();
-    for (int d = threadIdx.x; d < kRsBins; d += kRsThreads) hist[(long long)d * gridDim.x + blockIdx.x] = cnt[d];
-}
-
-// Stable scatter of one block's tile: warp w ranks the keys [w * 256, (w + 1) * 256) of
-// the tile in order (per-warp digit counts, a prefix over the warps per digit on top of
-// the block's scanned offsets, then ranks by __match_any_sync round by round).
-__global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const uint32_t* __restrict__ keys_in,
-                                                           const uint32_t* __restrict__ vals_in,
-                                                           uint32_t* __restrict__ keys_out,
-                                                           uint32_t* __restrict__ vals_out, long long nq,
-                                                           const unsigned long long* __restrict__ nq_dev, int shift,
-                                                           const uint32_t* __restrict__ offsets) {
-    __shared__ uint32_t wc[kRsWarps][kRsBins];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const unsigned lt = (1u << lane) - 1u;
-    for (int k = threadIdx.x; k < kRsWarps * kRsBins; k += kRsThreads) (&wc[0][0])[k] = 0;
-    __syncthreads();
-    if (nq_dev) nq = (long long)min(*nq_dev, (unsigned long long)nq);
-    const long long wbase = (long long)blockIdx.x * kRsTile + (long long)warp * kRsPerWarp;
-    for (int r = 0; r < kRsPerWarp / 32; ++r) {
-        const long long i = wbase + r * 32 + lane;
-        const bool valid = i < nq;
-        const uint32_t d = valid ? (keys_in[i] >> shift) & (kRsBins - 1) : 0xffffffffu;
-        const unsigned peers = __match_any_sync(kFull, d);
-        if (valid && (peers & lt) == 0u) wc[warp][d] += (uint32_t)__popc(peers);
-        __syncwarp();
-    }
-    __syncthreads();
-    for (int d = threadIdx.x; d < kRsBins; d += kRsThreads) {
-        uint32_t run = offsets[(long long)d * gridDim.x + blockIdx.x];
-        for (int w = 0; w < kRsWarps; ++w) {
-            const uint32_t c = wc[w][d];
-            wc[w][d] = run;
-            run += c;
-        }
-    }
-    __syncthreads();
-    for (int r = 0; r < kRsPerWarp / 32; ++r) {
-        const long long i = wbase + r * 32 + lane;
-        const bool valid = i < nq;
-        uint32_t key = 0, val = 0, d = 0xffffffffu;
-        if (valid) {
-            key = keys_in[i];
-            val = vals_in[i];
-            d = (key >> shift) & (kRsBins - 1);
-        }
-        const unsigned peers = __match_any_sync(kFull, d);
-        uint32_t pos = 0;
-        if (valid) pos = wc[warp][d] + (uint32_t)__popc(peers & lt);
-        __syncwarp();
-        if (valid) {
-            keys_out[pos] = key;
-            vals_out[pos] = val;
-            if ((peers & lt) == 0u) wc[warp][d] += (uint32_t)__popc(peers);
-        }
-        __syncwarp();
-    }
-}
-
-// Chunk boxes: one warp per chunk reduces its (at most 32) photons' coordinates.
-__global__ void k_chunk_boxes(const float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ z,
-                              long long n, int lc, float4* __restrict__ lo, float4* __restrict__ hi) {
-    const long long w = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    const long long m = 1LL << lc;
-    if (w >= m) return;
-    const long long e = m + w;
-    const long long s = kd_node_start(e, lc, n);
-    const long long end = (w + 1 < m) ? kd_node_start(e + 1, lc, n) : n;
-    const long long c = end - s;   // <= 32: the node's range plus at most one median
-    float mnx = INFINITY, mny = INFINITY, mnz = INFINITY, mxx = -INFINITY, mxy = -INFINITY, mxz = -INFINITY;
-    if (lane < c) {
-        mnx = mxx = x[s + lane];
-        mny = mxy = y[s + lane];
-        mnz = mxz = z[s + lane];
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        mnx = fminf(mnx, __shfl_xor_sync(kFull, mnx, o)); mny = fminf(mny, __shfl_xor_sync(kFull, mny, o));
-        mnz = fminf(mnz, __shfl_xor_sync(kFull, mnz, o)); mxx = fmaxf(mxx, __shfl_xor_sync(kFull, mxx, o));
-        mxy = fmaxf(mxy, __shfl_xor_sync(kFull, mxy, o)); mxz = fmaxf(mxz, __shfl_xor_sync(kFull, mxz, o));
-    }
-    if (lane == 0) {
-        lo[e] = make_float4(mnx, mny, mnz, __uint_as_float((uint32_t)s));
-        hi[e] = make_float4(mxx, mxy, mxz, __uint_as_float((uint32_t)c));
-    }
-}
-
-// Boxes of the nodes on one level: the union of their children's.
-__device__ __forceinline__ void unite_children(float4* lo, float4* hi, long long e) {
-    const float4 a = lo[2 * e], b = lo[2 * e + 1], c = hi[2 * e], d = hi[2 * e + 1];
-    lo[e] = make_float4(fminf(a.x, b.x), fminf(a.y, b.y), fminf(a.z, b.z), 0.0f);
-    hi[e] = make_float4(fmaxf(c.x, d.x), fmaxf(c.y, d.y), fmaxf(c.z, d.z), 0.0f);
-}
-__global__ void k_level_boxes(int level, float4* lo, float4* hi) {
-    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i < (1LL << level)) unite_children(lo, hi, (1LL << level) + i);
-}
-// levels [0, top] in one CTA, bottom-up
-constexpr int kTopLevels = 11;
-__global__ void __launch_bounds__(1024) k_top_boxes(int top, float4* lo, float4* hi) {
-    for (int l = top; l >= 0; --l) {
-        for (long long i = threadIdx.x; i < (1LL << l); i += blockDim.x) unite_children(lo, hi, (1LL << l) + i);
-        __syncthreads();
-    }
-}
-
-// Photon records gathered into tree order, so the gather reads them contiguously
-// (positions only when ph.dir is null).
-__global__ void k_tree_records(PhotonBuf ph, const uint32_t* __restrict__ id, long long n, TreePhotons tp) {
-    const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    const uint32_t i = id[p];
-    tp.t0[p] = ph.pos[i];
-    if (ph.dir) {
-        tp.t1[p] = ph.dir[i];
-        tp.t2[p] = ph.tp[i];
-    }
-}
-
-ChunkTree chunk_tree(const KdTree& tree, const float4* t0) {
-    return ChunkTree{tree.box_lo, tree.box_hi, t0, (tree.n > 0 && tree.box_lo) ? tree.box_levels - 1 : -1};
+ChunkTree chunk_tree(const PhotonTree& tree, const float4* t0) {
+    return ChunkTree{tree.box_lo, tree.box_hi, t0, photon_chunk_level(tree.n)};
 }
 
 // Launch shapes: (resident blocks per SM, queries per group, levels per expansion step).
@@ -766,99 +514,6 @@ void launch_variant(int v, const ChunkTree& t, const float* qpos, int qstride, c
 
 }  // namespace
 
-int kd_chunk_level(long long n) {
-    if (n <= 0) return -1;
-    int l = 0;
-    while ((n >> l) > kChunkNode) ++l;
-    return l;
-}
-
-int kd_box_levels(long long n) { return n > 0 ? kd_chunk_level(n) + 1 : 0; }
-
-void launch_kd_boxes(const KdTree& tree, cudaStream_t s, int* launches) {
-    if (tree.n <= 0 || !tree.box_lo) return;
-    const int lc = tree.box_levels - 1;
-    const long long chunks = 1LL << lc;
-    k_chunk_boxes<<<(unsigned)((chunks * 32 + 255) / 256), 256, 0, s>>>(tree.x, tree.y, tree.z, tree.n, lc,
-                                                                        tree.box_lo, tree.box_hi);
-    int nl = 1;
-    int l = lc - 1;
-    for (; l > kTopLevels; --l) {
-        k_level_boxes<<<(unsigned)(((1LL << l) + 255) / 256), 256, 0, s>>>(l, tree.box_lo, tree.box_hi);
-        ++nl;
-    }
-    if (l >= 0) {
-        k_top_boxes<<<1, 1024, 0, s>>>(l, tree.box_lo, tree.box_hi);
-        ++nl;
-    }
-    if (launches) *launches += nl;
-}
-
-namespace {
-long long rs_blocks(long long nq) { return (nq + kRsTile - 1) / kRsTile; }
-}  // namespace
-
-size_t query_order_scratch_bytes(long long nq) {
-    const long long n = nq > 0 ? nq : 1;
-    const long long m = rs_blocks(n) * kRsBins;
-    auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
-    return 3 * al(4 * (size_t)n) + al(4 * (size_t)m) + al(4 * scan_scratch_words(m));
-}
-
-QueryFrame query_frame(const float lo[3], const float hi[3]) {
-    QueryFrame f;
-    for (int k = 0; k < 3; ++k) {
-        const float ext = hi[k] - lo[k];
-        f.lo[k] = lo[k];
-        f.scale[k] = ext > 0.0f ? 1023.99f / ext : 0.0f;
-    }
-    return f;
-}
-
-void launch_query_order(const float* qpos, int stride, long long nq, const QueryFrame& frame, void* scratch,
-                        uint32_t* order, int* launches, cudaStream_t s, const unsigned long long* nq_dev) {
-    if (nq <= 0) return;
-    const long long B = rs_blocks(nq), m = B * kRsBins;
-    auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
-    char* p = (char*)scratch;
-    uint32_t* keys_a = (uint32_t*)p; p += al(4 * (size_t)nq);
-    uint32_t* keys_b = (uint32_t*)p; p += al(4 * (size_t)nq);
-    uint32_t* vals_a = (uint32_t*)p; p += al(4 * (size_t)nq);
-    uint32_t* hist = (uint32_t*)p; p += al(4 * (size_t)m);
-    uint32_t* tiles = (uint32_t*)p;
-    k_query_keys<<<(unsigned)((nq + 255) / 256), 256, 0, s>>>(qpos, stride, nq, nq_dev, frame, keys_a, vals_a);
-    int nl = 1;
-    // passes: a -> (keys_b, order), (keys_b, order) -> (keys_a, vals_a), (keys_a, vals_a) -> (keys_b, order)
-    const uint32_t* kin[3] = {keys_a, keys_b, keys_a};
-    const uint32_t* vin[3] = {vals_a, order, vals_a};
-    uint32_t* kout[3] = {keys_b, keys_a, keys_b};
-    uint32_t* vout[3] = {order, vals_a, order};
-    for (int pass = 0; pass < 3; ++pass) {
-        k_rs_hist<<<(unsigned)B, kRsThreads, 0, s>>>(kin[pass], nq, nq_dev, pass * kRsBits, hist);
-        launch_scan_counts(hist, m, tiles, s);
-        k_rs_scatter<<<(unsigned)B, kRsThreads, 0, s>>>(kin[pass], vin[pass], kout[pass], vout[pass], nq, nq_dev,
-                                                         pass * kRsBits, hist);
-        nl += 2 + (m > 4 * kScanTile ? 3 : 1);
-    }
-    if (launches) *launches += nl;
-}
-
-size_t scan_scratch_words(long long m) { return (size_t)(m / kScanTile + 2); }
-
-void launch_scan_counts(uint32_t* counts, long long m, uint32_t* tile_scratch, cudaStream_t s) {
-    if (m <= 0) return;
-    if (m <= 4 * kScanTile || !tile_scratch) { k_scan_counts<<<1, 1024, 0, s>>>(counts, m); return; }
-    const long long tiles = (m + kScanTile - 1) / kScanTile;
-    k_scan_tile<<<(unsigned)tiles, 1024, 0, s>>>(counts, m, tile_scratch);
-    k_scan_counts<<<1, 1024, 0, s>>>(tile_scratch, tiles);
-    k_scan_tile_add<<<(unsigned)((m + 255) / 256), 256, 0, s>>>(counts, m, tile_scratch);
-}
-
-void launch_tree_records(PhotonBuf ph, const KdTree& tree, TreePhotons tp, cudaStream_t s) {
-    if (tree.n <= 0) return;
-    k_tree_records<<<(unsigned)((tree.n + 255) / 256), 256, 0, s>>>(ph, tree.id, tree.n, tp);
-}
-
 int gather_variants() { return kNumShapes; }
 int gather_default_variant() { return kDefaultShape; }
 
@@ -871,7 +526,7 @@ const char* gather_variant_name(int v) {
     return (v >= 0 && v < kNumShapes) ? names[v] : "?";
 }
 
-void launch_gather(const VMParams& p, const KdTree& tree, TreePhotons tp, QueryBuf qb, const uint32_t* order,
+void launch_gather(const VMParams& p, const PhotonTree& tree, TreePhotons tp, QueryBuf qb, const uint32_t* order,
                    long long nq, double* accum, unsigned long long* counters, cudaStream_t s, int variant,
                    const unsigned long long* nq_dev, const int* skip) {
     if (nq <= 0 || tree.n <= 0) return;
@@ -880,7 +535,7 @@ void launch_gather(const VMParams& p, const KdTree& tree, TreePhotons tp, QueryB
                    skip, p.radius_sqr, sink, counters, p.error + ERR_GATHER, s);
 }
 
-void launch_gather_sets(const KdTree& tree, const float4* t0, const float* qpos, int qstride, const uint32_t* order,
+void launch_gather_sets(const PhotonTree& tree, const float4* t0, const float* qpos, int qstride, const uint32_t* order,
                         long long nq, float r2, int* counts, const long long* offsets, int* cursor, int* idx,
                         int variant, unsigned long long* counters, int* err, cudaStream_t s) {
     if (nq <= 0 || tree.n <= 0) return;

@@ -1,4 +1,6 @@
-// Photon KD-tree built on the GPU by parallel median splits.
+// Photon KD-tree built on the GPU by parallel median splits, for the callers that ask for
+// the tree itself (rc_kd_build_nodes, rc_kd_build_noalloc); the render's gather walks
+// spatially sorted photons instead (photon_order.cu).
 //
 // Same tree as KD_Tree::build_kd_tree (src/KD_Tree.cpp:110-190): an implicit heap
 // of 8-byte nodes, root at 1, children 2e and 2e+1.  A node over `count` photons
@@ -32,10 +34,6 @@ struct KdTree {
     // photons in tree order (SoA) and their photon-buffer index
     float* x = nullptr; float* y = nullptr; float* z = nullptr;
     uint32_t* id = nullptr;
-    // optional node bounding boxes for levels [0, box_levels) (launch_kd_boxes)
-    float4* box_lo = nullptr;
-    float4* box_hi = nullptr;
-    int box_levels = 0;
 };
 
 // Start of node e's photon range (root e = 1, level = floor(log2 e)).

@@ -15,6 +15,7 @@
 
 #include "bvh_build.h"
 #include "host_scene.h"
+#include "kdtree.cuh"
 #include "mlp.cuh"
 #include "proposal.cuh"
 #include "realcaustics.h"
@@ -56,7 +57,7 @@ struct DeviceState {
     bool ready = false;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev[8] = {};
-    // the camera pass's stream, beside the light pass and the KD build: fork and join
+    // the camera pass's stream, beside the light pass and the photon order: fork and join
     // events (timing disabled)
     cudaStream_t side = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
@@ -75,10 +76,8 @@ struct DeviceState {
     DevBuf<float4> q0, q1, q2, q3, q4;
     DevBuf<unsigned long long> counters;   // [0] photons, [1] queries
     DevBuf<int> errors;
-    DevBuf<uint2> kd_nodes;
-    DevBuf<float> kd_x, kd_y, kd_z;
-    DevBuf<uint32_t> kd_id;
-    DevBuf<unsigned char> kd_scratch;
+    DevBuf<uint32_t> ph_order;              // sorted photons (launch_photon_order) and its scratch
+    DevBuf<unsigned char> ph_scratch;
     DevBuf<float4> tp0, tp1, box_lo, box_hi;
     DevBuf<float2> tp2;
     DevBuf<uint32_t> qorder;
@@ -122,7 +121,7 @@ struct DeviceState {
         for (auto* b : f4) b->release();
         world_mesh.release(); mesh_root.release(); lights.release(); cdf.release(); materials.release();
         ph_tp.release(); ph_path.release(); counters.release(); errors.release();
-        kd_nodes.release(); kd_x.release(); kd_y.release(); kd_z.release(); kd_id.release(); kd_scratch.release();
+        ph_order.release(); ph_scratch.release();
         tp0.release(); tp1.release(); tp2.release(); qorder.release(); qscratch.release();
         box_lo.release(); box_hi.release();
         accum.release();
@@ -436,13 +435,25 @@ int prepare() {
     return RC_OK;
 }
 
-// Frame of the merge queries' Morton order: the scene's bounding box (every camera
-// vertex lies on a scene surface).
-QueryFrame scene_query_frame(const HostScene& sc) {
+// Frame of the photons' and merge queries' spatial order: the scene's bounding box (every
+// path vertex lies on a scene surface).
+CurveFrame scene_frame(const HostScene& sc, const VMParams& p) {
     const float lo[3] = {sc.bounds.mn.x, sc.bounds.mn.y, sc.bounds.mn.z};
     const float hi[3] = {sc.bounds.mx.x, sc.bounds.mx.y, sc.bounds.mx.z};
-    return query_frame(lo, hi);
+    return curve_frame(lo, hi, std::sqrt(p.radius_sqr));
 }
+
+// The gather's photon structure over n photons, in the context's buffers.
+int reserve_photon_tree(long long n) {
+    DeviceState& d = ctx().dev;
+    const size_t m = (size_t)std::max<long long>(n, 1), boxes = (size_t)2 << std::max(photon_chunk_level(n), 0);
+    RC_CUDA(d.ph_order.reserve(m));
+    RC_CUDA(d.ph_scratch.reserve(order_scratch_bytes(n)));
+    RC_CUDA(d.tp0.reserve(m)); RC_CUDA(d.tp1.reserve(m)); RC_CUDA(d.tp2.reserve(m));
+    RC_CUDA(d.box_lo.reserve(boxes)); RC_CUDA(d.box_hi.reserve(boxes));
+    return RC_OK;
+}
+PhotonTree photon_tree(const DeviceState& d, long long n) { return {n, d.ph_order.p, d.box_lo.p, d.box_hi.p}; }
 
 int check_errors() {
     int h[ERR_COUNT];
@@ -505,9 +516,9 @@ cudaError_t record(cudaEvent_t e, cudaStream_t s) {
                                                : cudaEventRecord(e, s);
 }
 
-// Device time from the light pass's start to the later of the KD build's end and the
+// Device time from the light pass's start to the later of the photon order's end and the
 // camera pass's end, for an iteration whose camera pass ran on the side stream (its
-// events ev[4], ev[5] overlap the light pass and the KD build).
+// events ev[4], ev[5] overlap the light pass and the photon order).
 double overlapped_ms(const DeviceState& d) {
     return std::max(ms_between(d.ev[0], d.ev[3]), ms_between(d.ev[0], d.ev[5]));
 }
@@ -769,7 +780,7 @@ int render_iteration(HostScene& sc, int redo_iteration = -1, bool tune_passes = 
     // Once its launch shape is tuned it then runs on the side stream: with uniformly
     // sampled light paths issued right before the light pass, so that its blocks take
     // the SMs that the light pass's tail frees and run through the host's read-back of
-    // the photon count and the KD build's launches; with a Metropolis sampler issued
+    // the photon count and the photon order's launches; with a Metropolis sampler issued
     // before the chains, whose one thread per chain leaves room on every SM.  It joins
     // the main stream before the query order.  (With the learned proposal the network's
     // inference ends before the fork and its training starts after the join: no
@@ -867,7 +878,7 @@ int render_iteration(HostScene& sc, int redo_iteration = -1, bool tune_passes = 
         if (attempt == 2) { ctx().err = "photon buffer overflow"; return RC_E_CAPACITY; }
     }
     if (nph >= (1ull << 28)) {
-        // the KD node word holds a photon index in 28 bits (src/KD_Tree.h:13-32)
+        // a KD node word holds a photon index in 28 bits (src/KD_Tree.h:13-32)
         ctx().err = "more than 2^28 photons stored in one iteration";
         return RC_E_CAPACITY;
     }
@@ -879,38 +890,18 @@ int render_iteration(HostScene& sc, int redo_iteration = -1, bool tune_passes = 
         p.merge_scale = vis;
         d.stats_mlt_visible = vis;
     }
-    // KD tree over the stored photons
-    long long n = (long long)nph;
-    long long nn = kd_node_array_len(n);
-    RC_CUDA(d.kd_nodes.reserve(std::max<long long>(nn, 2)));
-    RC_CUDA(d.kd_x.reserve(std::max<long long>(n, 1))); RC_CUDA(d.kd_y.reserve(std::max<long long>(n, 1)));
-    RC_CUDA(d.kd_z.reserve(std::max<long long>(n, 1))); RC_CUDA(d.kd_id.reserve(std::max<long long>(n, 1)));
-    size_t sb = kd_scratch_bytes(n);
-    RC_CUDA(d.kd_scratch.reserve(sb));
-    KdTree tree;
-    tree.nodes = d.kd_nodes.p; tree.x = d.kd_x.p; tree.y = d.kd_y.p; tree.z = d.kd_z.p; tree.id = d.kd_id.p;
-    int kd_launches = 0;
+    // the stored photons sorted for the gather, with their boxes
+    const long long n = (long long)nph;
+    const CurveFrame frame = scene_frame(sc, p);
+    r = reserve_photon_tree(n);
+    if (r) return r;
+    const PhotonTree tree = photon_tree(d, n);
+    const TreePhotons tph{d.tp0.p, d.tp1.p, d.tp2.p};
+    int order_launches = 0;
     RC_CUDA(cudaEventRecord(d.ev[2], s));
-    if (kd_build(d.ph_pos.p, n, tree, d.kd_scratch.p, d.kd_scratch.n, s, &kd_launches, d.errors.p + ERR_KD)) {
-        ctx().err = "KD scratch too small"; return RC_E_CAPACITY;
-    }
+    launch_photon_order(PhotonBuf{d.ph_pos.p, d.ph_dir.p, d.ph_tp.p, d.ph_path.p, (long long)d.ph_pos.n, d.counters.p}, n,
+                        nullptr, frame, d.ph_scratch.p, tree, tph, &order_launches, s);
     RC_CUDA(cudaGetLastError());
-    RC_CUDA(d.tp0.reserve(std::max<long long>(n, 1))); RC_CUDA(d.tp1.reserve(std::max<long long>(n, 1)));
-    RC_CUDA(d.tp2.reserve(std::max<long long>(n, 1)));
-    TreePhotons tph{d.tp0.p, d.tp1.p, d.tp2.p};
-    tree.box_levels = kd_box_levels(n);
-    if (tree.box_levels > 0) {
-        RC_CUDA(d.box_lo.reserve((size_t)1 << tree.box_levels));
-        RC_CUDA(d.box_hi.reserve((size_t)1 << tree.box_levels));
-        tree.box_lo = d.box_lo.p; tree.box_hi = d.box_hi.p;
-        launch_kd_boxes(tree, s, &kd_launches);
-        RC_CUDA(cudaGetLastError());
-    }
-    {
-        PhotonBuf phb{d.ph_pos.p, d.ph_dir.p, d.ph_tp.p, d.ph_path.p, (long long)d.ph_pos.n, d.counters.p};
-        launch_tree_records(phb, tree, tph, s);
-        RC_CUDA(cudaGetLastError());
-    }
     RC_CUDA(cudaEventRecord(d.ev[3], s));
     // camera pass -> merge queries (joined from the side stream, or run here: untuned
     // launch shape, a Metropolis sampler, or a query overflow)
@@ -958,10 +949,10 @@ int render_iteration(HostScene& sc, int redo_iteration = -1, bool tune_passes = 
     if (r) return r;
     QueryBuf qb{d.q0.p, d.q1.p, d.q2.p, d.q3.p, d.q4.p, (long long)d.q0.n, d.counters.p + 1};
     RC_CUDA(d.qorder.reserve(std::max<unsigned long long>(nq, 1)));
-    RC_CUDA(d.qscratch.reserve(query_order_scratch_bytes((long long)nq)));
+    RC_CUDA(d.qscratch.reserve(order_scratch_bytes((long long)nq)));
     RC_CUDA(cudaEventRecord(d.ev[6], s));
     int qlaunch = 0;
-    launch_query_order(reinterpret_cast<const float*>(d.q0.p), 4, (long long)nq, scene_query_frame(sc), d.qscratch.p,
+    launch_query_order(reinterpret_cast<const float*>(d.q0.p), 4, (long long)nq, frame, d.qscratch.p,
                        d.qorder.p, &qlaunch, s);
     int variant = gather_default_variant();
     if (cfg().autotune && nq > 0) {
@@ -1031,7 +1022,7 @@ int render_iteration(HostScene& sc, int redo_iteration = -1, bool tune_passes = 
     st[10] = d.iterations_done;
     st[11] = sc.scene_radius;
     st[12] = std::sqrt(p.radius_sqr);
-    st[13] = kd_launches + 3 + qlaunch;
+    st[13] = order_launches + 3 + qlaunch;
     d.acc_gather_ms += ms_between(d.evg[0], d.evg[1]);   // the gather kernel alone
     // gather algorithmic bytes: each photon record read once (40 B), each query record
     // read once (64 B), each pixel's FP64 RGB sum read and written once (48 B)
@@ -1049,7 +1040,7 @@ int render_iteration(HostScene& sc, int redo_iteration = -1, bool tune_passes = 
 // ---------------------------------------------------------------- asynchronous iterations
 // After one iteration with host round trips has fixed the sizes, further iterations of
 // the uniform sampler are enqueued without any: photon and query capacities are fixed
-// (the KD tree is built over the whole photon capacity, unused slots padded far away,
+// (the photon order covers the whole photon capacity, unused slots padded far away,
 // which leaves every radius query's answer unchanged), the query order and the gather
 // read the query count on the device, and a per-iteration flag records a count that
 // overflowed its capacity (that iteration's gather is skipped and the iteration is
@@ -1085,14 +1076,10 @@ int async_setup(const HostScene& sc) {
     RC_CUDA(d.q0.reserve(d.async_qcap)); RC_CUDA(d.q1.reserve(d.async_qcap)); RC_CUDA(d.q2.reserve(d.async_qcap));
     RC_CUDA(d.q3.reserve(d.async_qcap)); RC_CUDA(d.q4.reserve(d.async_qcap));
     const long long n = d.async_pcap;
-    RC_CUDA(d.kd_nodes.reserve(std::max<long long>(kd_node_array_len(n), 2)));
-    RC_CUDA(d.kd_x.reserve(n)); RC_CUDA(d.kd_y.reserve(n)); RC_CUDA(d.kd_z.reserve(n)); RC_CUDA(d.kd_id.reserve(n));
-    RC_CUDA(d.kd_scratch.reserve(kd_scratch_bytes(n)));
-    RC_CUDA(d.tp0.reserve(n)); RC_CUDA(d.tp1.reserve(n)); RC_CUDA(d.tp2.reserve(n));
-    const int bl = kd_box_levels(n);
-    if (bl > 0) { RC_CUDA(d.box_lo.reserve((size_t)1 << bl)); RC_CUDA(d.box_hi.reserve((size_t)1 << bl)); }
+    int r = reserve_photon_tree(n);
+    if (r) return r;
     RC_CUDA(d.qorder.reserve(d.async_qcap));
-    RC_CUDA(d.qscratch.reserve(query_order_scratch_bytes(d.async_qcap)));
+    RC_CUDA(d.qscratch.reserve(order_scratch_bytes(d.async_qcap)));
     RC_CUDA(d.accum.reserve(3 * npix));
     auto var = [](int v, int dflt) { return v >= 0 ? v : dflt; };
     d.async_lvar = var(light_slot(cfg().photons_per_iter > 0 ? cfg().photons_per_iter : npix).load(), kUntunedPass);
@@ -1102,7 +1089,7 @@ int async_setup(const HostScene& sc) {
     // the staged passes' scratch: reserved before any capture
     const long long paths = cfg().photons_per_iter > 0 ? cfg().photons_per_iter : npix;
     void* park = nullptr;
-    int r = reserve_park(d.light_park, d.async_lvar, paths, &park);
+    r = reserve_park(d.light_park, d.async_lvar, paths, &park);
     if (!r) r = reserve_park(d.camera_park, d.async_cvar, npix, &park);
     if (r) return r;
     return RC_OK;
@@ -1120,41 +1107,32 @@ int async_head(VMParams& p, cudaStream_t s) {
     return RC_OK;
 }
 
-// async_tail, on s after the light pass: the photon capacity padded, the KD tree and its
-// boxes, the tree-order records; then, once the camera pass has recorded `camera_done`,
+// async_tail, on s after the light pass: the photon capacity padded, the photon order with
+// its boxes and records; then, once the camera pass has recorded `camera_done`,
 // the count check (`flag` = 1 on an overflow), the query order and the gather.
 int async_tail(HostScene& sc, const VMParams& p, cudaStream_t s, cudaEvent_t camera_done, int* flag) {
     DeviceState& d = ctx().dev;
     const long long pc = d.async_pcap, qc = d.async_qcap;
     QueryBuf qb{d.q0.p, d.q1.p, d.q2.p, d.q3.p, d.q4.p, qc, d.counters.p + 1};
     // pads one scene extent (plus four base radii) beyond the scene's +x face: outside
-    // every merge radius, and close enough that the KD build's largest-extent rule
-    // separates them from the stored photons along x within a few levels
+    // every merge radius (they are sorted behind the stored photons)
     const float ext = std::max(std::max(sc.bounds.mx.x - sc.bounds.mn.x, sc.bounds.mx.y - sc.bounds.mn.y),
                                sc.bounds.mx.z - sc.bounds.mn.z);
     const float4 pad = make_float4(sc.bounds.mx.x + ext + 4.0f * sc.base_radius + 1.0f,
                                    0.5f * (sc.bounds.mn.y + sc.bounds.mx.y), 0.5f * (sc.bounds.mn.z + sc.bounds.mx.z),
                                    0.0f);
     launch_pad_photons(d.ph_pos.p, d.counters.p, pc, pad, s);
-    KdTree tree{};
-    tree.nodes = d.kd_nodes.p; tree.x = d.kd_x.p; tree.y = d.kd_y.p; tree.z = d.kd_z.p; tree.id = d.kd_id.p;
     RC_CUDA(record(d.ev[2], s));
-    int kl = 0;
-    if (kd_build(d.ph_pos.p, pc, tree, d.kd_scratch.p, d.kd_scratch.n, s, &kl, d.errors.p + ERR_KD)) {
-        ctx().err = "KD scratch too small"; return RC_E_CAPACITY;
-    }
-    TreePhotons tph{d.tp0.p, d.tp1.p, d.tp2.p};
-    tree.box_levels = kd_box_levels(pc);
-    if (tree.box_levels > 0) {
-        tree.box_lo = d.box_lo.p; tree.box_hi = d.box_hi.p;
-        launch_kd_boxes(tree, s, nullptr);
-    }
-    launch_tree_records(PhotonBuf{d.ph_pos.p, d.ph_dir.p, d.ph_tp.p, d.ph_path.p, pc, d.counters.p}, tree, tph, s);
+    const CurveFrame frame = scene_frame(sc, p);
+    const PhotonTree tree = photon_tree(d, pc);
+    const TreePhotons tph{d.tp0.p, d.tp1.p, d.tp2.p};
+    launch_photon_order(PhotonBuf{d.ph_pos.p, d.ph_dir.p, d.ph_tp.p, d.ph_path.p, pc, d.counters.p}, pc, d.counters.p, frame,
+                        d.ph_scratch.p, tree, tph, nullptr, s);
     RC_CUDA(record(d.ev[3], s));
     RC_CUDA(cudaStreamWaitEvent(s, camera_done, 0));
     launch_check_counts(d.counters.p, pc, d.counters.p + 1, qc, flag, s);
     RC_CUDA(record(d.ev[6], s));
-    launch_query_order(reinterpret_cast<const float*>(d.q0.p), 4, qc, scene_query_frame(sc), d.qscratch.p, d.qorder.p,
+    launch_query_order(reinterpret_cast<const float*>(d.q0.p), 4, qc, frame, d.qscratch.p, d.qorder.p,
                        nullptr, s, d.counters.p + 1);
     RC_CUDA(cudaMemsetAsync(d.counters.p + 2, 0, 4 * sizeof(unsigned long long), s));
     RC_CUDA(record(d.evg[0], s));
@@ -1175,8 +1153,8 @@ int enqueue_async_iteration(HostScene& sc, int it, int* flag) {
     QueryBuf qb{d.q0.p, d.q1.p, d.q2.p, d.q3.p, d.q4.p, qc, d.counters.p + 1};
     int r = async_head(p, s);
     if (r) return r;
-    // the camera pass on a branch of its own beside the light pass's tail and the KD
-    // build (it reads nothing they write), joined before the count check
+    // the camera pass on a branch of its own beside the light pass's tail and the photon
+    // order (it reads nothing they write), joined before the count check
     r = light_pass(p, ph, s, d.async_lvar, d.fork);   // the camera branch forks where
     if (r) return r;                                   // the light pass stops filling the GPU
     RC_CUDA(record(d.ev[1], s));
@@ -1301,8 +1279,7 @@ int render_iterations(HostScene& sc, int iterations) {
         ++i;
         if (r) return r;
         // Replay pays where host round trips and launch gaps are a visible share of an
-        // iteration; for long iterations the KD tree over the padded capacity costs more
-        // than it saves (measured: 64-scene batch +6%, 37 ms water-pool iterations -2%).
+        // iteration (the photon order over the padded capacity costs a little more).
         if (d.stats[9] > kReplayMaxIterationMs && cfg().graph_replay != 2) d.async_pcap = -1;
         else {
             r = async_setup(sc);
@@ -1332,7 +1309,7 @@ int render_iterations(HostScene& sc, int iterations) {
 // Several resident scenes (one context each) rendered as one launch set per iteration:
 // one persistent light pass over every scene's light paths and one persistent camera
 // pass over every scene's pixels (scene index found per work item), and per scene its
-// light-path order, KD build, query order and gather on a branch of its own; the whole
+// light-path order, photon order, query order and gather on a branch of its own; the whole
 // iteration is captured as one CUDA graph, updated in place and replayed per iteration.
 // Capacities are each scene's asynchronous ones (async_setup: fixed from a first
 // iteration with host round trips), so the graph holds no host round trip, whatever
@@ -2209,9 +2186,14 @@ int rc_proposal_state(long long n, float* prop4, float* contrib) {
 }
 
 int rc_camera_queries(int iteration, float* out, long long cap, long long* count) {
+    return rc_camera_queries_shape(0, iteration, out, cap, count);
+}
+
+int rc_camera_queries_shape(int shape, int iteration, float* out, long long cap, long long* count) {
     int r = prepare();
     if (r) return r;
     if (iteration < 0 || (cap > 0 && !out)) { ctx().err = "bad query output"; return RC_E_INVALID; }
+    if (shape < 0 || shape >= pass_variants()) { ctx().err = "camera pass shape out of range"; return RC_E_INVALID; }
     HostScene& sc = *ctx().scene;
     DeviceState& d = ctx().dev;
     cudaStream_t s = d.stream;
@@ -2225,7 +2207,7 @@ int rc_camera_queries(int iteration, float* out, long long cap, long long* count
         RC_CUDA(d.counters.reserve(10));
         RC_CUDA(cudaMemsetAsync(d.counters.p + 1, 0, sizeof(unsigned long long), s));
         QueryBuf qb{d.q0.p, d.q1.p, d.q2.p, d.q3.p, d.q4.p, (long long)d.q0.n, d.counters.p + 1};
-        r = camera_pass(p, qb, s, 0);
+        r = camera_pass(p, qb, s, shape);
         if (r) return r;
         RC_CUDA(cudaGetLastError());
         RC_CUDA(cudaMemcpyAsync(&nq, d.counters.p + 1, sizeof(nq), cudaMemcpyDeviceToHost, s));
@@ -2391,42 +2373,25 @@ int rc_trace_rays_shape(int n, const float* origins, const float* directions, fl
     return check_errors();
 }
 
-static int kd_build_host(int n, const float* positions, DevBuf<float4>& pos, DevBuf<uint2>& nodes, DevBuf<float>& x,
-                         DevBuf<float>& y, DevBuf<float>& z, DevBuf<uint32_t>& id, DevBuf<unsigned char>& scratch,
-                         DevBuf<float4>& boxes, DevBuf<float4>& t0, KdTree& tree, cudaStream_t s) {
-    DevBuf<int> err;
-    RC_CUDA(err.reserve(1));
-    RC_CUDA(cudaMemsetAsync(err.p, 0, sizeof(int), s));
+// n host positions as the device's float4 records.
+static int upload_positions(int n, const float* positions, DevBuf<float4>& pos, cudaStream_t s) {
     std::vector<float4> p4((size_t)n);
     for (int i = 0; i < n; ++i) p4[i] = make_float4(positions[3 * i], positions[3 * i + 1], positions[3 * i + 2], 0.0f);
     RC_CUDA(pos.reserve(std::max(n, 1)));
     if (n) RC_CUDA(cudaMemcpyAsync(pos.p, p4.data(), 16 * (size_t)n, cudaMemcpyHostToDevice, s));
-    long long nn = kd_node_array_len(n);
-    RC_CUDA(nodes.reserve(std::max<long long>(nn, 2)));
-    RC_CUDA(x.reserve(std::max(n, 1))); RC_CUDA(y.reserve(std::max(n, 1)));
-    RC_CUDA(z.reserve(std::max(n, 1))); RC_CUDA(id.reserve(std::max(n, 1)));
-    RC_CUDA(scratch.reserve(kd_scratch_bytes(n)));
-    tree.nodes = nodes.p; tree.x = x.p; tree.y = y.p; tree.z = z.p; tree.id = id.p;
-    if (kd_build(pos.p, n, tree, scratch.p, scratch.n, s, nullptr, err.p)) { ctx().err = "KD scratch"; return RC_E_CAPACITY; }
-    RC_CUDA(cudaGetLastError());
-    tree.box_levels = kd_box_levels(n);
-    if (tree.box_levels > 0) {
-        RC_CUDA(boxes.reserve((size_t)2 << tree.box_levels));
-        tree.box_lo = boxes.p;
-        tree.box_hi = boxes.p + ((size_t)1 << tree.box_levels);
-        launch_kd_boxes(tree, s, nullptr);
-        RC_CUDA(cudaGetLastError());
-        RC_CUDA(t0.reserve(std::max(n, 1)));
-        launch_tree_records(PhotonBuf{pos.p, nullptr, nullptr, nullptr, n, nullptr}, tree, TreePhotons{t0.p, nullptr, nullptr},
-                            s);
-        RC_CUDA(cudaGetLastError());
-    }
-    int h = 0;
-    RC_CUDA(cudaMemcpyAsync(&h, err.p, sizeof(int), cudaMemcpyDeviceToHost, s));
-    RC_CUDA(cudaStreamSynchronize(s));
-    err.release();
-    if (h) { ctx().err = "KD-tree build found inconsistent counts"; return RC_E_INVALID; }
+    RC_CUDA(cudaStreamSynchronize(s));   // (p4 ends here)
     return RC_OK;
+}
+
+// Frame over the given points for queries of squared radius r2.
+static CurveFrame points_frame(int n, const float* p, float r2) {
+    float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+    for (int j = 0; j < n; ++j)
+        for (int k = 0; k < 3; ++k) {
+            lo[k] = std::min(lo[k], p[3 * (size_t)j + k]);
+            hi[k] = std::max(hi[k], p[3 * (size_t)j + k]);
+        }
+    return curve_frame(lo, hi, std::sqrt(std::max(r2, 0.0f)));
 }
 
 int rc_gather_variants(void) { return gather_variants(); }
@@ -2446,26 +2411,30 @@ int rc_gather_query(int variant, int n, const float* positions, int q, const flo
     if (variant < 0) variant = gather_default_variant();
     cudaStream_t s = nullptr;
     RC_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-    DevBuf<float4> pos, boxes, t0; DevBuf<uint2> nodes; DevBuf<float> x, y, z, qp; DevBuf<uint32_t> id, ord;
+    DevBuf<float4> pos, boxes, t0; DevBuf<float> qp; DevBuf<uint32_t> id, ord;
     DevBuf<unsigned char> scratch, osc; DevBuf<int> cnt, cur, out, err; DevBuf<long long> off;
-    KdTree tree;
-    int r = kd_build_host(n, positions, pos, nodes, x, y, z, id, scratch, boxes, t0, tree, s);
+    PhotonTree tree;
+    int r = upload_positions(n, positions, pos, s);
+    if (!r) r = [&]() -> int {
+        const size_t m = (size_t)2 << std::max(photon_chunk_level(n), 0);
+        RC_CUDA(id.reserve(std::max(n, 1))); RC_CUDA(t0.reserve(std::max(n, 1))); RC_CUDA(boxes.reserve(2 * m));
+        RC_CUDA(scratch.reserve(order_scratch_bytes(n)));
+        tree = PhotonTree{n, id.p, boxes.p, boxes.p + m};
+        launch_photon_order(PhotonBuf{pos.p, nullptr, nullptr, nullptr, n, nullptr}, n, nullptr,
+                            points_frame(n, positions, r2), scratch.p, tree, TreePhotons{t0.p, nullptr, nullptr}, nullptr, s);
+        RC_CUDA(cudaGetLastError());
+        return RC_OK;
+    }();
     if (!r && total) *total = 0;
     if (!r && q > 0) {
         r = [&]() -> int {
             RC_CUDA(qp.reserve(3 * (size_t)q)); RC_CUDA(cnt.reserve(q)); RC_CUDA(cur.reserve(q)); RC_CUDA(off.reserve(q));
             RC_CUDA(err.reserve(1)); RC_CUDA(ord.reserve(q));
-            RC_CUDA(osc.reserve(query_order_scratch_bytes(q)));
+            RC_CUDA(osc.reserve(order_scratch_bytes(q)));
             RC_CUDA(cudaMemcpyAsync(qp.p, queries, 12 * (size_t)q, cudaMemcpyHostToDevice, s));
             RC_CUDA(cudaMemsetAsync(cnt.p, 0, 4 * (size_t)q, s));
             RC_CUDA(cudaMemsetAsync(err.p, 0, sizeof(int), s));
-            float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-            for (int j = 0; j < q; ++j)
-                for (int k = 0; k < 3; ++k) {
-                    lo[k] = std::min(lo[k], queries[3 * j + k]);
-                    hi[k] = std::max(hi[k], queries[3 * j + k]);
-                }
-            launch_query_order(qp.p, 3, q, query_frame(lo, hi), osc.p, ord.p, nullptr, s);
+            launch_query_order(qp.p, 3, q, points_frame(q, queries, r2), osc.p, ord.p, nullptr, s);
             launch_gather_sets(tree, t0.p, qp.p, 3, ord.p, q, r2, cnt.p, nullptr, nullptr, nullptr, variant, nullptr,
                                err.p, s);
             RC_CUDA(cudaGetLastError());
@@ -2491,7 +2460,7 @@ int rc_gather_query(int variant, int n, const float* positions, int q, const flo
             return RC_OK;
         }();
     }
-    pos.release(); nodes.release(); x.release(); y.release(); z.release(); id.release(); scratch.release();
+    pos.release(); id.release(); scratch.release();
     cnt.release(); cur.release(); out.release(); off.release(); qp.release(); ord.release(); osc.release();
     boxes.release(); t0.release(); err.release();
     cudaStreamDestroy(s);
@@ -2508,9 +2477,25 @@ int rc_kd_build_nodes(int n, const float* positions, unsigned* nodes_out, long l
     cudaStream_t s = nullptr;
     RC_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
     DevBuf<float4> pos; DevBuf<uint2> nodes; DevBuf<float> x, y, z; DevBuf<uint32_t> id; DevBuf<unsigned char> scratch;
-    KdTree tree;
-    DevBuf<float4> boxes, t0;
-    int r = kd_build_host(n, positions, pos, nodes, x, y, z, id, scratch, boxes, t0, tree, s);
+    DevBuf<int> err;
+    int r = upload_positions(n, positions, pos, s);
+    if (!r) r = [&]() -> int {
+        const size_t m = (size_t)std::max(n, 1);
+        RC_CUDA(err.reserve(1));
+        RC_CUDA(cudaMemsetAsync(err.p, 0, sizeof(int), s));
+        RC_CUDA(nodes.reserve(std::max<long long>(kd_node_array_len(n), 2)));
+        RC_CUDA(x.reserve(m)); RC_CUDA(y.reserve(m)); RC_CUDA(z.reserve(m)); RC_CUDA(id.reserve(m));
+        RC_CUDA(scratch.reserve(kd_scratch_bytes(n)));
+        KdTree tree;
+        tree.nodes = nodes.p; tree.x = x.p; tree.y = y.p; tree.z = z.p; tree.id = id.p;
+        if (kd_build(pos.p, n, tree, scratch.p, scratch.n, s, nullptr, err.p)) { ctx().err = "KD scratch"; return RC_E_CAPACITY; }
+        RC_CUDA(cudaGetLastError());
+        int h = 0;
+        RC_CUDA(cudaMemcpyAsync(&h, err.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+        RC_CUDA(cudaStreamSynchronize(s));
+        if (h) { ctx().err = "KD-tree build found inconsistent counts"; return RC_E_INVALID; }
+        return RC_OK;
+    }();
     if (!r) {
         long long nn = kd_node_array_len(n);
         if (num_nodes) *num_nodes = nn;
@@ -2521,8 +2506,7 @@ int rc_kd_build_nodes(int n, const float* positions, unsigned* nodes_out, long l
             if (e != cudaSuccess) { ctx().err = cudaGetErrorString(e); r = RC_E_CUDA; }
         }
     }
-    pos.release(); nodes.release(); x.release(); y.release(); z.release(); id.release(); scratch.release();
-    boxes.release(); t0.release();
+    pos.release(); nodes.release(); x.release(); y.release(); z.release(); id.release(); scratch.release(); err.release();
     cudaStreamDestroy(s);
     return r;
 }

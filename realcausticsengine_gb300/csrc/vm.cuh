@@ -4,7 +4,7 @@
 // One progressive iteration (src/Vertex_Merging.cpp:196-366):
 //   light pass   - light sub-paths, photons stored at non-delta vertices reached by a
 //                  glossy event (Path_Vertex records)
-//   KD build     - photon KD-tree over the stored photons (kdtree.cu)
+//   photon order - the stored photons sorted in space, with a tree of boxes (photon_order.cu)
 //   camera pass  - one camera sub-path per pixel; every non-delta vertex becomes a
 //                  merge query
 //   gather       - photons within the merge radius of each query, MIS-weighted BSDF
@@ -14,7 +14,6 @@
 #include <cuda_runtime.h>
 #include "rc_device_types.h"
 #include "trace.cuh"
-#include "kdtree.cuh"
 
 namespace rc {
 
@@ -40,7 +39,7 @@ struct QueryBuf {
     unsigned long long* count;
 };
 
-// Photon records in KD-tree order (filled after the build by launch_tree_records):
+// Photon records in sorted order (filled by launch_photon_order):
 //   t0 = position.xyz | dVM   t1 = direction_world.xyz | throughput.r   t2 = throughput.gb
 struct TreePhotons {
     float4* t0;
@@ -109,8 +108,8 @@ int mlt_variants();
 // Every path keeps its samples and index: only the order of tracing changes.
 size_t light_order_scratch_bytes(long long n);
 void launch_light_order(const VMParams& p, void* scratch, uint32_t* order, cudaStream_t s);
-// Exclusive scan of m counters in place; large m in three passes over 8192-counter tiles
-// with tile_scratch (scan_scratch_words(m) words) for the tile totals.
+// Exclusive scan of m counters in place, in three passes over 8192-counter tiles with
+// tile_scratch (scan_scratch_words(m) words) for the tile totals.
 size_t scan_scratch_words(long long m);
 void launch_scan_counts(uint32_t* counts, long long m, uint32_t* tile_scratch, cudaStream_t s);
 // next_path: device counter for the persistent shapes; rays (optional): receives the number
@@ -135,8 +134,8 @@ void launch_debug_view(const VMParams& p, int mode, float ior, double* accum, cu
 // FP32 mean image (n floats) from the FP64 running sum.
 void launch_image_mean(const double* acc, float* out, long long n, double scale, cudaStream_t s);
 // Photon slots [*count, capacity) get position `pad` (chosen outside the scene by more
-// than any merge radius: a KD tree over the full capacity then answers the same radius
-// queries as one over the stored photons), and *flag = 1 when a count overflowed its
+// than any merge radius: radius queries over the full capacity then find what they find
+// over the stored photons), and *flag = 1 when a count overflowed its
 // capacity.
 void launch_pad_photons(float4* pos, const unsigned long long* count, long long capacity, float4 pad,
                         cudaStream_t s);
@@ -146,25 +145,31 @@ void launch_check_counts(const unsigned long long* photons, long long photon_cap
 // (the reference's form).  found: n records of scratch.
 void launch_trace_rays(const SceneView& s, int n, const float* o, const float* d, float tmin, HitRec* found,
                        float* out_full, unsigned* out_words, int* err, cudaStream_t st, int shape = 0);
-// Photon records in tree order (tp.t0/t1/t2 from ph.pos/dir/tp; only t0 when ph.dir is null).
-void launch_tree_records(PhotonBuf ph, const KdTree& tree, TreePhotons tp, cudaStream_t s);
-// Node bounding boxes used by the gather to prune exactly: the photons in tree order
-// are cut into 2^Lc chunks of at most 32 (Lc = kd_chunk_level(n), the shallowest level
-// whose nodes hold at most 31 photons: a chunk is such a node's range plus the median
-// photon that may follow it); the chunk boxes carry their first position and count in
-// .w, every node above has the union of its children's.  Levels [0, kd_box_levels(n)),
-// arrays of 2^kd_box_levels(n) float4 each, filled from the tree's x/y/z.
-int kd_chunk_level(long long n);
-int kd_box_levels(long long n);
-void launch_kd_boxes(const KdTree& tree, cudaStream_t s, int* launches);
-// Spatial order of queries (positions at qpos + stride*i): order[] receives the query
-// indices sorted by the 30-bit Morton code of their cell in a 1024^3 grid over the box
-// `frame` describes (query_frame(lo, hi); positions outside are clamped), by a stable
-// radix sort.  scratch: query_order_scratch_bytes(nq) bytes.
-struct QueryFrame { float lo[3], scale[3]; };
-QueryFrame query_frame(const float lo[3], const float hi[3]);
-size_t query_order_scratch_bytes(long long nq);
-void launch_query_order(const float* qpos, int stride, long long nq, const QueryFrame& frame, void* scratch,
+// Spatial order of the photons and queries (photon_order.cu): cells of a grid over a box,
+// 2^bits per axis, along the Hilbert curve.  radius: the merge radius, which sets how fine
+// the grid has to be.
+struct CurveFrame { float lo[3], scale[3]; int bits; };
+CurveFrame curve_frame(const float lo[3], const float hi[3], float radius);
+size_t order_scratch_bytes(long long n);   // scratch of either order over n points, any frame
+// The gather's photon structure.  id[p]: photon buffer index of sorted position p (n
+// entries); box_lo / box_hi: a box per node of the tree over the 2^photon_chunk_level(n)
+// chunks (heap order, 2^(level + 1) entries each).
+struct PhotonTree {
+    long long n = 0;
+    uint32_t* id = nullptr;
+    float4* box_lo = nullptr;
+    float4* box_hi = nullptr;
+};
+int photon_chunk_level(long long n);
+// Sorts the n photons of ph (positions outside the frame are clamped to its border cells),
+// fills tree.id and the boxes, and gathers the records into sorted order (tp.t0/t1/t2 from
+// ph.pos/dir/tp; only t0 when ph.dir is null).  count: device word with the number of
+// photons stored (at most n); the slots beyond hold pad positions and are sorted last.
+void launch_photon_order(const PhotonBuf& ph, long long n, const unsigned long long* count, const CurveFrame& frame,
+                         void* scratch, const PhotonTree& tree, TreePhotons tp, int* launches, cudaStream_t s);
+// order[] receives the query indices (positions at qpos + stride*i) in sorted order.  With
+// nq_dev the number of queries is read on the device (at most nq).
+void launch_query_order(const float* qpos, int stride, long long nq, const CurveFrame& frame, void* scratch,
                         uint32_t* order, int* launches, cudaStream_t s, const unsigned long long* nq_dev = nullptr);
 // The gather: one fused kernel over groups of ordered queries (gather.cu).  Photon sets
 // are the reference's; each accepted photon's merge (BSDF, MIS weight, throughput) is
@@ -173,17 +178,17 @@ void launch_query_order(const float* qpos, int stride, long long nq, const Query
 // photon-query pairs, photon tests (chunk photons x overlapping queries), chunks
 // tested, boxes tested.  With nq_dev the query count is read on the device (bounded by
 // num_queries, the capacity the grid is sized for) and a non-zero *skip makes the
-// launch a no-op.  Needs the boxes (launch_kd_boxes) and the tree-order records.
-void launch_gather(const VMParams& p, const KdTree& tree, TreePhotons tp, QueryBuf qb, const uint32_t* order,
+// launch a no-op.  Needs the boxes and the sorted records (launch_photon_order).
+void launch_gather(const VMParams& p, const PhotonTree& tree, TreePhotons tp, QueryBuf qb, const uint32_t* order,
                    long long num_queries, double* accum, unsigned long long* counters, cudaStream_t s, int variant,
                    const unsigned long long* nq_dev = nullptr, const int* skip = nullptr);
 // Parity hook: the same kernel with a sink that records each query's photon ids
 // (tree.id of the accepted positions).  Without offsets it adds each query's count into
 // counts[] (zeroed by the caller); with offsets it writes the ids at offsets[q] +
-// cursor[q]++ (cursor zeroed by the caller).  t0: tree-order positions
-// (launch_tree_records); queries at qpos + qstride*i in the order `order`.  *err is set
+// cursor[q]++ (cursor zeroed by the caller).  t0: sorted positions
+// (launch_photon_order); queries at qpos + qstride*i in the order `order`.  *err is set
 // if a traversal stack would overflow (cannot happen for n < 2^28).
-void launch_gather_sets(const KdTree& tree, const float4* t0, const float* qpos, int qstride, const uint32_t* order,
+void launch_gather_sets(const PhotonTree& tree, const float4* t0, const float* qpos, int qstride, const uint32_t* order,
                         long long nq, float r2, int* counts, const long long* offsets, int* cursor, int* idx,
                         int variant, unsigned long long* counters, int* err, cudaStream_t s);
 int gather_variants();

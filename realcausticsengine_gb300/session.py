@@ -141,12 +141,14 @@ class Renderer:
                                          int(shape)), "rc_trace_rays_shape")
         return out
 
-    def camera_queries(self, iteration: int) -> np.ndarray:
-        """Merge queries of one camera pass: (n, 4) float32 [position xyz, camera dVM]."""
+    def camera_queries(self, iteration: int, shape: int = 0) -> np.ndarray:
+        """Merge queries of one camera pass in launch shape `shape` (0-3 persistent, 4-6
+        staged): (n, 4) float32 [position xyz, camera dVM]."""
         n = C.c_longlong()
-        check(self.L.rc_camera_queries(int(iteration), None, 0, C.byref(n)), "rc_camera_queries")
+        check(self.L.rc_camera_queries_shape(shape, int(iteration), None, 0, C.byref(n)), "rc_camera_queries_shape")
         out = np.zeros((max(n.value, 1), 4), np.float32)
-        check(self.L.rc_camera_queries(int(iteration), out.ctypes.data, len(out), C.byref(n)), "rc_camera_queries")
+        check(self.L.rc_camera_queries_shape(shape, int(iteration), out.ctypes.data, len(out), C.byref(n)),
+              "rc_camera_queries_shape")
         return out[:n.value]
 
     def light_photons_shape(self, shape: int, iteration: int) -> np.ndarray:
