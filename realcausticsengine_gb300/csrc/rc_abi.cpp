@@ -1,6 +1,8 @@
 // C ABI of librealcaustics.so: the reference's init()/main() plus the additive rc_*
 // entry points, over the host scene (host_scene.cpp) and the sm_103a kernels.
 #include <cuda_runtime.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <atomic>
@@ -1826,6 +1828,19 @@ int write_exr(const char* path, const float* rgb, int w, int h) {
     return RC_OK;
 }
 
+// Backs the pages of [p, p + bytes) with memory, their contents untouched.  A copy from the
+// device into pages that nothing has written yet has the device's accesses fault them in,
+// page by page: 21 ms for a fresh 25 MB numpy array (1080p image) against 0.9 ms here and
+// 0.16 ms for the copy.  (Best effort: without it the copy still works.)
+void back_pages(void* p, size_t bytes) {
+#ifndef MADV_POPULATE_WRITE
+#define MADV_POPULATE_WRITE 23
+#endif
+    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
+    const uintptr_t a = (uintptr_t)p & ~(page - 1), b = ((uintptr_t)p + bytes + page - 1) & ~(page - 1);
+    (void)madvise((void*)a, b - a, MADV_POPULATE_WRITE);
+}
+
 int read_image(float* rgb, int w, int h) {
     if (!ctx().scene) { ctx().err = "no scene"; return RC_E_NO_SCENE; }
     if (!rgb || w != ctx().scene->camera.width || h != ctx().scene->camera.height) { ctx().err = "bad image buffer"; return RC_E_INVALID; }
@@ -1841,6 +1856,7 @@ int read_image(float* rgb, int w, int h) {
     RC_CUDA(d.image.reserve(n));
     launch_image_mean(d.accum.p, d.image.p, (long long)n, sc, d.stream);
     RC_CUDA(cudaGetLastError());
+    back_pages(rgb, n * sizeof(float));   // (while the mean runs)
     RC_CUDA(cudaMemcpyAsync(rgb, d.image.p, n * sizeof(float), cudaMemcpyDeviceToHost, d.stream));
     RC_CUDA(cudaStreamSynchronize(d.stream));
     return RC_OK;
