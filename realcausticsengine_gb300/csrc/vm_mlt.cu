@@ -78,11 +78,9 @@ __device__ __forceinline__ bool mlt_path_start(const VMParams& P, const float* u
     return true;
 }
 
-__device__ __forceinline__ bool mlt_path_bounce(const VMParams& P, const float* u, const PathRng& rr, int maxlen,
-                                                MltPath& t, PhotonRec* out) {
-    const F3 ro = t.o + t.d * kRayEps;
-    HitRec h;
-    if (!scene_hit(P.scene, ro, t.d, kRayEps, h, P.error + ERR_STACK)) return false;
+// The shading half of a segment, at hit h of the ray from ro.
+__device__ __forceinline__ bool mlt_path_shade(const VMParams& P, const float* u, const PathRng& rr, int maxlen,
+                                               MltPath& t, PhotonRec* out, const HitRec& h, F3 ro) {
     Isect is;
     fill_isect(P.scene, h, ro, t.d, is);
     if ((unsigned)is.material >= (unsigned)P.num_materials) { atomicOr(P.error + ERR_MATERIAL, 1); return false; }
@@ -120,6 +118,14 @@ __device__ __forceinline__ bool mlt_path_bounce(const VMParams& P, const float* 
     else t.dVM = (smp.cos_out / smp.fwd) * (1.0f + smp.rev * t.dVM);
     t.len++;
     return true;
+}
+
+__device__ __forceinline__ bool mlt_path_bounce(const VMParams& P, const float* u, const PathRng& rr, int maxlen,
+                                                MltPath& t, PhotonRec* out) {
+    const F3 ro = t.o + t.d * kRayEps;
+    HitRec h;
+    if (!scene_hit(P.scene, ro, t.d, kRayEps, h, P.error + ERR_STACK)) return false;
+    return mlt_path_shade(P, u, rr, maxlen, t, out, h, ro);
 }
 
 // The whole path; returns the number of photons.
@@ -176,66 +182,168 @@ __device__ __forceinline__ void mutate(const VMParams& P, uint64_t key, float m,
     }
 }
 
+// A proposal's sample vector, drawn as its path needs it: `done` Philox blocks have been
+// written, 4 coordinates each (a large step) or 2 (a mutation of `from`).  Most proposals
+// end after a few segments and are rejected; only an accepted one is completed.
+struct Proposal {
+    PathRng g;
+    int done;
+    bool large;
+    float scale;        // mutation: exp(-1/m)
+};
+constexpr int kLargeBlocks = (kMltDims + 3) / 4, kMutationBlocks = (kMltDims + 1) / 2;
+
+__device__ __forceinline__ void propose_large(const VMParams& P, long long pidx, uint32_t salt, Proposal& r) {
+    r.g.init(P.seed, (uint64_t)pidx, P.iteration ^ (salt << 20), STREAM_LIGHT);
+    r.done = 0;
+    r.large = true;
+}
+__device__ __forceinline__ void propose_mutation(const VMParams& P, uint64_t key, float m, Proposal& r) {
+    r.g.init(P.seed, key, P.iteration, STREAM_MLT);
+    r.done = 0;
+    r.large = false;
+    r.scale = powf(0.36787944117f, 1.0f / m);
+}
+// Coordinates [0, upto) of u at least (the same values as uniform_samples and mutate).
+__device__ __forceinline__ void propose_extend(Proposal& r, int upto, float* u, const float* from) {
+    upto = min(upto, kMltDims);
+    if (r.large) {
+        for (; 4 * r.done < upto; ++r.done) {
+            const U4 w = r.g.block(r.done);
+            const float v[4] = {u01(w.a), u01(w.b), u01(w.c), u01(w.d)};
+            for (int k = 0; k < 4 && 4 * r.done + k < kMltDims; ++k) u[4 * r.done + k] = v[k];
+        }
+    } else {
+        for (; 2 * r.done < upto; ++r.done) {
+            const U4 w = r.g.block(r.done);
+            const float e0 = u01(w.a), s0 = u01(w.b), e1 = u01(w.c), s1 = u01(w.d);
+            const int i0 = 2 * r.done, i1 = i0 + 1;
+            float a = from[i0];
+            a += s0 < 0.5f ? e0 * r.scale : -e0 * r.scale;
+            a -= floorf(a);
+            u[i0] = a;
+            if (i1 < kMltDims) {
+                float b = from[i1];
+                b += s1 < 0.5f ? e1 * r.scale : -e1 * r.scale;
+                b -= floorf(b);
+                u[i1] = b;
+            }
+        }
+    }
+}
+// The coordinates an emission reads.
+__device__ __forceinline__ int emission_dims(const VMParams& P) { return P.proposal_table ? kMltDims : 5; }
+
+// The chains run one per thread: few warps (65,536 chains are 13 per SM), long dependent
+// searches.  A warp's lanes search in phases (search_run); once kServeLanes lanes' searches
+// have ended they shade and go on to their next segment while the others' searches wait,
+// so that no lane waits for the longest search of its warp, and once enough lanes'
+// proposals have ended (or no lane searches) those settle their steps together (accept
+// or reject, the adaptive mutation size) and start their next proposals.  Each chain takes
+// the same steps with the same random numbers in the same order as a step-at-a-time loop.
+// Issue-bound by the searches (2,000 gems, 65,536 chains, 4.2M steps; light pass by lanes
+// served: 4, 8, 12, 16, 20 -> 57.9, 55.8, 53.2, 52.5, 53.4 ms; by lanes settled, 8 served:
+// 4, 8, 16 -> 54.1, 55.8, 60.4 ms); 76.8 ms with a segment per lane and round and whole
+// sample vectors.  Hybrid (water pool, 518,400 paths): 16 served, 16 settled 2.25 ms,
+// 16 / 8 2.42, 8 / 8 2.69; 2.83 ms step at a time.
+constexpr int kServeLanes = 16, kSettlePss = 8, kSettleHybrid = 16;
+
+// Hybrid chain (the reference's scheme): every index first traces a large step; if it
+// stores no photon, the last state is mutated and the mutation traced.
 __global__ void __launch_bounds__(128) k_mlt_hybrid(const VMParams P, PhotonBuf ph, int chains,
                                                     unsigned long long* __restrict__ stats) {
     const int chain = blockIdx.x * blockDim.x + threadIdx.x;
-    if (chain >= chains) return;
     const long long N = P.num_light_paths;
     const long long per = (N + chains - 1) / chains;
     const long long p0 = (long long)chain * per;
     const long long p1 = p0 + per < N ? p0 + per : N;
-    if (p0 >= p1) return;
+    // lanes without a chain stay in the loop (its votes take the whole warp), idle
+    bool alive = chain < chains && p0 < p1;
     const int maxlen = P.max_path_length < kMltMaxLen ? P.max_path_length : kMltMaxLen;
-    float cur[kMltDims], prop[kMltDims];
+    float su[2][kMltDims];
     PhotonRec buf[kPhotonBuf];
-    // MLT_Sampler constructor: uniform initial state
-    uniform_samples(P, p0, 1u, cur);
+    int ci = 0;
     float m = 1.0f;
     int accepted = 1, mutated = 0;
     unsigned long long visible_large = 0;
-    for (long long p = p0; p < p1; ++p) {
-        // large step (Init_Uniform)
-        uniform_samples(P, p, 0u, prop);
-        PathRng rr;
-        rr.init(P.seed, (uint64_t)p * 2u, P.iteration, STREAM_MLT + 1u);
-        int n = trace_light_samples(P, prop, rr, maxlen, buf);
-        if (n > 0) {
-            ++visible_large;
-            store_photons(ph, buf, n, 1.0f, (uint32_t)p);
-            for (int k = 0; k < kMltDims; ++k) cur[k] = prop[k];
-            continue;
-        }
-        // Reject the large step, Mutate from the last state, trace the mutation
-        for (int k = 0; k < kMltDims; ++k) prop[k] = cur[k];
-        mutate(P, (uint64_t)p, m, prop);
-        ++mutated;
-        rr.init(P.seed, (uint64_t)p * 2u + 1u, P.iteration, STREAM_MLT + 1u);
-        n = trace_light_samples(P, prop, rr, maxlen, buf);
-        if (n > 0) {
-            ++accepted;
-            store_photons(ph, buf, n, 1.0f, (uint32_t)p);
-            for (int k = 0; k < kMltDims; ++k) cur[k] = prop[k];
-        }
-        const float R = (float)accepted / (float)mutated;
-        m += (R - 0.234f) / (float)mutated;
+    long long p = p0;
+    Proposal prop;
+    PathRng rr;
+    MltPath path;
+    path.n = 0;
+    SearchStack st;
+    Search q;
+    q.w0 = kSearchIdle;
+    bool ended = false;             // the proposal's path has ended, its step is not settled
+    bool first = true;              // nothing proposed yet
+    if (alive) {
+        // MLT_Sampler constructor: uniform initial state
+        uniform_samples(P, p0, 1u, su[0]);
+        ended = true;
     }
-    atomicAdd(&stats[0], visible_large);
-    atomicAdd(&stats[1], (unsigned long long)(p1 - p0));
+    while (__any_sync(0xffffffffu, alive)) {
+        const unsigned waiting = __ballot_sync(0xffffffffu, ended);
+        const unsigned searching = __ballot_sync(0xffffffffu, q.w0 != kSearchIdle);
+        if (ended && (__popc(waiting) >= kSettleHybrid || !searching)) {
+            bool mutate_next = false;
+            if (!first) {
+                const int n = path.n;
+                if (n > 0) {
+                    store_photons(ph, buf, n, 1.0f, (uint32_t)p);
+                    propose_extend(prop, kMltDims, su[ci ^ 1], su[ci]);
+                    ci ^= 1;
+                }
+                if (prop.large) {
+                    if (n > 0) { ++visible_large; ++p; }
+                    else mutate_next = true;
+                } else {
+                    if (n > 0) ++accepted;
+                    const float R = (float)accepted / (float)mutated;
+                    m += (R - 0.234f) / (float)mutated;
+                    ++p;
+                }
+            }
+            first = false;
+            if (p >= p1) {
+                alive = ended = false;
+                atomicAdd(&stats[0], visible_large);
+                atomicAdd(&stats[1], (unsigned long long)(p1 - p0));
+            } else {
+                if (mutate_next) {
+                    propose_mutation(P, (uint64_t)p, m, prop);
+                    ++mutated;
+                    rr.init(P.seed, (uint64_t)p * 2u + 1u, P.iteration, STREAM_MLT + 1u);
+                } else {
+                    propose_large(P, p, 0u, prop);
+                    rr.init(P.seed, (uint64_t)p * 2u, P.iteration, STREAM_MLT + 1u);
+                }
+                propose_extend(prop, emission_dims(P), su[ci ^ 1], su[ci]);
+                path.n = 0;
+                if (mlt_path_start(P, su[ci ^ 1], path)) {
+                    ended = false;
+                    search_begin(q, st, path.o + path.d * kRayEps, path.d);
+                }
+            }
+        }
+        __syncwarp();
+        const int n = __popc(__ballot_sync(0xffffffffu, q.w0 != kSearchIdle));
+        search_run(P.scene, q, st, path.d, kRayEps, n > kServeLanes ? n - kServeLanes : max(n - 1, 0),
+                   P.error + ERR_STACK);
+        if (alive && !ended && q.w0 == kSearchIdle) {
+            bool more = q.out.slot >= 0;
+            if (more) {
+                propose_extend(prop, 8 + 3 * path.len, su[ci ^ 1], su[ci]);
+                more = mlt_path_shade(P, su[ci ^ 1], rr, maxlen, path, buf, q.out, q.origin());
+            }
+            if (more) search_begin(q, st, path.o + path.d * kRayEps, path.d);
+            else ended = true;
+        }
+        __syncwarp();
+    }
 }
 
-// PSSMLT, one chain per thread, advanced one path segment per loop iteration: lanes
-// whose proposal's path has ended wait until kSettleLanes lanes of the warp (or all
-// that still have steps) have, then settle their steps together (accept or reject,
-// dwell, the adaptive mutation size) and start their chains' next proposals, so that
-// the lanes of a warp neither wait for the warp's longest path at every step nor draw
-// their proposals' random numbers (dozens of Philox blocks) a few lanes at a time.
-// Each chain takes the same steps with the same random numbers in the same order as a
-// step-at-a-time loop: burn-in large steps t = 0 .. (first visible, at most 256) from
-// the chain's first path index, then one step per further path index.
-// (gem cluster, 65,536 chains, 32M steps: 1, 4, 8, 16, 24 lanes -> 680, 681, 679, 700,
-// 779 ms per iteration)
-constexpr int kSettleLanes = 8;
-
+// PSSMLT chain: burn-in large steps t = 0 .. (first visible, at most 256) from the chain's
+// first path index, then one step per further path index.
 __global__ void __launch_bounds__(128) k_mlt_pss(const VMParams P, PhotonBuf ph, int chains, float p_large,
                                                  unsigned long long* __restrict__ stats) {
     const int chain = blockIdx.x * blockDim.x + threadIdx.x;
@@ -243,7 +351,6 @@ __global__ void __launch_bounds__(128) k_mlt_pss(const VMParams P, PhotonBuf ph,
     const long long per = (N + chains - 1) / chains;
     const long long p0 = (long long)chain * per;
     const long long p1 = p0 + per < N ? p0 + per : N;
-    // lanes without a chain stay in the loop (its votes take the whole warp), idle
     bool alive = chain < chains && p0 < p1;
     const int maxlen = P.max_path_length < kMltMaxLen ? P.max_path_length : kMltMaxLen;
     // the current state and the proposal: sample vectors and photon lists, swapped on
@@ -259,72 +366,92 @@ __global__ void __launch_bounds__(128) k_mlt_pss(const VMParams P, PhotonBuf ph,
     int t = 0;                       // burn-in step (t < 256), then main steps
     bool burn_in = true;
     long long p = p0 + 1;
-    bool is_large = true;
+    Proposal prop;
     PathRng rr;
     MltPath path;
     path.n = 0;
-    bool tracing = false;
-    if (alive) {
-        // first proposal: burn-in step 0
-        uniform_samples(P, p0, 16u, su[ci ^ 1]);
-        rr.init(P.seed, (uint64_t)p0 << 9, P.iteration, STREAM_MLT + 2u);
-        tracing = mlt_path_start(P, su[ci ^ 1], path);
-        if (!tracing) path.n = 0;
-    }
+    SearchStack st;
+    Search q;
+    q.w0 = kSearchIdle;
+    bool ended = alive;
+    bool first = true;
     while (__any_sync(0xffffffffu, alive)) {
-        if (alive && tracing) tracing = mlt_path_bounce(P, su[ci ^ 1], rr, maxlen, path, sph[ci ^ 1]);
-        const unsigned waiting = __ballot_sync(0xffffffffu, alive && !tracing);
-        const unsigned live = __ballot_sync(0xffffffffu, alive);
-        if (!waiting || (__popc(waiting) < kSettleLanes && waiting != live)) continue;
-        if (!(alive && !tracing)) continue;
-        // the proposal's path has ended: settle its step
-        const int n = path.n;
-        if (burn_in) {
-            ++large;
-            if (n > 0) { ++large_visible; ci ^= 1; cur_n = n; burn_in = false; }
-            else if (++t == 256) { ci ^= 1; cur_n = 0; burn_in = false; }   // go on from the last state tried
-        } else {
-            if (is_large) { ++large; if (n > 0) ++large_visible; }
-            if (n > 0) {
-                if (cur_n > 0) store_photons(ph, sph[ci], cur_n, dwell, (uint32_t)p);
-                ci ^= 1;
-                cur_n = n;
-                dwell = 1.0f;
-                if (!is_large) ++accepted;
-            } else {
-                dwell += 1.0f;
+        const unsigned waiting = __ballot_sync(0xffffffffu, ended);
+        const unsigned searching = __ballot_sync(0xffffffffu, q.w0 != kSearchIdle);
+        if (ended && (__popc(waiting) >= kSettlePss || !searching)) {
+            // the proposal's path has ended: settle its step
+            const int n = path.n;
+            if (!first) {
+                bool take = n > 0;
+                if (burn_in) {
+                    ++large;
+                    if (n > 0) { ++large_visible; burn_in = false; }
+                    else if (++t == 256) { take = true; burn_in = false; }   // go on from the last state tried
+                } else {
+                    if (prop.large) { ++large; if (n > 0) ++large_visible; }
+                    if (n > 0) {
+                        if (cur_n > 0) store_photons(ph, sph[ci], cur_n, dwell, (uint32_t)p);
+                        dwell = 1.0f;
+                        if (!prop.large) ++accepted;
+                    } else {
+                        dwell += 1.0f;
+                    }
+                    if (!prop.large && mutated > 0) {
+                        const float R = (float)accepted / (float)mutated;
+                        m += (R - 0.234f) / (float)mutated;
+                    }
+                    ++p;
+                }
+                if (take) {
+                    propose_extend(prop, kMltDims, su[ci ^ 1], su[ci]);
+                    ci ^= 1;
+                    cur_n = n;
+                }
             }
-            if (!is_large && mutated > 0) {
-                const float R = (float)accepted / (float)mutated;
-                m += (R - 0.234f) / (float)mutated;
-            }
-            ++p;
-        }
-        // the next proposal
-        if (burn_in) {
-            uniform_samples(P, p0, 16u + (uint32_t)t, su[ci ^ 1]);
-            rr.init(P.seed, ((uint64_t)p0 << 9) | (uint64_t)t, P.iteration, STREAM_MLT + 2u);
-        } else {
-            if (p >= p1) {
-                alive = false;
+            first = false;
+            // the next proposal
+            if (burn_in) {
+                propose_large(P, p0, 16u + (uint32_t)t, prop);
+                rr.init(P.seed, ((uint64_t)p0 << 9) | (uint64_t)t, P.iteration, STREAM_MLT + 2u);
+            } else if (p >= p1) {
+                alive = ended = false;
                 if (cur_n > 0) store_photons(ph, sph[ci], cur_n, dwell, (uint32_t)p0);
                 atomicAdd(&stats[0], large_visible);
                 atomicAdd(&stats[1], large);
-                continue;
+            } else {
+                PathRng g;
+                g.init(P.seed, (uint64_t)p, P.iteration, STREAM_MLT + 3u);
+                if (u01(g.block(0).a) < p_large) {
+                    propose_large(P, p, 0u, prop);
+                } else {
+                    propose_mutation(P, (uint64_t)p, m, prop);
+                    ++mutated;
+                }
+                rr.init(P.seed, (uint64_t)p * 2u, P.iteration, STREAM_MLT + 1u);
             }
-            PathRng g;
-            g.init(P.seed, (uint64_t)p, P.iteration, STREAM_MLT + 3u);
-            is_large = u01(g.block(0).a) < p_large;
-            if (is_large) uniform_samples(P, p, 0u, su[ci ^ 1]);
-            else {
-                for (int k = 0; k < kMltDims; ++k) su[ci ^ 1][k] = su[ci][k];
-                mutate(P, (uint64_t)p, m, su[ci ^ 1]);
-                ++mutated;
+            if (alive) {
+                propose_extend(prop, emission_dims(P), su[ci ^ 1], su[ci]);
+                path.n = 0;
+                if (mlt_path_start(P, su[ci ^ 1], path)) {
+                    ended = false;
+                    search_begin(q, st, path.o + path.d * kRayEps, path.d);
+                }
             }
-            rr.init(P.seed, (uint64_t)p * 2u, P.iteration, STREAM_MLT + 1u);
         }
-        tracing = mlt_path_start(P, su[ci ^ 1], path);
-        if (!tracing) path.n = 0;
+        __syncwarp();
+        const int n = __popc(__ballot_sync(0xffffffffu, q.w0 != kSearchIdle));
+        search_run(P.scene, q, st, path.d, kRayEps, n > kServeLanes ? n - kServeLanes : max(n - 1, 0),
+                   P.error + ERR_STACK);
+        if (alive && !ended && q.w0 == kSearchIdle) {
+            bool more = q.out.slot >= 0;
+            if (more) {
+                propose_extend(prop, 8 + 3 * path.len, su[ci ^ 1], su[ci]);
+                more = mlt_path_shade(P, su[ci ^ 1], rr, maxlen, path, sph[ci ^ 1], q.out, q.origin());
+            }
+            if (more) search_begin(q, st, path.o + path.d * kRayEps, path.d);
+            else ended = true;
+        }
+        __syncwarp();
     }
 }
 
