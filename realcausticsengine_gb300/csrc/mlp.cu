@@ -20,49 +20,30 @@ constexpr uint32_t kWait = 1u << 22;
 // sin/cos(2^k pi c) for k = 0..11: sincospi at k = 0, then the double-angle identities
 // sin 2a = 2 sin a cos a, cos 2a = 1 - 2 sin^2 a (rounding error doubles per step:
 // below 3e-4 at k = 11, under the BF16 rounding of the network input).
-__device__ __forceinline__ void encode(float px, float py, float pz, float* x) {
-    const float c[3] = {px, py, pz};
+constexpr int kMlpCoord = 1 + 2 * kMlpFreqs;   // inputs per coordinate
+__device__ __forceinline__ void encode_coord(float c, float* x) {
+    float sn, cs;
+    sincospif(c, &sn, &cs);
+    x[0] = c;
 #pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        float sn, cs;
-        sincospif(c[i], &sn, &cs);
-        x[25 * i] = c[i];
-#pragma unroll
-        for (int k = 0; k < kMlpFreqs; ++k) {
-            x[25 * i + 1 + 2 * k] = sn;
-            x[25 * i + 2 + 2 * k] = cs;
-            const float s2 = 2.0f * sn * cs;
-            cs = 1.0f - 2.0f * sn * sn;
-            sn = s2;
-        }
+    for (int k = 0; k < kMlpFreqs; ++k) {
+        x[1 + 2 * k] = sn;
+        x[2 + 2 * k] = cs;
+        const float s2 = 2.0f * sn * cs;
+        cs = 1.0f - 2.0f * sn * sn;
+        sn = s2;
     }
+}
+__device__ __forceinline__ void encode(float px, float py, float pz, float* x) {
+    encode_coord(px, x);
+    encode_coord(py, x + kMlpCoord);
+    encode_coord(pz, x + 2 * kMlpCoord);
 #pragma unroll
-    for (int o = 3 * (1 + 2 * kMlpFreqs); o < kMlpIn; ++o) x[o] = 0.0f;
+    for (int o = 3 * kMlpCoord; o < kMlpIn; ++o) x[o] = 0.0f;
 }
 
 __device__ __forceinline__ float softplus(float v) { return v > 20.0f ? v : log1pf(expf(v)); }
 __device__ __forceinline__ float sigmoid(float v) { return 1.0f / (1.0f + expf(-v)); }
-
-// Mixture parameters from the 80 network outputs.
-struct Lobes {
-    float pi[kMlpLobes], mx[kMlpLobes], my[kMlpLobes], mz[kMlpLobes], kappa[kMlpLobes], rlen[kMlpLobes];
-};
-
-__device__ __forceinline__ void lobes_from(const float* o, Lobes& L) {
-    float mxl = -INFINITY;
-    for (int k = 0; k < kMlpLobes; ++k) mxl = fmaxf(mxl, o[5 * k]);
-    float sum = 0.0f;
-    for (int k = 0; k < kMlpLobes; ++k) { L.pi[k] = expf(o[5 * k] - mxl); sum += L.pi[k]; }
-    for (int k = 0; k < kMlpLobes; ++k) {
-        L.pi[k] /= sum;
-        float x = o[5 * k + 1], y = o[5 * k + 2], z = o[5 * k + 3];
-        float len = sqrtf(x * x + y * y + z * z);
-        len = fmaxf(len, 1e-6f);
-        L.rlen[k] = len;
-        L.mx[k] = x / len; L.my[k] = y / len; L.mz[k] = z / len;
-        L.kappa[k] = fminf(kKappaMin + softplus(o[5 * k + 4]), kKappaMax);
-    }
-}
 
 __device__ __forceinline__ float vmf_pdf(float kappa, float cosang) {
     return kappa / (2.0f * 3.14159265f * (1.0f - expf(-2.0f * kappa))) * expf(kappa * (cosang - 1.0f));
@@ -301,42 +282,9 @@ __global__ void k_norm_weights(float4* dir4, int n, const float* wsum) {
     if (mean > 0.0f) dir4[i].w /= mean;
 }
 
-// ----------------------------------------------------------------------------- loss gradient
-// Per row: L = -w log q(dir) with q = a p_light + (1 - a) sum_k pi_k vMF_k (w = dir.w,
-// the light's own density at dir = pl).  g = dL/d(outputs) * inv_n; returns L * inv_n.
-__device__ float loss_grad_row(const float* o, float4 d, float pl, float inv_n, float* g) {
-    Lobes L;
-    lobes_from(o, L);
-    const float w = d.w;
-    float s[kMlpLobes], ca[kMlpLobes];
-    float S = 0.0f;
-#pragma unroll
-    for (int k = 0; k < kMlpLobes; ++k) {
-        ca[k] = L.mx[k] * d.x + L.my[k] * d.y + L.mz[k] * d.z;
-        s[k] = L.pi[k] * vmf_pdf(L.kappa[k], ca[k]);
-        S += s[k];
-    }
-    const float q = fmaxf(kMlpDefensive * pl + (1.0f - kMlpDefensive) * S, 1e-20f);
-    const float c = -(1.0f - kMlpDefensive) * w * inv_n / q;
-#pragma unroll
-    for (int k = 0; k < kMlpLobes; ++k) {
-        g[5 * k] = c * (s[k] - L.pi[k] * S);
-        const float kap = L.kappa[k];
-        const float gm = c * s[k] * kap / L.rlen[k];
-        g[5 * k + 1] = gm * (d.x - ca[k] * L.mx[k]);
-        g[5 * k + 2] = gm * (d.y - ca[k] * L.my[k]);
-        g[5 * k + 3] = gm * (d.z - ca[k] * L.mz[k]);
-        const float e2 = expf(-2.0f * kap);
-        const float dlog = 1.0f / kap - 2.0f * e2 / (1.0f - e2) + (ca[k] - 1.0f);
-        const float dk = (kap >= kKappaMax) ? 0.0f : sigmoid(o[5 * k + 4]);
-        g[5 * k + 4] = c * s[k] * dlog * dk;
-    }
-    return -w * logf(q) * inv_n;
-}
-
 // ----------------------------------------------------------------------------- fused training step
-// One CTA of 128 threads takes 128-row tiles of the batch (thread = row) and runs, per
-// tile, the forward pass, the loss gradient and the backward pass on the tensor cores:
+// One CTA takes 128-row tiles of the batch and runs, per tile, the forward pass, the loss
+// gradient and the backward pass on the tensor cores:
 //   dW_l += dY_l^T . In_l        (M = 128 (out rows, zero-padded), N = in,  K = 128 rows)
 //   db_l += dY_l^T . 1           (N = 16 columns of ones)
 //   dX_l  = dY_l . W_l           (M = 128 rows, N = in, K = out), dY_{l-1} = dX_l * relu'(In_l)
@@ -344,6 +292,16 @@ __device__ float loss_grad_row(const float* o, float4 d, float pl, float inv_n, 
 // written once per CTA as a partial sum; k_reduce_adam adds the partials.
 // Operands with the batch rows as the reduction dimension (In_l^T, dY_l^T) are written
 // transposed by the epilogues: element (feature i, row r) at kmajor_offset(i, r, 128).
+//
+// A step of 16,384 rows gives each CTA one tile, so its time is one chain of latencies.
+// Four groups of four warps share it: all groups see the tile's 128 rows (TMEM lanes), each
+// takes a quarter of every epilogue's columns (a coordinate of the encoding, 16 features
+// of a hidden layer, 4 lobes of the output).  The weights come in as one 62 KB image, kept in
+// the shared-memory layout beside them.  With 128 threads, a thread per row, and the
+// weights laid out per CTA element by element, the step took 107 us (the layout 27, the
+// forward layers 18, the loss 12, the backward layers 20, the partial sums' scattered
+// stores 11) and its reduction 12.6; now 27 and 6.7 (GB300, 16,384 rows).
+constexpr int kTrainThreads = 512;
 struct SmemTrain {
     static constexpr int wf0 = 0;                       // forward weights (out x in), K-major over in
     static constexpr int wf1 = wf0 + 64 * 80 * 2;
@@ -352,7 +310,8 @@ struct SmemTrain {
     static constexpr int wt1 = wf3 + 80 * 64 * 2;       // W_l^T (in x out), K-major over out
     static constexpr int wt2 = wt1 + 64 * 64 * 2;
     static constexpr int wt3 = wt2 + 64 * 64 * 2;
-    static constexpr int act = wt3 + 64 * 80 * 2;       // 128 x 80 activations (forward A operand)
+    static constexpr int image = wt3 + 64 * 80 * 2;     // (the bytes before: MlpParams::image)
+    static constexpr int act = image;                   // 128 x 80 activations (forward A operand)
     static constexpr int xt = act + 128 * 80 * 2;       // X^T 80 x 128
     static constexpr int ht0 = xt + 80 * 128 * 2;       // H_l^T 64 x 128
     static constexpr int ht1 = ht0 + 64 * 128 * 2;
@@ -361,21 +320,28 @@ struct SmemTrain {
     static constexpr int dyt = dy + 128 * 80 * 2;       // dY^T 128 x 128, rows >= out zero
     static constexpr int ones = dyt + 128 * 128 * 2;    // 16 x 128 ones
     static constexpr int bias = ones + 16 * 128 * 2;    // 272 floats
-    static constexpr int total = bias + 272 * 4;
+    static constexpr int swap = bias + 272 * 4;         // 3 x 4 groups x 128 rows: the loss's sums over groups
+    static constexpr int total = swap + 3 * 4 * 128 * 4;
 };
 static_assert(SmemTrain::total <= 227 * 1024, "training step shared memory");
+__host__ __device__ constexpr int image_wf(int l) {
+    return l == 0 ? SmemTrain::wf0 : l == 1 ? SmemTrain::wf1 : l == 2 ? SmemTrain::wf2 : SmemTrain::wf3;
+}
+__host__ __device__ constexpr int image_wt(int l) {
+    return l == 1 ? SmemTrain::wt1 : l == 2 ? SmemTrain::wt2 : SmemTrain::wt3;
+}
+// Weight (o, c) of layer l into the image.
+__device__ __forceinline__ void image_put(unsigned char* image, int l, int o, int c, __nv_bfloat16 w) {
+    const int in = mlp_in_dim(l), out = mlp_out_dim(l);
+    *reinterpret_cast<__nv_bfloat16*>(image + image_wf(l) + tc::kmajor_offset(o, c, in)) = w;
+    if (l > 0) *reinterpret_cast<__nv_bfloat16*>(image + image_wt(l) + tc::kmajor_offset(c, o, out)) = w;
+}
 
 // TMEM columns: dW_l accumulators (N = in_l) at 0, 80, 144, 208; db_l (N = 16) at
 // 272 + 16 l; per-tile products (N <= 80) at 336.
 __device__ __forceinline__ uint32_t col_w(int l) { return l == 0 ? 0u : 16u + 64u * (uint32_t)l; }
 __device__ __forceinline__ uint32_t col_b(int l) { return 272u + 16u * (uint32_t)l; }
 constexpr uint32_t kColT = 336;
-
-__device__ __forceinline__ void store_col_bf16(unsigned char* base, int r, const float* v, int cnt) {
-#pragma unroll
-    for (int i = 0; i < cnt; ++i)
-        *reinterpret_cast<__nv_bfloat16*>(base + tc::kmajor_offset(i, r, 128)) = __float2bfloat16_rn(v[i]);
-}
 
 // MMAs of one K extent without the completion commit (several products share one).
 __device__ __forceinline__ void gemm_issue_nc(uint32_t d_tmem, const void* a_smem, const void* b_smem, int K, int N,
@@ -407,160 +373,280 @@ __device__ __forceinline__ void publish_smem() {
     __syncthreads();
 }
 
-__global__ void __launch_bounds__(128, 1) k_mlp_train(const MlpParams P, const float4* __restrict__ pos,
-                                                       const float4* __restrict__ dir, int n, float inv_n,
-                                                       float* __restrict__ part, int part_stride,
-                                                       float* __restrict__ loss, int* err) {
+// `cnt` values of row r from column c0 (even): row-major K-major (the A operand, K columns)
+// and transposed (columns = the 128 rows).
+template <int cnt>
+__device__ __forceinline__ void store_both_bf16(unsigned char* rows, unsigned char* cols, int r, int c0, const float* v,
+                                                int K) {
+    if (cnt == 16) {
+#pragma unroll
+        for (int k = 0; k < 16; k += 8)
+            *reinterpret_cast<uint4*>(rows + tc::kmajor_offset(r, c0 + k, K)) =
+                make_uint4(pack_bf16x2(v[k], v[k + 1]), pack_bf16x2(v[k + 2], v[k + 3]), pack_bf16x2(v[k + 4], v[k + 5]),
+                           pack_bf16x2(v[k + 6], v[k + 7]));
+    } else {
+#pragma unroll
+        for (int k = 0; k < cnt; k += 2)
+            *reinterpret_cast<uint32_t*>(rows + tc::kmajor_offset(r, c0 + k, K)) = pack_bf16x2(v[k], v[k + 1]);
+    }
+#pragma unroll
+    for (int k = 0; k < cnt; ++k)
+        *reinterpret_cast<__nv_bfloat16*>(cols + tc::kmajor_offset(c0 + k, r, 128)) = __float2bfloat16_rn(v[k]);
+}
+
+// This CTA's state and position: row r of the tile, column group grp.
+struct TrainCta {
+    unsigned char* sm;
+    uint64_t* mbar;
+    uint32_t tm, lane_base, phase;
+    int r, grp;
+    int* err;
+    __device__ __forceinline__ unsigned char* in_t(int l) const {   // In_l^T
+        return sm + (l == 0 ? SmemTrain::xt : l == 1 ? SmemTrain::ht0 : l == 2 ? SmemTrain::ht1 : SmemTrain::ht2);
+    }
+};
+
+// Forward layer L: the thread's columns (16 of a hidden layer, stored as the next layer's
+// input; 20 of the output layer) in v.
+template <int L>
+__device__ __forceinline__ bool train_forward(TrainCta& t, float* v) {
+    constexpr int K = mlp_in_dim(L), N = mlp_out_dim(L);
+    unsigned char* act = t.sm + SmemTrain::act;
+    publish_smem();
+    if (threadIdx.x == 0) {
+        tc::fence_after_sync();
+        tc::gemm_issue(t.tm + kColT, act, t.sm + image_wf(L), K, N, false, t.mbar);
+    }
+    if (!cta_sync_wait(t.mbar, t.phase, t.err, 4)) return false;
+    const float* b = reinterpret_cast<const float*>(t.sm + SmemTrain::bias) + 64 * L + (N / 4) * t.grp;
+    const uint32_t col = t.tm + t.lane_base + kColT + (uint32_t)((N / 4) * t.grp);
+    tc::tmem_ld16(col, v);
+    if (L < 3) {
+#pragma unroll
+        for (int c = 0; c < 16; ++c) v[c] = fmaxf(v[c] + b[c], 0.0f);
+        store_both_bf16<16>(act, t.in_t(L + 1), t.r, 16 * t.grp, v, N);
+    } else {
+        tc::tmem_ld4(col + 16u, v + 16);
+#pragma unroll
+        for (int c = 0; c < 20; ++c) v[c] += b[c];
+    }
+    return true;
+}
+
+// Sum (or maximum) of x over the four groups of the thread's row, through swap slot `slot`.
+__device__ __forceinline__ float4 over_groups(const TrainCta& t, int slot, float x) {
+    float* s = reinterpret_cast<float*>(t.sm + SmemTrain::swap) + slot * 512;
+    s[t.grp * 128 + t.r] = x;
+    __syncthreads();
+    return make_float4(s[t.r], s[128 + t.r], s[256 + t.r], s[384 + t.r]);
+}
+
+// Per row: L = -w log q(dir) with q = a p_light + (1 - a) sum_k pi_k vMF_k (w = dir.w, the
+// light's own density at dir = pl), over the thread's four lobes (outputs o).
+// g = dL/d(outputs) * inv_n; returns L * inv_n.
+__device__ __forceinline__ float loss_grad(const TrainCta& t, const float* o, float4 d, float pl, float inv_n, float* g) {
+    const float4 m4 = over_groups(t, 0, fmaxf(fmaxf(o[0], o[5]), fmaxf(o[10], o[15])));
+    const float mx = fmaxf(fmaxf(m4.x, m4.y), fmaxf(m4.z, m4.w));
+    float pi[4], sum = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) { pi[k] = expf(o[5 * k] - mx); sum += pi[k]; }
+    const float4 s4 = over_groups(t, 1, sum);
+    sum = ((s4.x + s4.y) + s4.z) + s4.w;
+    float s[4], ca[4], kap[4], len[4], mu[4][3], S = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        pi[k] /= sum;
+        const float x = o[5 * k + 1], y = o[5 * k + 2], z = o[5 * k + 3];
+        len[k] = fmaxf(sqrtf(x * x + y * y + z * z), 1e-6f);
+        mu[k][0] = x / len[k]; mu[k][1] = y / len[k]; mu[k][2] = z / len[k];
+        kap[k] = fminf(kKappaMin + softplus(o[5 * k + 4]), kKappaMax);
+        ca[k] = mu[k][0] * d.x + mu[k][1] * d.y + mu[k][2] * d.z;
+        s[k] = pi[k] * vmf_pdf(kap[k], ca[k]);
+        S += s[k];
+    }
+    const float4 q4 = over_groups(t, 2, S);
+    S = ((q4.x + q4.y) + q4.z) + q4.w;
+    const float q = fmaxf(kMlpDefensive * pl + (1.0f - kMlpDefensive) * S, 1e-20f);
+    const float c = -(1.0f - kMlpDefensive) * d.w * inv_n / q;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        g[5 * k] = c * (s[k] - pi[k] * S);
+        const float gm = c * s[k] * kap[k] / len[k];
+        g[5 * k + 1] = gm * (d.x - ca[k] * mu[k][0]);
+        g[5 * k + 2] = gm * (d.y - ca[k] * mu[k][1]);
+        g[5 * k + 3] = gm * (d.z - ca[k] * mu[k][2]);
+        const float e2 = expf(-2.0f * kap[k]);
+        const float dlog = 1.0f / kap[k] - 2.0f * e2 / (1.0f - e2) + (ca[k] - 1.0f);
+        const float dk = (kap[k] >= kKappaMax) ? 0.0f : sigmoid(o[5 * k + 4]);
+        g[5 * k + 4] = c * s[k] * dlog * dk;
+    }
+    return -d.w * logf(q) * inv_n;
+}
+
+// Backward layer L: its gradients into TMEM, the previous layer's output gradients into Dy.
+template <int L>
+__device__ __forceinline__ bool train_backward(TrainCta& t, bool first) {
+    constexpr int in = mlp_in_dim(L), out = mlp_out_dim(L);
+    unsigned char* dy = t.sm + SmemTrain::dy;
+    unsigned char* dyt = t.sm + SmemTrain::dyt;
+    publish_smem();
+    if (threadIdx.x == 0) {
+        tc::fence_after_sync();
+        gemm_issue_nc(t.tm + col_w(L), dyt, t.in_t(L), 128, in, !first);
+        gemm_issue_nc(t.tm + col_b(L), dyt, t.sm + SmemTrain::ones, 128, 16, !first);
+        if (L > 0) gemm_issue_nc(t.tm + kColT, dy, t.sm + image_wt(L), out, in, false);
+        tc::mma_commit(t.mbar);
+    }
+    if (!cta_sync_wait(t.mbar, t.phase, t.err, 8)) return false;
+    if (L == 3) {
+        // rows 64..79 of dY^T held the output layer's extra gradients
+        uint4* z = reinterpret_cast<uint4*>(dyt + tc::kmajor_offset(64, 0, 128));
+        for (int i = threadIdx.x; i < 16 * 128 * 2 / 16; i += kTrainThreads) z[i] = make_uint4(0, 0, 0, 0);
+    }
+    if (L > 0) {
+        float g[16];
+        const int c0 = 16 * t.grp;
+        tc::tmem_ld16(t.tm + t.lane_base + kColT + (uint32_t)c0, g);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const float h = __bfloat162float(
+                *reinterpret_cast<const __nv_bfloat16*>(t.in_t(L) + tc::kmajor_offset(c0 + i, t.r, 128)));
+            if (!(h > 0.0f)) g[i] = 0.0f;
+        }
+        store_both_bf16<16>(dy, dyt, t.r, c0, g, in);
+    }
+    return true;
+}
+
+__global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_train(const MlpParams P, const float4* __restrict__ pos,
+                                                                const float4* __restrict__ dir, int n, float inv_n,
+                                                                float* __restrict__ part, int* err) {
     extern __shared__ __align__(1024) unsigned char sm[];
     __shared__ __align__(8) uint64_t mbar;
     __shared__ uint32_t tmem_base;
+    __shared__ float loss_warp[4];
     const int tid = threadIdx.x, warp = tid >> 5;
-    unsigned char* Wf[4] = {sm + SmemTrain::wf0, sm + SmemTrain::wf1, sm + SmemTrain::wf2, sm + SmemTrain::wf3};
-    unsigned char* Wt[4] = {nullptr, sm + SmemTrain::wt1, sm + SmemTrain::wt2, sm + SmemTrain::wt3};
-    unsigned char* InT[4] = {sm + SmemTrain::xt, sm + SmemTrain::ht0, sm + SmemTrain::ht1, sm + SmemTrain::ht2};
-    unsigned char* Act = sm + SmemTrain::act;
-    unsigned char* Dy = sm + SmemTrain::dy;
     unsigned char* DyT = sm + SmemTrain::dyt;
-    unsigned char* Ones = sm + SmemTrain::ones;
-    for (int l = 0; l < 4; ++l) {
-        const int in = mlp_in_dim(l), out = mlp_out_dim(l);
-        for (int i = tid; i < in * out; i += 128) {
-            const int o = i / in, c = i % in;
-            const __nv_bfloat16 v = P.w[l][i];
-            *reinterpret_cast<__nv_bfloat16*>(Wf[l] + tc::kmajor_offset(o, c, in)) = v;
-            if (l > 0) *reinterpret_cast<__nv_bfloat16*>(Wt[l] + tc::kmajor_offset(c, o, out)) = v;
-        }
+    {
+        const uint4* src = reinterpret_cast<const uint4*>(P.image);
+        uint4* to = reinterpret_cast<uint4*>(sm);
+#pragma unroll 8
+        for (int i = tid; i < SmemTrain::image / 16; i += kTrainThreads) to[i] = src[i];
     }
-    for (int i = tid; i < 128 * 128 * 2 / 16; i += 128) reinterpret_cast<uint4*>(DyT)[i] = make_uint4(0, 0, 0, 0);
-    for (int i = tid; i < 16 * 128 * 2 / 16; i += 128)
-        reinterpret_cast<uint4*>(Ones)[i] = make_uint4(0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u);
-    float* bias = reinterpret_cast<float*>(sm + SmemTrain::bias);
-    for (int i = tid; i < 272; i += 128) {
-        const int l = i < 64 ? 0 : (i < 128 ? 1 : (i < 192 ? 2 : 3));
-        bias[i] = P.b[l][i - 64 * l];
+    for (int i = tid; i < 128 * 128 * 2 / 16; i += kTrainThreads) reinterpret_cast<uint4*>(DyT)[i] = make_uint4(0, 0, 0, 0);
+    for (int i = tid; i < 16 * 128 * 2 / 16; i += kTrainThreads)
+        reinterpret_cast<uint4*>(sm + SmemTrain::ones)[i] = make_uint4(0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u);
+    if (tid < 272) {
+        const int l = tid < 64 ? 0 : (tid < 128 ? 1 : (tid < 192 ? 2 : 3));
+        reinterpret_cast<float*>(sm + SmemTrain::bias)[tid] = P.b[l][tid - 64 * l];
     }
     if (tid == 0) tc::mbar_init(&mbar, 1);
     if (warp == 0) tc::tmem_alloc(&tmem_base, 512);
     publish_smem();
     tc::fence_after_sync();
-    const uint32_t tm = tmem_base;
-    const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
-    uint32_t phase = 0;
+    // warp w reads TMEM lanes 32 (w % 4) ..: its row of the tile; w / 4 is its column group
+    TrainCta t{sm, &mbar, tmem_base, (uint32_t)((warp & 3) * 32) << 16, 0u, (warp & 3) * 32 + (tid & 31), warp >> 2, err};
     bool failed = false, first = true;
-    float loss_acc = 0.0f;
+    float loss = 0.0f;
     for (long long tile = blockIdx.x; tile * 128 < n && !failed; tile += gridDim.x) {
-        const long long row = tile * 128 + tid;
+        const long long row = tile * 128 + t.r;
         const bool valid = row < n;
         const float4 pd = valid ? pos[row] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         const float4 dd = valid ? dir[row] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        float v[kMlpOut];
-        {
-            float x[kMlpIn];
-            if (valid) encode(pd.x, pd.y, pd.z, x);
-            else for (int i = 0; i < kMlpIn; ++i) x[i] = 0.0f;
-            store_row_bf16(Act, tid, x, kMlpIn);
-            store_col_bf16(InT[0], tid, x, kMlpIn);
-        }
-        for (int l = 0; l < 4 && !failed; ++l) {
-            const int K = mlp_in_dim(l), N = mlp_out_dim(l);
-            publish_smem();
-            if (tid == 0) {
-                tc::fence_after_sync();
-                tc::gemm_issue(tm + kColT, Act, Wf[l], K, N, false, &mbar);
+        unsigned char* act = sm + SmemTrain::act;
+        if (t.grp < 3) {
+            float x[kMlpCoord];
+            encode_coord(t.grp == 0 ? pd.x : t.grp == 1 ? pd.y : pd.z, x);
+#pragma unroll
+            for (int k = 0; k < kMlpCoord; ++k) {
+                const __nv_bfloat16 w = __float2bfloat16_rn(valid ? x[k] : 0.0f);
+                const int c = kMlpCoord * t.grp + k;
+                *reinterpret_cast<__nv_bfloat16*>(act + tc::kmajor_offset(t.r, c, kMlpIn)) = w;
+                *reinterpret_cast<__nv_bfloat16*>(t.in_t(0) + tc::kmajor_offset(c, t.r, 128)) = w;
             }
-            if (!cta_sync_wait(&mbar, phase, err, 4)) { failed = true; break; }
+        } else {
 #pragma unroll
-            for (int c = 0; c < N; c += 16) tc::tmem_ld16(tm + lane_base + kColT + (uint32_t)c, v + c);
-            const float* bl = bias + 64 * l;
-            if (l < 3) {
-#pragma unroll
-                for (int c = 0; c < N; ++c) v[c] = fmaxf(v[c] + bl[c], 0.0f);
-                store_row_bf16(Act, tid, v, N);
-                store_col_bf16(InT[l + 1], tid, v, N);
-            } else {
-#pragma unroll
-                for (int c = 0; c < N; ++c) v[c] += bl[c];
+            for (int c = 3 * kMlpCoord; c < kMlpIn; ++c) {
+                *reinterpret_cast<__nv_bfloat16*>(act + tc::kmajor_offset(t.r, c, kMlpIn)) = __float2bfloat16_rn(0.0f);
+                *reinterpret_cast<__nv_bfloat16*>(t.in_t(0) + tc::kmajor_offset(c, t.r, 128)) = __float2bfloat16_rn(0.0f);
             }
         }
+        float v[20];
+        failed = !train_forward<0>(t, v) || !train_forward<1>(t, v) || !train_forward<2>(t, v) || !train_forward<3>(t, v);
         if (failed) break;
-        {
-            float g[kMlpOut];
-            if (valid) loss_acc += loss_grad_row(v, dd, pd.w, inv_n, g);
-            else for (int i = 0; i < kMlpOut; ++i) g[i] = 0.0f;
-            store_row_bf16(Dy, tid, g, kMlpOut);
-            store_col_bf16(DyT, tid, g, kMlpOut);
-        }
-        for (int l = 3; l >= 0 && !failed; --l) {
-            const int in = mlp_in_dim(l), out = mlp_out_dim(l);
-            publish_smem();
-            if (tid == 0) {
-                tc::fence_after_sync();
-                gemm_issue_nc(tm + col_w(l), DyT, InT[l], 128, in, !first);
-                gemm_issue_nc(tm + col_b(l), DyT, Ones, 128, 16, !first);
-                if (l > 0) gemm_issue_nc(tm + kColT, Dy, Wt[l], out, in, false);
-                tc::mma_commit(&mbar);
-            }
-            if (!cta_sync_wait(&mbar, phase, err, 8)) { failed = true; break; }
-            if (l == 3) {
-                // rows 64..79 of dY^T held the output layer's extra gradients
-                uint4* z = reinterpret_cast<uint4*>(DyT + tc::kmajor_offset(64, 0, 128));
-                for (int i = tid; i < 16 * 128 * 2 / 16; i += 128) z[i] = make_uint4(0, 0, 0, 0);
-            }
-            if (l > 0) {
-                float g[kMlpHid];
-#pragma unroll
-                for (int c = 0; c < in; c += 16) tc::tmem_ld16(tm + lane_base + kColT + (uint32_t)c, g + c);
-#pragma unroll
-                for (int i = 0; i < in; ++i) {
-                    const float h = __bfloat162float(
-                        *reinterpret_cast<const __nv_bfloat16*>(InT[l] + tc::kmajor_offset(i, tid, 128)));
-                    if (!(h > 0.0f)) g[i] = 0.0f;
-                }
-                store_row_bf16(Dy, tid, g, in);
-                store_col_bf16(DyT, tid, g, in);
-            }
-        }
+        float g[20];
+        const float l = loss_grad(t, v, dd, pd.w, inv_n, g);
+        if (valid && t.grp == 0) loss += l;
+        if (!valid)
+            for (int i = 0; i < 20; ++i) g[i] = 0.0f;
+        store_both_bf16<20>(sm + SmemTrain::dy, DyT, t.r, 20 * t.grp, g, kMlpOut);
+        failed = !train_backward<3>(t, first) || !train_backward<2>(t, first) || !train_backward<1>(t, first) ||
+                 !train_backward<0>(t, first);
         first = false;
     }
-    for (int o = 16; o > 0; o >>= 1) loss_acc += __shfl_xor_sync(0xffffffffu, loss_acc, o);
-    if ((tid & 31) == 0 && loss_acc != 0.0f) atomicAdd(loss, loss_acc);
+    for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
+    if ((tid & 31) == 0 && warp < 4) loss_warp[warp] = loss;
+    // this CTA's gradient sums, packed like the parameters (per layer: W out x in, b), and loss
+    float* mine = part + (size_t)blockIdx.x * kMlpPartStride;
     if (!failed && !first) {
-        // this CTA's gradient sums, packed like the parameters (per layer: W out x in, b)
-        float* mine = part + (size_t)blockIdx.x * part_stride;
         int off = 0;
+#pragma unroll
         for (int l = 0; l < 4; ++l) {
             const int in = mlp_in_dim(l), out = mlp_out_dim(l);
-            float t[16];
+            float q[16];
+            for (int c = 16 * t.grp; c < in; c += 64) {
+                tc::tmem_ld16(t.tm + t.lane_base + col_w(l) + (uint32_t)c, q);
+                if (t.r < out)
 #pragma unroll
-            for (int c = 0; c < in; c += 16) {
-                tc::tmem_ld16(tm + lane_base + col_w(l) + (uint32_t)c, t);
-                if (tid < out)
-                    for (int j = 0; j < 16; ++j) mine[off + tid * in + c + j] = t[j];
+                    for (int j = 0; j < 16; j += 4)
+                        *reinterpret_cast<float4*>(mine + off + t.r * in + c + j) =
+                            make_float4(q[j], q[j + 1], q[j + 2], q[j + 3]);
             }
-            tc::tmem_ld16(tm + lane_base + col_b(l), t);
-            if (tid < out) mine[off + out * in + tid] = t[0];
+            if (t.grp == 3) {
+                tc::tmem_ld16(t.tm + t.lane_base + col_b(l), q);
+                if (t.r < out) mine[off + out * in + t.r] = q[0];
+            }
             off += out * in + out;
         }
+    } else {
+        for (int i = tid; i < kMlpPartStride - 4; i += kTrainThreads) mine[i] = 0.0f;
     }
     tc::fence_before_sync();
     __syncthreads();
-    if (warp == 0) tc::tmem_dealloc(tm, 512);
+    if (tid == 0) mine[kMlpPartStride - 4] = ((loss_warp[0] + loss_warp[1]) + loss_warp[2]) + loss_warp[3];
+    if (warp == 0) tc::tmem_dealloc(t.tm, 512);
 }
 
-// Sum of the per-CTA partial gradients into gw/gb, then (apply) one Adam step.
-__global__ void k_reduce_adam(const MlpParams P, const float* __restrict__ part, int nparts, int total, int apply,
-                              float lr, float b1t, float b2t) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= total) return;
+// Sum of the per-CTA partial gradients into gw/gb (and the loss), then (apply) one Adam
+// step.  A block takes 32 consecutive parameters, its 8 warps an eighth of the partial
+// rows each.
+constexpr int kReduceWarps = 8;
+__global__ void __launch_bounds__(32 * kReduceWarps) k_reduce_adam(const MlpParams P, const float* __restrict__ part,
+                                                                   int nparts, int apply, float lr, float b1t, float b2t,
+                                                                   float* __restrict__ loss) {
+    __shared__ float sums[kReduceWarps][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int j = blockIdx.x * 32 + lane;   // parameter, or the loss
+    constexpr int total = kMlpPartStride - 4;
     float g = 0.0f;
-    for (int b = 0; b < nparts; ++b) g += part[(size_t)b * total + j];
+    if (j <= total) {
+#pragma unroll 8
+        for (int b = warp; b < nparts; b += kReduceWarps) g += part[(size_t)b * kMlpPartStride + j];
+    }
+    sums[warp][lane] = g;
+    __syncthreads();
+    if (warp != 0 || j > total) return;
+    g = 0.0f;
+#pragma unroll
+    for (int w = 0; w < kReduceWarps; ++w) g += sums[w][lane];
+    if (j == total) { *loss = g; return; }
     int l = 0, idx = j;
     for (; l < 3; ++l) {
         const int sz = mlp_in_dim(l) * mlp_out_dim(l) + mlp_out_dim(l);
         if (idx < sz) break;
         idx -= sz;
     }
-    const int nw = mlp_in_dim(l) * mlp_out_dim(l);
+    const int in = mlp_in_dim(l), nw = in * mlp_out_dim(l);
     const bool is_w = idx < nw;
     const int i = is_w ? idx : idx - nw;
     float* w = is_w ? P.wm[l] : P.b[l];
@@ -575,12 +661,24 @@ __global__ void k_reduce_adam(const MlpParams P, const float* __restrict__ part,
     v[i] = vi;
     const float wi = w[i] - lr * (mi / (1.0f - b1t)) / (sqrtf(vi / (1.0f - b2t)) + eps);
     w[i] = wi;
-    if (is_w) P.w[l][i] = __float2bfloat16_rn(wi);
+    if (is_w) {
+        const __nv_bfloat16 h = __float2bfloat16_rn(wi);
+        P.w[l][i] = h;
+        image_put(P.image, l, i / in, i % in, h);
+    }
 }
 
-__global__ void k_to_bf16(const float* w, __nv_bfloat16* wb, int n) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) wb[i] = __float2bfloat16_rn(w[i]);
+// Layer l's BF16 weights and its part of the image, from the FP32 weights.
+__global__ void k_to_bf16(const MlpParams P, int l) {
+    const int in = mlp_in_dim(l), i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= in * mlp_out_dim(l)) return;
+    const __nv_bfloat16 h = __float2bfloat16_rn(P.wm[l][i]);
+    P.w[l][i] = h;
+    image_put(P.image, l, i / in, i % in, h);
+}
+
+void to_bf16(const MlpParams& p, int l, cudaStream_t s) {
+    k_to_bf16<<<(mlp_in_dim(l) * mlp_out_dim(l) + 255) / 256, 256, 0, s>>>(p, l);
 }
 
 int sm_count() {
@@ -631,7 +729,7 @@ int mlp_import(MlpParams& p, const float* in, int adam_step, cudaStream_t s) {
             if (cudaMemcpyAsync(dst[k], in + o, 4 * cnt[k], cudaMemcpyHostToDevice, s) != cudaSuccess) return -1;
             o += cnt[k];
         }
-        k_to_bf16<<<(unsigned)((nw + 255) / 256), 256, 0, s>>>(p.wm[l], p.w[l], (int)nw);
+        to_bf16(p, l, s);
     }
     p.adam_step = adam_step;
     return cudaStreamSynchronize(s) == cudaSuccess ? 0 : -1;
@@ -660,7 +758,7 @@ int mlp_init(MlpParams& p, uint64_t seed, cudaStream_t s) {
         cudaMemsetAsync(p.vw[l], 0, 4 * w.size(), s);
         cudaMemsetAsync(p.mb[l], 0, 4 * b.size(), s);
         cudaMemsetAsync(p.vb[l], 0, 4 * b.size(), s);
-        k_to_bf16<<<(unsigned)((w.size() + 255) / 256), 256, 0, s>>>(p.wm[l], p.w[l], (int)w.size());
+        to_bf16(p, l, s);
     }
     p.adam_step = 0;
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
@@ -746,15 +844,14 @@ int mlp_train_step(MlpParams& p, MlpBatch& b, const float4* pos4, const float4* 
     const size_t smem = SmemTrain::total;
     static std::once_flag attr[kOnceDevices];   // once per device (contexts on several threads launch)
     once_per_device(attr, [&] { cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); });
-    const int total = (int)mlp_param_floats();
     const int tiles = (n + 127) / 128;
     const int grid = std::min(std::min(tiles, sm_count()), b.part_rows);
-    cudaMemsetAsync(b.loss, 0, sizeof(float), s);
-    k_mlp_train<<<grid, 128, smem, s>>>(p, pos4, dir4, n, 1.0f / (float)n, b.part, total, b.loss, err);
+    k_mlp_train<<<grid, kTrainThreads, smem, s>>>(p, pos4, dir4, n, 1.0f / (float)n, b.part, err);
     if (apply) p.adam_step++;
     const float b1t = std::pow(0.9f, (float)std::max(p.adam_step, 1));
     const float b2t = std::pow(0.999f, (float)std::max(p.adam_step, 1));
-    k_reduce_adam<<<(total + 255) / 256, 256, 0, s>>>(p, b.part, grid, total, apply ? 1 : 0, lr, b1t, b2t);
+    k_reduce_adam<<<(kMlpPartStride - 4) / 32 + 1, 32 * kReduceWarps, 0, s>>>(p, b.part, grid, apply ? 1 : 0, lr, b1t, b2t,
+                                                                           b.loss);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -786,6 +883,7 @@ bool MlpStore::setup(int n) {
         p.gw[l] = alloc<float>(nw); p.gb[l] = alloc<float>(nb); p.mw[l] = alloc<float>(nw);
         p.vw[l] = alloc<float>(nw); p.mb[l] = alloc<float>(nb); p.vb[l] = alloc<float>(nb);
     }
+    p.image = alloc<unsigned char>(SmemTrain::image);
     b.n = n;
     b.pos = alloc<float4>(n); b.dir = alloc<float4>(n);
     b.out = alloc<float>((size_t)n * kMlpOut);
@@ -794,7 +892,7 @@ bool MlpStore::setup(int n) {
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     b.part_rows = std::max(sms, 1);
-    b.part = alloc<float>((size_t)b.part_rows * mlp_param_floats());
+    b.part = alloc<float>((size_t)b.part_rows * kMlpPartStride);
     for (void* a : allocs) if (!a) return false;
     return true;
 }
@@ -819,7 +917,7 @@ struct HostMlp : MlpStore {
             const size_t nw = (size_t)mlp_in_dim(l) * mlp_out_dim(l), nb = mlp_out_dim(l);
             cudaMemcpy(p.wm[l], packed + o, 4 * nw, cudaMemcpyHostToDevice); o += nw;
             cudaMemcpy(p.b[l], packed + o, 4 * nb, cudaMemcpyHostToDevice); o += nb;
-            k_to_bf16<<<(unsigned)((nw + 255) / 256), 256>>>(p.wm[l], p.w[l], (int)nw);
+            to_bf16(p, l, 0);
         }
     }
     void get(float* const* src_w, float* const* src_b, float* packed) {

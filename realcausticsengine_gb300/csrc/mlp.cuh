@@ -24,6 +24,7 @@ namespace rc {
 constexpr int kMlpIn = 80, kMlpInReal = 75, kMlpHid = 64, kMlpOut = 80, kMlpLobes = 16, kMlpFreqs = 12;
 constexpr int kMlpLayers = 4;
 constexpr float kMlpDefensive = 0.2f;
+constexpr int kMlpPartStride = 64 * 80 + 64 + 2 * (64 * 64 + 64) + 80 * 64 + 80 + 4;   // parameters, loss, padding
 
 __host__ __device__ constexpr int mlp_in_dim(int l) { return l == 0 ? kMlpIn : kMlpHid; }
 __host__ __device__ constexpr int mlp_out_dim(int l) { return l == 3 ? kMlpOut : kMlpHid; }
@@ -38,6 +39,7 @@ struct MlpParams {
     float* vw[kMlpLayers];
     float* mb[kMlpLayers];
     float* vb[kMlpLayers];
+    unsigned char* image;           // the BF16 weights as the training step holds them in shared memory
     int adam_step;
 };
 
@@ -47,7 +49,7 @@ struct MlpBatch {
     float4* dir;                    // sampled direction (xyz) | weight f / q_old
     float* out;                     // n x 80 network outputs (forward test)
     float* loss;                    // weighted loss of the last step (1 float)
-    float* part;                    // per-CTA partial gradients (part_rows x parameters)
+    float* part;                    // per-CTA partial gradients and loss (part_rows x kMlpPartStride)
     int part_rows;
     int n;
 };

@@ -188,6 +188,40 @@ def test_mlp_gradients_match_fp64():
             assert cos > 0.999 and rel < 0.03, (l, cos, rel)
 
 
+@pytest.mark.parametrize("n", [1, 64, 127, 128, 129, 152 * 128, 152 * 128 + 1])
+def test_mlp_gradients_at_tile_edges(n):
+    """Rows of weight zero change nothing: twice the gradients of a batch of 2 n rows whose
+    second half weighs nothing are those of its first half.  1 / n against 1 / (2 n) is an
+    exact power of two and every row's products are the same, so only the order of FP32 sums
+    differs: at most 128 partial sums of 19,457 rows, 1e-5 of each layer's norm.  The first
+    half agrees with the FP64 model where rows enough average its BF16 roundings."""
+    L = lib()
+    rng = np.random.default_rng(3)
+    ps = init_params(rng)
+    flat = pack(ps)
+    pos4, dir4 = batch(rng, 2 * n)
+    dir4[n:, 3] = 0.0
+    grads, losses = [], []
+    for m in (n, 2 * n):
+        g, loss = np.zeros_like(flat), np.zeros(1, np.float32)
+        assert L.rc_mlp_grad_test(m, flat.ctypes.data, pos4.ctypes.data, dir4.ctypes.data, g.ctypes.data,
+                                  loss.ctypes.data) == 0
+        grads.append(g)
+        losses.append(float(loss[0]))
+    assert abs(losses[0] - 2 * losses[1]) <= 1e-5 * abs(losses[0])
+    for a, b in zip(unpack(grads[0]), unpack(grads[1])):
+        for x, y in zip(a, b):
+            assert np.linalg.norm(x) > 0
+            assert np.linalg.norm(x - 2 * y) <= 1e-5 * np.linalg.norm(x)
+    if n >= 4096:
+        out, acts = forward_np(ps, pos4[:n, :3])
+        _, dout = loss_and_dout(out, *(dir4[:n, :3].astype(np.float64), dir4[:n, 3].astype(np.float64),
+                                       pos4[:n, 3].astype(np.float64)))
+        for a, b in zip(unpack(grads[0]), backward_np(ps, acts, dout)):
+            for x, y in zip(a, b):
+                assert np.linalg.norm(x - y) < 0.03 * np.linalg.norm(y)
+
+
 def test_mlp_training_lowers_loss():
     L = lib()
     rng = np.random.default_rng(2)
