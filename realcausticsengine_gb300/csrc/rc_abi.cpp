@@ -814,7 +814,7 @@ int render_iteration(HostScene& sc, int redo_iteration = -1, bool tune_passes = 
             RC_CUDA(cudaEventRecord(d.evm[1], s));
         }
         RC_CUDA(cudaEventRecord(d.ev[0], s));
-        if (sampler == RC_SAMPLER_UNIFORM && attempt == 0) {
+        if (sampler == RC_SAMPLER_UNIFORM && attempt == 0 && light_order_pays(p.num_light_paths)) {
             // coherent processing order of the light paths (their samples unchanged)
             RC_CUDA(d.path_order.reserve(std::max<long long>(p.num_light_paths, 1)));
             RC_CUDA(d.order_scratch.reserve(light_order_scratch_bytes(p.num_light_paths)));
@@ -1099,11 +1099,12 @@ int async_setup(const HostScene& sc) {
 
 // The two ends of an asynchronous iteration (no host synchronisation), shared by the
 // single-scene replay and the batch (batch_render).  async_head, on s: the iteration's
-// photon and query counters reset, the light-path order.
-int async_head(VMParams& p, cudaStream_t s) {
+// photon and query counters reset, the light-path order (if `order`).
+int async_head(VMParams& p, cudaStream_t s, bool order) {
     DeviceState& d = ctx().dev;
     RC_CUDA(cudaMemsetAsync(d.counters.p, 0, sizeof(unsigned long long) * 2, s));
     RC_CUDA(record(d.ev[0], s));
+    if (!order) return RC_OK;
     launch_light_order(p, d.order_scratch.p, d.path_order.p, s);
     p.path_order = d.path_order.p;
     return RC_OK;
@@ -1153,7 +1154,7 @@ int enqueue_async_iteration(HostScene& sc, int it, int* flag) {
     const long long pc = d.async_pcap, qc = d.async_qcap;
     PhotonBuf ph{d.ph_pos.p, d.ph_dir.p, d.ph_tp.p, d.ph_path.p, pc, d.counters.p};
     QueryBuf qb{d.q0.p, d.q1.p, d.q2.p, d.q3.p, d.q4.p, qc, d.counters.p + 1};
-    int r = async_head(p, s);
+    int r = async_head(p, s, light_order_pays(p.num_light_paths));
     if (r) return r;
     // the camera pass on a branch of its own beside the light pass's tail and the photon
     // order (it reads nothing they write), joined before the count check
@@ -1529,7 +1530,7 @@ int batch_render(Context* const* cs, int n, int iterations, double* out) {
                 t_bound = cs[i];
                 VMParams p = entries[entry_at[j] + a].p;
                 RC_CUDA(cudaStreamWaitEvent(branch(i), B.start, 0));
-                int rr = async_head(p, branch(i));
+                int rr = async_head(p, branch(i), true);
                 if (rr) return scene_fail(i, rr);
                 RC_CUDA(cudaEventRecord(B.join, branch(i)));
                 RC_CUDA(cudaStreamWaitEvent(B.main, B.join, 0));

@@ -106,6 +106,9 @@ int mlt_variants();
 // u, v, direction u, v; with p.proposal, the proposed direction's octahedral coordinates
 // for the direction), so that each warp of the persistent pass starts coherent rays.
 // Every path keeps its samples and index: only the order of tracing changes.
+// light_order_pays: not where the passes spread few paths over many warps (its five launches
+// take 25 us and coherence gains nothing there).
+bool light_order_pays(long long n);
 size_t light_order_scratch_bytes(long long n);
 void launch_light_order(const VMParams& p, void* scratch, uint32_t* order, cudaStream_t s);
 // Exclusive scan of m counters in place, in three passes over 8192-counter tiles with

@@ -174,11 +174,12 @@ __global__ void k_light_scatter(const uint32_t* __restrict__ keys, long long n, 
 }
 
 constexpr int kRefillLanes = 24;
+__device__ __forceinline__ int refill_lanes(int lanes) { return (kRefillLanes * lanes + 31) / 32; }
 
 // kMinBlocks caps the registers per thread (resident blocks per SM the allocation must
 // allow); traversal stacks are per-traversal local-memory arrays.
 template <int kBlock, int kMinBlocks>
-__global__ void __launch_bounds__(kBlock, kMinBlocks) k_light_pass_persistent(const VMParams P, PhotonBuf ph,
+__global__ void __launch_bounds__(kBlock, kMinBlocks) k_light_pass_persistent(const VMParams P, PhotonBuf ph, int lanes,
                                                                                unsigned long long* __restrict__ next_path,
                                                                                unsigned long long* __restrict__ rays) {
     CallStack stk;
@@ -187,6 +188,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) k_light_pass_persistent(co
     bool alive = false;
     bool pool_left = true;
     unsigned traced = 0;      // closest-hit queries of this lane (one per bounce)
+    const int refill = refill_lanes(lanes);
     while (true) {
         // refill lanes without a path, once at least kRefillLanes are free (or none has
         // a path): lanes refilled together take consecutive, coherent paths (the order
@@ -195,12 +197,12 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) k_light_pass_persistent(co
         // any free lane 14.2 ms, at 16 free 13.6, at 20-24 free 13.4, at 32 free 14.5;
         // with the children tested at the parent, per iteration at 20 / 24 / 28 / 32
         // free: 20.49 / 20.48 / 20.82 / 21.13 ms)
-        const unsigned need = __ballot_sync(0xffffffffu, !alive);
-        if (need && pool_left && (__popc(need) >= kRefillLanes || need == 0xffffffffu)) {
+        const unsigned need = __ballot_sync(0xffffffffu, !alive && lane < lanes);
+        if (pool_left && __popc(need) >= refill) {
             unsigned long long base = 0;
             if (lane == __ffs(need) - 1) base = atomicAdd(next_path, (unsigned long long)__popc(need));
             base = __shfl_sync(0xffffffffu, base, __ffs(need) - 1);
-            if (!alive) {
+            if (!alive && lane < lanes) {
                 const unsigned long long mine = base + __popc(need & ((1u << lane) - 1u));
                 if (mine < (unsigned long long)P.num_light_paths)
                     alive = light_path_start(P, P.path_order ? (long long)__ldg(&P.path_order[mine]) : (long long)mine,
@@ -311,7 +313,7 @@ __device__ __forceinline__ bool camera_path_bounce(const VMParams& P, const Quer
 }
 
 template <int kBlock, int kMinBlocks>
-__global__ void __launch_bounds__(kBlock, kMinBlocks) k_camera_pass_persistent(const VMParams P, QueryBuf qb,
+__global__ void __launch_bounds__(kBlock, kMinBlocks) k_camera_pass_persistent(const VMParams P, QueryBuf qb, int lanes,
                                                                                 unsigned long long* __restrict__ next_pixel) {
     CallStack stk;
     const int lane = threadIdx.x & 31;
@@ -319,20 +321,21 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) k_camera_pass_persistent(c
     CameraPath s;
     bool alive = false;
     bool pool_left = true;
+    const int refill = refill_lanes(lanes);
     while (true) {
         // refill as in the light pass: once kRefillLanes lanes are free (2.43 -> 2.35 ms on
         // the water pool), drawing again for samples that fall outside the buffer
-        unsigned need = __ballot_sync(0xffffffffu, !alive);
-        while (need && pool_left && (__popc(need) >= kRefillLanes || need == 0xffffffffu)) {
+        unsigned need = __ballot_sync(0xffffffffu, !alive && lane < lanes);
+        while (pool_left && __popc(need) >= refill) {
             unsigned long long base = 0;
             if (lane == __ffs(need) - 1) base = atomicAdd(next_pixel, (unsigned long long)__popc(need));
             base = __shfl_sync(0xffffffffu, base, __ffs(need) - 1);
-            if (!alive) {
+            if (!alive && lane < lanes) {
                 const unsigned long long mine = base + __popc(need & ((1u << lane) - 1u));
                 if (mine < (unsigned long long)npix) alive = camera_path_start(P, (long long)mine, s);
             }
             if (base + __popc(need) >= (unsigned long long)npix) pool_left = false;
-            need = __ballot_sync(0xffffffffu, !alive);   // samples outside the buffer: draw again
+            need = __ballot_sync(0xffffffffu, !alive && lane < lanes);   // samples outside the buffer: draw again
         }
         if (!__any_sync(0xffffffffu, alive)) break;
         if (alive) alive = camera_path_bounce(P, qb, s, stk);
@@ -713,19 +716,36 @@ unsigned persistent_grid(K kernel, int block, size_t smem, long long work_items)
     return (unsigned)(need < blocks ? need : blocks);
 }
 
+// Paths that a warp of the persistent passes holds.  A pass too small to give 12 warps per
+// SM 32 paths each is spread over the warps of the whole GPU: its time is then the longest
+// warp, and a warp of few paths executes fewer of the others' steps (sphere of 5k triangles,
+// light / camera pass in us: 6,144 paths 248 / 237 with 32 lanes, 191 / 163 with 4; 19,200:
+// 261 / 274 with 32, 193 / 223 with 8; 49,152: 306 / 299 with 32, 265 / 256 with 16).  12 warps
+// leave room for the other pass beside it: an update of 6,144 paths and pixels takes 566 us
+// with 32 lanes, 502 / 495 / 497 / 500 / 515 with 8 / 12 / 16 / 24 / 32 warps per SM.
+int path_lanes(long long n) {
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const long long warps = 12LL * std::max(sms, 1);
+    return (int)std::min(std::max((n + warps / 2) / warps, 1LL), 32LL);
+}
+
 template <int B, int MB>
 void launch_light_t(const VMParams& p, PhotonBuf ph, unsigned long long* next_path, unsigned long long* rays,
                     cudaStream_t s) {
     // per host thread: contexts on different threads launch concurrently
     static thread_local unsigned grid_cache = 0;
     static thread_local long long grid_for = -1;
+    static thread_local int lanes = 32;
     if (grid_for != p.num_light_paths) {
-        grid_cache = persistent_grid(k_light_pass_persistent<B, MB>, B, 0, p.num_light_paths);
+        lanes = path_lanes(p.num_light_paths);
+        grid_cache = persistent_grid(k_light_pass_persistent<B, MB>, B, 0, p.num_light_paths * 32 / lanes);
         grid_for = p.num_light_paths;
     }
     cudaMemsetAsync(next_path, 0, sizeof(unsigned long long), s);
     if (rays) cudaMemsetAsync(rays, 0, sizeof(unsigned long long), s);
-    k_light_pass_persistent<B, MB><<<grid_cache, B, 0, s>>>(p, ph, next_path, rays);
+    k_light_pass_persistent<B, MB><<<grid_cache, B, 0, s>>>(p, ph, lanes, next_path, rays);
 }
 
 template <int B, int MB>
@@ -734,12 +754,14 @@ void launch_camera_t(const VMParams& p, QueryBuf qb, unsigned long long* next_pi
     // per host thread: contexts on different threads launch concurrently
     static thread_local unsigned grid_cache = 0;
     static thread_local long long grid_for = -1;
+    static thread_local int lanes = 32;
     if (grid_for != n) {
-        grid_cache = persistent_grid(k_camera_pass_persistent<B, MB>, B, 0, n);
+        lanes = path_lanes(n);
+        grid_cache = persistent_grid(k_camera_pass_persistent<B, MB>, B, 0, n * 32 / lanes);
         grid_for = n;
     }
     cudaMemsetAsync(next_pixel, 0, sizeof(unsigned long long), s);
-    k_camera_pass_persistent<B, MB><<<grid_cache, B, 0, s>>>(p, qb, next_pixel);
+    k_camera_pass_persistent<B, MB><<<grid_cache, B, 0, s>>>(p, qb, lanes, next_pixel);
 }
 
 template <int B, int MB>
@@ -773,6 +795,8 @@ void launch_camera_batch_t(const BatchScene* scenes, const long long* prefix, in
 size_t light_order_scratch_bytes(long long n) {
     return 4 * (size_t)(n > 0 ? n : 1) + 4 * (size_t)kOrderCells + 4 * scan_scratch_words(kOrderCells) + 512;
 }
+
+bool light_order_pays(long long n) { return path_lanes(n) >= 32; }
 
 void launch_light_order(const VMParams& p, void* scratch, uint32_t* order, cudaStream_t s) {
     const long long n = p.num_light_paths;

@@ -44,6 +44,20 @@ def test_staged_camera_pass_writes_the_same_queries(size):
     r.release()
 
 
+@pytest.mark.parametrize("lanes,paths", [(1, 2735), (2, 2737), (31, 57455), (32, 57457)])
+def test_small_passes_spread_over_warps_store_the_same(lanes, paths):
+    """On 152 SMs a warp of the persistent shapes holds `lanes` paths at these sizes."""
+    r = Renderer(scenes.test_scene(paths // 97, 97, subdiv=2, rough_glass=True, dispersion=0.03), max_path_length=6,
+                 photons_per_iter=paths, seed=5)
+    r.prepare()
+    photons, queries = _canonical(r.light_photons_shape(4, 1)), _canonical(r.camera_queries(1, 4))
+    for shape in range(4):
+        for got, want in ((r.light_photons_shape(shape, 1), photons), (r.camera_queries(1, shape), queries)):
+            got = _canonical(got)
+            assert got.shape == want.shape and (got == want).all(), f"shape {shape}"
+    r.release()
+
+
 @pytest.mark.parametrize("radius", [0.4, 2e-3, 1e-5])
 @pytest.mark.parametrize("n", [1, 31, 32, 33, 63, 4095, 4097, 20011])
 def test_spatial_order_finds_every_photon(n, radius):
