@@ -58,11 +58,11 @@ struct DevBuf {
 struct DeviceState {
     bool ready = false;
     cudaStream_t stream = nullptr;
-    cudaEvent_t ev[8] = {};
-    // the camera pass's stream, beside the light pass and the photon order: fork and join
-    // events (timing disabled)
+    cudaEvent_t ev[9] = {};
+    // the stream of the camera pass (and a replayed iteration's query order) beside the light
+    // pass and the photon order: fork, camera-done and join events (timing disabled)
     cudaStream_t side = nullptr;
-    cudaEvent_t fork = nullptr, join = nullptr;
+    cudaEvent_t fork = nullptr, camera = nullptr, join = nullptr;
     // scene
     DevBuf<float4> nodes, wnode_lo, wnode_hi, tris, tri_n0, tri_n1, tri_n2;   // layouts: trace.cuh SceneView
     long long num_mesh_nodes = 0, num_tris = 0;
@@ -146,6 +146,7 @@ struct DeviceState {
         if (t0) { cudaEventDestroy(t0); t0 = nullptr; }
         if (t1) { cudaEventDestroy(t1); t1 = nullptr; }
         if (fork) { cudaEventDestroy(fork); fork = nullptr; }
+        if (camera) { cudaEventDestroy(camera); camera = nullptr; }
         if (join) { cudaEventDestroy(join); join = nullptr; }
         if (side) { cudaStreamDestroy(side); side = nullptr; }
         if (stream) { cudaStreamDestroy(stream); stream = nullptr; }
@@ -242,6 +243,7 @@ int ensure_device() {
         RC_CUDA(cudaEventCreate(&d.t1));
         RC_CUDA(cudaStreamCreateWithFlags(&d.side, cudaStreamNonBlocking));
         RC_CUDA(cudaEventCreateWithFlags(&d.fork, cudaEventDisableTiming));
+        RC_CUDA(cudaEventCreateWithFlags(&d.camera, cudaEventDisableTiming));
         RC_CUDA(cudaEventCreateWithFlags(&d.join, cudaEventDisableTiming));
     }
     return RC_OK;
@@ -519,10 +521,10 @@ cudaError_t record(cudaEvent_t e, cudaStream_t s) {
 }
 
 // Device time from the light pass's start to the later of the photon order's end and the
-// camera pass's end, for an iteration whose camera pass ran on the side stream (its
-// events ev[4], ev[5] overlap the light pass and the photon order).
-double overlapped_ms(const DeviceState& d) {
-    return std::max(ms_between(d.ev[0], d.ev[3]), ms_between(d.ev[0], d.ev[5]));
+// side stream's (ev[side_end]: the camera pass ev[5], a replayed iteration's query order
+// ev[8]), for an iteration whose camera pass ran beside the light pass.
+double overlapped_ms(const DeviceState& d, int side_end) {
+    return std::max(ms_between(d.ev[0], d.ev[3]), ms_between(d.ev[0], d.ev[side_end]));
 }
 
 ProposalCtx proposal_ctx(const HostScene& sc, const VMParams& p) {
@@ -1020,7 +1022,7 @@ int render_iteration(HostScene& sc, int redo_iteration = -1, bool tune_passes = 
     st[6] = t_cam;
     st[7] = ms_between(d.ev[6], d.ev[7]);
     st[8] = t_mlp;           // proposal inference + training
-    st[9] = (cam_side ? overlapped_ms(d) : st[4] + st[5] + st[6]) + st[7] + st[8];
+    st[9] = (cam_side ? overlapped_ms(d, 5) : st[4] + st[5] + st[6]) + st[7] + st[8];
     st[10] = d.iterations_done;
     st[11] = sc.scene_radius;
     st[12] = std::sqrt(p.radius_sqr);
@@ -1111,9 +1113,10 @@ int async_head(VMParams& p, cudaStream_t s, bool order) {
 }
 
 // async_tail, on s after the light pass: the photon capacity padded, the photon order with
-// its boxes and records; then, once the camera pass has recorded `camera_done`,
-// the count check (`flag` = 1 on an overflow), the query order and the gather.
-int async_tail(HostScene& sc, const VMParams& p, cudaStream_t s, cudaEvent_t camera_done, int* flag) {
+// its boxes and records; beside it, on `side` once the camera pass has recorded
+// `camera_done`, the query order; then the count check (`flag` = 1 on an overflow) and
+// the gather.  (A batch passes s itself: its scenes' tails run beside one another already.)
+int async_tail(HostScene& sc, const VMParams& p, cudaStream_t s, cudaStream_t side, cudaEvent_t camera_done, int* flag) {
     DeviceState& d = ctx().dev;
     const long long pc = d.async_pcap, qc = d.async_qcap;
     QueryBuf qb{d.q0.p, d.q1.p, d.q2.p, d.q3.p, d.q4.p, qc, d.counters.p + 1};
@@ -1132,11 +1135,14 @@ int async_tail(HostScene& sc, const VMParams& p, cudaStream_t s, cudaEvent_t cam
     launch_photon_order(PhotonBuf{d.ph_pos.p, d.ph_dir.p, d.ph_tp.p, d.ph_path.p, pc, d.counters.p}, pc, d.counters.p, frame,
                         d.ph_scratch.p, tree, tph, nullptr, s);
     RC_CUDA(record(d.ev[3], s));
-    RC_CUDA(cudaStreamWaitEvent(s, camera_done, 0));
+    RC_CUDA(cudaStreamWaitEvent(side, camera_done, 0));
+    launch_query_order(reinterpret_cast<const float*>(d.q0.p), 4, qc, frame, d.qscratch.p, d.qorder.p,
+                       nullptr, side, d.counters.p + 1);
+    RC_CUDA(record(d.ev[8], side));
+    RC_CUDA(cudaEventRecord(d.join, side));
+    RC_CUDA(cudaStreamWaitEvent(s, d.join, 0));
     launch_check_counts(d.counters.p, pc, d.counters.p + 1, qc, flag, s);
     RC_CUDA(record(d.ev[6], s));
-    launch_query_order(reinterpret_cast<const float*>(d.q0.p), 4, qc, frame, d.qscratch.p, d.qorder.p,
-                       nullptr, s, d.counters.p + 1);
     RC_CUDA(cudaMemsetAsync(d.counters.p + 2, 0, 4 * sizeof(unsigned long long), s));
     RC_CUDA(record(d.evg[0], s));
     launch_gather(p, tree, tph, qb, d.qorder.p, qc, d.accum.p, d.counters.p + 2, s, d.async_gvar, d.counters.p + 1,
@@ -1156,8 +1162,10 @@ int enqueue_async_iteration(HostScene& sc, int it, int* flag) {
     QueryBuf qb{d.q0.p, d.q1.p, d.q2.p, d.q3.p, d.q4.p, qc, d.counters.p + 1};
     int r = async_head(p, s, light_order_pays(p.num_light_paths));
     if (r) return r;
-    // the camera pass on a branch of its own beside the light pass's tail and the photon
-    // order (it reads nothing they write), joined before the count check
+    // the camera pass and the query order on a branch of their own beside the light pass's
+    // tail and the photon order (they read nothing those write), joined before the count
+    // check (the query order on the main stream, after the photon order: an update of 6,144
+    // pixels 495 us, now 420; four iterations of the 518,400-path water pool 6.95 ms, now 6.64)
     r = light_pass(p, ph, s, d.async_lvar, d.fork);   // the camera branch forks where
     if (r) return r;                                   // the light pass stops filling the GPU
     RC_CUDA(record(d.ev[1], s));
@@ -1166,8 +1174,8 @@ int enqueue_async_iteration(HostScene& sc, int it, int* flag) {
     r = camera_pass(p, qb, d.side, d.async_cvar);
     if (r) return r;
     RC_CUDA(record(d.ev[5], d.side));
-    RC_CUDA(cudaEventRecord(d.join, d.side));
-    return async_tail(sc, p, s, d.join, flag);
+    RC_CUDA(cudaEventRecord(d.camera, d.side));
+    return async_tail(sc, p, s, d.side, d.camera, flag);
 }
 
 // Capture iteration `it` as a graph, update the instantiated graph with it (or
@@ -1236,7 +1244,7 @@ int async_finish(HostScene& sc, int first_it, int n_async, bool windows) {
     st[6] = windows ? ms_between(d.ev[4], d.ev[5]) : 0.0;
     st[7] = ms_between(d.ev[6], d.ev[7]);
     st[8] = 0.0;
-    st[9] = windows ? overlapped_ms(d) + st[7] : ms_between(d.ev[2], d.ev[7]);
+    st[9] = windows ? overlapped_ms(d, 8) + st[7] : ms_between(d.ev[2], d.ev[7]);
     st[10] = d.iterations_done;
     st[11] = sc.scene_radius;
     st[12] = std::sqrt(p.radius_sqr);
@@ -1554,7 +1562,7 @@ int batch_render(Context* const* cs, int n, int iterations, double* out) {
                 const int i = active[j][a];
                 t_bound = cs[i];
                 RC_CUDA(cudaStreamWaitEvent(branch(i), B.light, 0));
-                int rr = async_tail(*ctx().scene, entries[entry_at[j] + a].p, branch(i), B.camera,
+                int rr = async_tail(*ctx().scene, entries[entry_at[j] + a].p, branch(i), branch(i), B.camera,
                                     ctx().dev.async_flags.p + j);
                 if (rr) return scene_fail(i, rr);
                 RC_CUDA(cudaEventRecord(B.join, branch(i)));
