@@ -333,7 +333,7 @@ int rc_kd_query(int n, const float* positions, int q, const float* queries, floa
 
 /* The same radius query run by the render's own gather kernel (KD_Tree::find_closest_in_radius,
  * src/KD_Tree.cpp:217-280, as the gather of Path_Vertices::get_contrib, src/Path_Vertices.h:46-68,
- * calls it): the tree's chunk boxes, the KD-cell query order, `variant`'s launch shape
+ * calls it): the chunks' boxes, the queries' curve order, `variant`'s launch shape
  * (0 .. rc_gather_variants()-1, -1 = the default; the autotuner picks among the same
  * shapes) and the pending-pair lists, with a sink that records photon ids where the
  * render evaluates merges.  rc_kd_query is this call with variant -1. */

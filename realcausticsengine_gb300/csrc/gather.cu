@@ -31,6 +31,7 @@
 // per-query BSDF state staged in shared memory when the group starts, sums them per
 // query in shared memory, and adds each query's sum into its FP64 pixel once.  The
 // parity hook's sink records photon ids instead; both are the same kernel template.
+#include <algorithm>
 #include "vm.cuh"
 #include "bsdf.cuh"
 
@@ -122,6 +123,19 @@ struct QState {
     float pad;
 };
 static_assert(sizeof(QState) == 29 * 4, "QState must keep an odd word stride");
+
+// Parking (the last two shapes).  A caustic's focus meets the spheres of a few groups with
+// most of the photons, and the warps of those groups are then the gather's time.  A warp that
+// has done kParkWork (chunks tested and eighths of accepted pairs: 32 pairs take as long as 4
+// chunks) leaves the rest to a second launch: the current step's untested chunks one by one,
+// its pending subtrees in kParkParts parts each (every kParkParts-th chunk).  An item is
+// (group, first | end << 8 of its sub-group's lanes, root, part) at parked[1 + i],
+// parked[0].x of them; void items have root 0.  216k queries and 20k photons behind a glass
+// ball under a point light: 783 us, parked 120 (102 with kParkWork 16; 258 with subtrees
+// only).  Without a focus the second launch costs more than it gives (3.7M queries on a water
+// pool's floor 1.79 ms against 2.17), so the autotuner chooses.
+constexpr unsigned kParkWork = 64, kParkParts = 16;
+constexpr int kParkedItems = (1 << 16) - 1;
 
 template <bool Eval> struct GroupExtra {};
 template <> struct GroupExtra<true> {
@@ -263,15 +277,18 @@ struct SetSink {
     __device__ __forceinline__ void finish(WarpSmem<false>&, int, bool, uint32_t) const {}
 };
 
-// One group of G queries per warp.  MinBlocks (resident blocks per SM the register
-// allocation must allow), G and E (levels per expansion step) are the launch shape the
-// autotuner picks.  counters (optional, 4 u64 accumulated): accepted pairs, photon
-// tests (chunk photons x overlapping queries), chunks tested, boxes tested.
-template <int MinBlocks, int G, int E, class Sink>
+// One group of G queries per warp (stage 0; 1: and it may park subtrees; 2: one parked item
+// at a time).  MinBlocks
+// (resident blocks per SM the register allocation must allow), G and E (levels per
+// expansion step) are the launch shape the autotuner picks.  counters (optional, 4 u64
+// accumulated): accepted pairs, photon tests (chunk photons x overlapping queries), chunks
+// tested, boxes tested.
+template <int kStage, int MinBlocks, int G, int E, class Sink>
 __global__ void __launch_bounds__(32 * kWarpsPerBlock, MinBlocks)
     k_gather(const ChunkTree t, const float* __restrict__ qpos, int qstride, const uint32_t* __restrict__ order,
              long long nq, const unsigned long long* __restrict__ nq_dev, const int* __restrict__ skip, float r2,
-             const Sink sink, unsigned long long* __restrict__ counters, int* __restrict__ err) {
+             const Sink sink, uint4* parked, unsigned long long* __restrict__ counters, int* __restrict__ err) {
+    constexpr bool kRest = kStage == 2;
     static_assert(G == 16 || G == 32, "a group is a half or a whole warp of queries");
     static_assert(E >= 1 && E <= 5, "an expansion step tests at most 32 descendants");
     // device-side count (bounded by the capacity nq) and an iteration-wide skip flag,
@@ -280,12 +297,21 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, MinBlocks)
     if (nq_dev) nq = (long long)min(*nq_dev, (unsigned long long)nq);
     __shared__ WarpSmem<Sink::kEval> smem[kWarpsPerBlock];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long long first = ((long long)blockIdx.x * kWarpsPerBlock + warp) * G;
-    if (first >= nq || t.lc < 0) return;
+    const unsigned lt = (1u << lane) - 1u;
     WarpSmem<Sink::kEval>& sm = smem[warp];
+    if (t.lc < 0) return;
+    const uint32_t items = kRest ? min(parked[0].x, (uint32_t)kParkedItems) : 0u;
+    for (long long w = (long long)blockIdx.x * kWarpsPerBlock + warp;; w += (long long)gridDim.x * kWarpsPerBlock) {
+    uint4 item = make_uint4((uint32_t)w, 0u, 1u, 0u);
+    if (kRest) {
+        if (w >= items) return;
+        item = parked[1 + w];
+        if (item.z == 0u) continue;
+    }
+    const long long first = (long long)item.x * G;
+    if (first >= nq) return;
     const int nslots = (int)min((long long)G, nq - first);
     const bool active = lane < nslots;
-    const unsigned lt = (1u << lane) - 1u;
     uint32_t qi = 0;
     F3 q = f3(0.0f);
     if (active) {
@@ -302,6 +328,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, MinBlocks)
     bool in = false;
     float4 glo, ghi;
 
+    bool park = kStage == 1 && t.lc > 0;
     int np = 0;
     unsigned n_acc = 0, n_tests = 0, n_chunks = 0, n_boxes = 0;
 
@@ -344,7 +371,8 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, MinBlocks)
     // lane j), then the photon tests chunk by chunk, the next chunk's photons loaded
     // while the current one's are tested; the queries of a chunk are tested two at a
     // time into a per-photon mask of accepting queries.
-    auto chunks = [&](unsigned bm, float4 blo, float4 bhi) {
+    // Returns the candidates it left (to park) because the warp's share of work was done.
+    auto chunks = [&](unsigned bm, float4 blo, float4 bhi) -> unsigned {
         uint32_t my_qm = 0;
         while (bm) {
             const int j = __ffs(bm) - 1;
@@ -357,13 +385,14 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, MinBlocks)
             if (lane == j) my_qm = qm;
         }
         unsigned cm = __ballot_sync(kFull, my_qm != 0u);
-        if (!cm) return;
+        if (!cm) return 0u;
         int j = __ffs(cm) - 1;
         uint32_t start = __shfl_sync(kFull, __float_as_uint(blo.w), j);
         uint32_t cnt = __shfl_sync(kFull, __float_as_uint(bhi.w), j);
         float4 pp = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         if ((uint32_t)lane < cnt) pp = __ldg(&t.pos[start + lane]);
         for (;;) {
+            if (kStage == 1 && park && n_chunks + n_acc / 8 >= kParkWork) return cm;
             const uint32_t qm = __shfl_sync(kFull, my_qm, j);
             cm &= cm - 1u;
             int jn = 0;
@@ -389,24 +418,39 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, MinBlocks)
             }
             if ((uint32_t)lane >= cnt) am = 0u;
             emit(am, start + (uint32_t)lane);
-            if (!cm) break;
+            if (!cm) return 0u;
             j = jn; start = sn; cnt = cn; pp = pn;
         }
     };
 
+    // Room for `add` parked items, from `at`; without it the items given below the end are
+    // void and the warp parks no more.
+    auto reserve_items = [&](uint32_t add) -> uint32_t {
+        uint32_t at = 0;
+        if (lane == 0) at = atomicAdd(&parked[0].x, add);
+        at = __shfl_sync(kFull, at, 0);
+        park = at + add <= (uint32_t)kParkedItems;
+        return at;
+    };
+    auto write_item = [&](uint32_t at, int a, int b, uint32_t root, uint32_t which) {
+        if (at < (uint32_t)kParkedItems)
+            parked[1 + at] = make_uint4(item.x, (uint32_t)a | ((uint32_t)b << 8), park ? root : 0u, which);
+    };
+
     const int lc = t.lc;
     const float4 rlo = __ldg(&t.lo[1]), rhi = __ldg(&t.hi[1]);
-    // Sub-groups.  Consecutive queries of the Morton order can straddle a jump of the
+    // Sub-groups.  Consecutive queries of the curve can straddle a jump of the
     // curve, and a group holding two distant clusters would walk every chunk between
     // them.  A range is therefore split at its largest gap between consecutive queries
     // when the two parts' boxes, grown by 4 radii, have less than half the surface of the
     // whole range's; the parts are traversed one after another.
     const float grow = 4.0f * sqrtf(r2);
-    int a = 0;
-    while (a < nslots) {
-        int b = nslots;
+    int a = kRest ? (int)(item.y & 255u) : 0;
+    const int end = kRest ? (int)(item.y >> 8) : nslots;
+    while (a < end) {
+        int b = end;
         warp_box(lane >= a && lane < b, q, glo, ghi);
-        while (b - a >= 4) {
+        while (!kRest && b - a >= 4) {
             const F3 qp = f3(__shfl_up_sync(kFull, q.x, 1), __shfl_up_sync(kFull, q.y, 1), __shfl_up_sync(kFull, q.z, 1));
             const float gap = (lane > a && lane < b) ? length_sq(q - qp) : -1.0f;
             const int c = warp_argmax(gap);
@@ -421,14 +465,21 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, MinBlocks)
         }
         in = lane >= a && lane < b;
         ++n_boxes;
-        if (!gap_outside(glo, ghi, rlo, rhi, r2)) {
+        if (kRest || !gap_outside(glo, ghi, rlo, rhi, r2)) {
         if (lc == 0) {
             chunks(1u, rlo, rhi);
         } else {
-            if (lane == 0) sm.stk[0] = 1u;
+            if (lane == 0) sm.stk[0] = item.z;
             __syncwarp();
             int sp = 1;
             while (sp > 0) {
+                if (kStage == 1 && park && n_chunks + n_acc / 8 >= kParkWork) {
+                    // this warp has done its share: the subtrees left, in kParkParts parts
+                    // each, to the second launch
+                    const uint32_t add = (uint32_t)sp * kParkParts, at = reserve_items(add);
+                    for (uint32_t i = lane; i < add; i += 32) write_item(at + i, a, b, sm.stk[i / kParkParts], i % kParkParts);
+                    if (park) break;
+                }
                 --sp;
                 const uint32_t e = sm.stk[sp];
                 __syncwarp();
@@ -441,12 +492,18 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, MinBlocks)
                 if ((uint32_t)lane < m) {
                     blo = __ldg(&t.lo[ce]);
                     bhi = __ldg(&t.hi[ce]);
-                    keep = !gap_outside(glo, ghi, blo, bhi, r2);
+                    keep = (!kRest || L + k < lc || ce % kParkParts == item.w) && !gap_outside(glo, ghi, blo, bhi, r2);
                 }
                 n_boxes += m;
                 const unsigned bm = __ballot_sync(kFull, keep);
                 if (L + k == lc) {
-                    chunks(bm, blo, bhi);
+                    unsigned left = chunks(bm, blo, bhi);
+                    while (kStage == 1 && left) {
+                        const uint32_t at = reserve_items((uint32_t)__popc(left));
+                        if ((left >> lane) & 1u) write_item(at + __popc(left & lt), a, b, ce, ce % kParkParts);
+                        if (park) break;
+                        left = chunks(left, blo, bhi);
+                    }
                 } else {
                     const int add = __popc(bm);
                     if (sp + add > kRootStack) {   // cannot happen (bound above); flagged, not silent
@@ -475,46 +532,63 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, MinBlocks)
         atomicAdd(&counters[2], (unsigned long long)n_chunks);
         atomicAdd(&counters[3], (unsigned long long)n_boxes);
     }
+    if (!kRest) return;
+    __syncwarp();
+    }
 }
 
 ChunkTree chunk_tree(const PhotonTree& tree, const float4* t0) {
     return ChunkTree{tree.box_lo, tree.box_hi, t0, photon_chunk_level(tree.n)};
 }
 
-// Launch shapes: (resident blocks per SM, queries per group, levels per expansion step).
-struct Shape { int mb, g, e; };
-constexpr Shape kShapes[] = {{2, 32, 5}, {3, 32, 5}, {4, 32, 5}, {3, 32, 4}, {4, 32, 4}, {3, 16, 5}, {4, 16, 4}, {4, 16, 5}};
-constexpr int kNumShapes = (int)(sizeof(kShapes) / sizeof(kShapes[0]));
+// Launch shapes: resident blocks per SM, queries per group, levels per expansion step, parking.
+constexpr int kNumShapes = 10;
 constexpr int kDefaultShape = 1;
 
-template <int MB, int G, int E, class Sink>
+int sm_count() {
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return std::max(sms, 1);
+}
+
+template <int MB, int G, int E, bool kPark, class Sink>
 void launch_shape(const ChunkTree& t, const float* qpos, int qstride, const uint32_t* order, long long nq,
                   const unsigned long long* nq_dev, const int* skip, float r2, const Sink& sink,
-                  unsigned long long* counters, int* err, cudaStream_t s) {
+                  uint4* parked, unsigned long long* counters, int* err, cudaStream_t s) {
     const long long warps = (nq + G - 1) / G;
-    k_gather<MB, G, E, Sink><<<(unsigned)((warps + kWarpsPerBlock - 1) / kWarpsPerBlock), 32 * kWarpsPerBlock, 0, s>>>(
-        t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, counters, err);
+    const unsigned blocks = (unsigned)((warps + kWarpsPerBlock - 1) / kWarpsPerBlock);
+    if (kPark) cudaMemsetAsync(parked, 0, sizeof(uint4), s);
+    k_gather<kPark ? 1 : 0, MB, G, E, Sink><<<blocks, 32 * kWarpsPerBlock, 0, s>>>(
+        t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, parked, counters, err);
+    if (kPark)
+        k_gather<2, MB, G, E, Sink><<<MB * sm_count(), 32 * kWarpsPerBlock, 0, s>>>(
+            t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, parked, counters, err);
 }
 
 template <class Sink>
 void launch_variant(int v, const ChunkTree& t, const float* qpos, int qstride, const uint32_t* order, long long nq,
                     const unsigned long long* nq_dev, const int* skip, float r2, const Sink& sink,
-                    unsigned long long* counters, int* err, cudaStream_t s) {
+                    uint4* parked, unsigned long long* counters, int* err, cudaStream_t s) {
     switch (v) {
-    case 0: launch_shape<2, 32, 5>(t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, counters, err, s); break;
-    case 2: launch_shape<4, 32, 5>(t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, counters, err, s); break;
-    case 3: launch_shape<3, 32, 4>(t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, counters, err, s); break;
-    case 4: launch_shape<4, 32, 4>(t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, counters, err, s); break;
-    case 5: launch_shape<3, 16, 5>(t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, counters, err, s); break;
-    case 6: launch_shape<4, 16, 4>(t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, counters, err, s); break;
-    case 7: launch_shape<4, 16, 5>(t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, counters, err, s); break;
-    default: launch_shape<3, 32, 5>(t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, counters, err, s); break;
+    case 0: launch_shape<2, 32, 5, false>(t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, parked, counters, err, s); break;
+    case 2: launch_shape<4, 32, 5, false>(t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, parked, counters, err, s); break;
+    case 3: launch_shape<3, 32, 4, false>(t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, parked, counters, err, s); break;
+    case 4: launch_shape<4, 32, 4, false>(t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, parked, counters, err, s); break;
+    case 5: launch_shape<3, 16, 5, false>(t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, parked, counters, err, s); break;
+    case 6: launch_shape<4, 16, 4, false>(t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, parked, counters, err, s); break;
+    case 7: launch_shape<4, 16, 5, false>(t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, parked, counters, err, s); break;
+    case 8: launch_shape<3, 16, 5, true>(t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, parked, counters, err, s); break;
+    case 9: launch_shape<3, 32, 5, true>(t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, parked, counters, err, s); break;
+    default: launch_shape<3, 32, 5, false>(t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, parked, counters, err, s); break;
     }
 }
 
 }  // namespace
 
+size_t gather_parked_bytes() { return sizeof(uint4) * (size_t)(1 + kParkedItems); }
 int gather_variants() { return kNumShapes; }
+bool gather_parks(int variant) { return variant >= 8 && variant < kNumShapes; }
 int gather_default_variant() { return kDefaultShape; }
 
 const char* gather_variant_name(int v) {
@@ -522,26 +596,27 @@ const char* gather_variant_name(int v) {
         "blocks/SM>=2, 32 queries/group, 5-level steps", "blocks/SM>=3, 32 queries/group, 5-level steps",
         "blocks/SM>=4, 32 queries/group, 5-level steps", "blocks/SM>=3, 32 queries/group, 4-level steps",
         "blocks/SM>=4, 32 queries/group, 4-level steps", "blocks/SM>=3, 16 queries/group, 5-level steps",
-        "blocks/SM>=4, 16 queries/group, 4-level steps", "blocks/SM>=4, 16 queries/group, 5-level steps"};
+        "blocks/SM>=4, 16 queries/group, 4-level steps", "blocks/SM>=4, 16 queries/group, 5-level steps",
+        "blocks/SM>=3, 16 queries/group, 5-level steps, parking", "blocks/SM>=3, 32 queries/group, 5-level steps, parking"};
     return (v >= 0 && v < kNumShapes) ? names[v] : "?";
 }
 
 void launch_gather(const VMParams& p, const PhotonTree& tree, TreePhotons tp, QueryBuf qb, const uint32_t* order,
-                   long long nq, double* accum, unsigned long long* counters, cudaStream_t s, int variant,
-                   const unsigned long long* nq_dev, const int* skip) {
+                   long long nq, double* accum, void* parked, unsigned long long* counters, cudaStream_t s,
+                   int variant, const unsigned long long* nq_dev, const int* skip) {
     if (nq <= 0 || tree.n <= 0) return;
     const EvalSink sink{p, qb, tp, tree.id, accum};
     launch_variant(variant, chunk_tree(tree, tp.t0), reinterpret_cast<const float*>(qb.q0), 4, order, nq, nq_dev,
-                   skip, p.radius_sqr, sink, counters, p.error + ERR_GATHER, s);
+                   skip, p.radius_sqr, sink, static_cast<uint4*>(parked), counters, p.error + ERR_GATHER, s);
 }
 
 void launch_gather_sets(const PhotonTree& tree, const float4* t0, const float* qpos, int qstride, const uint32_t* order,
                         long long nq, float r2, int* counts, const long long* offsets, int* cursor, int* idx,
-                        int variant, unsigned long long* counters, int* err, cudaStream_t s) {
+                        int variant, void* parked, unsigned long long* counters, int* err, cudaStream_t s) {
     if (nq <= 0 || tree.n <= 0) return;
     const SetSink sink{tree.id, counts, offsets, cursor, idx};
-    launch_variant(variant, chunk_tree(tree, t0), qpos, qstride, order, nq, nullptr, nullptr, r2, sink, counters, err,
-                   s);
+    launch_variant(variant, chunk_tree(tree, t0), qpos, qstride, order, nq, nullptr, nullptr, r2, sink,
+                   static_cast<uint4*>(parked), counters, err, s);
 }
 
 }  // namespace rc

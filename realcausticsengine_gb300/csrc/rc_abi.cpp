@@ -84,6 +84,7 @@ struct DeviceState {
     DevBuf<float2> tp2;
     DevBuf<uint32_t> qorder;
     DevBuf<unsigned char> qscratch;
+    DevBuf<unsigned char> gather_parked;    // launch_gather's scratch
     DevBuf<double> accum;
     DevBuf<float> image;          // FP32 mean for readback
     // light-path processing order (launch_light_order) and its scratch
@@ -124,7 +125,7 @@ struct DeviceState {
         world_mesh.release(); mesh_root.release(); lights.release(); cdf.release(); materials.release();
         ph_tp.release(); ph_path.release(); counters.release(); errors.release();
         ph_order.release(); ph_scratch.release();
-        tp0.release(); tp1.release(); tp2.release(); qorder.release(); qscratch.release();
+        tp0.release(); tp1.release(); tp2.release(); qorder.release(); qscratch.release(); gather_parked.release();
         box_lo.release(); box_hi.release();
         accum.release();
         image.release();
@@ -156,17 +157,18 @@ struct DeviceState {
 };
 
 // Autotuner choices: launch variant per size class (log2 of light paths or pixels, and of
-// the scene's triangles; log2 of queries), -1 = untuned.  Kept for the process and shared
-// by every context (a new scene, or a scene in another context, reuses them).  The
-// triangles are in the key because the light and camera passes' best shape depends on how
+// the scene's triangles; log2 of queries and of photons), -1 = untuned.  Kept for the
+// process and shared by every context (a new scene, or a scene in another context, reuses
+// them).  The triangles are in the key because the light and camera passes' best shape depends on how
 // long a search is: at 4.2M light paths 2,000 gems (261k triangles) run 20.7 ms staged
-// against 35.4, at 1M a glass sphere (20k) 0.53 ms staged against 0.38.
+// against 35.4, at 1M a glass sphere (20k) 0.53 ms staged against 0.38.  The photons are in
+// the gather's because they tell a caustic's focus from a wide floor: 216k queries take 120
+// us parked against 783 with 20k photons of one; without one parking only costs.
 struct TuneTables {
-    std::atomic<int> light[64][32], camera[64][32], gather[64];
+    std::atomic<int> light[64][32], camera[64][32], gather[64][32];
     TuneTables() {
         for (int i = 0; i < 64; ++i) {
-            gather[i] = -1;
-            for (int j = 0; j < 32; ++j) { light[i][j] = -1; camera[i][j] = -1; }
+            for (int j = 0; j < 32; ++j) { light[i][j] = -1; camera[i][j] = -1; gather[i][j] = -1; }
         }
     }
 };
@@ -453,6 +455,7 @@ int reserve_photon_tree(long long n) {
     const size_t m = (size_t)std::max<long long>(n, 1), boxes = (size_t)2 << std::max(photon_chunk_level(n), 0);
     RC_CUDA(d.ph_order.reserve(m));
     RC_CUDA(d.ph_scratch.reserve(order_scratch_bytes(n)));
+    RC_CUDA(d.gather_parked.reserve(gather_parked_bytes()));
     RC_CUDA(d.tp0.reserve(m)); RC_CUDA(d.tp1.reserve(m)); RC_CUDA(d.tp2.reserve(m));
     RC_CUDA(d.box_lo.reserve(boxes)); RC_CUDA(d.box_hi.reserve(boxes));
     return RC_OK;
@@ -632,6 +635,9 @@ std::atomic<int>& light_slot(long long paths) {
 }
 std::atomic<int>& camera_slot(long long pixels) {
     return g_tune.camera[size_class(pixels)][std::min(size_class(ctx().dev.num_tris), 31)];
+}
+std::atomic<int>& gather_slot(long long queries, long long photons) {
+    return g_tune.gather[size_class(queries)][std::min(size_class(photons), 31)];
 }
 constexpr int kUntunedPass = 2;   // the light and camera passes' shape where nothing was timed
 
@@ -960,34 +966,34 @@ int render_iteration(HostScene& sc, int redo_iteration = -1, bool tune_passes = 
                        d.qorder.p, &qlaunch, s);
     int variant = gather_default_variant();
     if (cfg().autotune && nq > 0) {
-        const int cls = 63 - __builtin_clzll((unsigned long long)nq);
-        if (g_tune.gather[cls].load() < 0) {
+        std::atomic<int>& slot = gather_slot((long long)nq, n);
+        if (slot.load() < 0) {
             // time every launch shape on this iteration's queries into a scratch image
             // (warm-up launch first: the first launch of a shape loads its code)
             RC_CUDA(d.tune_accum.reserve(std::max<long long>(3 * npix, 1)));
             float best = 1e30f;
             int best_v = variant;
             for (int v = 0; v < gather_variants(); ++v) {
-                launch_gather(p, tree, tph, qb, d.qorder.p, (long long)nq, d.tune_accum.p, nullptr, s, v);
+                launch_gather(p, tree, tph, qb, d.qorder.p, (long long)nq, d.tune_accum.p, d.gather_parked.p, nullptr, s, v);
                 RC_CUDA(cudaEventRecord(d.evm[0], s));
-                launch_gather(p, tree, tph, qb, d.qorder.p, (long long)nq, d.tune_accum.p, nullptr, s, v);
+                launch_gather(p, tree, tph, qb, d.qorder.p, (long long)nq, d.tune_accum.p, d.gather_parked.p, nullptr, s, v);
                 RC_CUDA(cudaEventRecord(d.evm[1], s));
                 RC_CUDA(cudaEventSynchronize(d.evm[1]));
                 const float ms = ms_between(d.evm[0], d.evm[1]);
                 if (cfg().verbose) std::printf("{\"gather_shape\": %d, \"ms\": %.4f}\n", v, ms);
                 if (ms < best) { best = ms; best_v = v; }
             }
-            g_tune.gather[cls] = best_v;
+            slot = best_v;
             if (cfg().verbose)
                 std::printf("{\"autotune\": \"gather\", \"queries\": %llu, \"variant\": \"%s\", \"ms\": %.3f}\n",
                             nq, gather_variant_name(best_v), best);
         }
-        variant = g_tune.gather[cls].load();
+        variant = slot.load();
     }
     unsigned long long gc[4] = {0, 0, 0, 0};
     RC_CUDA(cudaMemsetAsync(d.counters.p + 2, 0, 4 * sizeof(unsigned long long), s));
     RC_CUDA(cudaEventRecord(d.evg[0], s));
-    launch_gather(p, tree, tph, qb, d.qorder.p, (long long)nq, d.accum.p, d.counters.p + 2, s, variant);
+    launch_gather(p, tree, tph, qb, d.qorder.p, (long long)nq, d.accum.p, d.gather_parked.p, d.counters.p + 2, s, variant);
     RC_CUDA(cudaEventRecord(d.evg[1], s));
     RC_CUDA(cudaGetLastError());
     RC_CUDA(cudaEventRecord(d.ev[7], s));
@@ -1026,7 +1032,7 @@ int render_iteration(HostScene& sc, int redo_iteration = -1, bool tune_passes = 
     st[10] = d.iterations_done;
     st[11] = sc.scene_radius;
     st[12] = std::sqrt(p.radius_sqr);
-    st[13] = order_launches + 3 + qlaunch;
+    st[13] = order_launches + (gather_parks(variant) ? 4 : 3) + qlaunch;
     d.acc_gather_ms += ms_between(d.evg[0], d.evg[1]);   // the gather kernel alone
     // gather algorithmic bytes: each photon record read once (40 B), each query record
     // read once (64 B), each pixel's FP64 RGB sum read and written once (48 B)
@@ -1088,7 +1094,7 @@ int async_setup(const HostScene& sc) {
     auto var = [](int v, int dflt) { return v >= 0 ? v : dflt; };
     d.async_lvar = var(light_slot(cfg().photons_per_iter > 0 ? cfg().photons_per_iter : npix).load(), kUntunedPass);
     d.async_cvar = var(camera_slot(npix).load(), kUntunedPass);
-    d.async_gvar = var(g_tune.gather[size_class((long long)d.last_queries)].load(), gather_default_variant());
+    d.async_gvar = var(gather_slot((long long)d.last_queries, (long long)d.last_photons).load(), gather_default_variant());
     if (!cfg().autotune) d.async_lvar = d.async_cvar = 0, d.async_gvar = gather_default_variant();
     // the staged passes' scratch: reserved before any capture
     const long long paths = cfg().photons_per_iter > 0 ? cfg().photons_per_iter : npix;
@@ -1145,8 +1151,8 @@ int async_tail(HostScene& sc, const VMParams& p, cudaStream_t s, cudaStream_t si
     RC_CUDA(record(d.ev[6], s));
     RC_CUDA(cudaMemsetAsync(d.counters.p + 2, 0, 4 * sizeof(unsigned long long), s));
     RC_CUDA(record(d.evg[0], s));
-    launch_gather(p, tree, tph, qb, d.qorder.p, qc, d.accum.p, d.counters.p + 2, s, d.async_gvar, d.counters.p + 1,
-                  flag);
+    launch_gather(p, tree, tph, qb, d.qorder.p, qc, d.accum.p, d.gather_parked.p, d.counters.p + 2, s, d.async_gvar,
+                  d.counters.p + 1, flag);
     RC_CUDA(record(d.evg[1], s));
     RC_CUDA(record(d.ev[7], s));
     return RC_OK;
@@ -2437,7 +2443,7 @@ int rc_gather_query(int variant, int n, const float* positions, int q, const flo
     cudaStream_t s = nullptr;
     RC_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
     DevBuf<float4> pos, boxes, t0; DevBuf<float> qp; DevBuf<uint32_t> id, ord;
-    DevBuf<unsigned char> scratch, osc; DevBuf<int> cnt, cur, out, err; DevBuf<long long> off;
+    DevBuf<unsigned char> scratch, osc, parked; DevBuf<int> cnt, cur, out, err; DevBuf<long long> off;
     PhotonTree tree;
     int r = upload_positions(n, positions, pos, s);
     if (!r) r = [&]() -> int {
@@ -2454,14 +2460,14 @@ int rc_gather_query(int variant, int n, const float* positions, int q, const flo
     if (!r && q > 0) {
         r = [&]() -> int {
             RC_CUDA(qp.reserve(3 * (size_t)q)); RC_CUDA(cnt.reserve(q)); RC_CUDA(cur.reserve(q)); RC_CUDA(off.reserve(q));
-            RC_CUDA(err.reserve(1)); RC_CUDA(ord.reserve(q));
+            RC_CUDA(err.reserve(1)); RC_CUDA(ord.reserve(q)); RC_CUDA(parked.reserve(gather_parked_bytes()));
             RC_CUDA(osc.reserve(order_scratch_bytes(q)));
             RC_CUDA(cudaMemcpyAsync(qp.p, queries, 12 * (size_t)q, cudaMemcpyHostToDevice, s));
             RC_CUDA(cudaMemsetAsync(cnt.p, 0, 4 * (size_t)q, s));
             RC_CUDA(cudaMemsetAsync(err.p, 0, sizeof(int), s));
             launch_query_order(qp.p, 3, q, points_frame(q, queries, r2), osc.p, ord.p, nullptr, s);
-            launch_gather_sets(tree, t0.p, qp.p, 3, ord.p, q, r2, cnt.p, nullptr, nullptr, nullptr, variant, nullptr,
-                               err.p, s);
+            launch_gather_sets(tree, t0.p, qp.p, 3, ord.p, q, r2, cnt.p, nullptr, nullptr, nullptr, variant, parked.p,
+                               nullptr, err.p, s);
             RC_CUDA(cudaGetLastError());
             int h = 0;
             RC_CUDA(cudaMemcpyAsync(counts, cnt.p, 4 * (size_t)q, cudaMemcpyDeviceToHost, s));
@@ -2476,8 +2482,8 @@ int rc_gather_query(int variant, int n, const float* positions, int q, const flo
                 RC_CUDA(out.reserve(t));
                 RC_CUDA(cudaMemcpyAsync(off.p, offs.data(), 8 * (size_t)q, cudaMemcpyHostToDevice, s));
                 RC_CUDA(cudaMemsetAsync(cur.p, 0, 4 * (size_t)q, s));
-                launch_gather_sets(tree, t0.p, qp.p, 3, ord.p, q, r2, nullptr, off.p, cur.p, out.p, variant, nullptr,
-                                   err.p, s);
+                launch_gather_sets(tree, t0.p, qp.p, 3, ord.p, q, r2, nullptr, off.p, cur.p, out.p, variant, parked.p,
+                                   nullptr, err.p, s);
                 RC_CUDA(cudaGetLastError());
                 RC_CUDA(cudaMemcpyAsync(idx, out.p, 4 * (size_t)t, cudaMemcpyDeviceToHost, s));
                 RC_CUDA(cudaStreamSynchronize(s));
@@ -2487,7 +2493,7 @@ int rc_gather_query(int variant, int n, const float* positions, int q, const flo
     }
     pos.release(); id.release(); scratch.release();
     cnt.release(); cur.release(); out.release(); off.release(); qp.release(); ord.release(); osc.release();
-    boxes.release(); t0.release(); err.release();
+    boxes.release(); t0.release(); err.release(); parked.release();
     cudaStreamDestroy(s);
     return r;
 }

@@ -75,3 +75,21 @@ def test_spatial_order_finds_every_photon(n, radius):
         inside = (d[:, 0] * d[:, 0] + d[:, 1] * d[:, 1]) + d[:, 2] * d[:, 2] < r2
         assert counts[j] == inside.sum()
         assert (np.sort(sets[j]) == np.nonzero(inside)[0]).all()
+
+
+@pytest.mark.parametrize("n,q", [(1, 40), (33, 400), (2011, 333), (3001, 4001)])
+def test_parking_gather_finds_every_photon(n, q):
+    """Every query's sphere holds most photons, so every warp parks (no subtrees with one
+    chunk, chunks only, whole subtrees, and more items than the list holds)."""
+    rng = np.random.default_rng(q)
+    p = rng.normal(scale=0.5, size=(n, 3)).astype(np.float32)
+    at = rng.normal(scale=0.1, size=(q, 3)).astype(np.float32)
+    want, sets = kd_query(p, at, 1.0, variant=0)
+    for j in range(0, q, 97):
+        d = at[j] - p
+        inside = (d[:, 0] * d[:, 0] + d[:, 1] * d[:, 1]) + d[:, 2] * d[:, 2] < np.float32(1.0)
+        assert (np.sort(sets[j]) == np.nonzero(inside)[0]).all()
+    for variant in (8, 9):
+        counts, got = kd_query(p, at, 1.0, variant=variant)
+        assert (counts == want).all()
+        assert all((np.sort(a) == np.sort(b)).all() for a, b in zip(got, sets))
