@@ -22,11 +22,13 @@
 //   finishes second computes the parent (per-node arrival counter; nothing waits).
 //
 // Work split.  Segments of more than kSmall (256) triangles go through level passes
-// over 2048-triangle chunks (bounds, bins, decision, partition, swap); smaller segments
-// are finished by one warp each, depth first, with the pending right halves on a stack
-// kept in the segment's own slice of a global array.  (A warp walks its subtree node by
-// node at L2 latency, so the per-warp size is kept small enough for thousands of warps
-// to share the subtrees.)
+// over 2048-triangle chunks (bounds, bins, decision, partition, swap).  A smaller segment
+// is taken by one warp, depth first, with the pending right halves on a stack kept in the
+// segment's own slice of a global array, down to ranges of at most kTiny (32) triangles:
+// those are the subtrees of a second launch, a warp each, one triangle per lane.  A warp
+// that walks a whole segment reads its triangles three times per node at L2 latency, 5 us a
+// node, and nearly all nodes are below 32 triangles: 100k triangles took 1721 us that way,
+// now 79 down to the small ranges and 110 below (kSmall 128, 512 and 1024 are no faster).
 #include "bvh_build.h"
 
 #include <algorithm>
@@ -40,6 +42,7 @@ namespace {
 
 constexpr int kBins = 12;
 constexpr int kSmall = 256;
+constexpr int kTiny = 32;
 constexpr int kChunk = 2048;
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
@@ -190,7 +193,7 @@ struct View {
     uint32_t* tf; int* pf;   // failing elements left of the split: triangle, position (by rank)
     uint32_t* tt; int* pt;   // passing elements right of the split: triangle, position (by rank)
     int4* stack;
-    NodeRec* small_pool;
+    NodeRec* small_pool;     // of the ranges below kSmall: a leaf at 2 start, a split at 2 mid - 1
     NodeRec* large_pool;
     int* large_count;
     int large_cap;
@@ -199,6 +202,8 @@ struct View {
     int* flags;
     int n;
     int next_cap, small_cap;   // capacities of the next-level and per-warp segment lists
+    int4* tiny;                // ranges of at most kTiny triangles (at most one per triangle)
+    int* tiny_count;
 };
 
 __device__ __forceinline__ void record_node(NodeRec* rec, const Keys12& k, int start, int depth, int count, int mid,
@@ -573,16 +578,26 @@ __global__ void __launch_bounds__(kThreads) k_lvl_swap(SegState* st, const int2*
 
 // ---- one warp per segment of at most kSmall triangles -------------------------------
 
+__device__ __forceinline__ NodeRec* small_record(const View& V, int a, int mid) {
+    return V.small_pool + (mid < 0 ? 2 * (size_t)a : 2 * (size_t)mid - 1);
+}
+
 __global__ void __launch_bounds__(kThreads) k_small_build(const int4* segs, const int* nsegs, View V) {
     const int lane = threadIdx.x & 31;
     const int nw = gridDim.x * kWarps;
     const int count = *nsegs;
-    for (int w = blockIdx.x * kWarps + (threadIdx.x >> 5); w < count; w += nw) {
+    auto push_tiny = [&](int a, int b, int depth) {
+        if (lane != 0) return;
+        const int i = atomicAdd(V.tiny_count, 1);
+        if (i < V.n) V.tiny[i] = make_int4(a, b, depth, 0);
+        else atomicOr(V.flags, kFlagIndex);
+    };
+    for (int w = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; w < count; w += nw) {   // spread over the SMs
         const int4 sg = segs[w];
         const int s0 = sg.x, e0 = sg.y;
-        NodeRec* pool = V.small_pool + 2 * (size_t)s0;
+        if (e0 - s0 <= kTiny) { push_tiny(s0, e0, sg.z); continue; }
         int4* stack = V.stack + s0;
-        int sp = 0, slot = 0;
+        int sp = 0;
         int a = sg.x, b = sg.y, depth = sg.z;
         bool bad = false;
         while (true) {
@@ -595,104 +610,99 @@ __global__ void __launch_bounds__(kThreads) k_small_build(const int4* segs, cons
             }
             keys_warp_reduce(k);
             int split_mid = -1;
-            if (n > 1) {
-                float clo, chi;
-                const int dim = keys_split_axis(k, clo, chi);
-                if (clo != chi) {
-                    if (n == 2) {
-                        // two triangles: ordered by centroid (src/BVH/BVH_mesh.cpp:80-88)
-                        if (lane == 0) {
-                            const uint32_t t0 = V.perm[a], t1 = V.perm[a + 1];
-                            const float c0 = comp(centroid(V.blo[t0], V.bhi[t0]), dim);
-                            const float c1 = comp(centroid(V.blo[t1], V.bhi[t1]), dim);
-                            if (!(c0 < c1)) { V.perm[a] = t1; V.perm[a + 1] = t0; }
+            float clo, chi;
+            const int dim = keys_split_axis(k, clo, chi);
+            if (clo != chi) {
+                int bc = 0;
+                uint32_t bk[6] = {kKeyPosInf, kKeyPosInf, kKeyPosInf, kKeyNegInf, kKeyNegInf, kKeyNegInf};
+                for (int base = a; base < b; base += 32) {
+                    const int i = base + lane;
+                    const bool valid = i < b;
+                    float4 lo = make_float4(0, 0, 0, 0), hi = lo;
+                    int bkt = 0;
+                    if (valid) {
+                        const uint32_t t = V.perm[i];
+                        lo = V.blo[t];
+                        hi = V.bhi[t];
+                        bkt = bucket_of(comp(centroid(lo, hi), dim), clo, chi);
+                    }
+                    unsigned pending = __ballot_sync(kFull, valid);
+                    while (pending) {
+                        const int leader = __ffs(pending) - 1;
+                        const int bl = __shfl_sync(kFull, bkt, leader);
+                        const bool in = valid && bkt == bl;
+                        const unsigned m = __ballot_sync(kFull, in);
+                        const uint32_t r0 = __reduce_min_sync(kFull, in ? fkey(lo.x) : kKeyPosInf);
+                        const uint32_t r1 = __reduce_min_sync(kFull, in ? fkey(lo.y) : kKeyPosInf);
+                        const uint32_t r2 = __reduce_min_sync(kFull, in ? fkey(lo.z) : kKeyPosInf);
+                        const uint32_t r3 = __reduce_max_sync(kFull, in ? fkey(hi.x) : kKeyNegInf);
+                        const uint32_t r4 = __reduce_max_sync(kFull, in ? fkey(hi.y) : kKeyNegInf);
+                        const uint32_t r5 = __reduce_max_sync(kFull, in ? fkey(hi.z) : kKeyNegInf);
+                        if (lane == bl) {
+                            bc += __popc(m);
+                            bk[0] = min(bk[0], r0); bk[1] = min(bk[1], r1); bk[2] = min(bk[2], r2);
+                            bk[3] = max(bk[3], r3); bk[4] = max(bk[4], r4); bk[5] = max(bk[5], r5);
                         }
-                        __syncwarp();
-                        split_mid = a + 1;
-                    } else {
-                        int bc = 0;
-                        uint32_t bk[6] = {kKeyPosInf, kKeyPosInf, kKeyPosInf, kKeyNegInf, kKeyNegInf, kKeyNegInf};
-                        for (int base = a; base < b; base += 32) {
-                            const int i = base + lane;
-                            const bool valid = i < b;
-                            float4 lo = make_float4(0, 0, 0, 0), hi = lo;
-                            int bkt = 0;
-                            if (valid) {
-                                const uint32_t t = V.perm[i];
-                                lo = V.blo[t];
-                                hi = V.bhi[t];
-                                bkt = bucket_of(comp(centroid(lo, hi), dim), clo, chi);
-                            }
-                            unsigned pending = __ballot_sync(kFull, valid);
-                            while (pending) {
-                                const int leader = __ffs(pending) - 1;
-                                const int bl = __shfl_sync(kFull, bkt, leader);
-                                const bool in = valid && bkt == bl;
-                                const unsigned m = __ballot_sync(kFull, in);
-                                const uint32_t r0 = __reduce_min_sync(kFull, in ? fkey(lo.x) : kKeyPosInf);
-                                const uint32_t r1 = __reduce_min_sync(kFull, in ? fkey(lo.y) : kKeyPosInf);
-                                const uint32_t r2 = __reduce_min_sync(kFull, in ? fkey(lo.z) : kKeyPosInf);
-                                const uint32_t r3 = __reduce_max_sync(kFull, in ? fkey(hi.x) : kKeyNegInf);
-                                const uint32_t r4 = __reduce_max_sync(kFull, in ? fkey(hi.y) : kKeyNegInf);
-                                const uint32_t r5 = __reduce_max_sync(kFull, in ? fkey(hi.z) : kKeyNegInf);
-                                if (lane == bl) {
-                                    bc += __popc(m);
-                                    bk[0] = min(bk[0], r0); bk[1] = min(bk[1], r1); bk[2] = min(bk[2], r2);
-                                    bk[3] = max(bk[3], r3); bk[4] = max(bk[4], r4); bk[5] = max(bk[5], r5);
-                                }
-                                pending &= ~m;
-                            }
-                        }
-                        int mb = warp_choose_split(bc, bk, keys_box_area(k), n, lane);
-                        const int T = __reduce_add_sync(kFull, (mb >= 0 && lane <= mb) ? bc : 0);
-                        if (mb >= 0 && (T <= 0 || T >= n)) { bad = true; mb = -1; }
-                        if (mb >= 0) {
-                            const int m = a + T;
-                            int run = 0, kfl = 0;
-                            for (int base = a; base < b; base += 32) {
-                                const int i = base + lane;
-                                const bool valid = i < b;
-                                uint32_t t = 0;
-                                bool pred = false;
-                                if (valid) {
-                                    t = V.perm[i];
-                                    pred = bucket_of(comp(centroid(V.blo[t], V.bhi[t]), dim), clo, chi) <= mb;
-                                }
-                                const unsigned bt = __ballot_sync(kFull, pred);
-                                const int true_rank = run + __popc(bt & ((1u << lane) - 1u));
-                                const bool left_fail = valid && i < m && !pred;
-                                if (left_fail) {
-                                    const int kk = (i - a) - true_rank;
-                                    if (kk >= 0 && kk < n) { V.tf[a + kk] = t; V.pf[a + kk] = i; }
-                                    else bad = true;
-                                }
-                                if (valid && i >= m && pred) {
-                                    const int kk = T - 1 - true_rank;
-                                    if (kk >= 0 && kk < n) { V.tt[a + kk] = t; V.pt[a + kk] = i; }
-                                    else bad = true;
-                                }
-                                kfl += __popc(__ballot_sync(kFull, left_fail));
-                                run += __popc(bt);
-                            }
-                            __syncwarp();
-                            for (int kk = lane; kk < kfl && kk < n; kk += 32) {
-                                const int pf = V.pf[a + kk], pt = V.pt[a + kk];
-                                if (pf < a || pf >= b || pt < a || pt >= b) { bad = true; continue; }
-                                V.perm[pf] = V.tt[a + kk];
-                                V.perm[pt] = V.tf[a + kk];
-                            }
-                            __syncwarp();
-                            split_mid = m;
-                        }
+                        pending &= ~m;
                     }
                 }
+                int mb = warp_choose_split(bc, bk, keys_box_area(k), n, lane);
+                const int T = __reduce_add_sync(kFull, (mb >= 0 && lane <= mb) ? bc : 0);
+                if (mb >= 0 && (T <= 0 || T >= n)) { bad = true; mb = -1; }
+                if (mb >= 0) {
+                    const int m = a + T;
+                    int run = 0, kfl = 0;
+                    for (int base = a; base < b; base += 32) {
+                        const int i = base + lane;
+                        const bool valid = i < b;
+                        uint32_t t = 0;
+                        bool pred = false;
+                        if (valid) {
+                            t = V.perm[i];
+                            pred = bucket_of(comp(centroid(V.blo[t], V.bhi[t]), dim), clo, chi) <= mb;
+                        }
+                        const unsigned bt = __ballot_sync(kFull, pred);
+                        const int true_rank = run + __popc(bt & ((1u << lane) - 1u));
+                        const bool left_fail = valid && i < m && !pred;
+                        if (left_fail) {
+                            const int kk = (i - a) - true_rank;
+                            if (kk >= 0 && kk < n) { V.tf[a + kk] = t; V.pf[a + kk] = i; }
+                            else bad = true;
+                        }
+                        if (valid && i >= m && pred) {
+                            const int kk = T - 1 - true_rank;
+                            if (kk >= 0 && kk < n) { V.tt[a + kk] = t; V.pt[a + kk] = i; }
+                            else bad = true;
+                        }
+                        kfl += __popc(__ballot_sync(kFull, left_fail));
+                        run += __popc(bt);
+                    }
+                    __syncwarp();
+                    for (int kk = lane; kk < kfl && kk < n; kk += 32) {
+                        const int pf = V.pf[a + kk], pt = V.pt[a + kk];
+                        if (pf < a || pf >= b || pt < a || pt >= b) { bad = true; continue; }
+                        V.perm[pf] = V.tt[a + kk];
+                        V.perm[pt] = V.tf[a + kk];
+                    }
+                    __syncwarp();
+                    split_mid = m;
+                }
             }
-            if (slot >= 2 * (e0 - s0) || (split_mid >= 0 && sp >= e0 - s0)) { bad = true; break; }
-            if (lane == 0) record_node(pool + slot, k, a, depth, split_mid < 0 ? n : -1, split_mid, V.cnt, V.topd);
-            ++slot;
+            if (split_mid >= 0 && sp >= e0 - s0) { bad = true; break; }
+            if (lane == 0)
+                record_node(small_record(V, a, split_mid), k, a, depth, split_mid < 0 ? n : -1, split_mid, V.cnt, V.topd);
+            bool descend = false;
             if (split_mid >= 0) {
-                if (lane == 0) stack[sp] = make_int4(split_mid, b, depth + 1, 0);
-                ++sp;
+                if (b - split_mid > kTiny) {
+                    if (lane == 0) stack[sp] = make_int4(split_mid, b, depth + 1, 0);
+                    ++sp;
+                } else {
+                    push_tiny(split_mid, b, depth + 1);
+                }
+                descend = split_mid - a > kTiny;
+                if (!descend) push_tiny(a, split_mid, depth + 1);
+            }
+            if (descend) {
                 b = split_mid;
                 depth += 1;
             } else {
@@ -704,6 +714,121 @@ __global__ void __launch_bounds__(kThreads) k_small_build(const int4* segs, cons
             }
         }
         if (__any_sync(kFull, bad) && lane == 0) atomicOr(V.flags, kFlagIndex);
+    }
+}
+
+// One warp per range of at most kTiny triangles, triangle i of the range in lane i.
+__global__ void __launch_bounds__(kThreads) k_tiny_build(View V) {
+    __shared__ int s_stack[kWarps][kTiny];     // pending right halves: first | end << 8 | depth << 16
+    __shared__ uint8_t s_lf[kWarps][kTiny], s_rt[kWarps][kTiny];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned lt = (1u << lane) - 1u;
+    const int count = min(*V.tiny_count, V.n);
+    int* const stack = s_stack[warp];
+    for (int w = warp * gridDim.x + blockIdx.x; w < count; w += gridDim.x * kWarps) {
+        const int4 sg = V.tiny[w];
+        const int s0 = sg.x, total = sg.y - sg.x;
+        uint32_t t = 0;
+        float4 lo = make_float4(0, 0, 0, 0), hi = lo;
+        if (lane < total) {
+            t = V.perm[s0 + lane];
+            lo = V.blo[t];
+            hi = V.bhi[t];
+        }
+        int sp = 0, a = 0, b = total, depth = 0;
+        bool bad = false;
+        while (true) {
+            const int n = b - a;
+            const bool in = lane >= a && lane < b;
+            int mid = -1;
+            if (n == 1) {
+                if (lane == a) {
+                    Keys12 k;
+                    keys_init(k);
+                    keys_add(k, lo, hi);
+                    record_node(small_record(V, s0 + a, -1), k, s0 + a, sg.z + depth, 1, -1, V.cnt, V.topd);
+                }
+            } else {
+                Keys12 k;
+                keys_init(k);
+                if (in) keys_add(k, lo, hi);
+                keys_warp_reduce(k);
+                float clo, chi;
+                const int dim = keys_split_axis(k, clo, chi);
+                int from = lane;   // the lane whose triangle this one takes
+                if (clo != chi) {
+                    const float c = comp(centroid(lo, hi), dim);
+                    if (n == 2) {
+                        // two triangles: ordered by centroid (src/BVH/BVH_mesh.cpp:80-88)
+                        const float c0 = __shfl_sync(kFull, c, a), c1 = __shfl_sync(kFull, c, a + 1);
+                        if (in && !(c0 < c1)) from = lane == a ? a + 1 : a;
+                        mid = a + 1;
+                    } else {
+                        const int bkt = in ? bucket_of(c, clo, chi) : 0;
+                        int bc = 0;
+                        uint32_t bk[6] = {kKeyPosInf, kKeyPosInf, kKeyPosInf, kKeyNegInf, kKeyNegInf, kKeyNegInf};
+                        unsigned pending = __ballot_sync(kFull, in);
+                        while (pending) {
+                            const int bl = __shfl_sync(kFull, bkt, __ffs(pending) - 1);
+                            const bool mine = in && bkt == bl;
+                            const unsigned m = __ballot_sync(kFull, mine);
+                            const uint32_t r0 = __reduce_min_sync(kFull, mine ? fkey(lo.x) : kKeyPosInf);
+                            const uint32_t r1 = __reduce_min_sync(kFull, mine ? fkey(lo.y) : kKeyPosInf);
+                            const uint32_t r2 = __reduce_min_sync(kFull, mine ? fkey(lo.z) : kKeyPosInf);
+                            const uint32_t r3 = __reduce_max_sync(kFull, mine ? fkey(hi.x) : kKeyNegInf);
+                            const uint32_t r4 = __reduce_max_sync(kFull, mine ? fkey(hi.y) : kKeyNegInf);
+                            const uint32_t r5 = __reduce_max_sync(kFull, mine ? fkey(hi.z) : kKeyNegInf);
+                            if (lane == bl) {
+                                bc = __popc(m);
+                                bk[0] = r0; bk[1] = r1; bk[2] = r2; bk[3] = r3; bk[4] = r4; bk[5] = r5;
+                            }
+                            pending &= ~m;
+                        }
+                        int mb = warp_choose_split(bc, bk, keys_box_area(k), n, lane);
+                        const int T = __reduce_add_sync(kFull, (mb >= 0 && lane <= mb) ? bc : 0);
+                        if (mb >= 0 && (T <= 0 || T >= n)) { bad = true; mb = -1; }
+                        if (mb >= 0) {
+                            // std::partition's swaps: the k-th failing triangle of the left part with
+                            // the k-th passing one from the end of the right part
+                            mid = a + T;
+                            const bool pred = in && bkt <= mb;
+                            const unsigned lf = __ballot_sync(kFull, in && lane < mid && !pred);
+                            const unsigned rt = __ballot_sync(kFull, pred && lane >= mid);
+                            if ((lf >> lane) & 1u) s_lf[warp][__popc(lf & lt)] = (uint8_t)lane;
+                            if ((rt >> lane) & 1u) s_rt[warp][__popc(rt & ~lt) - 1] = (uint8_t)lane;
+                            __syncwarp();
+                            if (__popc(lf) != __popc(rt)) bad = true;
+                            else if ((lf >> lane) & 1u) from = s_rt[warp][__popc(lf & lt)];
+                            else if ((rt >> lane) & 1u) from = s_lf[warp][__popc(rt & ~lt) - 1];
+                            __syncwarp();
+                        }
+                    }
+                    t = __shfl_sync(kFull, t, from);
+                    lo.x = __shfl_sync(kFull, lo.x, from); lo.y = __shfl_sync(kFull, lo.y, from);
+                    lo.z = __shfl_sync(kFull, lo.z, from); hi.x = __shfl_sync(kFull, hi.x, from);
+                    hi.y = __shfl_sync(kFull, hi.y, from); hi.z = __shfl_sync(kFull, hi.z, from);
+                }
+                if (lane == 0)
+                    record_node(small_record(V, s0 + a, mid < 0 ? -1 : s0 + mid), k, s0 + a, sg.z + depth, mid < 0 ? n : -1,
+                                mid < 0 ? -1 : s0 + mid, V.cnt, V.topd);
+            }
+            if (mid >= 0) {   // (at most total - 1 pending halves)
+                if (lane == 0) stack[sp] = mid | (b << 8) | ((depth + 1) << 16);
+                ++sp;
+                b = mid;
+                depth += 1;
+            } else {
+                if (sp == 0) break;
+                --sp;
+                __syncwarp();
+                const int e = stack[sp];
+                __syncwarp();
+                a = e & 255; b = (e >> 8) & 255; depth = e >> 16;
+            }
+        }
+        if (lane < total) V.perm[s0 + lane] = t;
+        if (__any_sync(kFull, bad) && lane == 0) atomicOr(V.flags, kFlagIndex);
+        __syncwarp();
     }
 }
 
@@ -876,7 +1001,7 @@ struct GpuBvhBuilder::Bufs {
     Buf<uint32_t> tri, mat, tri_off, vert_off, perm, tf, tt;
     Buf<float4> blo, bhi;
     Buf<int> pf, pt, chunk_cnt, chunk_off, cnt, topd, prefix, tile, parent, arrive, ctr;
-    Buf<int4> stack, lvl0, lvl1, small;
+    Buf<int4> stack, lvl0, lvl1, small, tiny;
     Buf<SegState> seg;
     Buf<int2> chunks;
     Buf<NodeRec> small_pool, large_pool;
@@ -887,7 +1012,7 @@ struct GpuBvhBuilder::Bufs {
         blo.release(); bhi.release();
         pf.release(); pt.release(); chunk_cnt.release(); chunk_off.release(); cnt.release(); topd.release();
         prefix.release(); tile.release(); parent.release(); arrive.release(); ctr.release();
-        stack.release(); lvl0.release(); lvl1.release(); small.release(); seg.release(); chunks.release();
+        stack.release(); lvl0.release(); lvl1.release(); small.release(); tiny.release(); seg.release(); chunks.release();
         small_pool.release(); large_pool.release();
     }
 };
@@ -944,7 +1069,7 @@ int GpuBvhBuilder::build(const std::vector<GpuMeshSrc>& meshes, cudaStream_t s, 
     BVH_CUDA(B.tri_off.reserve(M + 1)); BVH_CUDA(B.vert_off.reserve(M));
     BVH_CUDA(B.blo.reserve(n)); BVH_CUDA(B.bhi.reserve(n)); BVH_CUDA(B.perm.reserve(n));
     BVH_CUDA(B.tf.reserve(n)); BVH_CUDA(B.tt.reserve(n)); BVH_CUDA(B.pf.reserve(n)); BVH_CUDA(B.pt.reserve(n));
-    BVH_CUDA(B.stack.reserve(n)); BVH_CUDA(B.small.reserve(n + M));
+    BVH_CUDA(B.stack.reserve(n)); BVH_CUDA(B.tiny.reserve(n)); BVH_CUDA(B.small.reserve(n + M));
     BVH_CUDA(B.lvl0.reserve(max_seg)); BVH_CUDA(B.lvl1.reserve(max_seg)); BVH_CUDA(B.seg.reserve(max_seg));
     BVH_CUDA(B.chunks.reserve(max_chunks)); BVH_CUDA(B.chunk_cnt.reserve(max_chunks * kBins));
     BVH_CUDA(B.chunk_off.reserve(max_chunks));
@@ -964,7 +1089,8 @@ int GpuBvhBuilder::build(const std::vector<GpuMeshSrc>& meshes, cudaStream_t s, 
     BVH_CUDA(cudaMemcpyAsync(B.tri_off.p, tri_off.data(), 4 * (M + 1), cudaMemcpyHostToDevice, s));
     BVH_CUDA(cudaMemcpyAsync(B.vert_off.p, vert_off.data(), 4 * M, cudaMemcpyHostToDevice, s));
     // ctr: [0] chunks of the level, [1]/[5] segment counts of the two level lists,
-    // [2] per-warp segments, [3] large node records, [4] flags, [6] non-empty levels
+    // [2] per-warp segments, [3] large node records, [4] flags, [6] non-empty levels,
+    // [7] ranges of at most kTiny triangles
     int h_ctr[8] = {0, (int)large0.size(), (int)small0.size(), 0, 0, 0, 0, 0};
     BVH_CUDA(cudaMemcpyAsync(B.ctr.p, h_ctr, sizeof(h_ctr), cudaMemcpyHostToDevice, s));
     if (!large0.empty())
@@ -986,6 +1112,7 @@ int GpuBvhBuilder::build(const std::vector<GpuMeshSrc>& meshes, cudaStream_t s, 
     V.stack = B.stack.p; V.small_pool = B.small_pool.p; V.large_pool = B.large_pool.p;
     V.large_count = B.ctr.p + 3; V.large_cap = B.large_cap;
     V.cnt = B.cnt.p; V.topd = B.topd.p; V.flags = flags; V.n = (int)N;
+    V.tiny = B.tiny.p; V.tiny_count = B.ctr.p + 7;
     V.next_cap = (int)max_seg; V.small_cap = (int)(n + M);
 
     // level passes, kLevelsPerSync at a time between reads of the remaining count
@@ -1016,6 +1143,7 @@ int GpuBvhBuilder::build(const std::vector<GpuMeshSrc>& meshes, cudaStream_t s, 
         // one warp per remaining segment (the count is read on the device)
         const int gs = (int)std::min<long long>((n + M + kWarps - 1) / kWarps, kMaxGrid);
         k_small_build<<<gs, kThreads, 0, s>>>(B.small.p, B.ctr.p + 2, V);
+        k_tiny_build<<<gs, kThreads, 0, s>>>(V);
         BVH_CUDA(cudaGetLastError());
     }
     const int ntiles = (int)((n + kScanTile - 1) / kScanTile);

@@ -150,3 +150,22 @@ def test_negative_zero_falls_back_to_host():
     assert not st_dev["device_bvh"]
     for a, b in zip(dev, host):
         assert (a == b).all()
+
+
+@pytest.mark.parametrize("spread", ["soup", "line", "copies"])
+def test_device_bvh_at_range_sizes(spread):
+    """Meshes of the sizes where a range changes hands (a lane's, a warp's, the level
+    passes'): random, all centroids on one axis in steps, and few distinct centroids."""
+    rng = np.random.default_rng(11)
+    meshes = []
+    for n in (1, 2, 3, 31, 32, 33, 63, 64, 65, 255, 256, 257, 511, 600):
+        c = rng.uniform(-2, 2, (n, 3))
+        if spread == "line":
+            c = np.stack([np.round(c[:, 0], 1), np.zeros(n), np.ones(n)], 1)
+        elif spread == "copies":
+            c = c[rng.integers(0, min(n, 5), n)]
+        V = (c[:, None, :] + 0.1 * rng.normal(size=(1, 3, 3))).reshape(-1, 3)
+        meshes.append(_mesh(V, np.arange(3 * n).reshape(n, 3)))
+    host, device = _dumps(_scene(meshes), gpu_bvh=False)[0], _dumps(_scene(meshes), gpu_bvh=True)[0]
+    for a, b in zip(host, device):
+        assert a.shape == b.shape and (np.asarray(a).view(np.uint32) == np.asarray(b).view(np.uint32)).all()
