@@ -31,7 +31,7 @@ namespace {
 
 // Largest photon count the fixed scratch holds (sized by kd_scratch_bytes).
 constexpr long long kNoAllocMaxPhotons = 1LL << 19;
-constexpr size_t kNoAllocScratchBytes = 16u * (size_t)kNoAllocMaxPhotons + (1u << 20);
+constexpr size_t kNoAllocScratchBytes = 16u * (size_t)kNoAllocMaxPhotons + (1u << 20) + (1u << 16);
 
 static __device__ __align__(256) unsigned char g_kd_scratch[kNoAllocScratchBytes];
 static __device__ __align__(16) int g_kd_error;

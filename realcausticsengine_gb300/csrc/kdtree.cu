@@ -2,10 +2,16 @@
 //
 // Levels whose nodes hold more than kSmemSeg photons are split with global passes,
 // one pass per step over all photons (SoA x/y/z/id, double buffered):
-//   bbox      per-node extent -> axis (largest extent)
-//   hist x4   8-bit radix select of the rank-count/2 key along the node's axis (the
-//             leading digits the node's box fixes are skipped)
-//   partition photons below / equal / above the median key to their halves
+//   hist x4   8-bit radix select of the rank-count/2 key along the node's axis (its box's
+//             largest extent; the leading digits the box fixes are skipped)
+//   partition photons below / equal / above the median key to their halves, and the halves'
+//             boxes (the next level's nodes)
+// Each pass first picks the previous digit: every CTA does it for its own nodes, from the
+// finished histogram, and the histograms, boxes and cursors of the next level are cleared by
+// the passes of this one, so a level is 5 launches, each started while the one before ends.
+// At a few hundred thousand photons a pass is mostly its launch and one chain of loads: with
+// the box, its axis and each digit's choice in launches of their own (12 a level) 300,001
+// photons took 750 us, with 5 a level 519, started early 472.
 // A CTA covers T x kItems consecutive positions (T = 256 threads on levels whose nodes
 // hold more than 2048 photons, else 128); because nodes on these levels hold more
 // than that many photons, a chunk meets at most two nodes (and one ancestor median
@@ -20,6 +26,7 @@
 #include <cmath>
 #include <cstdio>
 #include <mutex>
+#include <utility>
 
 namespace rc {
 
@@ -71,12 +78,30 @@ __device__ __forceinline__ long long locate(long long i, int level, long long n,
     return e;
 }
 
+// Passes are launched programmatically: a pass's CTAs start while the pass before ends and
+// wait here for it (its memory is then visible) before they touch what it wrote.
+__device__ __forceinline__ void pass_wait() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// The global passes' state.  Levels alternate between two box and two cursor arrays.
+struct LevelState {
+    int* box;          // 6 per node of this level: min xyz, max xyz (f2ord)
+    int* cnt;          // 3 per node of this level: partition cursors (below / equal / above)
+    int* next_box;     // the next level's
+    int* next_cnt;
+    uint32_t* hist;    // [pass][node][256]
+    uint2* sel;        // [pass][node]: (selected high bits of the median key, rank left) after the pass
+    long long nodes;   // nodes the arrays hold
+};
+
+// A node's selection before `pass` (4: complete).
 struct NodeSel {
     uint32_t prefix;   // selected high bits of the median key
     int krem;          // remaining rank inside the selected bin
-    int eq;            // photons whose key equals the median key
+    int eq;            // photons whose key equals the median key (pass 4)
     int axis;
-    int cnt[3];        // partition cursors (below / equal / above)
     int first;         // first digit pass that runs (earlier digits fixed by the node's box)
 };
 
@@ -121,18 +146,7 @@ __device__ __forceinline__ int which(long long i, const ChunkNodes& cn) {
     return -1;
 }
 
-__global__ void k_level_init(int level, long long first, long long count, int* nbox, NodeSel* sel, long long n) {
-    long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (t >= count) return;
-    int* b = nbox + 6 * t;
-    b[0] = b[1] = b[2] = 0x7fffffff;
-    b[3] = b[4] = b[5] = (int)0x80000000;
-    NodeSel& s = sel[t];
-    s.prefix = 0; s.krem = (int)((n >> level) >> 1); s.eq = 0; s.axis = 0;
-    s.cnt[0] = s.cnt[1] = s.cnt[2] = 0;
-    s.first = 0;
-}
-
+// The root's box (the partition computes the other nodes').
 template <int T>
 __global__ void __launch_bounds__(T) k_bbox(Buffers B, int cur, int level, long long n, long long first, int* nbox) {
     __shared__ ChunkNodes cn;
@@ -186,68 +200,128 @@ __global__ void __launch_bounds__(T) k_bbox(Buffers B, int cur, int level, long 
     }
 }
 
-__device__ __forceinline__ int node_axis(const int* nbox, long long t) {
-    const int* b = nbox + 6 * t;
-    float ex = ord2f(b[3]) - ord2f(b[0]);
-    float ey = ord2f(b[4]) - ord2f(b[1]);
-    float ez = ord2f(b[5]) - ord2f(b[2]);
-    return biggest_axis(ex, ey, ez);
+// One warp: node t's selection before `pass`.  Every key of the node
+// lies between the keys of its box's ends along its axis (both orders are IEEE total
+// order), so the whole leading digits those two keys share are the median's digits too:
+// they go into the prefix, and the radix-select passes over them are skipped (the last pass
+// always runs: it gives the split and the count of keys equal to the median).  Otherwise
+// the digit of pass - 1 is the bin of its histogram that holds rank krem.  `keep` (one CTA
+// per node) stores the result for the next passes.
+__device__ __forceinline__ NodeSel node_select(const LevelState& S, long long t, int count, int pass, bool keep,
+                                               int* err) {
+    const int lane = threadIdx.x & 31;
+    const int* b = S.box + 6 * t;
+    const int b0 = b[0], b1 = b[1], b2 = b[2], b3 = b[3], b4 = b[4], b5 = b[5];
+    // (all loads in flight together, used or not)
+    uint2 prev = make_uint2(0u, 0u);
+    uint4 h0 = make_uint4(0u, 0u, 0u, 0u), h1 = h0;
+    if (pass >= 2) prev = S.sel[(pass - 2) * S.nodes + t];
+    if (pass >= 1) {
+        const uint4* h = reinterpret_cast<const uint4*>(S.hist + ((pass - 1) * S.nodes + t) * 256) + 2 * lane;
+        h0 = h[0];
+        h1 = h[1];
+    }
+    NodeSel s;
+    s.axis = biggest_axis(ord2f(b3) - ord2f(b0), ord2f(b4) - ord2f(b1), ord2f(b5) - ord2f(b2));
+    const uint32_t lo = f2key(ord2f(s.axis == 0 ? b0 : (s.axis == 1 ? b1 : b2)));
+    const uint32_t hi = f2key(ord2f(s.axis == 0 ? b3 : (s.axis == 1 ? b4 : b5)));
+    s.first = min(__clz(lo ^ hi) >> 3, 3);
+    s.prefix = lo & ~(0xffffffffu >> (8 * s.first));
+    s.krem = count >> 1;
+    s.eq = 0;
+    if (pass <= s.first) return s;
+    if (pass - 1 > s.first) {
+        s.prefix = prev.x;
+        s.krem = (int)prev.y;
+    }
+    const uint32_t v[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
+    uint32_t sum = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) sum += v[k];
+    uint32_t incl = sum;
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    uint32_t cum = incl - sum;
+    // lane whose range [cum, incl) contains krem
+    const unsigned bal = __ballot_sync(0xffffffffu, (uint32_t)s.krem >= cum && (uint32_t)s.krem < incl);
+    if (!bal) {
+        if (lane == 0) atomicOr(err, 1);   // histogram does not hold rank krem
+        return s;
+    }
+    int bin = lane * 8 + 7;
+    uint32_t at = cum, eq = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        if (eq == 0 && (uint32_t)s.krem < at + v[k]) { bin = lane * 8 + k; cum = at; eq = v[k]; }
+        at += v[k];
+    }
+    const int owner = __ffs(bal) - 1;
+    s.krem -= (int)__shfl_sync(0xffffffffu, cum, owner);
+    s.prefix |= (uint32_t)__shfl_sync(0xffffffffu, bin, owner) << (24 - 8 * (pass - 1));
+    s.eq = (int)__shfl_sync(0xffffffffu, eq, owner);
+    if (keep && lane == 0 && pass < 4) S.sel[(pass - 1) * S.nodes + t] = make_uint2(s.prefix, (uint32_t)s.krem);
+    return s;
 }
 
-// The node's split axis.  Every key of the node lies between the keys of its box's
-// ends along that axis (both orders are IEEE total order), so the whole leading digits
-// those two keys share are the median's digits too: they go into the prefix, and the
-// radix-select passes over them are skipped (the last pass always runs: it writes the
-// split and the count of keys equal to the median).
-__global__ void k_axis(long long count, const int* nbox, NodeSel* sel) {
-    long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (t >= count) return;
-    const int a = node_axis(nbox, t);
-    const uint32_t lo = f2key(ord2f(nbox[6 * t + a])), hi = f2key(ord2f(nbox[6 * t + 3 + a]));
-    const int d = min(__clz(lo ^ hi) >> 3, 3);
-    NodeSel& s = sel[t];
-    s.axis = a;
-    s.first = d;
-    s.prefix = lo & ~(0xffffffffu >> (8 * d));
+// Grid-wide clear of histogram `pass` for `nodes` nodes.
+__device__ __forceinline__ void clear_hist(const LevelState& S, int pass, long long nodes) {
+    uint4* h = reinterpret_cast<uint4*>(S.hist + pass * S.nodes * 256);
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < 64 * nodes; i += (long long)gridDim.x * blockDim.x)
+        h[i] = make_uint4(0u, 0u, 0u, 0u);
 }
 
 __device__ __forceinline__ float coord(const Side& S, long long i, int axis) {
     return axis == 0 ? S.x[i] : (axis == 1 ? S.y[i] : S.z[i]);
 }
 
+// next: nodes of the next level (0: there is none).
 template <int T>
-__global__ void __launch_bounds__(T) k_hist(Buffers B, int cur, int level, long long n, long long first,
-                                                   const NodeSel* sel, uint32_t* hist, int pass) {
+__global__ void __launch_bounds__(T) k_hist(Buffers B, int cur, int level, long long n, long long first, LevelState S,
+                                            long long next, int pass, int* err) {
     __shared__ ChunkNodes cn;
     __shared__ uint32_t sh[2][256];
     __shared__ uint32_t pre[2];
     __shared__ int ax[2];
     __shared__ bool live[2];   // the node's digit for this pass is not fixed by its box
     long long a = blockIdx.x * (long long)(T * kItems);
-    if (threadIdx.x == 0) {
-        chunk_nodes(a, T * kItems, level, n, cn);
-        const NodeSel* sa = sel + (cn.eA - first);
-        ax[0] = sa->axis; pre[0] = sa->prefix; live[0] = pass >= sa->first;
-        live[1] = false;
-        if (cn.eB) {
-            const NodeSel* sb = sel + (cn.eB - first);
-            ax[1] = sb->axis; pre[1] = sb->prefix; live[1] = pass >= sb->first;
+    if (threadIdx.x == 0) chunk_nodes(a, T * kItems, level, n, cn);
+    for (int k = threadIdx.x; k < 512; k += T) (&sh[0][0])[k] = 0;
+    pass_wait();
+    if (pass == 0) {
+        clear_hist(S, 3, first);
+        for (long long t = blockIdx.x * (long long)T + threadIdx.x; t < next; t += (long long)gridDim.x * T) {
+            for (int k = 0; k < 6; ++k) S.next_box[6 * t + k] = k < 3 ? 0x7fffffff : (int)0x80000000;
+            for (int k = 0; k < 3; ++k) S.next_cnt[3 * t + k] = 0;
+        }
+    } else if (pass >= 2) {
+        clear_hist(S, pass - 2, next);
+    }
+    __syncthreads();
+    if (threadIdx.x < 64) {
+        const int w = threadIdx.x >> 5;
+        const long long e = w ? cn.eB : cn.eA, s = w ? cn.sB : cn.sA;
+        if (e) {
+            const NodeSel q = node_select(S, e - first, (int)cn.c, pass, s >= a, err);
+            if ((threadIdx.x & 31) == 0) { ax[w] = q.axis; pre[w] = q.prefix; live[w] = pass >= q.first; }
+        } else if ((threadIdx.x & 31) == 0) {
+            live[w] = false;
         }
     }
-    for (int k = threadIdx.x; k < 512; k += T) (&sh[0][0])[k] = 0;
     __syncthreads();
     if (!live[0] && !live[1]) return;
     const int shift = 24 - 8 * pass;
     // all rounds' coordinates first (independent loads in flight together), then bins
     float val[kItems];
     int wh[kItems];
-    const Side S = side(B, cur);
+    const Side P = side(B, cur);
 #pragma unroll
     for (int it = 0; it < kItems; ++it) {
         long long i = a + it * T + threadIdx.x;
         const int w = i < n ? which(i, cn) : -1;
         wh[it] = w >= 0 && live[w] ? w : -1;
-        val[it] = wh[it] >= 0 ? coord(S, i, ax[wh[it]]) : 0.0f;
+        val[it] = wh[it] >= 0 ? coord(P, i, ax[wh[it]]) : 0.0f;
     }
 #pragma unroll
     for (int it = 0; it < kItems; ++it) {   // every lane runs every round (full-warp match)
@@ -269,74 +343,38 @@ __global__ void __launch_bounds__(T) k_hist(Buffers B, int cur, int level, long 
         int q = k >> 8;
         uint32_t v = (&sh[0][0])[k];
         long long e = q == 0 ? cn.eA : cn.eB;
-        if (v && e) atomicAdd(&hist[(e - first) * 256 + (k & 255)], v);
-    }
-}
-
-// One warp per node: find the bin holding rank krem, narrow the prefix, clear the
-// histogram for the next pass.  After the last pass, write the node's split.
-__global__ void k_select(long long count, long long first, int level, long long n, NodeSel* sel, uint32_t* hist,
-                         int pass, uint2* nodes, int* err) {
-    long long t = blockIdx.x * (long long)(blockDim.x / 32) + threadIdx.x / 32;
-    int lane = threadIdx.x & 31;
-    if (t >= count) return;
-    if (pass < sel[t].first) return;   // digit fixed by the node's box (k_axis); no counts
-    uint32_t* h = hist + t * 256;
-    uint32_t v[8];
-    uint32_t sum = 0;
-    for (int k = 0; k < 8; ++k) { v[k] = h[lane * 8 + k]; sum += v[k]; h[lane * 8 + k] = 0; }
-    uint32_t incl = sum;
-    for (int o = 1; o < 32; o <<= 1) {
-        uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += y;
-    }
-    uint32_t excl = incl - sum;
-    int krem = sel[t].krem;
-    // lane whose range [excl, incl) contains krem
-    bool mine = (uint32_t)krem >= excl && (uint32_t)krem < incl;
-    unsigned bal = __ballot_sync(0xffffffffu, mine);
-    int owner = __ffs(bal) - 1;
-    if (owner < 0) {
-        if (lane == 0) atomicOr(err, 1);   // histogram does not hold rank krem
-        return;
-    }
-    if (lane == owner) {
-        uint32_t cum = excl;
-        int bin = 0;
-        for (int k = 0; k < 8; ++k) {
-            if ((uint32_t)krem < cum + v[k]) { bin = lane * 8 + k; break; }
-            cum += v[k];
-        }
-        NodeSel& s = sel[t];
-        s.krem = krem - (int)cum;
-        s.prefix |= (uint32_t)bin << (24 - 8 * pass);
-        if (pass == 3) {
-            s.eq = (int)v[bin - lane * 8];
-            long long c = n >> level;
-            float m = key2f(s.prefix);
-            long long e = first + t;
-            nodes[e].y = __float_as_uint((c & 1) ? m : m + kSplitBias);
-            if (!(c & 1)) nodes[e].x = even_mask(s.axis);
-        }
+        if (v && e) atomicAdd(&S.hist[(pass * S.nodes + e - first) * 256 + (k & 255)], v);
     }
 }
 
 template <int T>
 __global__ void __launch_bounds__(T) k_partition(Buffers B, int cur, int level, long long n, long long first,
-                                                        NodeSel* sel, uint2* nodes, int* err) {
+                                                 LevelState L, long long next, uint2* nodes, int* err) {
     __shared__ ChunkNodes cn;
     __shared__ int ax[2], krem[2], eq[2];
     __shared__ uint32_t med[2];
     __shared__ int base[6];
     __shared__ int woff[kItems][T / 32][6];
+    __shared__ int sb[4][6];   // boxes of the halves: node A left, right, node B left, right
     long long a = blockIdx.x * (long long)(T * kItems);
-    if (threadIdx.x == 0) {
-        chunk_nodes(a, T * kItems, level, n, cn);
-        NodeSel s = sel[cn.eA - first];
-        ax[0] = s.axis; krem[0] = s.krem; eq[0] = s.eq; med[0] = s.prefix;
-        if (cn.eB) {
-            s = sel[cn.eB - first];
-            ax[1] = s.axis; krem[1] = s.krem; eq[1] = s.eq; med[1] = s.prefix;
+    if (threadIdx.x == 0) chunk_nodes(a, T * kItems, level, n, cn);
+    if (threadIdx.x < 24) sb[threadIdx.x / 6][threadIdx.x % 6] = (threadIdx.x % 6) < 3 ? 0x7fffffff : (int)0x80000000;
+    pass_wait();
+    clear_hist(L, 2, next);
+    __syncthreads();
+    if (threadIdx.x < 64) {
+        const int w = threadIdx.x >> 5;
+        const long long e = w ? cn.eB : cn.eA, s = w ? cn.sB : cn.sA;
+        if (e) {
+            const NodeSel q = node_select(L, e - first, (int)cn.c, 4, false, err);
+            if ((threadIdx.x & 31) == 0) {
+                ax[w] = q.axis; krem[w] = q.krem; eq[w] = q.eq; med[w] = q.prefix;
+                if (s >= a) {   // the node's split, written by the CTA its range starts in
+                    const float m = key2f(q.prefix);
+                    nodes[e].y = __float_as_uint((cn.c & 1) ? m : m + kSplitBias);
+                    if (!(cn.c & 1)) nodes[e].x = even_mask(q.axis);
+                }
+            }
         }
     }
     __syncthreads();
@@ -388,15 +426,17 @@ __global__ void __launch_bounds__(T) k_partition(Buffers B, int cur, int level, 
                 run += v;
             }
         long long e = q < 3 ? cn.eA : cn.eB;
-        base[q] = (e && run) ? atomicAdd(&sel[e - first].cnt[q % 3], run) : 0;
+        base[q] = (e && run) ? atomicAdd(&L.cnt[3 * (e - first) + q % 3], run) : 0;
     }
     __syncthreads();
     const long long c = cn.c;
     const long long k = c >> 1, odd = c & 1;
+    int half[kItems];   // the half the photon goes to (2 w + right), -1: none
 #pragma unroll
     for (int it = 0; it < kItems; ++it) {
         long long i = a + it * T + threadIdx.x;
         int q = cls[it];
+        half[it] = -1;
         if (q == -2) continue;
         const float xv = px[it], yv = py[it], zv = pz[it];
         const uint32_t idv = pid[it];
@@ -419,13 +459,44 @@ __global__ void __launch_bounds__(T) k_partition(Buffers B, int cur, int level, 
                 } else d = s + k + odd + (r - kl - odd);
             } else d = s + k + odd + (eq[w] - kl - odd) + r;
             if (d < s || d >= s + c) { atomicOr(err, 2); continue; }   // inconsistent counts
+            if (!(odd && d == s + k)) half[it] = 2 * w + (d >= s + k);
         }
         D.x[d] = xv; D.y[d] = yv; D.z[d] = zv; D.id[d] = idv;
     }
+    if (!next) return;
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+        if (h >= 2 && !cn.eB) break;
+        int mn[3] = {0x7fffffff, 0x7fffffff, 0x7fffffff};
+        int mx[3] = {(int)0x80000000, (int)0x80000000, (int)0x80000000};
+#pragma unroll
+        for (int it = 0; it < kItems; ++it) {
+            if (half[it] != h) continue;
+            const int vx = f2ord(px[it]), vy = f2ord(py[it]), vz = f2ord(pz[it]);
+            mn[0] = min(mn[0], vx); mn[1] = min(mn[1], vy); mn[2] = min(mn[2], vz);
+            mx[0] = max(mx[0], vx); mx[1] = max(mx[1], vy); mx[2] = max(mx[2], vz);
+        }
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            const int v = __reduce_min_sync(0xffffffffu, mn[j]), u = __reduce_max_sync(0xffffffffu, mx[j]);
+            if (lane == 0) { atomicMin(&sb[h][j], v); atomicMax(&sb[h][3 + j], u); }
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < 24) {
+        const int h = threadIdx.x / 6, j = threadIdx.x % 6;
+        const long long e = h < 2 ? cn.eA : cn.eB;
+        if (e) {
+            int* dst2 = L.next_box + 6 * (2 * (e - first) + (h & 1)) + j;
+            if (j < 3) atomicMin(dst2, sb[h][j]); else atomicMax(dst2, sb[h][j]);
+        }
+    }
 }
 
-__global__ void k_load(const float4* __restrict__ pos4, long long n, Buffers B) {
+__global__ void k_load(const float4* __restrict__ pos4, long long n, Buffers B, LevelState S) {
     long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (S.nodes > 0 && i < 6) S.box[i] = i < 3 ? 0x7fffffff : (int)0x80000000;
+    if (S.nodes > 0 && i < 3) S.cnt[i] = 0;
     if (i >= n) return;
     float4 p = pos4[i];
     B.x[0][i] = p.x; B.y[0][i] = p.y; B.z[0][i] = p.z; B.id[0][i] = (uint32_t)i;
@@ -503,6 +574,7 @@ __global__ void __launch_bounds__(kSmemThreads) k_smem_build(Buffers B, int src,
     const int tid = threadIdx.x, nt = blockDim.x;
     const int lane = tid & 31, wid = tid >> 5;
     const Side S = side(B, src);
+    pass_wait();
     for (int i = tid; i < c0; i += nt) {
         X[i] = S.x[s0 + i]; Y[i] = S.y[s0 + i]; Z[i] = S.z[s0 + i]; I[i] = S.id[s0 + i];
     }
@@ -701,11 +773,31 @@ size_t kd_scratch_bytes(long long n) {
     long long maxnodes = l0 > 0 ? (1LL << (l0 - 1)) : 1;
     size_t b = 0;
     b += 16 * (size_t)n;                      // second buffer x/y/z/id
-    b += 24 * (size_t)maxnodes;               // boxes
-    b += sizeof(NodeSel) * (size_t)maxnodes;  // selection state
-    b += 1024 * (size_t)maxnodes;             // histograms
+    b += 2 * 36 * (size_t)maxnodes;           // boxes and cursors of two levels
+    b += 3 * 8 * (size_t)maxnodes;            // selection state after passes 0 .. 2
+    b += 4 * 1024 * (size_t)maxnodes;         // histograms of the four passes
     return b + 1024;
 }
+
+namespace {
+
+// A launch that may start before the one before it in the stream has ended (pass_wait).
+template <class... P, class... A>
+void launch_pass(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(block);
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+}
+
+}  // namespace
 
 int kd_build(const float4* pos4, long long n, KdTree& tree, void* scratch, size_t scratch_bytes,
              cudaStream_t stream, int* launches, int* err) {
@@ -725,42 +817,45 @@ int kd_build(const float4* pos4, long long n, KdTree& tree, void* scratch, size_
     B.z[1] = (float*)p; p += 4 * (size_t)n;
     B.id[1] = (uint32_t*)p; p += 4 * (size_t)n;
     p = (char*)(((uintptr_t)p + 255) & ~(uintptr_t)255);
-    int* nbox = (int*)p; p += 24 * (size_t)maxnodes;
-    p = (char*)(((uintptr_t)p + 15) & ~(uintptr_t)15);
-    NodeSel* sel = (NodeSel*)p; p += sizeof(NodeSel) * (size_t)maxnodes;
-    p = (char*)(((uintptr_t)p + 255) & ~(uintptr_t)255);
-    uint32_t* hist = (uint32_t*)p;
+    LevelState S{};
+    S.nodes = l0 > 0 ? maxnodes : 0;
+    S.hist = (uint32_t*)p; p += 4 * 1024 * (size_t)maxnodes;
+    S.sel = (uint2*)p; p += 3 * 8 * (size_t)maxnodes;
+    S.box = (int*)p; p += 24 * (size_t)maxnodes;
+    S.next_box = (int*)p; p += 24 * (size_t)maxnodes;
+    S.cnt = (int*)p; p += 12 * (size_t)maxnodes;
+    S.next_cnt = (int*)p;
 
     cudaMemsetAsync(tree.nodes, 0, sizeof(uint2) * (size_t)tree.num_nodes, stream);
-    k_load<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(pos4, n, B);
+    k_load<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(pos4, n, B, S);
     nl++;
-    if (l0 > 0) cudaMemsetAsync(hist, 0, 1024 * (size_t)maxnodes, stream);
     int cur = 0;
+    if (l0 > 0) {
+        // the root's histograms; the passes clear those of the levels below
+        for (int pass = 0; pass < 4; ++pass)
+            cudaMemsetAsync(S.hist + pass * maxnodes * 256, 0, 1024, stream);
+        const long long span = (long long)kWideThreads * kItems;
+        k_bbox<kWideThreads><<<(unsigned)((n + span - 1) / span), kWideThreads, 0, stream>>>(B, 0, 0, n, 1, S.box);
+        nl++;
+    }
     for (int l = 0; l < l0; ++l) {
-        long long first = 1LL << l, count = 1LL << l;
-        unsigned g = (unsigned)((count + 255) / 256);
+        const long long first = 1LL << l, next = l + 1 < l0 ? 2 * first : 0;
         // half as many CTAs, each twice as wide, while a wide chunk still meets at most
         // two nodes: the passes' per-CTA fixed cost (chunk location, shared-memory
         // reduction) is paid half as often
         const bool wide = (n >> l) > (long long)kWideThreads * kItems;
         const long long span = (long long)(wide ? kWideThreads : kThreads) * kItems;
         const unsigned chunks = (unsigned)((n + span - 1) / span);
-        k_level_init<<<g, 256, 0, stream>>>(l, first, count, nbox, sel, n);
-        if (wide) k_bbox<kWideThreads><<<chunks, kWideThreads, 0, stream>>>(B, cur, l, n, first, nbox);
-        else k_bbox<kThreads><<<chunks, kThreads, 0, stream>>>(B, cur, l, n, first, nbox);
-        k_axis<<<g, 256, 0, stream>>>(count, nbox, sel);
-        nl += 3;
-        for (int pass = 0; pass < 4; ++pass) {
-            if (wide) k_hist<kWideThreads><<<chunks, kWideThreads, 0, stream>>>(B, cur, l, n, first, sel, hist, pass);
-            else k_hist<kThreads><<<chunks, kThreads, 0, stream>>>(B, cur, l, n, first, sel, hist, pass);
-            k_select<<<(unsigned)((count + 7) / 8), 256, 0, stream>>>(count, first, l, n, sel, hist, pass, tree.nodes,
-                                                                       err);
-            nl += 2;
+        for (int pass = 0; pass < 4; ++pass, ++nl) {
+            if (wide) launch_pass(k_hist<kWideThreads>, chunks, kWideThreads, 0, stream, B, cur, l, n, first, S, next, pass, err);
+            else launch_pass(k_hist<kThreads>, chunks, kThreads, 0, stream, B, cur, l, n, first, S, next, pass, err);
         }
-        if (wide) k_partition<kWideThreads><<<chunks, kWideThreads, 0, stream>>>(B, cur, l, n, first, sel, tree.nodes, err);
-        else k_partition<kThreads><<<chunks, kThreads, 0, stream>>>(B, cur, l, n, first, sel, tree.nodes, err);
+        if (wide) launch_pass(k_partition<kWideThreads>, chunks, kWideThreads, 0, stream, B, cur, l, n, first, S, next, tree.nodes, err);
+        else launch_pass(k_partition<kThreads>, chunks, kThreads, 0, stream, B, cur, l, n, first, S, next, tree.nodes, err);
         nl++;
         cur ^= 1;
+        std::swap(S.box, S.next_box);
+        std::swap(S.cnt, S.next_cnt);
     }
     if (cur == 1 && l0 > 0) {
         long long cnt = (1LL << l0) - 1;
@@ -772,7 +867,7 @@ int kd_build(const float4* pos4, long long n, KdTree& tree, void* scratch, size_
     // several threads build concurrently
     static std::once_flag attr_set[kOnceDevices];
     once_per_device(attr_set, [&] { cudaFuncSetAttribute(k_smem_build, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); });
-    k_smem_build<<<(unsigned)(1LL << l0), kSmemThreads, smem, stream>>>(B, cur, l0, n, tree.nodes);
+    launch_pass(k_smem_build, (unsigned)(1LL << l0), kSmemThreads, smem, stream, B, cur, l0, n, tree.nodes);
     nl++;
     if (launches) *launches = nl;
     return 0;

@@ -89,3 +89,38 @@ def test_noalloc_rejects_counts_beyond_fixed_scratch():
                                  d.data_ptr(), d.data_ptr(), None)
     assert rc == -5
     assert b"524288" in lib.rc_kd_noalloc_last_error()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1023, 1025, 2049, 4097, 8193, 70003])
+def test_kd_build_is_the_median_split_tree(n):
+    """Around a subtree's 1024 photons, the passes' 1024 and 2048 positions per block and
+    several levels of them, against the split written out in NumPy.  Distinct coordinates
+    (whatever their leading digits: one axis spans 2^-20 .. 1, one is all in one octave)."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    rng = np.random.default_rng(n)
+    cols = [np.linspace(-1, 1, n), np.exp2(np.linspace(-20, 0, n)), np.linspace(3.0, 3.9, n)]
+    pos = np.stack([rng.permutation(c.astype(np.float32)) for c in cols], 1)
+    assert all(len(np.unique(pos[:, k])) == n for k in range(3))
+    want = {}
+    pending = [(1, np.arange(n))]
+    while pending:
+        e, ids = pending.pop()
+        if len(ids) == 1:
+            want[e] = (int(ids[0]), 0)
+            continue
+        p = pos[ids]
+        ext = p.max(0) - p.min(0)
+        axis = int(np.argmax(ext == ext.max()))
+        order = ids[np.argsort(p[:, axis])]
+        half, odd = len(ids) // 2, len(ids) & 1
+        m = pos[order[half], axis]
+        word = (int(order[half]) | (0x90000000, 0xB0000000, 0xF0000000)[axis]) if odd else (0x80000000, 0xA0000000, 0xE0000000)[axis]
+        want[e] = (word, int((m if odd else np.float32(m + np.float32(1.175494e-38))).view(np.uint32)))
+        pending += [(2 * e, order[:half]), (2 * e + 1, order[half + odd:])]
+    nodes = _call_noalloc(torch, pos)[0]
+    e = np.fromiter(want, np.int64)
+    got = nodes[e].astype(np.int64)
+    assert (got == np.array([want[k] for k in e])).all()
