@@ -23,6 +23,7 @@
 // lists per level, writing nodes and final order.
 #include "kdtree.cuh"
 #include "dev_once.h"
+#include "early_launch.cuh"
 #include <cmath>
 #include <cstdio>
 #include <mutex>
@@ -76,13 +77,6 @@ __device__ __forceinline__ long long locate(long long i, int level, long long n,
     }
     *start = s;
     return e;
-}
-
-// Passes are launched programmatically: a pass's CTAs start while the pass before ends and
-// wait here for it (its memory is then visible) before they touch what it wrote.
-__device__ __forceinline__ void pass_wait() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // The global passes' state.  Levels alternate between two box and two cursor arrays.
@@ -288,7 +282,7 @@ __global__ void __launch_bounds__(T) k_hist(Buffers B, int cur, int level, long 
     long long a = blockIdx.x * (long long)(T * kItems);
     if (threadIdx.x == 0) chunk_nodes(a, T * kItems, level, n, cn);
     for (int k = threadIdx.x; k < 512; k += T) (&sh[0][0])[k] = 0;
-    pass_wait();
+    early_launch_wait();
     if (pass == 0) {
         clear_hist(S, 3, first);
         for (long long t = blockIdx.x * (long long)T + threadIdx.x; t < next; t += (long long)gridDim.x * T) {
@@ -359,7 +353,7 @@ __global__ void __launch_bounds__(T) k_partition(Buffers B, int cur, int level, 
     long long a = blockIdx.x * (long long)(T * kItems);
     if (threadIdx.x == 0) chunk_nodes(a, T * kItems, level, n, cn);
     if (threadIdx.x < 24) sb[threadIdx.x / 6][threadIdx.x % 6] = (threadIdx.x % 6) < 3 ? 0x7fffffff : (int)0x80000000;
-    pass_wait();
+    early_launch_wait();
     clear_hist(L, 2, next);
     __syncthreads();
     if (threadIdx.x < 64) {
@@ -574,7 +568,7 @@ __global__ void __launch_bounds__(kSmemThreads) k_smem_build(Buffers B, int src,
     const int tid = threadIdx.x, nt = blockDim.x;
     const int lane = tid & 31, wid = tid >> 5;
     const Side S = side(B, src);
-    pass_wait();
+    early_launch_wait();
     for (int i = tid; i < c0; i += nt) {
         X[i] = S.x[s0 + i]; Y[i] = S.y[s0 + i]; Z[i] = S.z[s0 + i]; I[i] = S.id[s0 + i];
     }
@@ -779,26 +773,6 @@ size_t kd_scratch_bytes(long long n) {
     return b + 1024;
 }
 
-namespace {
-
-// A launch that may start before the one before it in the stream has ended (pass_wait).
-template <class... P, class... A>
-void launch_pass(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, A... args) {
-    cudaLaunchConfig_t c{};
-    c.gridDim = dim3(grid);
-    c.blockDim = dim3(block);
-    c.dynamicSmemBytes = smem;
-    c.stream = s;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    c.attrs = &at;
-    c.numAttrs = 1;
-    cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
-}
-
-}  // namespace
-
 int kd_build(const float4* pos4, long long n, KdTree& tree, void* scratch, size_t scratch_bytes,
              cudaStream_t stream, int* launches, int* err) {
     int nl = 0;
@@ -847,11 +821,11 @@ int kd_build(const float4* pos4, long long n, KdTree& tree, void* scratch, size_
         const long long span = (long long)(wide ? kWideThreads : kThreads) * kItems;
         const unsigned chunks = (unsigned)((n + span - 1) / span);
         for (int pass = 0; pass < 4; ++pass, ++nl) {
-            if (wide) launch_pass(k_hist<kWideThreads>, chunks, kWideThreads, 0, stream, B, cur, l, n, first, S, next, pass, err);
-            else launch_pass(k_hist<kThreads>, chunks, kThreads, 0, stream, B, cur, l, n, first, S, next, pass, err);
+            if (wide) launch_early(k_hist<kWideThreads>, chunks, kWideThreads, 0, stream, B, cur, l, n, first, S, next, pass, err);
+            else launch_early(k_hist<kThreads>, chunks, kThreads, 0, stream, B, cur, l, n, first, S, next, pass, err);
         }
-        if (wide) launch_pass(k_partition<kWideThreads>, chunks, kWideThreads, 0, stream, B, cur, l, n, first, S, next, tree.nodes, err);
-        else launch_pass(k_partition<kThreads>, chunks, kThreads, 0, stream, B, cur, l, n, first, S, next, tree.nodes, err);
+        if (wide) launch_early(k_partition<kWideThreads>, chunks, kWideThreads, 0, stream, B, cur, l, n, first, S, next, tree.nodes, err);
+        else launch_early(k_partition<kThreads>, chunks, kThreads, 0, stream, B, cur, l, n, first, S, next, tree.nodes, err);
         nl++;
         cur ^= 1;
         std::swap(S.box, S.next_box);
@@ -867,7 +841,7 @@ int kd_build(const float4* pos4, long long n, KdTree& tree, void* scratch, size_
     // several threads build concurrently
     static std::once_flag attr_set[kOnceDevices];
     once_per_device(attr_set, [&] { cudaFuncSetAttribute(k_smem_build, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); });
-    launch_pass(k_smem_build, (unsigned)(1LL << l0), kSmemThreads, smem, stream, B, cur, l0, n, tree.nodes);
+    launch_early(k_smem_build, (unsigned)(1LL << l0), kSmemThreads, smem, stream, B, cur, l0, n, tree.nodes);
     nl++;
     if (launches) *launches = nl;
     return 0;

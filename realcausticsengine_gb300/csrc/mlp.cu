@@ -2,6 +2,7 @@
 #include "mlp.cuh"
 #include "lights.cuh"
 #include "proposal.cuh"
+#include "early_launch.cuh"
 #include "tc_gemm.cuh"
 #include "rng.cuh"
 #include "dev_once.h"
@@ -331,7 +332,8 @@ __global__ void k_norm_weights(float4* dir4, int n, const float* wsum) {
 // the shared-memory layout beside them.  With 128 threads, a thread per row, and the
 // weights laid out per CTA element by element, the step took 107 us (the layout 27, the
 // forward layers 18, the loss 12, the backward layers 20, the partial sums' scattered
-// stores 11) and its reduction 12.6; now 27 and 6.7 (GB300, 16,384 rows).
+// stores 11) and its reduction 12.6; now 27 and 6.7 (GB300, 16,384 rows), and a step is
+// launched while the one before ends (a 1280x720 learned pass 13.3 -> 12.7 ms).
 constexpr int kTrainThreads = 512;
 struct SmemTrain {
     static constexpr int wf0 = 0;                       // forward weights (out x in), K-major over in
@@ -558,21 +560,22 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_train(const MlpParams 
     __shared__ float loss_warp[4];
     const int tid = threadIdx.x, warp = tid >> 5;
     unsigned char* DyT = sm + SmemTrain::dyt;
+    for (int i = tid; i < 128 * 128 * 2 / 16; i += kTrainThreads) reinterpret_cast<uint4*>(DyT)[i] = make_uint4(0, 0, 0, 0);
+    for (int i = tid; i < 16 * 128 * 2 / 16; i += kTrainThreads)
+        reinterpret_cast<uint4*>(sm + SmemTrain::ones)[i] = make_uint4(0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u);
+    if (tid == 0) tc::mbar_init(&mbar, 1);
+    if (warp == 0) tc::tmem_alloc(&tmem_base, 512);
+    early_launch_wait();   // the weights of the step before
     {
         const uint4* src = reinterpret_cast<const uint4*>(P.image);
         uint4* to = reinterpret_cast<uint4*>(sm);
 #pragma unroll 8
         for (int i = tid; i < SmemTrain::image / 16; i += kTrainThreads) to[i] = src[i];
     }
-    for (int i = tid; i < 128 * 128 * 2 / 16; i += kTrainThreads) reinterpret_cast<uint4*>(DyT)[i] = make_uint4(0, 0, 0, 0);
-    for (int i = tid; i < 16 * 128 * 2 / 16; i += kTrainThreads)
-        reinterpret_cast<uint4*>(sm + SmemTrain::ones)[i] = make_uint4(0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u);
     if (tid < 272) {
         const int l = tid < 64 ? 0 : (tid < 128 ? 1 : (tid < 192 ? 2 : 3));
         reinterpret_cast<float*>(sm + SmemTrain::bias)[tid] = P.b[l][tid - 64 * l];
     }
-    if (tid == 0) tc::mbar_init(&mbar, 1);
-    if (warp == 0) tc::tmem_alloc(&tmem_base, 512);
     publish_smem();
     tc::fence_after_sync();
     // warp w reads TMEM lanes 32 (w % 4) ..: its row of the tile; w / 4 is its column group
@@ -660,6 +663,7 @@ __global__ void __launch_bounds__(32 * kReduceWarps) k_reduce_adam(const MlpPara
     const int j = blockIdx.x * 32 + lane;   // parameter, or the loss
     constexpr int total = kMlpPartStride - 4;
     float g = 0.0f;
+    early_launch_wait();   // the partial sums
     if (j <= total) {
 #pragma unroll 8
         for (int b = warp; b < nparts; b += kReduceWarps) g += part[(size_t)b * kMlpPartStride + j];
@@ -877,12 +881,12 @@ int mlp_train_step(MlpParams& p, MlpBatch& b, const float4* pos4, const float4* 
     once_per_device(attr, [&] { cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); });
     const int tiles = (n + 127) / 128;
     const int grid = std::min(std::min(tiles, sm_count()), b.part_rows);
-    k_mlp_train<<<grid, kTrainThreads, smem, s>>>(p, pos4, dir4, n, 1.0f / (float)n, b.part, err);
+    launch_early(k_mlp_train, grid, kTrainThreads, smem, s, p, pos4, dir4, n, 1.0f / (float)n, b.part, err);
     if (apply) p.adam_step++;
     const float b1t = std::pow(0.9f, (float)std::max(p.adam_step, 1));
     const float b2t = std::pow(0.999f, (float)std::max(p.adam_step, 1));
-    k_reduce_adam<<<(kMlpPartStride - 4) / 32 + 1, 32 * kReduceWarps, 0, s>>>(p, b.part, grid, apply ? 1 : 0, lr, b1t, b2t,
-                                                                           b.loss);
+    launch_early(k_reduce_adam, (kMlpPartStride - 4) / 32 + 1, 32 * kReduceWarps, 0, s, p, b.part, grid, apply ? 1 : 0,
+                 lr, b1t, b2t, b.loss);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
