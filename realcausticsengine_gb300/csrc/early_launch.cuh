@@ -5,12 +5,14 @@
 
 namespace rc {
 
-// In a kernel launched with launch_early: lets the next such launch start, then waits until
-// the launch before has ended and its memory is visible.  Nothing that launch reads or
-// writes may be touched above.
+// In a kernel launched with launch_early: waits until the launch before has ended and its
+// memory is visible, then lets the next such launch start.  Above it nothing may be touched
+// that the launch before writes, and nothing written that it reads; what the launch before
+// that one wrote is complete (read past L1: __ldcg), because the launch before let this one
+// start after its own wait.
 __device__ __forceinline__ void early_launch_wait() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 template <class... P, class... A>

@@ -11,7 +11,8 @@
 // the passes of this one, so a level is 5 launches, each started while the one before ends.
 // At a few hundred thousand photons a pass is mostly its launch and one chain of loads: with
 // the box, its axis and each digit's choice in launches of their own (12 a level) 300,001
-// photons took 750 us, with 5 a level 519, started early 472.
+// photons took 750 us, with 5 a level 519, started early 395 (472 without loading the
+// photons before the wait).
 // A CTA covers T x kItems consecutive positions (T = 256 threads on levels whose nodes
 // hold more than 2048 photons, else 128); because nodes on these levels hold more
 // than that many photons, a chunk meets at most two nodes (and one ancestor median
@@ -266,10 +267,6 @@ __device__ __forceinline__ void clear_hist(const LevelState& S, int pass, long l
         h[i] = make_uint4(0u, 0u, 0u, 0u);
 }
 
-__device__ __forceinline__ float coord(const Side& S, long long i, int axis) {
-    return axis == 0 ? S.x[i] : (axis == 1 ? S.y[i] : S.z[i]);
-}
-
 // next: nodes of the next level (0: there is none).
 template <int T>
 __global__ void __launch_bounds__(T) k_hist(Buffers B, int cur, int level, long long n, long long first, LevelState S,
@@ -280,9 +277,22 @@ __global__ void __launch_bounds__(T) k_hist(Buffers B, int cur, int level, long 
     __shared__ int ax[2];
     __shared__ bool live[2];   // the node's digit for this pass is not fixed by its box
     long long a = blockIdx.x * (long long)(T * kItems);
+    // the chunk's coordinates, loaded before the wait: the level's partition wrote them, at
+    // least two launches ago (pass 0: one, so it loads them after)
+    const Side P = side(B, cur);
+    float px[kItems], py[kItems], pz[kItems];
+    auto load = [&]() {
+#pragma unroll
+        for (int it = 0; it < kItems; ++it) {
+            const long long i = a + it * T + threadIdx.x, j = i < n ? i : a;
+            px[it] = __ldcg(&P.x[j]); py[it] = __ldcg(&P.y[j]); pz[it] = __ldcg(&P.z[j]);
+        }
+    };
+    if (pass > 0) load();
     if (threadIdx.x == 0) chunk_nodes(a, T * kItems, level, n, cn);
     for (int k = threadIdx.x; k < 512; k += T) (&sh[0][0])[k] = 0;
     early_launch_wait();
+    if (pass == 0) load();
     if (pass == 0) {
         clear_hist(S, 3, first);
         for (long long t = blockIdx.x * (long long)T + threadIdx.x; t < next; t += (long long)gridDim.x * T) {
@@ -306,16 +316,15 @@ __global__ void __launch_bounds__(T) k_hist(Buffers B, int cur, int level, long 
     __syncthreads();
     if (!live[0] && !live[1]) return;
     const int shift = 24 - 8 * pass;
-    // all rounds' coordinates first (independent loads in flight together), then bins
     float val[kItems];
     int wh[kItems];
-    const Side P = side(B, cur);
 #pragma unroll
     for (int it = 0; it < kItems; ++it) {
         long long i = a + it * T + threadIdx.x;
         const int w = i < n ? which(i, cn) : -1;
         wh[it] = w >= 0 && live[w] ? w : -1;
-        val[it] = wh[it] >= 0 ? coord(P, i, ax[wh[it]]) : 0.0f;
+        const int axis = wh[it] >= 0 ? ax[wh[it]] : 0;
+        val[it] = axis == 0 ? px[it] : (axis == 1 ? py[it] : pz[it]);
     }
 #pragma unroll
     for (int it = 0; it < kItems; ++it) {   // every lane runs every round (full-warp match)
@@ -353,6 +362,15 @@ __global__ void __launch_bounds__(T) k_partition(Buffers B, int cur, int level, 
     long long a = blockIdx.x * (long long)(T * kItems);
     if (threadIdx.x == 0) chunk_nodes(a, T * kItems, level, n, cn);
     if (threadIdx.x < 24) sb[threadIdx.x / 6][threadIdx.x % 6] = (threadIdx.x % 6) < 3 ? 0x7fffffff : (int)0x80000000;
+    // the chunk's photons, loaded before the wait (the partition before wrote them)
+    float px[kItems], py[kItems], pz[kItems];
+    uint32_t pid[kItems];
+    const Side S = side(B, cur);
+#pragma unroll
+    for (int it = 0; it < kItems; ++it) {
+        const long long i = a + it * T + threadIdx.x, j = i < n ? i : a;
+        px[it] = __ldcg(&S.x[j]); py[it] = __ldcg(&S.y[j]); pz[it] = __ldcg(&S.z[j]); pid[it] = __ldcg(&S.id[j]);
+    }
     early_launch_wait();
     clear_hist(L, 2, next);
     __syncthreads();
@@ -378,17 +396,12 @@ __global__ void __launch_bounds__(T) k_partition(Buffers B, int cur, int level, 
     // ballots within a warp, then per-(round, warp) offsets
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const unsigned lt_mask = (1u << lane) - 1u;
-    // the photons of all rounds are loaded once, up front (independent loads in flight
-    // together); position past n: -2, ancestor median (stays in place): -1
-    float px[kItems], py[kItems], pz[kItems];
-    uint32_t pid[kItems];
+    // position past n: -2, ancestor median (stays in place): -1
     int cls[kItems], rank[kItems];
-    const Side S = side(B, cur), D = side(B, dst);
+    const Side D = side(B, dst);
 #pragma unroll
     for (int it = 0; it < kItems; ++it) {
         const long long i = a + it * T + threadIdx.x;
-        const long long j = i < n ? i : a;
-        px[it] = S.x[j]; py[it] = S.y[j]; pz[it] = S.z[j]; pid[it] = S.id[j];
         cls[it] = i < n ? which(i, cn) : -2;
     }
 #pragma unroll
