@@ -107,6 +107,7 @@ struct DeviceState {
     DevBuf<int> async_flags;
     cudaGraphExec_t graph_exec = nullptr;
     unsigned long long last_photons = 0, last_queries = 0;
+    bool tuned = false;      // the last eager iteration timed launch shapes
     int mlp_rounds = 0;          // training rounds done (the proposal is used after the first)
     double mlp_last_rows = 0;    // training samples collected in the last round
     int iterations_done = 0;
@@ -611,6 +612,7 @@ int proposal_train(const HostScene& sc, const VMParams& p) {
 template <class Run>
 int autotune_variants(int nvariants, Run&& run, const char* what, long long size) {
     DeviceState& d = ctx().dev;
+    d.tuned = true;
     float best = 1e30f;
     int best_v = 0;
     for (int v = 0; v < nvariants; ++v) {
@@ -750,6 +752,7 @@ int debug_bvh_obj(HostScene& sc) {
 int render_iteration(HostScene& sc, int redo_iteration = -1, bool tune_passes = true) {
     DeviceState& d = ctx().dev;
     cudaStream_t s = d.stream;
+    d.tuned = false;
     int r0 = RC_OK;
     const int it = redo_iteration >= 0 ? redo_iteration : d.iterations_done;
     VMParams p = make_params(sc, it);
@@ -968,6 +971,7 @@ int render_iteration(HostScene& sc, int redo_iteration = -1, bool tune_passes = 
     if (cfg().autotune && nq > 0) {
         std::atomic<int>& slot = gather_slot((long long)nq, n);
         if (slot.load() < 0) {
+            d.tuned = true;
             // time every launch shape on this iteration's queries into a scratch image
             // (warm-up launch first: the first launch of a shape loads its code)
             RC_CUDA(d.tune_accum.reserve(std::max<long long>(3 * npix, 1)));
@@ -1281,8 +1285,9 @@ int async_finish(HostScene& sc, int first_it, int n_async, bool windows) {
 }
 
 
-// `iterations` progressive iterations: the first with host round trips, the rest
-// replayed asynchronously when eligible; overflowed iterations are rendered again.
+// `iterations` progressive iterations: the first (and those that time launch shapes) with
+// host round trips, the rest replayed asynchronously when eligible; overflowed iterations
+// are rendered again.
 int render_iterations(HostScene& sc, int iterations) {
     DeviceState& d = ctx().dev;
     int r = RC_OK;
@@ -1291,10 +1296,13 @@ int render_iterations(HostScene& sc, int iterations) {
         for (; i < iterations && !r; ++i) r = render_iteration(sc);
         return r;
     }
-    if (d.async_pcap == 0 && i < iterations) {
+    while (d.async_pcap == 0 && i < iterations) {
         r = render_iteration(sc);
         ++i;
         if (r) return r;
+        // an iteration that timed launch shapes says nothing of an iteration's length (and its
+        // time kept every scene that met a new size class from being replayed for good)
+        if (d.tuned && cfg().graph_replay != 2) continue;
         // Replay pays where host round trips and launch gaps are a visible share of an
         // iteration (the photon order over the padded capacity costs a little more).
         if (d.stats[9] > kReplayMaxIterationMs && cfg().graph_replay != 2) d.async_pcap = -1;
