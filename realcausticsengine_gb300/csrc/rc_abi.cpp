@@ -639,7 +639,7 @@ std::atomic<int>& camera_slot(long long pixels) {
     return g_tune.camera[size_class(pixels)][std::min(size_class(ctx().dev.num_tris), 31)];
 }
 std::atomic<int>& gather_slot(long long queries, long long photons) {
-    return g_tune.gather[size_class(queries)][std::min(size_class(photons), 31)];
+    return g_tune.gather[size_class(queries)][size_class(photons) / 2];   // (classes of 4x: fewer timings)
 }
 constexpr int kUntunedPass = 2;   // the light and camera passes' shape where nothing was timed
 

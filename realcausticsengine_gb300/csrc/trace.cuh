@@ -300,7 +300,7 @@ __device__ __forceinline__ bool scene_hit(const SceneView& s, F3 o, F3 d, float 
     out.t = INFINITY; out.u = 0.0f; out.v = 0.0f; out.slot = -1;
     bool hit = false;
     if (s.num_world_nodes == 1) {
-        // single world leaf: the common case (one leaf holding every mesh)
+        // single world leaf (a scene of one mesh)
         float4 lo = __ldg(&s.wnode_lo[0]);
         float4 hi = __ldg(&s.wnode_hi[0]);
         if (!box_hit(lo, hi, o, inv, tmin, out.t)) return false;
