@@ -3,9 +3,9 @@ workload (512x512-vertex water heightfield, GGX dielectric roughness 0.02 IOR 1.
 diffuse floor 1.5 below, 2x2 area light, 1920x1080, 16M photons per iteration, max
 path depth 8), one JSON line on stdout.
 
-A step is one progressive iteration: light pass (16M light paths, photon store), GPU
-KD-tree build over the stored photons, camera pass (one path per pixel, merge
-queries), radius gather with FP64 accumulation.
+A step is one progressive iteration: light pass (16M light paths, photon store), the
+stored photons sorted in space with a tree of boxes over them, camera pass (one path
+per pixel, merge queries), radius gather with FP64 accumulation.
 
   value   photons/s with the scene already resident in HBM (device-timed with CUDA
           events recorded by the library on its stream around the K steps)
@@ -53,10 +53,10 @@ PHOTON_BYTES, QUERY_BYTES, PIXEL_BYTES = 40, 64, 48
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) over algorithmic bytes of one
 # k_gather launch on the 960x540 / 4M-path water pool (profiles/k_gather_water_pool_960x540.md)
 GATHER_TRAFFIC_OVER_ALGORITHMIC = 1.161
-# SM issue efficiency of the persistent light pass from the same kind of capture
-# (profiles/k_light_pass_water_pool_960x540.md): issue-active cycles and thread
+# SM issue efficiency of the staged light pass from the same kind of capture, its two
+# launches together (profiles/light_pass_staged_water_pool_960x540.md): issue-active cycles and thread
 # instructions per warp instruction
-LIGHT_ISSUE_ACTIVE_PCT, LIGHT_LANES_ACTIVE = 62.2, 10.3
+LIGHT_ISSUE_ACTIVE_PCT, LIGHT_LANES_ACTIVE = 51.7, 17.1
 
 
 def dist_env():
@@ -334,7 +334,7 @@ def run_ours(args):
                      "bytes_formula": "40 B x stored photons + 64 B x merge queries + 48 B x pixels",
                      "touched_bytes": touched,
                      "touched_frac": (touched / (gather_ms_mean / 1000.0) / 1e9) / peak if gather_ms_mean > 0 else 0.0},
-        "kd_roofline": kd_roofline(nph, st["kd_ms"], peak, peak_kind),
+        "photon_order_roofline": photon_order_roofline(nph, st["kd_ms"], peak, peak_kind),
         "gpu_launches": int(dev[3]),
         "clocks": clk.summary(),
         "phase_ms_per_step": {k: st[k] for k in ("light_ms", "kd_ms", "camera_ms", "gather_ms")},
@@ -342,11 +342,11 @@ def run_ours(args):
             "paths_per_s": paths / (st["light_ms"] / 1000.0) if st["light_ms"] > 0 else None,
             "rays_per_s": st["light_rays"] / (st["light_ms"] / 1000.0) if st["light_ms"] > 0 and st["light_rays"] else None,
             "rays_per_path": st["light_rays"] / paths if st["light_rays"] else None,
-            # ncu on the 960x540 / 4M-path case (profiles/k_light_pass_water_pool_960x540.md)
+            # ncu on the 960x540 / 4M-path case (profiles/light_pass_staged_water_pool_960x540.md)
             "issue_active_pct_ncu": LIGHT_ISSUE_ACTIVE_PCT, "lanes_active_per_warp_instruction_ncu": LIGHT_LANES_ACTIVE,
             "note": "window of the last iteration's light pass (the coherent path order included)"},
         "phase_note": "event windows of the last iteration; the camera pass runs on a second stream "
-                      "beside the light pass's last launch and the KD build, its window opening there",
+                      "beside the light pass and the photon order (kd_ms), its window opening at the fork",
         "wall_s": wall,
     }
     if not args.no_learned:
@@ -361,9 +361,8 @@ def kd_roofline(nph: float, kd_ms: float, peak: float, peak_kind: str) -> dict:
     """The KD build against the HBM roofline with the algorithmic bytes of a median-split
     build over P photons: 12 P (positions read once) + 2 x 16 P per level over ceil(log2 P)
     levels (x, y, z, id read and written) + 8 B per node of the 2^(floor(log2 P) + 1)-node
-    array.  kd_ms is the event window of the build, its boxes and the tree-order records,
-    with the camera pass running beside them on the other stream (so a lower bound on
-    the build's own rate)."""
+    array.  For a build of the reference's tree (rc_kd_build_noalloc) that took kd_ms; an
+    iteration sorts its photons instead (photon_order_roofline)."""
     import math
     P = float(nph)
     if P < 2 or kd_ms <= 0:
@@ -373,6 +372,20 @@ def kd_roofline(nph: float, kd_ms: float, peak: float, peak_kind: str) -> dict:
     return {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
             "peak_source": peak_kind, "algorithmic_bytes": b, "window_ms": kd_ms,
             "bytes_formula": "12 P + 32 P ceil(log2 P) + 8 x 2^(floor(log2 P) + 1)"}
+
+
+def photon_order_roofline(nph: float, kd_ms: float, peak: float, peak_kind: str) -> dict | None:
+    """The photon order against the HBM roofline: P photons' 40-byte records read and written
+    in sorted order once.  kd_ms is the event window of the keys, the sort, the records and
+    the boxes, with the camera pass running beside them on the other stream (so a lower
+    bound on the order's own rate)."""
+    P = float(nph)
+    if P < 2 or kd_ms <= 0:
+        return None
+    b = 80.0 * P
+    achieved = b / (kd_ms / 1000.0) / 1e9
+    return {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
+            "peak_source": peak_kind, "algorithmic_bytes": b, "window_ms": kd_ms, "bytes_formula": "80 P"}
 
 
 def same_config_anchor(cpu: dict | None, width: int = 960, height: int = 540, steps: int = 8, warmup: int = 2):
@@ -476,7 +489,7 @@ def run_batch(args):
     device buffers); --batch-threads host threads load the scenes through init() and
     prepare them (BVH build, upload).  Then rc_batch_render renders all of them as one
     launch set per iteration (one light pass and one camera pass over every scene, the
-    per-scene KD builds and gathers as branches of one CUDA graph): --warmup iterations
+    per-scene photon orders and gathers as branches of one CUDA graph): --warmup iterations
     (each scene's first iteration alone, the batch passes' shape tuning, the graph's
     instantiation), then --steps timed iterations.  value = photons of all scenes over
     the device time of the timed iterations (CUDA events on the batch stream, all scenes

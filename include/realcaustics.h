@@ -133,7 +133,7 @@ typedef struct rc_config {
     /* 1 (default): with the uniform sampler and no learned proposal, when an iteration
      * takes under 20 ms of device time, the iterations after the first of a
      * configuration are enqueued without host round trips (fixed photon and query
-     * capacities from the previous counts, KD tree over the padded photon capacity) and
+     * capacities from the previous counts, photon order over the padded capacity) and
      * replayed as an updated CUDA graph; an iteration whose counts outgrow the
      * capacities is rendered again at the end of the call.  0: every iteration reads its
      * counts back.  2: as 1 with capacities equal to the measured counts and no time
@@ -193,7 +193,7 @@ int rc_context_destroy(rc_context* ctx);
  * (distinct contexts, each with a scene from init() and the uniform sampler without the
  * learned proposal) as one launch set per iteration: one persistent light pass over all
  * scenes' light paths, one persistent camera pass over all scenes' pixels, and each
- * scene's light-path order, KD build, query order and gather as parallel branches of the
+ * scene's light-path order, photon order, query order and gather as parallel branches of the
  * same CUDA graph, which is captured, updated in place and replayed per iteration.  A
  * scene that has rendered no iteration yet renders its first one alone first (it fixes
  * the photon and query capacities of the graph); an iteration whose counts outgrow
