@@ -1124,7 +1124,7 @@ int async_head(VMParams& p, cudaStream_t s, bool order) {
 
 // async_tail, on s after the light pass: the photon capacity padded, the photon order with
 // its boxes and records; beside it, on `side` once the camera pass has recorded
-// `camera_done`, the query order; then the count check (`flag` = 1 on an overflow) and
+// `camera_done` and a pass that fills the GPU has ended, the query order; then the count check (`flag` = 1 on an overflow) and
 // the gather.  (A batch passes s itself: its scenes' tails run beside one another already.)
 int async_tail(HostScene& sc, const VMParams& p, cudaStream_t s, cudaStream_t side, cudaEvent_t camera_done, int* flag) {
     DeviceState& d = ctx().dev;
@@ -1139,6 +1139,16 @@ int async_tail(HostScene& sc, const VMParams& p, cudaStream_t s, cudaStream_t si
                                    0.0f);
     launch_pad_photons(d.ph_pos.p, d.counters.p, pc, pad, s);
     RC_CUDA(record(d.ev[2], s));
+    if (side != s && light_order_pays(p.num_light_paths)) {
+        // the query order not before the light pass has ended: its sort takes most of an SM's
+        // L1 as shared memory, and the light pass's blocks placed on that SM meanwhile ran with
+        // what was left to their end.  1080p water pool (16.7M paths): iterations of 13.5, 14.8
+        // or 15.9 ms as it fell out, now 13.5 to 13.8; a 1283x717 update 7.45 ms, now 7.19.
+        // (Passes too small to fill the GPU: 414 us an update of 6,144 paths either way, and
+        // there the query order is worth starting early.)
+        RC_CUDA(cudaEventRecord(d.fork, s));
+        RC_CUDA(cudaStreamWaitEvent(side, d.fork, 0));
+    }
     const CurveFrame frame = scene_frame(sc, p);
     const PhotonTree tree = photon_tree(d, pc);
     const TreePhotons tph{d.tp0.p, d.tp1.p, d.tp2.p};
