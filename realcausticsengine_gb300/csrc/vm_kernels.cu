@@ -434,7 +434,8 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) k_camera_pass_batch(const 
 //
 // What bounds the passes is the instruction issue of the closest-hit search (repeating the
 // search doubles k_pass_first's time); a step of 32 lanes at different places of the tree
-// had 9 to 10 of them active.  The search by phases (search_run) has 13 to 15.  Measured
+// had 9 to 10 of them active.  With the search by phases (search_run) k_pass_first has 21,
+// k_pass_rest 13 (960x540 water pool, 4.2M paths).  Measured
 // against the best persistent shape: light pass of the 1080p water pool (16.7M paths)
 // 11.3 -> 9.6 ms, of 2,000 gems (4.2M paths) 35.9 -> 21.1 ms.  Tried and lost: one
 // kernel that holds the continuing paths back per warp in global memory and switches
