@@ -9,7 +9,9 @@ namespace rc {
 // memory is visible, then lets the next such launch start.  Above it nothing may be touched
 // that the launch before writes, and nothing written that it reads; what the launch before
 // that one wrote is complete (read past L1: __ldcg), because the launch before let this one
-// start after its own wait.
+// start after its own wait.  The kernel's pointers carry no __restrict__: a load through a
+// const restrict pointer may be taken for a read of constant memory, past the wait's clobber
+// and past L1 coherence.
 __device__ __forceinline__ void early_launch_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -551,9 +551,9 @@ __device__ __forceinline__ bool train_backward(TrainCta& t, bool first) {
     return true;
 }
 
-__global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_train(const MlpParams P, const float4* __restrict__ pos,
-                                                                const float4* __restrict__ dir, int n, float inv_n,
-                                                                float* __restrict__ part, int* err) {
+__global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_train(const MlpParams P, const float4* pos,
+                                                                const float4* dir, int n, float inv_n, float* part,
+                                                                int* err) {
     extern __shared__ __align__(1024) unsigned char sm[];
     __shared__ __align__(8) uint64_t mbar;
     __shared__ uint32_t tmem_base;
@@ -655,9 +655,8 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_train(const MlpParams 
 // step.  A block takes 32 consecutive parameters, its 8 warps an eighth of the partial
 // rows each.
 constexpr int kReduceWarps = 8;
-__global__ void __launch_bounds__(32 * kReduceWarps) k_reduce_adam(const MlpParams P, const float* __restrict__ part,
-                                                                   int nparts, int apply, float lr, float b1t, float b2t,
-                                                                   float* __restrict__ loss) {
+__global__ void __launch_bounds__(32 * kReduceWarps) k_reduce_adam(const MlpParams P, const float* part, int nparts,
+                                                                   int apply, float lr, float b1t, float b2t, float* loss) {
     __shared__ float sums[kReduceWarps][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int j = blockIdx.x * 32 + lane;   // parameter, or the loss
