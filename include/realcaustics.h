@@ -341,6 +341,11 @@ int rc_gather_query(int variant, int n, const float* positions, int q, const flo
                     int* counts, int* idx, long long cap, long long* total);
 int rc_gather_variants(void);
 
+/* Items that the calling thread's last rc_gather_query asked the parked list for in its
+ * count pass (shapes that park a focus's work for a second launch; 0 for the others).  The
+ * list holds 65,535; what does not fit is done where it was found. */
+long long rc_gather_parked_items(void);
+
 /* PCI bus id ("domain:bus:device.function") of the CUDA device the calling thread
  * uses, for tools that address GPUs by bus id (nvidia-smi numbers GPUs physically and
  * ignores CUDA_VISIBLE_DEVICES).  len >= 13. */

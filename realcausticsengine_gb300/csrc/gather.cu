@@ -424,10 +424,12 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, MinBlocks)
     };
 
     // Room for `add` parked items, from `at`; without it the items given below the end are
-    // void and the warp parks no more.
+    // void and the warp parks no more.  A full list is not asked again: the count stays
+    // below kParkedItems and one request of every warp in flight, however many groups the
+    // launch has (counted for all of them it wraps at 2^32: 3.6M groups of some 1,200).
     auto reserve_items = [&](uint32_t add) -> uint32_t {
-        uint32_t at = 0;
-        if (lane == 0) at = atomicAdd(&parked[0].x, add);
+        uint32_t at = (uint32_t)kParkedItems;
+        if (lane == 0 && __ldcg(&parked[0].x) < (uint32_t)kParkedItems) at = atomicAdd(&parked[0].x, add);
         at = __shfl_sync(kFull, at, 0);
         park = at + add <= (uint32_t)kParkedItems;
         return at;

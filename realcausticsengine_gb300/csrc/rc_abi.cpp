@@ -2453,6 +2453,10 @@ int rc_device_bus_id(char* out, int len) {
     return RC_OK;
 }
 
+static thread_local uint32_t t_parked_items = 0;
+
+long long rc_gather_parked_items(void) { return t_parked_items; }
+
 int rc_gather_query(int variant, int n, const float* positions, int q, const float* queries, float r2, int* counts,
                     int* idx, long long cap, long long* total) {
     if (n < 0 || q < 0 || (n > 0 && !positions) || (q > 0 && (!queries || !counts))) { ctx().err = "bad KD arrays"; return RC_E_INVALID; }
@@ -2488,6 +2492,9 @@ int rc_gather_query(int variant, int n, const float* positions, int q, const flo
                                nullptr, err.p, s);
             RC_CUDA(cudaGetLastError());
             int h = 0;
+            t_parked_items = 0;
+            if (gather_parks(variant))
+                RC_CUDA(cudaMemcpyAsync(&t_parked_items, parked.p, 4, cudaMemcpyDeviceToHost, s));
             RC_CUDA(cudaMemcpyAsync(counts, cnt.p, 4 * (size_t)q, cudaMemcpyDeviceToHost, s));
             RC_CUDA(cudaMemcpyAsync(&h, err.p, sizeof(int), cudaMemcpyDeviceToHost, s));
             RC_CUDA(cudaStreamSynchronize(s));
