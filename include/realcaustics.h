@@ -149,6 +149,14 @@ typedef struct rc_config {
 int rc_default_config(rc_config* cfg);
 int rc_set_config(const rc_config* cfg);
 
+/* The device memory that the bound context's light and camera passes may each take for the
+ * paths a staged launch shape parks between its two launches (48 bytes a path, at most
+ * 800 MB), and a batch rendered by it for each of its two passes; negative (the default): no
+ * limit.  A pass whose scratch is over the limit, or cannot be allocated, runs in a
+ * persistent shape, which needs none: the same photons and queries, slower where the
+ * searches are long.  Nothing is timed there, so no shape is chosen for other contexts. */
+int rc_pass_scratch_limit(long long bytes);
+
 /* Stage the scene: BVH build + upload + light conversion (the pre-render half of main,
  * src/main.cpp:150-168).  Called implicitly by rc_render/main. */
 int rc_prepare(void);

@@ -32,6 +32,7 @@ def lib() -> C.CDLL:
     L.main.restype = C.c_int
     L.rc_default_config.argtypes = [C.POINTER(abi.RcConfig)]
     L.rc_set_config.argtypes = [C.POINTER(abi.RcConfig)]
+    L.rc_pass_scratch_limit.argtypes = [C.c_longlong]
     L.rc_prepare.argtypes = []
     L.rc_prepare_host.argtypes = [C.POINTER(C.c_float)]
     L.rc_host_mesh_bvh.argtypes = [C.c_int, C.c_void_p, C.c_int, C.c_void_p, C.c_int, C.POINTER(C.c_float)]
@@ -85,7 +86,7 @@ def check(rc: int, what: str = "") -> None:
         raise NativeError(f"{what} failed ({rc}): {msg}")
 
 
-EXPORTS = ["init", "main", "rc_default_config", "rc_set_config", "rc_prepare", "rc_prepare_host",
+EXPORTS = ["init", "main", "rc_default_config", "rc_set_config", "rc_pass_scratch_limit", "rc_prepare", "rc_prepare_host",
            "rc_host_mesh_bvh", "rc_host_world_bvh", "rc_render", "rc_read_image", "rc_release",
            "rc_last_error", "rc_get_stats", "rc_trace_rays", "rc_trace_rays_full", "rc_trace_rays_shape", "rc_kd_query",
            "rc_kd_build_nodes", "rc_light_photons", "rc_render_timed", "rc_kd_build_noalloc",

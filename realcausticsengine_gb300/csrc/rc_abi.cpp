@@ -187,6 +187,7 @@ struct Context {
     bool host_ready = false;
     double prep[5] = {};                   // rc_prepare_stats
     std::unique_ptr<GpuBvhBuilder> bvh;    // device BVH scratch, kept for the context (grow-only)
+    long long park_limit = -1;             // bytes a staged pass's parked paths may take (-1: no limit)
 };
 
 Context& default_ctx() {
@@ -608,7 +609,9 @@ int proposal_train(const HostScene& sc, const VMParams& p) {
 }
 
 // Autotuner: time each launch variant of a pass (warm-up launch, then one timed launch;
-// `run(v)` must reset whatever the pass appends to) and return the fastest.
+// `run(v)` must reset whatever the pass appends to) and return the fastest.  Called only
+// where every variant's scratch can be had: one that could not run would measure as the
+// fastest, and the choice is kept for every context of the process.
 template <class Run>
 int autotune_variants(int nvariants, Run&& run, const char* what, long long size) {
     DeviceState& d = ctx().dev;
@@ -643,14 +646,23 @@ std::atomic<int>& gather_slot(long long queries, long long photons) {
 }
 constexpr int kUntunedPass = 2;   // the light and camera passes' shape where nothing was timed
 
-// The scratch of a staged pass over n paths (nullptr for a persistent shape); a capturing
+// A pass over n paths in shape v: its scratch (nullptr for a persistent shape), or a persistent
+// shape where a staged one's scratch (48 B a path, at most 800 MB) cannot be had.  A capturing
 // stream needs it reserved before (async_setup).
-int reserve_park(DevBuf<unsigned char>& b, int v, long long n, void** park) {
+int fitting_shape(const Context& c, DevBuf<unsigned char>& b, int v, long long n, void** park) {
     *park = nullptr;
-    if (!pass_is_staged(v)) return RC_OK;
-    RC_CUDA(b.reserve(pass_park_bytes(n)));
-    *park = b.p;
-    return RC_OK;
+    if (!pass_is_staged(v)) return v;
+    const size_t bytes = pass_park_bytes(n);
+    if (c.park_limit < 0 || bytes <= (size_t)c.park_limit) {
+        if (b.reserve(bytes) == cudaSuccess) { *park = b.p; return v; }
+        cudaGetLastError();   // (the allocation's error)
+    }
+    return kUntunedPass;
+}
+constexpr int kStagedPass = 4;   // any staged shape: all take the same scratch
+bool staged_fits(const Context& c, DevBuf<unsigned char>& b, long long n) {
+    void* park;
+    return fitting_shape(c, b, kStagedPass, n, &park) == kStagedPass;
 }
 
 // The light pass in launch shape v.  `tail`, if given, is recorded first: work forked from
@@ -659,8 +671,7 @@ int reserve_park(DevBuf<unsigned char>& b, int v, long long n, void** park) {
 int light_pass(const VMParams& p, PhotonBuf ph, cudaStream_t s, int v, cudaEvent_t tail = nullptr) {
     DeviceState& d = ctx().dev;
     void* park = nullptr;
-    const int r = reserve_park(d.light_park, v, p.num_light_paths, &park);
-    if (r) return r;
+    v = fitting_shape(ctx(), d.light_park, v, p.num_light_paths, &park);
     if (tail) RC_CUDA(cudaEventRecord(tail, s));
     launch_light_pass(p, ph, d.counters.p + 6, s, v, d.counters.p + 8, park);
     return RC_OK;
@@ -669,8 +680,7 @@ int light_pass(const VMParams& p, PhotonBuf ph, cudaStream_t s, int v, cudaEvent
 int camera_pass(const VMParams& p, QueryBuf qb, cudaStream_t s, int v) {
     DeviceState& d = ctx().dev;
     void* park = nullptr;
-    const int r = reserve_park(d.camera_park, v, (long long)p.camera.width * p.camera.height, &park);
-    if (r) return r;
+    v = fitting_shape(ctx(), d.camera_park, v, (long long)p.camera.width * p.camera.height, &park);
     launch_camera_pass(p, qb, d.counters.p + 7, s, v, park);
     return RC_OK;
 }
@@ -846,7 +856,7 @@ int render_iteration(HostScene& sc, int redo_iteration = -1, bool tune_passes = 
         int lvar = 0;
         if (sampler == RC_SAMPLER_UNIFORM && cfg().autotune) {
             std::atomic<int>& slot = light_slot(p.num_light_paths);
-            if (slot.load() < 0 && tune_passes)
+            if (slot.load() < 0 && tune_passes && staged_fits(ctx(), d.light_park, p.num_light_paths))
                 slot = autotune_variants(pass_variants(), [&](int v) {
                     cudaMemsetAsync(d.counters.p, 0, sizeof(unsigned long long), s);
                     light_pass(p, ph, s, v);
@@ -938,7 +948,7 @@ int render_iteration(HostScene& sc, int redo_iteration = -1, bool tune_passes = 
         int cvar = 0;
         if (cfg().autotune) {
             std::atomic<int>& slot = camera_slot(npix);
-            if (slot.load() < 0 && tune_passes)
+            if (slot.load() < 0 && tune_passes && staged_fits(ctx(), d.camera_park, npix))
                 slot = autotune_variants(pass_variants(), [&](int v) {
                     cudaMemsetAsync(d.counters.p + 1, 0, sizeof(unsigned long long), s);
                     camera_pass(p, qb, s, v);
@@ -1103,9 +1113,8 @@ int async_setup(const HostScene& sc) {
     // the staged passes' scratch: reserved before any capture
     const long long paths = cfg().photons_per_iter > 0 ? cfg().photons_per_iter : npix;
     void* park = nullptr;
-    r = reserve_park(d.light_park, d.async_lvar, paths, &park);
-    if (!r) r = reserve_park(d.camera_park, d.async_cvar, npix, &park);
-    if (r) return r;
+    d.async_lvar = fitting_shape(ctx(), d.light_park, d.async_lvar, paths, &park);
+    d.async_cvar = fitting_shape(ctx(), d.camera_park, d.async_cvar, npix, &park);
     return RC_OK;
 }
 
@@ -1482,11 +1491,8 @@ int batch_render(Context* const* cs, int n, int iterations, double* out) {
     RC_CUDA(B.scenes.reserve(entries.size()));
     RC_CUDA(B.prefix.reserve(prefix.size()));
     RC_CUDA(B.next.reserve(2));
-    const bool tuned = g_batch_light.load() >= 0 && g_batch_camera.load() >= 0;
-    if (!tuned || pass_is_staged(g_batch_light.load()))
-        RC_CUDA(B.light_park.reserve(pass_park_bytes(*std::max_element(total_paths.begin(), total_paths.end()))));
-    if (!tuned || pass_is_staged(g_batch_camera.load()))
-        RC_CUDA(B.camera_park.reserve(pass_park_bytes(*std::max_element(total_pixels.begin(), total_pixels.end()))));
+    const long long most_paths = *std::max_element(total_paths.begin(), total_paths.end());
+    const long long most_pixels = *std::max_element(total_pixels.begin(), total_pixels.end());
     RC_CUDA(cudaMemcpy(B.scenes.p, entries.data(), entries.size() * sizeof(BatchScene), cudaMemcpyHostToDevice));
     RC_CUDA(cudaMemcpy(B.prefix.p, prefix.data(), prefix.size() * sizeof(long long), cudaMemcpyHostToDevice));
     RC_CUDA(cudaStreamCreateWithFlags(&B.main, cudaStreamNonBlocking));
@@ -1503,8 +1509,9 @@ int batch_render(Context* const* cs, int n, int iterations, double* out) {
         RC_CUDA(cudaEventCreate(e));
     // 3. launch shapes of the batch passes, timed once per process on the first
     //    iteration's scenes (warm-up launch, then a timed one; the graph resets every
-    //    counter the passes append to)
-    if (g_batch_light.load() < 0 || g_batch_camera.load() < 0) {
+    //    counter the passes append to), where every shape's scratch can be had
+    if ((g_batch_light.load() < 0 || g_batch_camera.load() < 0) && staged_fits(*caller, B.light_park, most_paths) &&
+        staged_fits(*caller, B.camera_park, most_pixels)) {
         const int m = (int)active[0].size();
         const BatchScene* sc0 = B.scenes.p + entry_at[0];
         const long long* pp = B.prefix.p + prefix_at[0];
@@ -1546,7 +1553,12 @@ int batch_render(Context* const* cs, int n, int iterations, double* out) {
             std::printf("{\"autotune\": \"batch passes\", \"light\": %d, \"camera\": %d}\n", g_batch_light.load(),
                         g_batch_camera.load());
     }
-    const int lvar = g_batch_light.load(), cvar = g_batch_camera.load();
+    auto batch_shape = [&](int tuned, DevBuf<unsigned char>& b, long long n_items) {
+        void* park = nullptr;
+        return fitting_shape(*caller, b, tuned >= 0 ? tuned : kUntunedPass, n_items, &park);
+    };
+    const int lvar = batch_shape(g_batch_light.load(), B.light_park, most_paths);
+    const int cvar = batch_shape(g_batch_camera.load(), B.camera_park, most_pixels);
     // 4. one graph per iteration: captured, the executable graph updated in place (or
     //    instantiated) and launched
     double kernels = 0;
@@ -2030,6 +2042,17 @@ int rc_set_config(const rc_config* c) {
     // sizes and shapes of asynchronous iterations are re-derived under the new settings
     ctx().dev.async_pcap = ctx().dev.async_qcap = 0;
     if (ctx().dev.graph_exec) { cudaGraphExecDestroy(ctx().dev.graph_exec); ctx().dev.graph_exec = nullptr; }
+    return RC_OK;
+}
+
+int rc_pass_scratch_limit(long long bytes) {
+    ctx().park_limit = bytes < 0 ? -1 : bytes;
+    // iterations recorded as a graph hold the shapes chosen under the old limit
+    DeviceState& d = ctx().dev;
+    d.light_park.release();
+    d.camera_park.release();
+    d.async_pcap = d.async_qcap = 0;
+    if (d.graph_exec) { cudaGraphExecDestroy(d.graph_exec); d.graph_exec = nullptr; }
     return RC_OK;
 }
 
