@@ -938,8 +938,9 @@ int render_iteration(HostScene& sc, int redo_iteration = -1, bool tune_passes = 
         if (!cam_done) qcap = (long long)nq + nq / 8 + 1024;
     }
     // a side-stream camera pass of an earlier iteration that returned an error may
-    // still be writing the query buffers (a wait before the event's first record is void)
-    if (!cam_side) RC_CUDA(cudaStreamWaitEvent(s, d.join, 0));
+    // still be writing the query buffers (not a wait for its event, which a replayed
+    // iteration may have recorded in its graph since)
+    if (!cam_side) RC_CUDA(cudaStreamSynchronize(d.side));
     for (int attempt = 0; attempt < 3 && !cam_done; ++attempt) {
         RC_CUDA(d.q0.reserve(qcap)); RC_CUDA(d.q1.reserve(qcap)); RC_CUDA(d.q2.reserve(qcap));
         RC_CUDA(d.q3.reserve(qcap)); RC_CUDA(d.q4.reserve(qcap));
