@@ -92,3 +92,40 @@ def test_no_shape_is_kept_from_a_context_without_scratch():
     passes = [[t for t in p if t != "gather"] for p in tuned]
     assert passes[0] == [] and passes[2] == []
     assert sorted(passes[1]) == ["batch passes", "camera pass", "light pass"]
+
+
+BATCH_FIRST = """
+import ctypes, sys, numpy as np
+sys.path.insert(0, {root!r})
+from realcausticsengine_gb300 import scenes
+from realcausticsengine_gb300.session import Context, Renderer, batch_render
+c = Context()
+with c:
+    r = Renderer(scenes.water_pool(160, 90, grid=24), photons_per_iter=300000, max_path_length=8, seed=4, verbose=True)
+    batch_render([c], 3)
+    ctypes.CDLL(None).fflush(None)
+    print("alone", flush=True)
+    r.render(2)
+    r.render(2)
+    assert r.stats()["iterations"] == 7
+    image = r.image()
+    r.release()
+    r = Renderer(scenes.water_pool(160, 90, grid=24), photons_per_iter=300000, max_path_length=8, seed=4)
+    r.render(7)
+    np.testing.assert_allclose(image, r.image(), rtol=1e-5, atol=1e-7)
+    r.release()
+c.destroy()
+"""
+
+
+def test_a_scene_first_rendered_in_a_batch_times_its_own_passes():
+    """The batch renders a scene's first iteration without timing the scene's own passes; the
+    first render of the scene alone does it, once, and goes on to replay."""
+    out = subprocess.run([sys.executable, "-c", BATCH_FIRST.format(root=str(ROOT))], capture_output=True, text=True,
+                         timeout=300)
+    assert out.returncode == 0, out.stderr
+    batch, alone = out.stdout.split("alone\n")
+    assert '{"autotune": "light pass"' not in batch and '{"autotune": "camera pass"' not in batch
+    for name in ("light pass", "camera pass"):
+        assert alone.count('{"autotune": "%s"' % name) == 1
+    assert '{"replayed_iterations": 2' in alone
