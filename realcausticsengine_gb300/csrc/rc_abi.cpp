@@ -157,19 +157,26 @@ struct DeviceState {
     }
 };
 
-// Autotuner choices: launch variant per size class (log2 of light paths or pixels, and of
-// the scene's triangles; log2 of queries and of photons), -1 = untuned.  Kept for the
-// process and shared by every context (a new scene, or a scene in another context, reuses
-// them).  The triangles are in the key because the light and camera passes' best shape depends on how
-// long a search is: at 4.2M light paths 2,000 gems (261k triangles) run 20.7 ms staged
-// against 35.4, at 1M a glass sphere (20k) 0.53 ms staged against 0.38.  The photons are in
-// the gather's because they tell a caustic's focus from a wide floor: 216k queries take 120
+// Autotuner choices: launch variant per size class (log2 of light paths or pixels, and
+// classes of 16x of the scene's triangles; log2 of queries, and classes of 4x of photons),
+// -1 = untuned.  Kept for the process and shared by every context (a new scene, or a scene
+// in another context, reuses them).  The triangles are in the key because the light and
+// camera passes' best shape depends on how long a search is: at 2.5M light paths 1,000 gems
+// (130k triangles) run 9.4 ms staged against 14.7, displaced spheres (16k) 0.97 staged
+// against 0.73.  No finer, because every new class is timed in some call: within a kind of
+// scene (displaced spheres, glass spheres, water; 1k to 1M triangles, 30k to 2.5M paths) the
+// better family changed once, by 6% (328k triangles of glass spheres), and twelve stills of
+// 2k to 300k triangles took 432 ms the first time with classes of 2x and every shape launched
+// twice, 234 now (and 122 when all classes are known).  The photons are in the gather's
+// because they tell a caustic's focus from a wide floor: 216k queries take 120
 // us parked against 783 with 20k photons of one; without one parking only costs.
 struct TuneTables {
-    std::atomic<int> light[64][32], camera[64][32], gather[64][32];
+    std::atomic<int> light[64][8], camera[64][8], gather[64][32];
     TuneTables() {
         for (int i = 0; i < 64; ++i) {
-            for (int j = 0; j < 32; ++j) { light[i][j] = -1; camera[i][j] = -1; gather[i][j] = -1; }
+            for (auto& a : light[i]) a = -1;
+            for (auto& a : camera[i]) a = -1;
+            for (auto& a : gather[i]) a = -1;
         }
     }
 };
@@ -608,41 +615,67 @@ int proposal_train(const HostScene& sc, const VMParams& p) {
     return RC_OK;
 }
 
-// Autotuner: time each launch variant of a pass (warm-up launch, then one timed launch;
-// `run(v)` must reset whatever the pass appends to) and return the fastest.  Called only
-// where every variant's scratch can be had: one that could not run would measure as the
-// fastest, and the choice is kept for every context of the process.
-template <class Run>
-int autotune_variants(int nvariants, Run&& run, const char* what, long long size) {
-    DeviceState& d = ctx().dev;
-    d.tuned = true;
+// Autotuner.  ShapeTimer times launch shapes on s between two events: each once, after one
+// untimed launch of the shape if the process has not launched it yet (the first launch loads
+// its code; `loaded` has a bit per shape).
+struct ShapeTimer {
+    cudaStream_t s;
+    cudaEvent_t from, to;
+    std::atomic<unsigned>& loaded;
+    const char* what;
+    bool verbose;
     float best = 1e30f;
     int best_v = 0;
-    for (int v = 0; v < nvariants; ++v) {
+    template <class Run> float time(int v, Run&& run) {
+        if (!((loaded.fetch_or(1u << v) >> v) & 1u)) run(v);
+        cudaEventRecord(from, s);
         run(v);
-        cudaEventRecord(d.evm[0], d.stream);
-        run(v);
-        cudaEventRecord(d.evm[1], d.stream);
-        cudaEventSynchronize(d.evm[1]);
-        const float ms = ms_between(d.evm[0], d.evm[1]);
-        if (cfg().verbose) std::printf("{\"autotune_shape\": \"%s\", \"variant\": %d, \"ms\": %.3f}\n", what, v, ms);
+        cudaEventRecord(to, s);
+        cudaEventSynchronize(to);
+        const float ms = ms_between(from, to);
+        if (verbose) std::printf("{\"autotune_shape\": \"%s\", \"variant\": %d, \"ms\": %.4f}\n", what, v, ms);
         if (ms < best) { best = ms; best_v = v; }
+        return ms;
     }
-    if (cfg().verbose)
-        std::printf("{\"autotune\": \"%s\", \"size\": %lld, \"variant\": %d, \"ms\": %.3f}\n", what, size, best_v,
-                    best);
-    return best_v;
+};
+std::atomic<unsigned> g_light_loaded{0}, g_camera_loaded{0}, g_gather_loaded{0};
+
+// The fastest shape of a light or camera pass (`run(v)` must reset whatever the pass appends
+// to).  Called only where every shape's scratch can be had: one that could not run would
+// measure as the fastest, and the choice is kept for every context of the process.  One
+// persistent and one staged shape are timed first; a family that is slower by more than
+// kFamilyMargin is not timed further (within a family the shapes differ by up to 15%; between
+// them by up to 1.9x): 5 to 9 launches for the 14 of two per shape, and fewer slow ones.
+constexpr float kFamilyMargin = 1.15f;
+template <class Run>
+int pick_pass_shape(ShapeTimer& t, Run&& run) {
+    constexpr int kPersistent = 0;
+    const int staged = pass_variants() - 1;
+    run(kPersistent);   // (the scene's data into L2)
+    const float p = t.time(kPersistent, run), q = t.time(staged, run);
+    for (int v = 0; v < pass_variants(); ++v) {
+        if (v == kPersistent || v == staged) continue;
+        if (pass_is_staged(v) ? q < kFamilyMargin * p : p < kFamilyMargin * q) t.time(v, run);
+    }
+    return t.best_v;
+}
+template <class Run>
+int autotune_pass(std::atomic<unsigned>& loaded, const char* what, long long size, Run&& run) {
+    DeviceState& d = ctx().dev;
+    d.tuned = true;
+    ShapeTimer t{d.stream, d.evm[0], d.evm[1], loaded, what, cfg().verbose != 0};
+    const int v = pick_pass_shape(t, run);
+    if (t.verbose)
+        std::printf("{\"autotune\": \"%s\", \"size\": %lld, \"variant\": %d, \"ms\": %.3f}\n", what, size, v, t.best);
+    return v;
 }
 
 int size_class(long long n) { return n > 0 ? 63 - __builtin_clzll((unsigned long long)n) : 0; }
-std::atomic<int>& light_slot(long long paths) {
-    return g_tune.light[size_class(paths)][std::min(size_class(ctx().dev.num_tris), 31)];
-}
-std::atomic<int>& camera_slot(long long pixels) {
-    return g_tune.camera[size_class(pixels)][std::min(size_class(ctx().dev.num_tris), 31)];
-}
+int triangle_class(long long n) { return std::min(size_class(n) / 4, 7); }
+std::atomic<int>& light_slot(long long paths) { return g_tune.light[size_class(paths)][triangle_class(ctx().dev.num_tris)]; }
+std::atomic<int>& camera_slot(long long pixels) { return g_tune.camera[size_class(pixels)][triangle_class(ctx().dev.num_tris)]; }
 std::atomic<int>& gather_slot(long long queries, long long photons) {
-    return g_tune.gather[size_class(queries)][size_class(photons) / 2];   // (classes of 4x: fewer timings)
+    return g_tune.gather[size_class(queries)][size_class(photons) / 2];
 }
 constexpr int kUntunedPass = 2;   // the light and camera passes' shape where nothing was timed
 
@@ -857,10 +890,10 @@ int render_iteration(HostScene& sc, int redo_iteration = -1, bool tune_passes = 
         if (sampler == RC_SAMPLER_UNIFORM && cfg().autotune) {
             std::atomic<int>& slot = light_slot(p.num_light_paths);
             if (slot.load() < 0 && tune_passes && staged_fits(ctx(), d.light_park, p.num_light_paths))
-                slot = autotune_variants(pass_variants(), [&](int v) {
+                slot = autotune_pass(g_light_loaded, "light pass", p.num_light_paths, [&](int v) {
                     cudaMemsetAsync(d.counters.p, 0, sizeof(unsigned long long), s);
                     light_pass(p, ph, s, v);
-                }, "light pass", p.num_light_paths);
+                });
             lvar = slot.load() >= 0 ? slot.load() : kUntunedPass;
             RC_CUDA(cudaMemsetAsync(d.counters.p, 0, sizeof(unsigned long long), s));
         }
@@ -950,10 +983,10 @@ int render_iteration(HostScene& sc, int redo_iteration = -1, bool tune_passes = 
         if (cfg().autotune) {
             std::atomic<int>& slot = camera_slot(npix);
             if (slot.load() < 0 && tune_passes && staged_fits(ctx(), d.camera_park, npix))
-                slot = autotune_variants(pass_variants(), [&](int v) {
+                slot = autotune_pass(g_camera_loaded, "camera pass", npix, [&](int v) {
                     cudaMemsetAsync(d.counters.p + 1, 0, sizeof(unsigned long long), s);
                     camera_pass(p, qb, s, v);
-                }, "camera pass", npix);
+                });
             cvar = slot.load() >= 0 ? slot.load() : kUntunedPass;
             RC_CUDA(cudaMemsetAsync(d.counters.p + 1, 0, sizeof(unsigned long long), s));
         }
@@ -984,24 +1017,17 @@ int render_iteration(HostScene& sc, int redo_iteration = -1, bool tune_passes = 
         if (slot.load() < 0) {
             d.tuned = true;
             // time every launch shape on this iteration's queries into a scratch image
-            // (warm-up launch first: the first launch of a shape loads its code)
             RC_CUDA(d.tune_accum.reserve(std::max<long long>(3 * npix, 1)));
-            float best = 1e30f;
-            int best_v = variant;
-            for (int v = 0; v < gather_variants(); ++v) {
+            ShapeTimer t{s, d.evm[0], d.evm[1], g_gather_loaded, "gather", cfg().verbose != 0};
+            auto run = [&](int v) {
                 launch_gather(p, tree, tph, qb, d.qorder.p, (long long)nq, d.tune_accum.p, d.gather_parked.p, nullptr, s, v);
-                RC_CUDA(cudaEventRecord(d.evm[0], s));
-                launch_gather(p, tree, tph, qb, d.qorder.p, (long long)nq, d.tune_accum.p, d.gather_parked.p, nullptr, s, v);
-                RC_CUDA(cudaEventRecord(d.evm[1], s));
-                RC_CUDA(cudaEventSynchronize(d.evm[1]));
-                const float ms = ms_between(d.evm[0], d.evm[1]);
-                if (cfg().verbose) std::printf("{\"gather_shape\": %d, \"ms\": %.4f}\n", v, ms);
-                if (ms < best) { best = ms; best_v = v; }
-            }
-            slot = best_v;
+            };
+            run(variant);   // (photons and queries into L2)
+            for (int v = 0; v < gather_variants(); ++v) t.time(v, run);
+            slot = t.best_v;
             if (cfg().verbose)
                 std::printf("{\"autotune\": \"gather\", \"queries\": %llu, \"variant\": \"%s\", \"ms\": %.3f}\n",
-                            nq, gather_variant_name(best_v), best);
+                            nq, gather_variant_name(t.best_v), t.best);
         }
         variant = slot.load();
     }
@@ -1375,6 +1401,7 @@ int render_iterations(HostScene& sc, int iterations) {
 
 // Launch shapes of the batch passes, tuned on the first batch (-1: untuned).
 std::atomic<int> g_batch_light{-1}, g_batch_camera{-1};
+std::atomic<unsigned> g_batch_light_loaded{0}, g_batch_camera_loaded{0};
 
 struct BatchRun {
     cudaStream_t main = nullptr, side = nullptr;
@@ -1522,8 +1549,8 @@ int batch_render(Context* const* cs, int n, int iterations, double* out) {
     for (cudaEvent_t* e : {&B.t0, &B.t1, &B.light_start, &B.light_end, &B.camera_start, &B.camera_end})
         RC_CUDA(cudaEventCreate(e));
     // 3. launch shapes of the batch passes, timed once per process on the first
-    //    iteration's scenes (warm-up launch, then a timed one; the graph resets every
-    //    counter the passes append to), where every shape's scratch can be had
+    //    iteration's scenes where every shape's scratch can be had (the graph resets every
+    //    counter the passes append to)
     if ((g_batch_light.load() < 0 || g_batch_camera.load() < 0) && staged_fits(*caller, B.light_park, most_paths) &&
         staged_fits(*caller, B.camera_park, most_pixels)) {
         const int m = (int)active[0].size();
@@ -1539,31 +1566,20 @@ int batch_render(Context* const* cs, int n, int iterations, double* out) {
             for (int a = 0; a < m; ++a)
                 cudaMemsetAsync(cs[active[0][a]]->dev.counters.p + which, 0, sizeof(unsigned long long), B.main);
         };
-        auto tune = [&](auto&& run) {
-            float best = 1e30f;
-            int best_v = 0;
-            for (int v = 0; v < pass_variants(); ++v) {
-                run(v);
-                cudaEventRecord(B.t0, B.main);
-                run(v);
-                cudaEventRecord(B.t1, B.main);
-                cudaEventSynchronize(B.t1);
-                const float ms = ms_between(B.t0, B.t1);
-                if (ms < best) { best = ms; best_v = v; }
-            }
-            return best_v;
-        };
-        g_batch_light = tune([&](int v) {
+        const bool verbose = caller->cfg_set && caller->cfg.verbose;
+        ShapeTimer light{B.main, B.t0, B.t1, g_batch_light_loaded, "batch light pass", verbose};
+        g_batch_light = pick_pass_shape(light, [&](int v) {
             reset(0);
             launch_light_pass_batch(sc0, pp, m, total_paths[0], B.next.p, B.main, v, B.light_park.p);
         });
-        g_batch_camera = tune([&](int v) {
+        ShapeTimer camera{B.main, B.t0, B.t1, g_batch_camera_loaded, "batch camera pass", verbose};
+        g_batch_camera = pick_pass_shape(camera, [&](int v) {
             reset(1);
             launch_camera_pass_batch(sc0, pp + m + 1, m, total_pixels[0], B.next.p + 1, B.main, v, B.camera_park.p);
         });
         RC_CUDA(cudaStreamSynchronize(B.main));
         RC_CUDA(cudaGetLastError());
-        if (caller->cfg_set && caller->cfg.verbose)
+        if (verbose)
             std::printf("{\"autotune\": \"batch passes\", \"light\": %d, \"camera\": %d}\n", g_batch_light.load(),
                         g_batch_camera.load());
     }
