@@ -172,11 +172,15 @@ struct DeviceState {
 // us parked against 783 with 20k photons of one; without one parking only costs.
 struct TuneTables {
     std::atomic<int> light[64][8], camera[64][8], gather[64][32];
+    // a batch's passes: its paths or pixels in all, its scenes' mean triangles
+    std::atomic<int> batch_light[64][8], batch_camera[64][8];
     TuneTables() {
         for (int i = 0; i < 64; ++i) {
             for (auto& a : light[i]) a = -1;
             for (auto& a : camera[i]) a = -1;
             for (auto& a : gather[i]) a = -1;
+            for (auto& a : batch_light[i]) a = -1;
+            for (auto& a : batch_camera[i]) a = -1;
         }
     }
 };
@@ -1399,8 +1403,6 @@ int render_iterations(HostScene& sc, int iterations) {
 // iteration with host round trips), so the graph holds no host round trip, whatever
 // an iteration's length; overflowed iterations are rendered again afterwards.
 
-// Launch shapes of the batch passes, tuned on the first batch (-1: untuned).
-std::atomic<int> g_batch_light{-1}, g_batch_camera{-1};
 std::atomic<unsigned> g_batch_light_loaded{0}, g_batch_camera_loaded{0};
 
 struct BatchRun {
@@ -1502,6 +1504,7 @@ int batch_render(Context* const* cs, int n, int iterations, double* out) {
     std::vector<long long> prefix;
     std::vector<size_t> entry_at(K), prefix_at(K);
     std::vector<long long> total_paths(K), total_pixels(K);
+    long long triangles = 0;   // of the first iteration's scenes
     for (int j = 0; j < K; ++j) {
         for (int i = 0; i < n; ++i) if (remaining[i] > j) active[j].push_back(i);
         entry_at[j] = entries.size();
@@ -1515,6 +1518,7 @@ int batch_render(Context* const* cs, int n, int iterations, double* out) {
             const int i = active[j][a];
             t_bound = cs[i];
             DeviceState& d = ctx().dev;
+            if (j == 0) triangles += d.num_tris;
             BatchScene b{};
             b.p = make_params(*ctx().scene, first_it[i] + j);
             b.p.path_order = d.path_order.p;
@@ -1548,11 +1552,17 @@ int batch_render(Context* const* cs, int n, int iterations, double* out) {
         RC_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
     for (cudaEvent_t* e : {&B.t0, &B.t1, &B.light_start, &B.light_end, &B.camera_start, &B.camera_end})
         RC_CUDA(cudaEventCreate(e));
-    // 3. launch shapes of the batch passes, timed once per process on the first
-    //    iteration's scenes where every shape's scratch can be had (the graph resets every
-    //    counter the passes append to)
-    if ((g_batch_light.load() < 0 || g_batch_camera.load() < 0) && staged_fits(*caller, B.light_park, most_paths) &&
-        staged_fits(*caller, B.camera_park, most_pixels)) {
+    // 3. launch shapes of the batch passes, timed once per process and size class on the
+    //    first iteration's scenes where every shape's scratch can be had (the graph resets
+    //    every counter the passes append to).  (Under no key, the shapes timed on four glass
+    //    balls gave a batch of four 2,000-gem scenes 103 ms an iteration, its own 53.7; the
+    //    gems' gave the balls 0.93 ms, their own 0.72.)
+    const int tri = triangle_class(triangles / (long long)active[0].size());
+    std::atomic<int>& light_choice = g_tune.batch_light[size_class(most_paths)][tri];
+    std::atomic<int>& camera_choice = g_tune.batch_camera[size_class(most_pixels)][tri];
+    const bool time_light = light_choice.load() < 0 && staged_fits(*caller, B.light_park, most_paths);
+    const bool time_camera = camera_choice.load() < 0 && staged_fits(*caller, B.camera_park, most_pixels);
+    if (time_light || time_camera) {
         const int m = (int)active[0].size();
         const BatchScene* sc0 = B.scenes.p + entry_at[0];
         const long long* pp = B.prefix.p + prefix_at[0];
@@ -1568,27 +1578,27 @@ int batch_render(Context* const* cs, int n, int iterations, double* out) {
         };
         const bool verbose = caller->cfg_set && caller->cfg.verbose;
         ShapeTimer light{B.main, B.t0, B.t1, g_batch_light_loaded, "batch light pass", verbose};
-        g_batch_light = pick_pass_shape(light, [&](int v) {
+        if (time_light) light_choice = pick_pass_shape(light, [&](int v) {
             reset(0);
             launch_light_pass_batch(sc0, pp, m, total_paths[0], B.next.p, B.main, v, B.light_park.p);
         });
         ShapeTimer camera{B.main, B.t0, B.t1, g_batch_camera_loaded, "batch camera pass", verbose};
-        g_batch_camera = pick_pass_shape(camera, [&](int v) {
+        if (time_camera) camera_choice = pick_pass_shape(camera, [&](int v) {
             reset(1);
             launch_camera_pass_batch(sc0, pp + m + 1, m, total_pixels[0], B.next.p + 1, B.main, v, B.camera_park.p);
         });
         RC_CUDA(cudaStreamSynchronize(B.main));
         RC_CUDA(cudaGetLastError());
         if (verbose)
-            std::printf("{\"autotune\": \"batch passes\", \"light\": %d, \"camera\": %d}\n", g_batch_light.load(),
-                        g_batch_camera.load());
+            std::printf("{\"autotune\": \"batch passes\", \"light\": %d, \"camera\": %d}\n", light_choice.load(),
+                        camera_choice.load());
     }
     auto batch_shape = [&](int tuned, DevBuf<unsigned char>& b, long long n_items) {
         void* park = nullptr;
         return fitting_shape(*caller, b, tuned >= 0 ? tuned : kUntunedPass, n_items, &park);
     };
-    const int lvar = batch_shape(g_batch_light.load(), B.light_park, most_paths);
-    const int cvar = batch_shape(g_batch_camera.load(), B.camera_park, most_pixels);
+    const int lvar = batch_shape(light_choice.load(), B.light_park, most_paths);
+    const int cvar = batch_shape(camera_choice.load(), B.camera_park, most_pixels);
     // 4. one graph per iteration: captured, the executable graph updated in place (or
     //    instantiated) and launched
     double kernels = 0;

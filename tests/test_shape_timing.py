@@ -47,3 +47,40 @@ def test_stills_of_other_meshes_time_no_shapes_again():
                 assert not {4, 5} & set(shapes), name
             if ms[0] > 1.16 * ms[6]:
                 assert not {1, 2, 3} & set(shapes), name
+
+
+BATCHES = """
+import ctypes, sys
+sys.path.insert(0, {root!r})
+from realcausticsengine_gb300 import scenes
+from realcausticsengine_gb300.session import Context, Renderer, batch_render
+for grid, paths in ((24, 20000), (28, 25000), (24, 200000), (300, 20000), (24, 20000)):
+    held = []
+    for k in range(2):
+        c = Context()
+        with c:
+            Renderer(scenes.water_pool(80, 45, grid=grid), photons_per_iter=paths, max_path_length=6, seed=4 + k)
+        held.append(c)
+    c = Context()
+    with c:
+        Renderer(scenes.water_pool(80, 45, grid=grid), photons_per_iter=1000, max_path_length=6, seed=2, verbose=True)
+        batch_render(held + [c], 2)
+        ctypes.CDLL(None).fflush(None)
+    for c in held + [c]:
+        c.destroy()
+    print("end of batch", flush=True)
+"""
+
+
+def test_batches_of_another_size_class_time_their_own_shapes():
+    """A batch's light and camera passes take the shapes timed on a batch of their size: the
+    second batch (the same classes of paths and triangles) times nothing, the third (more
+    paths) its light pass, the fourth (larger meshes) both, and the first again nothing."""
+    out = subprocess.run([sys.executable, "-c", BATCHES.format(root=str(ROOT))], capture_output=True, text=True, timeout=300)
+    assert out.returncode == 0, out.stderr
+    timed = []
+    for part in out.stdout.split("end of batch\n")[:5]:
+        rows = [json.loads(line) for line in part.splitlines() if line.startswith('{"autotune_shape"')]
+        timed.append({r["autotune_shape"] for r in rows if r["autotune_shape"].startswith("batch")})
+    both = {"batch light pass", "batch camera pass"}
+    assert timed == [both, set(), {"batch light pass"}, both, set()]
