@@ -309,10 +309,9 @@ int rc_light_photons(int iteration, float* out, long long cap, long long* count)
 
 /* One Metropolis light pass (the configured sampler, iteration `iteration`); the stored
  * photons as rc_light_photons writes them, large_steps (NULL or 2) = visible large
- * steps, large steps.  PSSMLT variant 0: the render's chains, advanced one path segment
- * per loop iteration; 1: the same chains one step at a time.  Both store the same
- * photons (in another order) and count the same steps; HYBRID ignores the variant.  No
- * counterpart in the reference (its sampler is src/Vertex_Merging.cpp:218-274). */
+ * steps, large steps.  Variant 0: the render's chains, their searches in phases; 1: the
+ * same chains one step at a time.  Both store the same photons (in another order) and
+ * count the same steps.  No counterpart in the reference (its sampler is src/Vertex_Merging.cpp:218-274). */
 int rc_mlt_photons(int variant, int iteration, float* out, long long cap, long long* count,
                    unsigned long long* large_steps);
 

@@ -191,7 +191,6 @@ struct Proposal {
     bool large;
     float scale;        // mutation: exp(-1/m)
 };
-constexpr int kLargeBlocks = (kMltDims + 3) / 4, kMutationBlocks = (kMltDims + 1) / 2;
 
 __device__ __forceinline__ void propose_large(const VMParams& P, long long pidx, uint32_t salt, Proposal& r) {
     r.g.init(P.seed, (uint64_t)pidx, P.iteration ^ (salt << 20), STREAM_LIGHT);
@@ -455,10 +454,58 @@ __global__ void __launch_bounds__(128) k_mlt_pss(const VMParams P, PhotonBuf ph,
     }
 }
 
+// The hybrid chain one step at a time: the scheme as defined (large step, and on failure a
+// mutation of the last state; whole sample vectors, whole paths), kept as a launch shape so
+// that tests can check that k_mlt_hybrid stores exactly its photons.
+__global__ void __launch_bounds__(128) k_mlt_hybrid_steps(const VMParams P, PhotonBuf ph, int chains,
+                                                          unsigned long long* __restrict__ stats) {
+    const int chain = blockIdx.x * blockDim.x + threadIdx.x;
+    if (chain >= chains) return;
+    const long long N = P.num_light_paths;
+    const long long per = (N + chains - 1) / chains;
+    const long long p0 = (long long)chain * per;
+    const long long p1 = p0 + per < N ? p0 + per : N;
+    if (p0 >= p1) return;
+    const int maxlen = P.max_path_length < kMltMaxLen ? P.max_path_length : kMltMaxLen;
+    float cur[kMltDims], prop[kMltDims];
+    PhotonRec buf[kPhotonBuf];
+    uniform_samples(P, p0, 1u, cur);   // MLT_Sampler constructor: uniform initial state
+    float m = 1.0f;
+    int accepted = 1, mutated = 0;
+    unsigned long long visible_large = 0;
+    for (long long p = p0; p < p1; ++p) {
+        uniform_samples(P, p, 0u, prop);
+        PathRng rr;
+        rr.init(P.seed, (uint64_t)p * 2u, P.iteration, STREAM_MLT + 1u);
+        int n = trace_light_samples(P, prop, rr, maxlen, buf);
+        const bool large = n > 0;
+        if (large) {
+            ++visible_large;
+        } else {
+            for (int k = 0; k < kMltDims; ++k) prop[k] = cur[k];
+            mutate(P, (uint64_t)p, m, prop);
+            ++mutated;
+            rr.init(P.seed, (uint64_t)p * 2u + 1u, P.iteration, STREAM_MLT + 1u);
+            n = trace_light_samples(P, prop, rr, maxlen, buf);
+        }
+        if (n > 0) {
+            store_photons(ph, buf, n, 1.0f, (uint32_t)p);
+            for (int k = 0; k < kMltDims; ++k) cur[k] = prop[k];
+        }
+        if (!large) {
+            if (n > 0) ++accepted;
+            const float R = (float)accepted / (float)mutated;
+            m += (R - 0.234f) / (float)mutated;
+        }
+    }
+    atomicAdd(&stats[0], visible_large);
+    atomicAdd(&stats[1], (unsigned long long)(p1 - p0));
+}
+
 // PSSMLT one step at a time per chain: the sampler as defined (propose, trace the whole
 // path, accept or reject, adapt the mutation size), kept as a launch shape so that tests
-// can check that k_mlt_pss (the same chains advanced one path segment per loop
-// iteration) stores exactly its photons.
+// can check that k_mlt_pss (the same chains, their searches in phases) stores exactly its
+// photons.
 __global__ void __launch_bounds__(128) k_mlt_pss_steps(const VMParams P, PhotonBuf ph, int chains, float p_large,
                                                  unsigned long long* __restrict__ stats) {
     const int chain = blockIdx.x * blockDim.x + threadIdx.x;
@@ -529,7 +576,8 @@ void launch_mlt_pass(const VMParams& p, PhotonBuf ph, int sampler, int chains, f
     if (p.num_light_paths <= 0 || chains <= 0) return;
     cudaMemsetAsync(stats, 0, 2 * sizeof(unsigned long long), s);
     const unsigned grid = (unsigned)((chains + 127) / 128);
-    if (sampler != RC_SAMPLER_PSSMLT) k_mlt_hybrid<<<grid, 128, 0, s>>>(p, ph, chains, stats);
+    if (sampler != RC_SAMPLER_PSSMLT && variant == 1) k_mlt_hybrid_steps<<<grid, 128, 0, s>>>(p, ph, chains, stats);
+    else if (sampler != RC_SAMPLER_PSSMLT) k_mlt_hybrid<<<grid, 128, 0, s>>>(p, ph, chains, stats);
     else if (variant == 1) k_mlt_pss_steps<<<grid, 128, 0, s>>>(p, ph, chains, p_large, stats);
     else k_mlt_pss<<<grid, 128, 0, s>>>(p, ph, chains, p_large, stats);
 }

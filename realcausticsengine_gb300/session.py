@@ -161,9 +161,8 @@ class Renderer:
         return out[:n.value]
 
     def mlt_photons(self, variant: int, iteration: int):
-        """Photons of one Metropolis light pass (PSSMLT variant 0: the render's chains, one
-        path segment per loop iteration; 1: one step at a time) and its (visible large
-        steps, large steps)."""
+        """Photons of one Metropolis light pass (variant 0: the render's chains, searches in
+        phases; 1: one step at a time) and its (visible large steps, large steps)."""
         n = C.c_longlong()
         st = np.zeros(2, np.uint64)
         check(self.L.rc_mlt_photons(variant, int(iteration), None, 0, C.byref(n), st.ctypes.data), "rc_mlt_photons")
