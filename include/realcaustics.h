@@ -330,6 +330,17 @@ int rc_camera_queries(int iteration, float* out, long long cap, long long* count
  * the queries of every shape are the same, only their storage order differs. */
 int rc_camera_queries_shape(int shape, int iteration, float* out, long long cap, long long* count);
 
+/* One light pass (pass 0) or camera pass (pass 1) of iteration `iteration` over the scenes of
+ * n distinct contexts as a batch runs it (one context: as rc_render does), in launch shape
+ * `shape`, a staged shape's launches `chunk` paths at a time (0: as many as its scratch may
+ * hold, 2^24).  Scene after scene, the photons (12 floats each, as rc_light_photons) or
+ * queries (20 floats: position xyz, camera dVM, shading normal xyz, material bits, geometric
+ * normal xyz, pixel bits, throughput xyz, 0, ray direction xyz, dispersion channel bits) go
+ * to out, at most cap of them; counts[i] receives the number scene i stored.  Every shape and
+ * chunk stores the same records. */
+int rc_pass_records(rc_context* const* ctxs, int n, int pass, int shape, long long chunk, int iteration, float* out,
+                    long long cap, long long* counts);
+
 /* Build the photon KD-tree on the GPU over n photon positions (3 floats each) and
  * answer q radius queries (squared radius r2): counts[j] = number of photons with
  * ((dx*dx + dy*dy) + dz*dz) < r2 (KD_Tree::find_closest_in_radius, src/KD_Tree.cpp:217-280),

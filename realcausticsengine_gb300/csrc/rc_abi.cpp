@@ -2335,6 +2335,27 @@ int rc_camera_queries_shape(int shape, int iteration, float* out, long long cap,
     return RC_OK;
 }
 
+// The first n photons of the context's buffers as 12 floats each.
+static int photons_out(const DeviceState& d, long long n, float* out) {
+    if (n <= 0) return RC_OK;
+    std::vector<float4> pos(n), dir(n);
+    std::vector<float2> tp(n);
+    std::vector<uint32_t> path(n);
+    RC_CUDA(cudaMemcpy(pos.data(), d.ph_pos.p, 16 * n, cudaMemcpyDeviceToHost));
+    RC_CUDA(cudaMemcpy(dir.data(), d.ph_dir.p, 16 * n, cudaMemcpyDeviceToHost));
+    RC_CUDA(cudaMemcpy(tp.data(), d.ph_tp.p, 8 * n, cudaMemcpyDeviceToHost));
+    RC_CUDA(cudaMemcpy(path.data(), d.ph_path.p, 4 * n, cudaMemcpyDeviceToHost));
+    for (long long i = 0; i < n; ++i) {
+        float* w = out + 12 * i;
+        w[0] = pos[i].x; w[1] = pos[i].y; w[2] = pos[i].z;
+        w[3] = dir[i].x; w[4] = dir[i].y; w[5] = dir[i].z;
+        w[6] = dir[i].w; w[7] = tp[i].x; w[8] = tp[i].y; w[9] = pos[i].w;
+        std::memcpy(&w[10], &path[i], 4);
+        w[11] = 0.0f;
+    }
+    return RC_OK;
+}
+
 int rc_light_photons(int iteration, float* out, long long cap, long long* count) {
     return rc_light_photons_shape(0, iteration, out, cap, count);
 }
@@ -2368,22 +2389,111 @@ int rc_light_photons_shape(int shape, int iteration, float* out, long long cap, 
     if (r) return r;
     if (count) *count = (long long)nph;
     long long n = std::min<long long>((long long)nph, cap);
-    if (n > 0) {
-        std::vector<float4> pos(n), dir(n);
-        std::vector<float2> tp(n);
-        std::vector<uint32_t> path(n);
-        RC_CUDA(cudaMemcpy(pos.data(), d.ph_pos.p, 16 * n, cudaMemcpyDeviceToHost));
-        RC_CUDA(cudaMemcpy(dir.data(), d.ph_dir.p, 16 * n, cudaMemcpyDeviceToHost));
-        RC_CUDA(cudaMemcpy(tp.data(), d.ph_tp.p, 8 * n, cudaMemcpyDeviceToHost));
-        RC_CUDA(cudaMemcpy(path.data(), d.ph_path.p, 4 * n, cudaMemcpyDeviceToHost));
-        for (long long i = 0; i < n; ++i) {
-            float* w = out + 12 * i;
-            w[0] = pos[i].x; w[1] = pos[i].y; w[2] = pos[i].z;
-            w[3] = dir[i].x; w[4] = dir[i].y; w[5] = dir[i].z;
-            w[6] = dir[i].w; w[7] = tp[i].x; w[8] = tp[i].y; w[9] = pos[i].w;
-            std::memcpy(&w[10], &path[i], 4);
-            w[11] = 0.0f;
+    return photons_out(d, n, out);
+}
+
+// One light (pass 0) or camera (pass 1) pass over the scenes cs[0 .. n), each with room for
+// room[i] records; counts[i] receives what scene i stored.
+static int pass_over(Context* const* cs, int n, int pass, int shape, long long chunk, int iteration,
+                     const std::vector<long long>& room, std::vector<unsigned long long>& counts) {
+    std::vector<BatchScene> scenes((size_t)n);
+    std::vector<long long> prefix((size_t)n + 1, 0);
+    for (int i = 0; i < n; ++i) {
+        t_bound = cs[i];
+        DeviceState& d = ctx().dev;
+        RC_CUDA(d.counters.reserve(10));
+        RC_CUDA(cudaMemsetAsync(d.counters.p, 0, 2 * sizeof(unsigned long long), d.stream));
+        BatchScene& b = scenes[i];
+        b = BatchScene{};
+        b.p = make_params(*ctx().scene, iteration);
+        if (pass == 0) {
+            RC_CUDA(d.ph_pos.reserve(room[i])); RC_CUDA(d.ph_dir.reserve(room[i]));
+            RC_CUDA(d.ph_tp.reserve(room[i])); RC_CUDA(d.ph_path.reserve(room[i]));
+            b.ph = PhotonBuf{d.ph_pos.p, d.ph_dir.p, d.ph_tp.p, d.ph_path.p, room[i], d.counters.p};
+            prefix[i + 1] = prefix[i] + b.p.num_light_paths;
+        } else {
+            RC_CUDA(d.q0.reserve(room[i])); RC_CUDA(d.q1.reserve(room[i])); RC_CUDA(d.q2.reserve(room[i]));
+            RC_CUDA(d.q3.reserve(room[i])); RC_CUDA(d.q4.reserve(room[i]));
+            b.qb = QueryBuf{d.q0.p, d.q1.p, d.q2.p, d.q3.p, d.q4.p, room[i], d.counters.p + 1};
+            prefix[i + 1] = prefix[i] + (long long)b.p.camera.width * b.p.camera.height;
         }
+        RC_CUDA(cudaStreamSynchronize(d.stream));
+    }
+    DeviceState& d0 = cs[0]->dev;
+    cudaStream_t s = d0.stream;
+    struct Scratch {
+        DevBuf<BatchScene> scenes;
+        DevBuf<long long> prefix;
+        DevBuf<unsigned char> park;
+        ~Scratch() { scenes.release(); prefix.release(); park.release(); }
+    } B;
+    RC_CUDA(B.park.reserve(pass_park_bytes(prefix[n])));
+    if (n == 1) {
+        if (pass == 0) launch_light_pass(scenes[0].p, scenes[0].ph, d0.counters.p + 6, s, shape, nullptr, B.park.p, chunk);
+        else launch_camera_pass(scenes[0].p, scenes[0].qb, d0.counters.p + 7, s, shape, B.park.p, chunk);
+    } else {
+        RC_CUDA(B.scenes.reserve(scenes.size()));
+        RC_CUDA(B.prefix.reserve(prefix.size()));
+        RC_CUDA(cudaMemcpyAsync(B.scenes.p, scenes.data(), scenes.size() * sizeof(BatchScene), cudaMemcpyHostToDevice, s));
+        RC_CUDA(cudaMemcpyAsync(B.prefix.p, prefix.data(), prefix.size() * sizeof(long long), cudaMemcpyHostToDevice, s));
+        if (pass == 0)
+            launch_light_pass_batch(B.scenes.p, B.prefix.p, n, prefix[n], d0.counters.p + 6, s, shape, B.park.p, chunk);
+        else
+            launch_camera_pass_batch(B.scenes.p, B.prefix.p, n, prefix[n], d0.counters.p + 7, s, shape, B.park.p, chunk);
+    }
+    RC_CUDA(cudaGetLastError());
+    RC_CUDA(cudaStreamSynchronize(s));
+    for (int i = 0; i < n; ++i) {
+        t_bound = cs[i];
+        RC_CUDA(cudaMemcpy(&counts[i], ctx().dev.counters.p + pass, sizeof(counts[i]), cudaMemcpyDeviceToHost));
+        const int r = check_errors();
+        if (r) return r;
+    }
+    return RC_OK;
+}
+
+int rc_pass_records(rc_context* const* ctxs, int n, int pass, int shape, long long chunk, int iteration, float* out,
+                    long long cap, long long* counts) {
+    Context* const* cs = reinterpret_cast<Context* const*>(ctxs);
+    BindGuard guard;
+    Context* caller = &ctx();
+    auto fail = [&](int code, const std::string& msg) { caller->err = "rc_pass_records: " + msg; return code; };
+    if (!ctxs || n < 1 || pass < 0 || pass > 1 || shape < 0 || shape >= pass_variants() || chunk < 0 || iteration < 0 ||
+        (cap > 0 && !out) || !counts)
+        return fail(RC_E_INVALID, "bad arguments");
+    for (int i = 0; i < n; ++i) {
+        if (!cs[i] || std::count(cs, cs + n, cs[i]) != 1) return fail(RC_E_INVALID, "null or repeated context");
+        t_bound = cs[i];
+        const int r = prepare();
+        if (r) return fail(r, "scene " + std::to_string(i) + ": " + cs[i]->err);
+    }
+    std::vector<unsigned long long> stored((size_t)n, 0);
+    std::vector<long long> room((size_t)n, 1024);
+    for (int attempt = 0; attempt < 2; ++attempt) {   // the first counts, the second has the room
+        const int r = pass_over(cs, n, pass, shape, chunk, iteration, room, stored);
+        if (r) return fail(r, (t_bound ? t_bound : caller)->err);
+        bool fits = true;
+        for (int i = 0; i < n; ++i) {
+            fits = fits && (long long)stored[i] <= room[i];
+            room[i] = std::max<long long>((long long)stored[i], 1024);
+        }
+        if (fits) break;
+    }
+    long long at = 0;
+    for (int i = 0; i < n; ++i) {
+        t_bound = cs[i];
+        counts[i] = (long long)stored[i];
+        const long long m = std::min(counts[i], cap - at);
+        if (m <= 0) continue;
+        int r = RC_OK;
+        const DeviceState& d = ctx().dev;
+        const float4* q[5] = {d.q0.p, d.q1.p, d.q2.p, d.q3.p, d.q4.p};
+        if (pass == 0) r = photons_out(d, m, out + 12 * at);
+        for (int k = 0; k < 5 && pass == 1; ++k)
+            if (cudaMemcpy2D(out + 20 * at + 4 * k, 80, q[k], 16, 16, (size_t)m, cudaMemcpyDeviceToHost) != cudaSuccess)
+                r = RC_E_CUDA;
+        if (r) return fail(r, "reading scene " + std::to_string(i));
+        at += m;
     }
     return RC_OK;
 }
@@ -2419,24 +2529,7 @@ int rc_mlt_photons(int variant, int iteration, float* out, long long cap, long l
     if (count) *count = (long long)nph;
     if (large_steps) { large_steps[0] = st[0]; large_steps[1] = st[1]; }
     long long n = std::min<long long>((long long)nph, cap);
-    if (n > 0) {
-        std::vector<float4> pos(n), dir(n);
-        std::vector<float2> tp(n);
-        std::vector<uint32_t> path(n);
-        RC_CUDA(cudaMemcpy(pos.data(), d.ph_pos.p, 16 * n, cudaMemcpyDeviceToHost));
-        RC_CUDA(cudaMemcpy(dir.data(), d.ph_dir.p, 16 * n, cudaMemcpyDeviceToHost));
-        RC_CUDA(cudaMemcpy(tp.data(), d.ph_tp.p, 8 * n, cudaMemcpyDeviceToHost));
-        RC_CUDA(cudaMemcpy(path.data(), d.ph_path.p, 4 * n, cudaMemcpyDeviceToHost));
-        for (long long i = 0; i < n; ++i) {
-            float* w = out + 12 * i;
-            w[0] = pos[i].x; w[1] = pos[i].y; w[2] = pos[i].z;
-            w[3] = dir[i].x; w[4] = dir[i].y; w[5] = dir[i].z;
-            w[6] = dir[i].w; w[7] = tp[i].x; w[8] = tp[i].y; w[9] = pos[i].w;
-            std::memcpy(&w[10], &path[i], 4);
-            w[11] = 0.0f;
-        }
-    }
-    return RC_OK;
+    return photons_out(d, n, out);
 }
 
 int rc_trace_rays(int n, const float* origins, const float* directions, float tmin, unsigned* out) {

@@ -117,20 +117,23 @@ size_t scan_scratch_words(long long m);
 void launch_scan_counts(uint32_t* counts, long long m, uint32_t* tile_scratch, cudaStream_t s);
 // next_path: device counter for the persistent shapes; rays (optional): receives the number
 // of closest-hit queries the pass traced; park: scratch of the staged shapes
-// (pass_park_bytes of the paths or pixels), without which a staged shape runs as shape 0.
+// (pass_park_bytes of the paths or pixels), without which a staged shape runs as shape 0;
+// chunk: paths per pair of a staged shape's launches (0: as many as the scratch may hold).
 void launch_light_pass(const VMParams& p, PhotonBuf ph, unsigned long long* next_path, cudaStream_t s, int variant = 0,
-                       unsigned long long* rays = nullptr, void* park = nullptr);
+                       unsigned long long* rays = nullptr, void* park = nullptr, long long chunk = 0);
 void launch_camera_pass(const VMParams& p, QueryBuf qb, unsigned long long* next_pixel, cudaStream_t s, int variant = 0,
-                        void* park = nullptr);
+                        void* park = nullptr, long long chunk = 0);
 // The light and camera passes over n resident scenes: scenes[i] (device memory) holds
 // scene i's parameters and buffers, path_prefix (pixel_prefix) n + 1 device words with the
 // first work index of each scene and the total at [n].  A scene's photons (queries) are
 // the ones its own pass stores, in another order.  variant: the launch shapes of the
 // single-scene passes.
 void launch_light_pass_batch(const BatchScene* scenes, const long long* path_prefix, int n, long long total_paths,
-                             unsigned long long* next_path, cudaStream_t s, int variant = 0, void* park = nullptr);
+                             unsigned long long* next_path, cudaStream_t s, int variant = 0, void* park = nullptr,
+                             long long chunk = 0);
 void launch_camera_pass_batch(const BatchScene* scenes, const long long* pixel_prefix, int n, long long total_pixels,
-                              unsigned long long* next_pixel, cudaStream_t s, int variant = 0, void* park = nullptr);
+                              unsigned long long* next_pixel, cudaStream_t s, int variant = 0, void* park = nullptr,
+                              long long chunk = 0);
 // Debug view `mode` (2 normals, 3 facing, 4 materials with IOR `ior`) added into the
 // FP64 image accumulation.
 void launch_debug_view(const VMParams& p, int mode, float ior, double* accum, cudaStream_t s);

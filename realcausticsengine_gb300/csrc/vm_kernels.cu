@@ -829,8 +829,8 @@ const char* pass_variant_name(int v) {
 namespace {
 
 template <class Kind, int kSegs, int kMinFirst, int kMinRest, int kKeep, int kFree, class Scenes>
-void launch_staged(Scenes S, long long n, void* scratch, unsigned long long* rays, cudaStream_t s) {
-    const long long chunk = std::min(n, kParkChunk);
+void launch_staged(Scenes S, long long n, long long most, void* scratch, unsigned long long* rays, cudaStream_t s) {
+    const long long chunk = std::min(n, most);
     float4* const m = static_cast<float4*>(scratch);
     const Parked park{m, m + chunk, m + 2 * chunk, reinterpret_cast<unsigned long long*>(m + 3 * chunk)};
     auto* const first = k_pass_first<Kind, Scenes, kMinFirst, kSegs>;
@@ -854,24 +854,25 @@ void launch_staged(Scenes S, long long n, void* scratch, unsigned long long* ray
 }
 
 template <class Kind, class Scenes>
-void launch_staged_variant(const Scenes& S, long long n, void* scratch, unsigned long long* rays, cudaStream_t s,
-                           int variant) {
+void launch_staged_variant(const Scenes& S, long long n, long long most, void* scratch, unsigned long long* rays,
+                           cudaStream_t s, int variant) {
+    if (most <= 0 || most > kParkChunk) most = kParkChunk;
     switch (variant) {
-    case 5: launch_staged<Kind, 2, 9, 9, 12, 4>(S, n, scratch, rays, s); break;
-    case 6: launch_staged<Kind, 1, 10, 8, 12, 4>(S, n, scratch, rays, s); break;
-    default: launch_staged<Kind, 2, 8, 8, 8, 8>(S, n, scratch, rays, s); break;
+    case 5: launch_staged<Kind, 2, 9, 9, 12, 4>(S, n, most, scratch, rays, s); break;
+    case 6: launch_staged<Kind, 1, 10, 8, 12, 4>(S, n, most, scratch, rays, s); break;
+    default: launch_staged<Kind, 2, 8, 8, 8, 8>(S, n, most, scratch, rays, s); break;
     }
 }
 
 }  // namespace
 
 void launch_light_pass(const VMParams& p, PhotonBuf ph, unsigned long long* next_path, cudaStream_t s, int variant,
-                       unsigned long long* rays, void* park) {
+                       unsigned long long* rays, void* park, long long chunk) {
     const long long n = p.num_light_paths;
     if (n <= 0) return;
     if (!next_path) return;
     if (pass_is_staged(variant) && park && n < (1LL << 32)) {
-        launch_staged_variant<LightKind>(OneScene<LightKind>{p, ph, 0, 0}, n, park, rays, s, variant);
+        launch_staged_variant<LightKind>(OneScene<LightKind>{p, ph, 0, 0}, n, chunk, park, rays, s, variant);
         return;
     }
     switch (variant) {
@@ -883,12 +884,12 @@ void launch_light_pass(const VMParams& p, PhotonBuf ph, unsigned long long* next
 }
 
 void launch_camera_pass(const VMParams& p, QueryBuf qb, unsigned long long* next_pixel, cudaStream_t s, int variant,
-                        void* park) {
+                        void* park, long long chunk) {
     const long long n = (long long)p.camera.width * p.camera.height;
     if (n <= 0) return;
     if (!next_pixel) return;
     if (pass_is_staged(variant) && park && n < (1LL << 31)) {
-        launch_staged_variant<CameraKind>(OneScene<CameraKind>{p, qb, 0, 0}, n, park, nullptr, s, variant);
+        launch_staged_variant<CameraKind>(OneScene<CameraKind>{p, qb, 0, 0}, n, chunk, park, nullptr, s, variant);
         return;
     }
     switch (variant) {
@@ -901,11 +902,11 @@ void launch_camera_pass(const VMParams& p, QueryBuf qb, unsigned long long* next
 
 // (a parked path names its scene in 16 bits; a scene's own indices fit 32)
 void launch_light_pass_batch(const BatchScene* scenes, const long long* path_prefix, int n, long long total_paths,
-                             unsigned long long* next_path, cudaStream_t s, int variant, void* park) {
+                             unsigned long long* next_path, cudaStream_t s, int variant, void* park, long long chunk) {
     if (n <= 0 || total_paths <= 0 || !next_path) return;
     if (pass_is_staged(variant) && park && n < (1 << 16)) {
-        launch_staged_variant<LightKind>(ManyScenes<LightKind>{scenes, path_prefix, n, 0, 0}, total_paths, park, nullptr,
-                                         s, variant);
+        launch_staged_variant<LightKind>(ManyScenes<LightKind>{scenes, path_prefix, n, 0, 0}, total_paths, chunk, park,
+                                         nullptr, s, variant);
         return;
     }
     switch (variant) {
@@ -917,10 +918,10 @@ void launch_light_pass_batch(const BatchScene* scenes, const long long* path_pre
 }
 
 void launch_camera_pass_batch(const BatchScene* scenes, const long long* pixel_prefix, int n, long long total_pixels,
-                              unsigned long long* next_pixel, cudaStream_t s, int variant, void* park) {
+                              unsigned long long* next_pixel, cudaStream_t s, int variant, void* park, long long chunk) {
     if (n <= 0 || total_pixels <= 0 || !next_pixel) return;
     if (pass_is_staged(variant) && park && n < (1 << 16)) {
-        launch_staged_variant<CameraKind>(ManyScenes<CameraKind>{scenes, pixel_prefix, n, 0, 0}, total_pixels, park,
+        launch_staged_variant<CameraKind>(ManyScenes<CameraKind>{scenes, pixel_prefix, n, 0, 0}, total_pixels, chunk, park,
                                           nullptr, s, variant);
         return;
     }

@@ -61,6 +61,21 @@ def batch_render(contexts, iterations: int) -> np.ndarray:
     return out
 
 
+def pass_records(contexts, which: int, shape: int, iteration: int, chunk: int = 0) -> list:
+    """Records of one light (which 0: photons, 12 floats) or camera pass (1: queries, 20 floats)
+    over the contexts' scenes in launch shape `shape`, one array per scene (rc_pass_records)."""
+    L = lib()
+    n = len(contexts)
+    handles = (C.c_void_p * n)(*[c.handle for c in contexts])
+    counts = (C.c_longlong * n)()
+    args = (handles, n, which, shape, chunk, iteration)
+    check(L.rc_pass_records(*args, None, 0, counts), "rc_pass_records")
+    out = np.zeros((max(sum(counts), 1), 20 if which else 12), np.float32)
+    check(L.rc_pass_records(*args, out.ctypes.data, len(out), counts), "rc_pass_records")
+    ends = np.cumsum(list(counts))
+    return [out[e - k:e] for e, k in zip(ends, counts)]
+
+
 class Renderer:
     """One scene loaded into the library (the library holds one scene at a time,
     like the reference's global `scene`)."""
