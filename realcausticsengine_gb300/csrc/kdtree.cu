@@ -142,57 +142,28 @@ __device__ __forceinline__ int which(long long i, const ChunkNodes& cn) {
 }
 
 // The root's box (the partition computes the other nodes').
-template <int T>
-__global__ void __launch_bounds__(T) k_bbox(Buffers B, int cur, int level, long long n, long long first, int* nbox) {
-    __shared__ ChunkNodes cn;
-    __shared__ int sb[2][6];
-    long long a = blockIdx.x * (long long)(T * kItems);
-    if (threadIdx.x == 0) chunk_nodes(a, T * kItems, level, n, cn);
-    if (threadIdx.x < 12) sb[threadIdx.x / 6][threadIdx.x % 6] = (threadIdx.x % 6) < 3 ? 0x7fffffff : (int)0x80000000;
-    __syncthreads();
-    int mn[2][3], mx[2][3];
-    for (int q = 0; q < 2; ++q) for (int k = 0; k < 3; ++k) { mn[q][k] = 0x7fffffff; mx[q][k] = (int)0x80000000; }
-    float px[kItems], py[kItems], pz[kItems];
-    int wh[kItems];
-    const Side S = side(B, cur);
+__global__ void __launch_bounds__(kWideThreads) k_root_box(Buffers B, long long n, int* box) {
+    __shared__ int sb[6];
+    if (threadIdx.x < 6) sb[threadIdx.x] = threadIdx.x < 3 ? 0x7fffffff : (int)0x80000000;
+    const long long a = blockIdx.x * (long long)(kWideThreads * kItems);
+    int mn[3] = {0x7fffffff, 0x7fffffff, 0x7fffffff};
+    int mx[3] = {(int)0x80000000, (int)0x80000000, (int)0x80000000};
 #pragma unroll
-    for (int it = 0; it < kItems; ++it) {   // loads of all rounds in flight together
-        long long i = a + it * T + threadIdx.x;
-        wh[it] = i < n ? which(i, cn) : -1;
-        const long long j = wh[it] >= 0 ? i : a;
-        px[it] = S.x[j]; py[it] = S.y[j]; pz[it] = S.z[j];
-    }
+    for (int it = 0; it < kItems; ++it) {   // (past the end: the chunk's first photon again)
+        const long long i = a + it * kWideThreads + threadIdx.x, j = i < n ? i : a;
+        const int v[3] = {f2ord(B.x[0][j]), f2ord(B.y[0][j]), f2ord(B.z[0][j])};
 #pragma unroll
-    for (int it = 0; it < kItems; ++it) {
-        const int w = wh[it];
-        if (w < 0) continue;
-        int vx = f2ord(px[it]), vy = f2ord(py[it]), vz = f2ord(pz[it]);
-        if (w == 0) {
-            mn[0][0] = min(mn[0][0], vx); mn[0][1] = min(mn[0][1], vy); mn[0][2] = min(mn[0][2], vz);
-            mx[0][0] = max(mx[0][0], vx); mx[0][1] = max(mx[0][1], vy); mx[0][2] = max(mx[0][2], vz);
-        } else {
-            mn[1][0] = min(mn[1][0], vx); mn[1][1] = min(mn[1][1], vy); mn[1][2] = min(mn[1][2], vz);
-            mx[1][0] = max(mx[1][0], vx); mx[1][1] = max(mx[1][1], vy); mx[1][2] = max(mx[1][2], vz);
-        }
+        for (int k = 0; k < 3; ++k) { mn[k] = min(mn[k], v[k]); mx[k] = max(mx[k], v[k]); }
     }
-    for (int q = 0; q < 2; ++q)
-        for (int k = 0; k < 3; ++k) {
-            int v = mn[q][k], u = mx[q][k];
-            for (int o = 16; o > 0; o >>= 1) {
-                v = min(v, __shfl_xor_sync(0xffffffffu, v, o));
-                u = max(u, __shfl_xor_sync(0xffffffffu, u, o));
-            }
-            if ((threadIdx.x & 31) == 0) { atomicMin(&sb[q][k], v); atomicMax(&sb[q][3 + k], u); }
-        }
     __syncthreads();
-    if (threadIdx.x < 12) {
-        int q = threadIdx.x / 6, k = threadIdx.x % 6;
-        long long e = q == 0 ? cn.eA : cn.eB;
-        if (e) {
-            int* dst = nbox + 6 * (e - first) + k;
-            if (k < 3) atomicMin(dst, sb[q][k]); else atomicMax(dst, sb[q][k]);
-        }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const int v = __reduce_min_sync(0xffffffffu, mn[k]), u = __reduce_max_sync(0xffffffffu, mx[k]);
+        if ((threadIdx.x & 31) == 0) { atomicMin(&sb[k], v); atomicMax(&sb[3 + k], u); }
     }
+    __syncthreads();
+    if (threadIdx.x < 3) atomicMin(&box[threadIdx.x], sb[threadIdx.x]);
+    else if (threadIdx.x < 6) atomicMax(&box[threadIdx.x], sb[threadIdx.x]);
 }
 
 // One warp: node t's selection before `pass`.  Every key of the node
@@ -822,7 +793,7 @@ int kd_build(const float4* pos4, long long n, KdTree& tree, void* scratch, size_
         for (int pass = 0; pass < 4; ++pass)
             cudaMemsetAsync(S.hist + pass * maxnodes * 256, 0, 1024, stream);
         const long long span = (long long)kWideThreads * kItems;
-        k_bbox<kWideThreads><<<(unsigned)((n + span - 1) / span), kWideThreads, 0, stream>>>(B, 0, 0, n, 1, S.box);
+        k_root_box<<<(unsigned)((n + span - 1) / span), kWideThreads, 0, stream>>>(B, n, S.box);
         nl++;
     }
     for (int l = 0; l < l0; ++l) {

@@ -480,7 +480,6 @@ int check_errors() {
     RC_CUDA(cudaMemcpy(h, ctx().dev.errors.p, sizeof(h), cudaMemcpyDeviceToHost));
     if (h[ERR_STACK]) { ctx().err = "BVH traversal stack overflow (depth > 64)"; return RC_E_CAPACITY; }
     if (h[ERR_MATERIAL]) { ctx().err = "triangle material index out of range"; return RC_E_INVALID; }
-    if (h[ERR_KD]) { ctx().err = "KD-tree build found inconsistent counts"; return RC_E_INVALID; }
     if (h[ERR_MLP]) { ctx().err = "tensor-core pipeline wait timed out in the MLP"; return RC_E_CUDA; }
     if (h[ERR_GATHER]) { ctx().err = "gather traversal stack overflow"; return RC_E_CAPACITY; }
     return RC_OK;
