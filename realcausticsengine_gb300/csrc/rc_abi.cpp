@@ -158,7 +158,7 @@ struct DeviceState {
 };
 
 // Autotuner choices: launch variant per size class (log2 of light paths or pixels, and
-// classes of 16x of the scene's triangles; log2 of queries, and classes of 4x of photons),
+// classes of 4x of the scene's triangles; log2 of queries, and classes of 4x of photons),
 // -1 = untuned.  Kept for the process and shared by every context (a new scene, or a scene
 // in another context, reuses them).  The triangles are in the key because the light and
 // camera passes' best shape depends on how long a search is: at 2.5M light paths 1,000 gems
@@ -167,13 +167,15 @@ struct DeviceState {
 // scene (displaced spheres, glass spheres, water; 1k to 1M triangles, 30k to 2.5M paths) the
 // better family changed once, by 6% (328k triangles of glass spheres), and twelve stills of
 // 2k to 300k triangles took 432 ms the first time with classes of 2x and every shape launched
-// twice, 234 now (and 122 when all classes are known).  The photons are in the gather's
+// twice, 258 now (and 124 when all classes are known).  No coarser, because kinds of scenes
+// differ: in one class of 16x, 2,000 gems (256k triangles) took the shapes of a water pool
+// (522k), 39.5 ms an update instead of 36.2.  The photons are in the gather's
 // because they tell a caustic's focus from a wide floor: 216k queries take 120
 // us parked against 783 with 20k photons of one; without one parking only costs.
 struct TuneTables {
-    std::atomic<int> light[64][8], camera[64][8], gather[64][32];
+    std::atomic<int> light[64][16], camera[64][16], gather[64][32];
     // a batch's passes: its paths or pixels in all, its scenes' mean triangles
-    std::atomic<int> batch_light[64][8], batch_camera[64][8];
+    std::atomic<int> batch_light[64][16], batch_camera[64][16];
     TuneTables() {
         for (int i = 0; i < 64; ++i) {
             for (auto& a : light[i]) a = -1;
@@ -674,7 +676,7 @@ int autotune_pass(std::atomic<unsigned>& loaded, const char* what, long long siz
 }
 
 int size_class(long long n) { return n > 0 ? 63 - __builtin_clzll((unsigned long long)n) : 0; }
-int triangle_class(long long n) { return std::min(size_class(n) / 4, 7); }
+int triangle_class(long long n) { return std::min(size_class(n) / 2, 15); }
 std::atomic<int>& light_slot(long long paths) { return g_tune.light[size_class(paths)][triangle_class(ctx().dev.num_tris)]; }
 std::atomic<int>& camera_slot(long long pixels) { return g_tune.camera[size_class(pixels)][triangle_class(ctx().dev.num_tris)]; }
 std::atomic<int>& gather_slot(long long queries, long long photons) {
