@@ -2650,7 +2650,7 @@ int rc_gather_query(int variant, int n, const float* positions, int q, const flo
             RC_CUDA(cudaGetLastError());
             int h = 0;
             t_parked_items = 0;
-            if (gather_parks(variant))
+            if (n > 0 && gather_parks(variant))
                 RC_CUDA(cudaMemcpyAsync(&t_parked_items, parked.p, 4, cudaMemcpyDeviceToHost, s));
             RC_CUDA(cudaMemcpyAsync(counts, cnt.p, 4 * (size_t)q, cudaMemcpyDeviceToHost, s));
             RC_CUDA(cudaMemcpyAsync(&h, err.p, sizeof(int), cudaMemcpyDeviceToHost, s));
