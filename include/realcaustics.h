@@ -359,6 +359,11 @@ int rc_gather_query(int variant, int n, const float* positions, int q, const flo
                     int* counts, int* idx, long long cap, long long* total);
 int rc_gather_variants(void);
 
+/* The order in which rc_gather_query's launch shape `variant` takes the q queries (indices,
+ * order[q]): shapes that park sort them along the photons' Hilbert curve, the others along
+ * the Morton curve. */
+int rc_query_order(int variant, int q, const float* queries, float r2, unsigned* order);
+
 /* Items that the calling thread's last rc_gather_query asked the parked list for in its
  * count pass (shapes that park a focus's work for a second launch; 0 for the others).  The
  * list holds 65,535; what does not fit is done where it was found. */

@@ -17,7 +17,7 @@
 // position and count in the spare .w words; every node above has the union of its
 // children's boxes.
 //
-// Work split (k_gather).  Queries are sorted along the same curve (launch_query_order) and a
+// Work split (k_gather).  Queries are sorted in space too (launch_query_order) and a
 // warp owns G consecutive ones (a group), one per lane.  The warp descends the box hierarchy
 // once for the whole group, E levels per step (lane j tests descendant j's box against
 // the group's bounding box grown by the radius), down to the candidate chunks.  At a

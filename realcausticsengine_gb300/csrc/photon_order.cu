@@ -1,8 +1,9 @@
 // Spatial orders of the iteration's photons and merge queries, and the gather's box tree.
 //
-// Photons and queries are sorted along a Hilbert curve over a grid of the scene's box
-// (Skilling, "Programming the Hilbert curve", AIP Conf. Proc. 707, 2004), so that any run
-// of consecutive ones is compact: unlike the Morton curve the Hilbert curve has no jumps.
+// Photons are sorted along a Hilbert curve over a grid of the scene's box (Skilling,
+// "Programming the Hilbert curve", AIP Conf. Proc. 707, 2004), so that any run of consecutive
+// ones is compact: unlike the Morton curve the Hilbert curve has no jumps.  Queries are
+// sorted along either (launch_query_order says which and why).
 // The gather's photon sets do not depend on how the photons are stored (gather.cu), so its
 // chunks are simply runs of the sorted photons, cut evenly into 2^Lc.  (They were the leaves
 // of the reference's median-split KD tree, built with four radix-select passes and a
@@ -159,9 +160,10 @@ __device__ __forceinline__ void hilbert_index(uint32_t x, uint32_t y, uint32_t z
           ((spread3(x & 1023u) << 2) | (spread3(y & 1023u) << 1) | spread3(z & 1023u));
 }
 
-// Keys of the points at pos + stride * i, i < n.  count (optional): the number of points on
-// the device; the ones from there to n sort last (kPadLast) or get no key.
-template <class Key, bool kPadLast>
+// Keys of the points at pos + stride * i, i < n: along the Hilbert curve, or (kMorton, 10
+// bits) the Morton curve.  count (optional): the number of points on the device; the ones
+// from there to n sort last (kPadLast) or get no key.
+template <class Key, bool kPadLast, bool kMorton>
 __global__ void k_curve_keys(const float* __restrict__ pos, int stride, long long n,
                              const unsigned long long* __restrict__ count, CurveFrame f, Key* __restrict__ keys) {
     const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -172,8 +174,11 @@ __global__ void k_curve_keys(const float* __restrict__ pos, int stride, long lon
     }
     const float* p = pos + (long long)stride * i;
     const float cells = (float)(1 << f.bits);
-    hilbert_index(cell_of((p[0] - f.lo[0]) * f.scale[0], cells), cell_of((p[1] - f.lo[1]) * f.scale[1], cells),
-                  cell_of((p[2] - f.lo[2]) * f.scale[2], cells), f.bits, keys[i]);
+    const uint32_t x = cell_of((p[0] - f.lo[0]) * f.scale[0], cells);
+    const uint32_t y = cell_of((p[1] - f.lo[1]) * f.scale[1], cells);
+    const uint32_t z = cell_of((p[2] - f.lo[2]) * f.scale[2], cells);
+    if (kMorton) keys[i] = spread3(x) | (spread3(y) << 1) | (spread3(z) << 2);
+    else hilbert_index(x, y, z, f.bits, keys[i]);
 }
 
 // ---------------------------------------------------------------- radix sort
@@ -368,15 +373,13 @@ void sort_keys(const SortSpace<Key>& sp, long long n, const unsigned long long* 
     if (launches) *launches += 4 * passes;
 }
 
-template <class Key>
-void order_points(const float* pos, int stride, long long n, const unsigned long long* count, bool pad_last,
-                  const CurveFrame& f, void* scratch, uint32_t* order, cudaStream_t s, int* launches) {
+template <class Key, bool kPadLast, bool kMorton>
+void order_points(const float* pos, int stride, long long n, const unsigned long long* count, const CurveFrame& f,
+                  void* scratch, uint32_t* order, cudaStream_t s, int* launches) {
     const SortSpace<Key> sp(scratch, n);
-    const unsigned g = (unsigned)((n + 255) / 256);
-    if (pad_last) k_curve_keys<Key, true><<<g, 256, 0, s>>>(pos, stride, n, count, f, sp.keys[0]);
-    else k_curve_keys<Key, false><<<g, 256, 0, s>>>(pos, stride, n, count, f, sp.keys[0]);
+    k_curve_keys<Key, kPadLast, kMorton><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(pos, stride, n, count, f, sp.keys[0]);
     if (launches) *launches += 1;
-    sort_keys<Key>(sp, n, pad_last ? nullptr : count, f.bits, order, s, launches);
+    sort_keys<Key>(sp, n, kPadLast ? nullptr : count, f.bits, order, s, launches);
 }
 
 // ---------------------------------------------------------------- records and boxes
@@ -472,11 +475,19 @@ size_t order_scratch_bytes(long long n) {
            round_up(4 * scan_scratch_words(m));
 }
 
-void launch_query_order(const float* qpos, int stride, long long nq, const CurveFrame& frame, void* scratch,
+void launch_query_order(const float* qpos, int stride, long long nq, const CurveFrame& frame, bool parks, void* scratch,
                         uint32_t* order, int* launches, cudaStream_t s, const unsigned long long* nq_dev) {
     if (nq <= 0) return;
-    if (frame.bits <= 10) order_points<uint32_t>(qpos, stride, nq, nq_dev, false, frame, scratch, order, s, launches);
-    else order_points<unsigned long long>(qpos, stride, nq, nq_dev, false, frame, scratch, order, s, launches);
+    if (!parks) {
+        CurveFrame f = frame;   // 10 bits per axis
+        for (float& k : f.scale) k *= 1023.99f / ((float)(1 << frame.bits) - 0.01f);
+        f.bits = 10;
+        order_points<uint32_t, false, true>(qpos, stride, nq, nq_dev, f, scratch, order, s, launches);
+    } else if (frame.bits <= 10) {
+        order_points<uint32_t, false, false>(qpos, stride, nq, nq_dev, frame, scratch, order, s, launches);
+    } else {
+        order_points<unsigned long long, false, false>(qpos, stride, nq, nq_dev, frame, scratch, order, s, launches);
+    }
 }
 
 int photon_chunk_level(long long n) {
@@ -490,8 +501,8 @@ void launch_photon_order(const PhotonBuf& ph, long long n, const unsigned long l
                          void* scratch, const PhotonTree& tree, TreePhotons tp, int* launches, cudaStream_t s) {
     if (n <= 0) return;
     const float* pos = reinterpret_cast<const float*>(ph.pos);
-    if (frame.bits <= 10) order_points<uint32_t>(pos, 4, n, count, true, frame, scratch, tree.id, s, launches);
-    else order_points<unsigned long long>(pos, 4, n, count, true, frame, scratch, tree.id, s, launches);
+    if (frame.bits <= 10) order_points<uint32_t, true, false>(pos, 4, n, count, frame, scratch, tree.id, s, launches);
+    else order_points<unsigned long long, true, false>(pos, 4, n, count, frame, scratch, tree.id, s, launches);
     const int lc = photon_chunk_level(n);
     k_chunks<<<(unsigned)(((32LL << lc) + 255) / 256), 256, 0, s>>>(ph, tree.id, n, lc, tp, tree.box_lo, tree.box_hi);
     int nl = 1;

@@ -1014,8 +1014,10 @@ int render_iteration(HostScene& sc, int redo_iteration = -1, bool tune_passes = 
     RC_CUDA(d.qscratch.reserve(order_scratch_bytes((long long)nq)));
     RC_CUDA(cudaEventRecord(d.ev[6], s));
     int qlaunch = 0;
-    launch_query_order(reinterpret_cast<const float*>(d.q0.p), 4, (long long)nq, frame, d.qscratch.p,
-                       d.qorder.p, &qlaunch, s);
+    auto order_queries = [&](int v, int* launches) {
+        launch_query_order(reinterpret_cast<const float*>(d.q0.p), 4, (long long)nq, frame, gather_parks(v), d.qscratch.p,
+                           d.qorder.p, launches, s);
+    };
     int variant = gather_default_variant();
     if (cfg().autotune && nq > 0) {
         std::atomic<int>& slot = gather_slot((long long)nq, n);
@@ -1027,8 +1029,13 @@ int render_iteration(HostScene& sc, int redo_iteration = -1, bool tune_passes = 
             auto run = [&](int v) {
                 launch_gather(p, tree, tph, qb, d.qorder.p, (long long)nq, d.tune_accum.p, d.gather_parked.p, nullptr, s, v);
             };
-            run(variant);   // (photons and queries into L2)
-            for (int v = 0; v < gather_variants(); ++v) t.time(v, run);
+            for (int v = 0; v < gather_variants(); ++v) {
+                if (v == 0 || gather_parks(v) != gather_parks(v - 1)) {   // another query order
+                    order_queries(v, nullptr);
+                    run(v);   // (photons and queries into L2)
+                }
+                t.time(v, run);
+            }
             slot = t.best_v;
             if (cfg().verbose)
                 std::printf("{\"autotune\": \"gather\", \"queries\": %llu, \"variant\": \"%s\", \"ms\": %.3f}\n",
@@ -1036,6 +1043,7 @@ int render_iteration(HostScene& sc, int redo_iteration = -1, bool tune_passes = 
         }
         variant = slot.load();
     }
+    order_queries(variant, &qlaunch);
     unsigned long long gc[4] = {0, 0, 0, 0};
     RC_CUDA(cudaMemsetAsync(d.counters.p + 2, 0, 4 * sizeof(unsigned long long), s));
     RC_CUDA(cudaEventRecord(d.evg[0], s));
@@ -1206,8 +1214,8 @@ int async_tail(HostScene& sc, const VMParams& p, cudaStream_t s, cudaStream_t si
                         d.ph_scratch.p, tree, tph, nullptr, s);
     RC_CUDA(record(d.ev[3], s));
     RC_CUDA(cudaStreamWaitEvent(side, camera_done, 0));
-    launch_query_order(reinterpret_cast<const float*>(d.q0.p), 4, qc, frame, d.qscratch.p, d.qorder.p,
-                       nullptr, side, d.counters.p + 1);
+    launch_query_order(reinterpret_cast<const float*>(d.q0.p), 4, qc, frame, gather_parks(d.async_gvar), d.qscratch.p,
+                       d.qorder.p, nullptr, side, d.counters.p + 1);
     RC_CUDA(record(d.ev[8], side));
     RC_CUDA(cudaEventRecord(d.join, side));
     RC_CUDA(cudaStreamWaitEvent(s, d.join, 0));
@@ -2602,6 +2610,25 @@ static CurveFrame points_frame(int n, const float* p, float r2) {
 
 int rc_gather_variants(void) { return gather_variants(); }
 
+int rc_query_order(int variant, int q, const float* queries, float r2, unsigned* order) {
+    if (q < 0 || (q > 0 && (!queries || !order))) { ctx().err = "bad query arrays"; return RC_E_INVALID; }
+    if (variant < -1 || variant >= gather_variants()) { ctx().err = "gather variant out of range"; return RC_E_INVALID; }
+    if (variant < 0) variant = gather_default_variant();
+    if (q == 0) return RC_OK;
+    struct Scratch {
+        DevBuf<float> pos;
+        DevBuf<uint32_t> ord;
+        DevBuf<unsigned char> sort;
+        ~Scratch() { pos.release(); ord.release(); sort.release(); }
+    } B;
+    RC_CUDA(B.pos.reserve(3 * (size_t)q)); RC_CUDA(B.ord.reserve((size_t)q)); RC_CUDA(B.sort.reserve(order_scratch_bytes(q)));
+    RC_CUDA(cudaMemcpy(B.pos.p, queries, 12 * (size_t)q, cudaMemcpyHostToDevice));
+    launch_query_order(B.pos.p, 3, q, points_frame(q, queries, r2), gather_parks(variant), B.sort.p, B.ord.p, nullptr, nullptr);
+    RC_CUDA(cudaGetLastError());
+    RC_CUDA(cudaMemcpy(order, B.ord.p, 4 * (size_t)q, cudaMemcpyDeviceToHost));
+    return RC_OK;
+}
+
 int rc_device_bus_id(char* out, int len) {
     if (!out || len < 13) { ctx().err = "bus id buffer too small"; return RC_E_INVALID; }
     int dev = 0;
@@ -2644,7 +2671,7 @@ int rc_gather_query(int variant, int n, const float* positions, int q, const flo
             RC_CUDA(cudaMemcpyAsync(qp.p, queries, 12 * (size_t)q, cudaMemcpyHostToDevice, s));
             RC_CUDA(cudaMemsetAsync(cnt.p, 0, 4 * (size_t)q, s));
             RC_CUDA(cudaMemsetAsync(err.p, 0, sizeof(int), s));
-            launch_query_order(qp.p, 3, q, points_frame(q, queries, r2), osc.p, ord.p, nullptr, s);
+            launch_query_order(qp.p, 3, q, points_frame(q, queries, r2), gather_parks(variant), osc.p, ord.p, nullptr, s);
             launch_gather_sets(tree, t0.p, qp.p, 3, ord.p, q, r2, cnt.p, nullptr, nullptr, nullptr, variant, parked.p,
                                nullptr, err.p, s);
             RC_CUDA(cudaGetLastError());

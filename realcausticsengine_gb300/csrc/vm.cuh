@@ -173,9 +173,17 @@ int photon_chunk_level(long long n);
 // photons stored (at most n); the slots beyond hold pad positions and are sorted last.
 void launch_photon_order(const PhotonBuf& ph, long long n, const unsigned long long* count, const CurveFrame& frame,
                          void* scratch, const PhotonTree& tree, TreePhotons tp, int* launches, cudaStream_t s);
-// order[] receives the query indices (positions at qpos + stride*i) in sorted order.  With
-// nq_dev the number of queries is read on the device (at most nq).
-void launch_query_order(const float* qpos, int stride, long long nq, const CurveFrame& frame, void* scratch,
+// order[] receives the query indices (positions at qpos + stride*i) in sorted order: for a
+// gather that parks (gather_parks) along the photons' Hilbert curve, else along the Morton
+// curve with 10 bits per axis.  (Without parking a
+// focus's groups are the gather's time, and in the Hilbert order they spread less evenly over
+// the SMs: the busiest took 11.0M cycles of a mean of 6.8M, in the Morton order 8.5M.  Gathers
+// of a displaced glass ball with 8M light paths 2.64 ms in the first, 2.11 in the second; with
+// 2M paths and 3 times the radius 4.77 and 3.57; of a 1080p water pool 1.70 and 1.66.  Parked,
+// the groups that straddle a jump of the Morton curve cost more: behind a glass ball, 4M
+// paths, 0.34 ms in the Hilbert order, 0.5 in the Morton one.)  With nq_dev the number of
+// queries is read on the device (at most nq).
+void launch_query_order(const float* qpos, int stride, long long nq, const CurveFrame& frame, bool parks, void* scratch,
                         uint32_t* order, int* launches, cudaStream_t s, const unsigned long long* nq_dev = nullptr);
 // The gather: one fused kernel over groups of ordered queries (gather.cu).  Photon sets
 // are the reference's; each accepted photon's merge (BSDF, MIS weight, throughput) is

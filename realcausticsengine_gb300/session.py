@@ -227,6 +227,14 @@ def kd_query(positions: np.ndarray, queries: np.ndarray, r2: float, with_indices
     return counts, [idx[offs[j]:offs[j + 1]] for j in range(len(q))]
 
 
+def query_order(queries: np.ndarray, r2: float, variant: int = -1) -> np.ndarray:
+    """The order in which the gather's launch shape `variant` takes the queries."""
+    q = np.ascontiguousarray(queries, np.float32)
+    out = np.zeros(len(q), np.uint32)
+    check(lib().rc_query_order(int(variant), len(q), q.ctypes.data, C.c_float(r2), out.ctypes.data), "rc_query_order")
+    return out
+
+
 def gather_variants() -> int:
     return int(lib().rc_gather_variants())
 
