@@ -366,8 +366,10 @@ int rc_query_order(int variant, int q, const float* queries, float r2, unsigned*
 
 /* Items that the calling thread's last rc_gather_query asked the parked list for in its
  * count pass (shapes that park a focus's work for a second launch; 0 for the others).  The
- * list holds 65,535; what does not fit is done where it was found. */
+ * list holds 65,535, or what rc_gather_parked_limit sets for the calling thread (1 to
+ * 1,048,575, which is a render's); what does not fit is done where it was found. */
 long long rc_gather_parked_items(void);
+int rc_gather_parked_limit(long long items);
 
 /* PCI bus id ("domain:bus:device.function") of the CUDA device the calling thread
  * uses, for tools that address GPUs by bus id (nvidia-smi numbers GPUs physically and

@@ -51,6 +51,7 @@ def lib() -> C.CDLL:
                                   C.c_void_p, C.c_longlong, C.POINTER(C.c_longlong)]
     L.rc_gather_variants.argtypes = []
     L.rc_query_order.argtypes = [C.c_int, C.c_int, C.c_void_p, C.c_float, C.c_void_p]
+    L.rc_gather_parked_limit.argtypes = [C.c_longlong]
     L.rc_gather_parked_items.argtypes = []
     L.rc_gather_parked_items.restype = C.c_longlong
     L.rc_device_bus_id.argtypes = [C.c_char_p, C.c_int]
@@ -96,6 +97,6 @@ EXPORTS = ["init", "main", "rc_default_config", "rc_set_config", "rc_pass_scratc
            "rc_kd_noalloc_last_error", "rc_proposal_state", "rc_render_debug",
            "rc_save_state", "rc_load_state", "rc_scene_dump", "rc_prepare_stats",
            "rc_context_create", "rc_context_bind", "rc_context_destroy", "rc_gather_query",
-           "rc_gather_variants", "rc_query_order", "rc_gather_parked_items", "rc_camera_queries", "rc_camera_queries_shape", "rc_device_bus_id", "rc_tc_gemm_selftest",
+           "rc_gather_variants", "rc_query_order", "rc_gather_parked_items", "rc_gather_parked_limit", "rc_camera_queries", "rc_camera_queries_shape", "rc_device_bus_id", "rc_tc_gemm_selftest",
            "rc_tc_wait_selftest", "rc_light_photons_shape", "rc_batch_render",
            "rc_pass_records", "rc_mlt_photons"]

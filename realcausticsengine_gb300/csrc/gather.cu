@@ -132,10 +132,14 @@ static_assert(sizeof(QState) == 29 * 4, "QState must keep an odd word stride");
 // (group, first | end << 8 of its sub-group's lanes, root, part) at parked[1 + i],
 // parked[0].x of them; void items have root 0.  216k queries and 20k photons behind a glass
 // ball under a point light: 783 us, parked 120 (102 with kParkWork 16; 258 with subtrees
-// only).  Without a focus the second launch costs more than it gives (3.7M queries on a water
+// only).  The list has to hold what the focus parks: the warps that find it full do their
+// rest alone, and are the gather's time again.  With 65,535 items, against a render's list of
+// 2^20 - 1 (kParkedItems), 512x512 queries behind the ball take 15.3 and 1.1 ms with 580k
+// photons, 12.5 and 3.1 with 18k and 20 times the radius (2^18: 12.5); 1920x1080 with 145k
+// photons 4.5 and 1.2.  Where 65,535 were enough the longer list costs nothing.
+// Without a focus the second launch costs more than it gives (3.7M queries on a water
 // pool's floor 1.79 ms against 2.17), so the autotuner chooses.
 constexpr unsigned kParkWork = 64, kParkParts = 16;
-constexpr int kParkedItems = (1 << 16) - 1;
 
 template <bool Eval> struct GroupExtra {};
 template <> struct GroupExtra<true> {
@@ -287,7 +291,8 @@ template <int kStage, int MinBlocks, int G, int E, class Sink>
 __global__ void __launch_bounds__(32 * kWarpsPerBlock, MinBlocks)
     k_gather(const ChunkTree t, const float* __restrict__ qpos, int qstride, const uint32_t* __restrict__ order,
              long long nq, const unsigned long long* __restrict__ nq_dev, const int* __restrict__ skip, float r2,
-             const Sink sink, uint4* parked, unsigned long long* __restrict__ counters, int* __restrict__ err) {
+             const Sink sink, uint4* parked, uint32_t room, unsigned long long* __restrict__ counters,
+             int* __restrict__ err) {
     constexpr bool kRest = kStage == 2;
     static_assert(G == 16 || G == 32, "a group is a half or a whole warp of queries");
     static_assert(E >= 1 && E <= 5, "an expansion step tests at most 32 descendants");
@@ -300,7 +305,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, MinBlocks)
     const unsigned lt = (1u << lane) - 1u;
     WarpSmem<Sink::kEval>& sm = smem[warp];
     if (t.lc < 0) return;
-    const uint32_t items = kRest ? min(parked[0].x, (uint32_t)kParkedItems) : 0u;
+    const uint32_t items = kRest ? min(parked[0].x, room) : 0u;
     for (long long w = (long long)blockIdx.x * kWarpsPerBlock + warp;; w += (long long)gridDim.x * kWarpsPerBlock) {
     uint4 item = make_uint4((uint32_t)w, 0u, 1u, 0u);
     if (kRest) {
@@ -425,17 +430,17 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, MinBlocks)
 
     // Room for `add` parked items, from `at`; without it the items given below the end are
     // void and the warp parks no more.  A full list is not asked again: the count stays
-    // below kParkedItems and one request of every warp in flight, however many groups the
+    // below `room` and one request of every warp in flight, however many groups the
     // launch has (counted for all of them it wraps at 2^32: 3.6M groups of some 1,200).
     auto reserve_items = [&](uint32_t add) -> uint32_t {
-        uint32_t at = (uint32_t)kParkedItems;
-        if (lane == 0 && __ldcg(&parked[0].x) < (uint32_t)kParkedItems) at = atomicAdd(&parked[0].x, add);
+        uint32_t at = room;
+        if (lane == 0 && __ldcg(&parked[0].x) < room) at = atomicAdd(&parked[0].x, add);
         at = __shfl_sync(kFull, at, 0);
-        park = at + add <= (uint32_t)kParkedItems;
+        park = at + add <= room;
         return at;
     };
     auto write_item = [&](uint32_t at, int a, int b, uint32_t root, uint32_t which) {
-        if (at < (uint32_t)kParkedItems)
+        if (at < room)
             parked[1 + at] = make_uint4(item.x, (uint32_t)a | ((uint32_t)b << 8), park ? root : 0u, which);
     };
 
@@ -557,38 +562,39 @@ int sm_count() {
 template <int MB, int G, int E, bool kPark, class Sink>
 void launch_shape(const ChunkTree& t, const float* qpos, int qstride, const uint32_t* order, long long nq,
                   const unsigned long long* nq_dev, const int* skip, float r2, const Sink& sink,
-                  uint4* parked, unsigned long long* counters, int* err, cudaStream_t s) {
+                  const ParkedList& list, unsigned long long* counters, int* err, cudaStream_t s) {
     const long long warps = (nq + G - 1) / G;
     const unsigned blocks = (unsigned)((warps + kWarpsPerBlock - 1) / kWarpsPerBlock);
+    uint4* const parked = static_cast<uint4*>(list.p);
     if (kPark) cudaMemsetAsync(parked, 0, sizeof(uint4), s);
     k_gather<kPark ? 1 : 0, MB, G, E, Sink><<<blocks, 32 * kWarpsPerBlock, 0, s>>>(
-        t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, parked, counters, err);
+        t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, parked, list.items, counters, err);
     if (kPark)
         k_gather<2, MB, G, E, Sink><<<MB * sm_count(), 32 * kWarpsPerBlock, 0, s>>>(
-            t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, parked, counters, err);
+            t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, parked, list.items, counters, err);
 }
 
 template <class Sink>
 void launch_variant(int v, const ChunkTree& t, const float* qpos, int qstride, const uint32_t* order, long long nq,
                     const unsigned long long* nq_dev, const int* skip, float r2, const Sink& sink,
-                    uint4* parked, unsigned long long* counters, int* err, cudaStream_t s) {
+                    const ParkedList& list, unsigned long long* counters, int* err, cudaStream_t s) {
     switch (v) {
-    case 0: launch_shape<2, 32, 5, false>(t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, parked, counters, err, s); break;
-    case 2: launch_shape<4, 32, 5, false>(t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, parked, counters, err, s); break;
-    case 3: launch_shape<3, 32, 4, false>(t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, parked, counters, err, s); break;
-    case 4: launch_shape<4, 32, 4, false>(t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, parked, counters, err, s); break;
-    case 5: launch_shape<3, 16, 5, false>(t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, parked, counters, err, s); break;
-    case 6: launch_shape<4, 16, 4, false>(t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, parked, counters, err, s); break;
-    case 7: launch_shape<4, 16, 5, false>(t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, parked, counters, err, s); break;
-    case 8: launch_shape<3, 16, 5, true>(t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, parked, counters, err, s); break;
-    case 9: launch_shape<3, 32, 5, true>(t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, parked, counters, err, s); break;
-    default: launch_shape<3, 32, 5, false>(t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, parked, counters, err, s); break;
+    case 0: launch_shape<2, 32, 5, false>(t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, list, counters, err, s); break;
+    case 2: launch_shape<4, 32, 5, false>(t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, list, counters, err, s); break;
+    case 3: launch_shape<3, 32, 4, false>(t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, list, counters, err, s); break;
+    case 4: launch_shape<4, 32, 4, false>(t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, list, counters, err, s); break;
+    case 5: launch_shape<3, 16, 5, false>(t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, list, counters, err, s); break;
+    case 6: launch_shape<4, 16, 4, false>(t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, list, counters, err, s); break;
+    case 7: launch_shape<4, 16, 5, false>(t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, list, counters, err, s); break;
+    case 8: launch_shape<3, 16, 5, true>(t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, list, counters, err, s); break;
+    case 9: launch_shape<3, 32, 5, true>(t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, list, counters, err, s); break;
+    default: launch_shape<3, 32, 5, false>(t, qpos, qstride, order, nq, nq_dev, skip, r2, sink, list, counters, err, s); break;
     }
 }
 
 }  // namespace
 
-size_t gather_parked_bytes() { return sizeof(uint4) * (size_t)(1 + kParkedItems); }
+size_t gather_parked_bytes(uint32_t items) { return sizeof(uint4) * ((size_t)items + 1); }
 int gather_variants() { return kNumShapes; }
 bool gather_parks(int variant) { return variant >= 8 && variant < kNumShapes; }
 int gather_default_variant() { return kDefaultShape; }
@@ -604,21 +610,21 @@ const char* gather_variant_name(int v) {
 }
 
 void launch_gather(const VMParams& p, const PhotonTree& tree, TreePhotons tp, QueryBuf qb, const uint32_t* order,
-                   long long nq, double* accum, void* parked, unsigned long long* counters, cudaStream_t s,
+                   long long nq, double* accum, const ParkedList& parked, unsigned long long* counters, cudaStream_t s,
                    int variant, const unsigned long long* nq_dev, const int* skip) {
     if (nq <= 0 || tree.n <= 0) return;
     const EvalSink sink{p, qb, tp, tree.id, accum};
     launch_variant(variant, chunk_tree(tree, tp.t0), reinterpret_cast<const float*>(qb.q0), 4, order, nq, nq_dev,
-                   skip, p.radius_sqr, sink, static_cast<uint4*>(parked), counters, p.error + ERR_GATHER, s);
+                   skip, p.radius_sqr, sink, parked, counters, p.error + ERR_GATHER, s);
 }
 
 void launch_gather_sets(const PhotonTree& tree, const float4* t0, const float* qpos, int qstride, const uint32_t* order,
                         long long nq, float r2, int* counts, const long long* offsets, int* cursor, int* idx,
-                        int variant, void* parked, unsigned long long* counters, int* err, cudaStream_t s) {
+                        int variant, const ParkedList& parked, unsigned long long* counters, int* err, cudaStream_t s) {
     if (nq <= 0 || tree.n <= 0) return;
     const SetSink sink{tree.id, counts, offsets, cursor, idx};
     launch_variant(variant, chunk_tree(tree, t0), qpos, qstride, order, nq, nullptr, nullptr, r2, sink,
-                   static_cast<uint4*>(parked), counters, err, s);
+                   parked, counters, err, s);
 }
 
 }  // namespace rc

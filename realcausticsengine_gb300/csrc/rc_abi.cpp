@@ -470,11 +470,18 @@ int reserve_photon_tree(long long n) {
     const size_t m = (size_t)std::max<long long>(n, 1), boxes = (size_t)2 << std::max(photon_chunk_level(n), 0);
     RC_CUDA(d.ph_order.reserve(m));
     RC_CUDA(d.ph_scratch.reserve(order_scratch_bytes(n)));
-    RC_CUDA(d.gather_parked.reserve(gather_parked_bytes()));
     RC_CUDA(d.tp0.reserve(m)); RC_CUDA(d.tp1.reserve(m)); RC_CUDA(d.tp2.reserve(m));
     RC_CUDA(d.box_lo.reserve(boxes)); RC_CUDA(d.box_hi.reserve(boxes));
     return RC_OK;
 }
+// The list of parked work for the gather's shape v, or the default shape where a parking one's
+// list (16 MB) cannot be had.  A capturing stream needs it reserved before (async_setup).
+int fitting_gather(DeviceState& d, int v) {
+    if (!gather_parks(v) || d.gather_parked.reserve(gather_parked_bytes(kParkedItems)) == cudaSuccess) return v;
+    cudaGetLastError();   // (the allocation's error)
+    return gather_default_variant();
+}
+ParkedList parked_list(const DeviceState& d) { return {d.gather_parked.p, kParkedItems}; }
 PhotonTree photon_tree(const DeviceState& d, long long n) { return {n, d.ph_order.p, d.box_lo.p, d.box_hi.p}; }
 
 int check_errors() {
@@ -1021,13 +1028,13 @@ int render_iteration(HostScene& sc, int redo_iteration = -1, bool tune_passes = 
     int variant = gather_default_variant();
     if (cfg().autotune && nq > 0) {
         std::atomic<int>& slot = gather_slot((long long)nq, n);
-        if (slot.load() < 0) {
+        if (slot.load() < 0 && gather_parks(fitting_gather(d, gather_variants() - 1))) {
             d.tuned = true;
             // time every launch shape on this iteration's queries into a scratch image
             RC_CUDA(d.tune_accum.reserve(std::max<long long>(3 * npix, 1)));
             ShapeTimer t{s, d.evm[0], d.evm[1], g_gather_loaded, "gather", cfg().verbose != 0};
             auto run = [&](int v) {
-                launch_gather(p, tree, tph, qb, d.qorder.p, (long long)nq, d.tune_accum.p, d.gather_parked.p, nullptr, s, v);
+                launch_gather(p, tree, tph, qb, d.qorder.p, (long long)nq, d.tune_accum.p, parked_list(d), nullptr, s, v);
             };
             for (int v = 0; v < gather_variants(); ++v) {
                 if (v == 0 || gather_parks(v) != gather_parks(v - 1)) {   // another query order
@@ -1041,13 +1048,13 @@ int render_iteration(HostScene& sc, int redo_iteration = -1, bool tune_passes = 
                 std::printf("{\"autotune\": \"gather\", \"queries\": %llu, \"variant\": \"%s\", \"ms\": %.3f}\n",
                             nq, gather_variant_name(t.best_v), t.best);
         }
-        variant = slot.load();
+        if (slot.load() >= 0) variant = fitting_gather(d, slot.load());
     }
     order_queries(variant, &qlaunch);
     unsigned long long gc[4] = {0, 0, 0, 0};
     RC_CUDA(cudaMemsetAsync(d.counters.p + 2, 0, 4 * sizeof(unsigned long long), s));
     RC_CUDA(cudaEventRecord(d.evg[0], s));
-    launch_gather(p, tree, tph, qb, d.qorder.p, (long long)nq, d.accum.p, d.gather_parked.p, d.counters.p + 2, s, variant);
+    launch_gather(p, tree, tph, qb, d.qorder.p, (long long)nq, d.accum.p, parked_list(d), d.counters.p + 2, s, variant);
     RC_CUDA(cudaEventRecord(d.evg[1], s));
     RC_CUDA(cudaGetLastError());
     RC_CUDA(cudaEventRecord(d.ev[7], s));
@@ -1159,6 +1166,7 @@ int async_setup(const HostScene& sc) {
     d.async_cvar = var(camera_slot(npix).load(), kUntunedPass);
     d.async_gvar = var(gather_slot((long long)d.last_queries, (long long)d.last_photons).load(), gather_default_variant());
     if (!cfg().autotune) d.async_lvar = d.async_cvar = 0, d.async_gvar = gather_default_variant();
+    d.async_gvar = fitting_gather(d, d.async_gvar);
     // the staged passes' scratch: reserved before any capture
     const long long paths = cfg().photons_per_iter > 0 ? cfg().photons_per_iter : npix;
     void* park = nullptr;
@@ -1223,7 +1231,7 @@ int async_tail(HostScene& sc, const VMParams& p, cudaStream_t s, cudaStream_t si
     RC_CUDA(record(d.ev[6], s));
     RC_CUDA(cudaMemsetAsync(d.counters.p + 2, 0, 4 * sizeof(unsigned long long), s));
     RC_CUDA(record(d.evg[0], s));
-    launch_gather(p, tree, tph, qb, d.qorder.p, qc, d.accum.p, d.gather_parked.p, d.counters.p + 2, s, d.async_gvar,
+    launch_gather(p, tree, tph, qb, d.qorder.p, qc, d.accum.p, parked_list(d), d.counters.p + 2, s, d.async_gvar,
                   d.counters.p + 1, flag);
     RC_CUDA(record(d.evg[1], s));
     RC_CUDA(record(d.ev[7], s));
@@ -2637,7 +2645,13 @@ int rc_device_bus_id(char* out, int len) {
     return RC_OK;
 }
 
-static thread_local uint32_t t_parked_items = 0;
+static thread_local uint32_t t_parked_items = 0, t_parked_room = (1u << 16) - 1u;
+
+int rc_gather_parked_limit(long long items) {
+    if (items < 1 || items > (long long)kParkedItems) { ctx().err = "parked list length out of range"; return RC_E_INVALID; }
+    t_parked_room = (uint32_t)items;
+    return RC_OK;
+}
 
 long long rc_gather_parked_items(void) { return t_parked_items; }
 
@@ -2666,14 +2680,14 @@ int rc_gather_query(int variant, int n, const float* positions, int q, const flo
     if (!r && q > 0) {
         r = [&]() -> int {
             RC_CUDA(qp.reserve(3 * (size_t)q)); RC_CUDA(cnt.reserve(q)); RC_CUDA(cur.reserve(q)); RC_CUDA(off.reserve(q));
-            RC_CUDA(err.reserve(1)); RC_CUDA(ord.reserve(q)); RC_CUDA(parked.reserve(gather_parked_bytes()));
+            RC_CUDA(err.reserve(1)); RC_CUDA(ord.reserve(q)); RC_CUDA(parked.reserve(gather_parked_bytes(t_parked_room)));
             RC_CUDA(osc.reserve(order_scratch_bytes(q)));
             RC_CUDA(cudaMemcpyAsync(qp.p, queries, 12 * (size_t)q, cudaMemcpyHostToDevice, s));
             RC_CUDA(cudaMemsetAsync(cnt.p, 0, 4 * (size_t)q, s));
             RC_CUDA(cudaMemsetAsync(err.p, 0, sizeof(int), s));
             launch_query_order(qp.p, 3, q, points_frame(q, queries, r2), gather_parks(variant), osc.p, ord.p, nullptr, s);
-            launch_gather_sets(tree, t0.p, qp.p, 3, ord.p, q, r2, cnt.p, nullptr, nullptr, nullptr, variant, parked.p,
-                               nullptr, err.p, s);
+            launch_gather_sets(tree, t0.p, qp.p, 3, ord.p, q, r2, cnt.p, nullptr, nullptr, nullptr, variant,
+                               ParkedList{parked.p, t_parked_room}, nullptr, err.p, s);
             RC_CUDA(cudaGetLastError());
             int h = 0;
             t_parked_items = 0;
@@ -2691,8 +2705,8 @@ int rc_gather_query(int variant, int n, const float* positions, int q, const flo
                 RC_CUDA(out.reserve(t));
                 RC_CUDA(cudaMemcpyAsync(off.p, offs.data(), 8 * (size_t)q, cudaMemcpyHostToDevice, s));
                 RC_CUDA(cudaMemsetAsync(cur.p, 0, 4 * (size_t)q, s));
-                launch_gather_sets(tree, t0.p, qp.p, 3, ord.p, q, r2, nullptr, off.p, cur.p, out.p, variant, parked.p,
-                                   nullptr, err.p, s);
+                launch_gather_sets(tree, t0.p, qp.p, 3, ord.p, q, r2, nullptr, off.p, cur.p, out.p, variant,
+                                   ParkedList{parked.p, t_parked_room}, nullptr, err.p, s);
                 RC_CUDA(cudaGetLastError());
                 RC_CUDA(cudaMemcpyAsync(idx, out.p, 4 * (size_t)t, cudaMemcpyDeviceToHost, s));
                 RC_CUDA(cudaStreamSynchronize(s));

@@ -192,11 +192,14 @@ void launch_query_order(const float* qpos, int stride, long long nq, const Curve
 // photon-query pairs, photon tests (chunk photons x overlapping queries), chunks
 // tested, boxes tested.  With nq_dev the query count is read on the device (bounded by
 // num_queries, the capacity the grid is sized for) and a non-zero *skip makes the
-// launch a no-op.  Needs the boxes and the sorted records (launch_photon_order) and
-// gather_parked_bytes() of scratch at `parked`, its own until the launch has ended.
-size_t gather_parked_bytes();
+// launch a no-op.  Needs the boxes and the sorted records (launch_photon_order) and, for a
+// shape that parks (gather_parks), the list of parked work: gather_parked_bytes(items) at p,
+// its own until the launch has ended.
+struct ParkedList { void* p; uint32_t items; };
+constexpr uint32_t kParkedItems = (1u << 20) - 1u;   // a render's list (16 MB)
+size_t gather_parked_bytes(uint32_t items);
 void launch_gather(const VMParams& p, const PhotonTree& tree, TreePhotons tp, QueryBuf qb, const uint32_t* order,
-                   long long num_queries, double* accum, void* parked, unsigned long long* counters, cudaStream_t s,
+                   long long num_queries, double* accum, const ParkedList& parked, unsigned long long* counters, cudaStream_t s,
                    int variant, const unsigned long long* nq_dev = nullptr, const int* skip = nullptr);
 // Parity hook: the same kernel with a sink that records each query's photon ids
 // (tree.id of the accepted positions).  Without offsets it adds each query's count into
@@ -206,7 +209,7 @@ void launch_gather(const VMParams& p, const PhotonTree& tree, TreePhotons tp, Qu
 // if a traversal stack would overflow (cannot happen for n < 2^28).
 void launch_gather_sets(const PhotonTree& tree, const float4* t0, const float* qpos, int qstride, const uint32_t* order,
                         long long nq, float r2, int* counts, const long long* offsets, int* cursor, int* idx,
-                        int variant, void* parked, unsigned long long* counters, int* err, cudaStream_t s);
+                        int variant, const ParkedList& parked, unsigned long long* counters, int* err, cudaStream_t s);
 int gather_variants();
 bool gather_parks(int variant);   // two launches
 int gather_default_variant();
