@@ -52,7 +52,7 @@ METRIC = "photons/s"
 PHOTON_BYTES, QUERY_BYTES, PIXEL_BYTES = 40, 64, 48
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) over algorithmic bytes of one
 # k_gather launch on the 960x540 / 4M-path water pool (profiles/k_gather_water_pool_960x540.md)
-GATHER_TRAFFIC_OVER_ALGORITHMIC = 1.161
+GATHER_TRAFFIC_OVER_ALGORITHMIC = 1.138
 # SM issue efficiency of the staged light pass from the same kind of capture, its two
 # launches together (profiles/light_pass_staged_water_pool_960x540.md): issue-active cycles and thread
 # instructions per warp instruction
@@ -310,8 +310,8 @@ def run_ours(args):
     e2e_value = paths * args.steps * world / e2e_s
     peak, peak_kind = measured_peaks()
     achieved = gather_bytes / (gather_ms_mean / 1000.0) / 1e9 if gather_ms_mean > 0 else 0.0
-    # DRAM bytes of one gather: the ncu capture on the 960x540 / 4M-path case moved
-    # 1.161x its algorithmic bytes; scaled to this workload's launch by its algorithmic
+    # DRAM bytes of one gather: what the ncu capture on the 960x540 / 4M-path case moved
+    # over its algorithmic bytes; scaled to this workload's launch by its algorithmic
     # bytes (photon, query and pixel records all scale with their counts)
     traffic = GATHER_TRAFFIC_OVER_ALGORITHMIC * gather_bytes
     touched = PHOTON_BYTES * st["merged"]
