@@ -1133,6 +1133,18 @@ bool passes_untimed(const HostScene& sc) {
            (camera_slot(npix).load() < 0 && staged_fits(ctx(), d.camera_park, npix));
 }
 
+// The launch shapes of replayed light and camera passes: the timed ones, or, where nothing
+// was timed, kUntunedPass.  Their scratch is reserved here, before any capture.
+void async_pass_shapes(const HostScene& sc) {
+    DeviceState& d = ctx().dev;
+    const long long npix = (long long)sc.camera.width * sc.camera.height;
+    const long long paths = cfg().photons_per_iter > 0 ? cfg().photons_per_iter : npix;
+    auto timed = [](int v) { return !cfg().autotune ? 0 : v >= 0 ? v : kUntunedPass; };
+    void* park = nullptr;
+    d.async_lvar = fitting_shape(ctx(), d.light_park, timed(light_slot(paths).load()), paths, &park);
+    d.async_cvar = fitting_shape(ctx(), d.camera_park, timed(camera_slot(npix).load()), npix, &park);
+}
+
 int async_setup(const HostScene& sc) {
     DeviceState& d = ctx().dev;
     const long long npix = (long long)sc.camera.width * sc.camera.height;
@@ -1161,17 +1173,9 @@ int async_setup(const HostScene& sc) {
     RC_CUDA(d.qorder.reserve(d.async_qcap));
     RC_CUDA(d.qscratch.reserve(order_scratch_bytes(d.async_qcap)));
     RC_CUDA(d.accum.reserve(3 * npix));
-    auto var = [](int v, int dflt) { return v >= 0 ? v : dflt; };
-    d.async_lvar = var(light_slot(cfg().photons_per_iter > 0 ? cfg().photons_per_iter : npix).load(), kUntunedPass);
-    d.async_cvar = var(camera_slot(npix).load(), kUntunedPass);
-    d.async_gvar = var(gather_slot((long long)d.last_queries, (long long)d.last_photons).load(), gather_default_variant());
-    if (!cfg().autotune) d.async_lvar = d.async_cvar = 0, d.async_gvar = gather_default_variant();
-    d.async_gvar = fitting_gather(d, d.async_gvar);
-    // the staged passes' scratch: reserved before any capture
-    const long long paths = cfg().photons_per_iter > 0 ? cfg().photons_per_iter : npix;
-    void* park = nullptr;
-    d.async_lvar = fitting_shape(ctx(), d.light_park, d.async_lvar, paths, &park);
-    d.async_cvar = fitting_shape(ctx(), d.camera_park, d.async_cvar, npix, &park);
+    const int g = gather_slot((long long)d.last_queries, (long long)d.last_photons).load();
+    d.async_gvar = fitting_gather(d, cfg().autotune && g >= 0 ? g : gather_default_variant());
+    async_pass_shapes(sc);
     return RC_OK;
 }
 
@@ -1355,8 +1359,10 @@ int async_finish(HostScene& sc, int first_it, int n_async, bool windows) {
         if (r) return r;
     }
     if (cfg().verbose)
-        std::printf("{\"replayed_iterations\": %d, \"redone\": %d, \"photon_capacity\": %lld, \"query_capacity\": %lld}\n",
-                    n_async, (int)std::count(flags.begin(), flags.end(), 1), d.async_pcap, d.async_qcap);
+        std::printf("{\"replayed_iterations\": %d, \"redone\": %d, \"photon_capacity\": %lld, \"query_capacity\": %lld, "
+                    "\"light_shape\": %d, \"camera_shape\": %d}\n",
+                    n_async, (int)std::count(flags.begin(), flags.end(), 1), d.async_pcap, d.async_qcap,
+                    windows ? d.async_lvar : -1, windows ? d.async_cvar : -1);
     return RC_OK;
 }
 
@@ -1397,6 +1403,8 @@ int render_iterations(HostScene& sc, int iterations) {
     }
     const int n_async = iterations - i;
     if (n_async <= 0) return RC_OK;
+    // (again here: another context may have timed the shapes since the capacities were set)
+    async_pass_shapes(sc);
     // the replayed iterations' camera branch writes the query buffers that an eager
     // iteration's side-stream camera pass may still be writing (after an error return)
     RC_CUDA(cudaStreamSynchronize(d.side));
