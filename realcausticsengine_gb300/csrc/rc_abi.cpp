@@ -11,7 +11,9 @@
 #include <cstdio>
 #include <cstring>
 #include <memory>
+#include <mutex>
 #include <new>
+#include <shared_mutex>
 #include <string>
 #include <vector>
 
@@ -627,6 +629,38 @@ int proposal_train(const HostScene& sc, const VMParams& p) {
     return RC_OK;
 }
 
+// Rendering calls of several threads run beside one another, but not beside the timing of
+// launch shapes: a shape timed beside another scene's passes measures those too, and the
+// choice is kept for every context (64 scenes rendered alone from two threads after a batch:
+// an iteration of each took 298 ms in shapes timed beside one another, 277 in shapes timed
+// quietly).  RenderCall is held for a rendering call; QuietGpu waits until no other
+// thread holds one, and lets none begin (g_quiet_gate) until it ends.
+std::mutex g_quiet_gate;
+std::shared_mutex g_rendering;
+thread_local int t_rendering = 0;   // RenderCalls of this thread, one within another
+struct RenderCall {
+    RenderCall() {
+        if (t_rendering++ > 0) return;
+        std::lock_guard<std::mutex> g(g_quiet_gate);
+        g_rendering.lock_shared();
+    }
+    ~RenderCall() { if (--t_rendering == 0) g_rendering.unlock_shared(); }
+    RenderCall(const RenderCall&) = delete;
+};
+struct QuietGpu {
+    QuietGpu() {
+        if (t_rendering > 0) g_rendering.unlock_shared();
+        g_quiet_gate.lock();
+        g_rendering.lock();
+    }
+    ~QuietGpu() {
+        g_rendering.unlock();
+        if (t_rendering > 0) g_rendering.lock_shared();
+        g_quiet_gate.unlock();
+    }
+    QuietGpu(const QuietGpu&) = delete;
+};
+
 // Autotuner.  ShapeTimer times launch shapes on s between two events: each once, after one
 // untimed launch of the shape if the process has not launched it yet (the first launch loads
 // its code; `loaded` has a bit per shape).
@@ -672,14 +706,16 @@ int pick_pass_shape(ShapeTimer& t, Run&& run) {
     return t.best_v;
 }
 template <class Run>
-int autotune_pass(std::atomic<unsigned>& loaded, const char* what, long long size, Run&& run) {
+void autotune_pass(std::atomic<int>& slot, std::atomic<unsigned>& loaded, const char* what, long long size, Run&& run) {
     DeviceState& d = ctx().dev;
+    QuietGpu quiet;
+    if (slot.load() >= 0) return;   // (timed by another thread meanwhile)
     d.tuned = true;
     ShapeTimer t{d.stream, d.evm[0], d.evm[1], loaded, what, cfg().verbose != 0};
-    const int v = pick_pass_shape(t, run);
+    slot = pick_pass_shape(t, run);
     if (t.verbose)
-        std::printf("{\"autotune\": \"%s\", \"size\": %lld, \"variant\": %d, \"ms\": %.3f}\n", what, size, v, t.best);
-    return v;
+        std::printf("{\"autotune\": \"%s\", \"size\": %lld, \"variant\": %d, \"ms\": %.3f}\n", what, size, slot.load(),
+                    t.best);
 }
 
 int size_class(long long n) { return n > 0 ? 63 - __builtin_clzll((unsigned long long)n) : 0; }
@@ -902,7 +938,7 @@ int render_iteration(HostScene& sc, int redo_iteration = -1, bool tune_passes = 
         if (sampler == RC_SAMPLER_UNIFORM && cfg().autotune) {
             std::atomic<int>& slot = light_slot(p.num_light_paths);
             if (slot.load() < 0 && tune_passes && staged_fits(ctx(), d.light_park, p.num_light_paths))
-                slot = autotune_pass(g_light_loaded, "light pass", p.num_light_paths, [&](int v) {
+                autotune_pass(slot, g_light_loaded, "light pass", p.num_light_paths, [&](int v) {
                     cudaMemsetAsync(d.counters.p, 0, sizeof(unsigned long long), s);
                     light_pass(p, ph, s, v);
                 });
@@ -995,7 +1031,7 @@ int render_iteration(HostScene& sc, int redo_iteration = -1, bool tune_passes = 
         if (cfg().autotune) {
             std::atomic<int>& slot = camera_slot(npix);
             if (slot.load() < 0 && tune_passes && staged_fits(ctx(), d.camera_park, npix))
-                slot = autotune_pass(g_camera_loaded, "camera pass", npix, [&](int v) {
+                autotune_pass(slot, g_camera_loaded, "camera pass", npix, [&](int v) {
                     cudaMemsetAsync(d.counters.p + 1, 0, sizeof(unsigned long long), s);
                     camera_pass(p, qb, s, v);
                 });
@@ -1029,24 +1065,27 @@ int render_iteration(HostScene& sc, int redo_iteration = -1, bool tune_passes = 
     if (cfg().autotune && nq > 0) {
         std::atomic<int>& slot = gather_slot((long long)nq, n);
         if (slot.load() < 0 && gather_parks(fitting_gather(d, gather_variants() - 1))) {
-            d.tuned = true;
-            // time every launch shape on this iteration's queries into a scratch image
-            RC_CUDA(d.tune_accum.reserve(std::max<long long>(3 * npix, 1)));
-            ShapeTimer t{s, d.evm[0], d.evm[1], g_gather_loaded, "gather", cfg().verbose != 0};
-            auto run = [&](int v) {
-                launch_gather(p, tree, tph, qb, d.qorder.p, (long long)nq, d.tune_accum.p, parked_list(d), nullptr, s, v);
-            };
-            for (int v = 0; v < gather_variants(); ++v) {
-                if (v == 0 || gather_parks(v) != gather_parks(v - 1)) {   // another query order
-                    order_queries(v, nullptr);
-                    run(v);   // (photons and queries into L2)
+            QuietGpu quiet;
+            if (slot.load() < 0) {   // (not timed by another thread meanwhile)
+                d.tuned = true;
+                // time every launch shape on this iteration's queries into a scratch image
+                RC_CUDA(d.tune_accum.reserve(std::max<long long>(3 * npix, 1)));
+                ShapeTimer t{s, d.evm[0], d.evm[1], g_gather_loaded, "gather", cfg().verbose != 0};
+                auto run = [&](int v) {
+                    launch_gather(p, tree, tph, qb, d.qorder.p, (long long)nq, d.tune_accum.p, parked_list(d), nullptr, s, v);
+                };
+                for (int v = 0; v < gather_variants(); ++v) {
+                    if (v == 0 || gather_parks(v) != gather_parks(v - 1)) {   // another query order
+                        order_queries(v, nullptr);
+                        run(v);   // (photons and queries into L2)
+                    }
+                    t.time(v, run);
                 }
-                t.time(v, run);
+                slot = t.best_v;
+                if (cfg().verbose)
+                    std::printf("{\"autotune\": \"gather\", \"queries\": %llu, \"variant\": \"%s\", \"ms\": %.3f}\n",
+                                nq, gather_variant_name(t.best_v), t.best);
             }
-            slot = t.best_v;
-            if (cfg().verbose)
-                std::printf("{\"autotune\": \"gather\", \"queries\": %llu, \"variant\": \"%s\", \"ms\": %.3f}\n",
-                            nq, gather_variant_name(t.best_v), t.best);
         }
         if (slot.load() >= 0) variant = fitting_gather(d, slot.load());
     }
@@ -1588,6 +1627,7 @@ int batch_render(Context* const* cs, int n, int iterations, double* out) {
     const bool time_light = light_choice.load() < 0 && staged_fits(*caller, B.light_park, most_paths);
     const bool time_camera = camera_choice.load() < 0 && staged_fits(*caller, B.camera_park, most_pixels);
     if (time_light || time_camera) {
+        QuietGpu quiet;
         const int m = (int)active[0].size();
         const BatchScene* sc0 = B.scenes.p + entry_at[0];
         const long long* pp = B.prefix.p + prefix_at[0];
@@ -2049,6 +2089,7 @@ int main(void) {
     // src/main.cpp:170-186: 1 = vertex merging, 2-4 = debug views (one pass, no
     // averaging), 5 = the mesh BVHs' boxes as OBJ files (host only, no image)
     const int mode = ctx().scene->debug_test;
+    RenderCall call;
     int r = mode == 5 ? prepare_host() : prepare();
     if (!r) {
         if (mode == 1) {
@@ -2230,6 +2271,7 @@ int rc_prepare_stats(double* out, int n) {
 
 int rc_render(int iterations) {
     if (iterations < 0) { ctx().err = "iterations < 0"; return RC_E_INVALID; }
+    RenderCall call;
     int r = prepare();
     if (!r) r = render_iterations(*ctx().scene, iterations);
     return r;
@@ -2251,11 +2293,13 @@ int rc_render_debug(int mode) {
 
 int rc_batch_render(rc_context* const* ctxs, int n, int iterations, double* out) {
     if (!ctxs || n < 1 || iterations < 0) { ctx().err = "rc_batch_render: bad arguments"; return RC_E_INVALID; }
+    RenderCall call;
     return batch_render(reinterpret_cast<Context* const*>(ctxs), n, iterations, out);
 }
 
 int rc_render_timed(int iterations, double* out) {
     if (iterations < 0 || !out) { ctx().err = "bad arguments"; return RC_E_INVALID; }
+    RenderCall call;
     int r = prepare();
     if (r) return r;
     DeviceState& d = ctx().dev;
