@@ -722,6 +722,17 @@ int size_class(long long n) { return n > 0 ? 63 - __builtin_clzll((unsigned long
 int triangle_class(long long n) { return std::min(size_class(n) / 2, 15); }
 std::atomic<int>& light_slot(long long paths) { return g_tune.light[size_class(paths)][triangle_class(ctx().dev.num_tris)]; }
 std::atomic<int>& camera_slot(long long pixels) { return g_tune.camera[size_class(pixels)][triangle_class(ctx().dev.num_tris)]; }
+// A shape timed for a class, or for the next one of paths (pixels); -1: none.  Scenes that
+// leave a batch take such a shape: 64 of them, rendered alone from two threads, need 0.32 s to
+// time what is missing (0.41 with a timing for every class), and an iteration of each takes
+// 272 ms (277).  Not the next one of triangles, where kinds of scenes differ (TuneTables).
+int near_shape(std::atomic<int> (&t)[64][16], long long n, long long tris) {
+    const int i = size_class(n), j = triangle_class(tris);
+    int v = t[i][j].load();
+    if (v < 0 && i > 0) v = t[i - 1][j].load();
+    if (v < 0 && i < 63) v = t[i + 1][j].load();
+    return v;
+}
 std::atomic<int>& gather_slot(long long queries, long long photons) {
     return g_tune.gather[size_class(queries)][size_class(photons) / 2];
 }
@@ -1163,25 +1174,26 @@ bool async_eligible() {
     return cfg().graph_replay && cfg().sampler == RC_SAMPLER_UNIFORM && !cfg().learned_proposal;
 }
 
-// The scene's light or camera pass has no timed shape and could be timed.
+// The scene's light or camera pass has no timed shape, nor a neighbouring class, and could be
+// timed.
 bool passes_untimed(const HostScene& sc) {
     DeviceState& d = ctx().dev;
     const long long npix = (long long)sc.camera.width * sc.camera.height;
     const long long paths = cfg().photons_per_iter > 0 ? cfg().photons_per_iter : npix;
-    return (light_slot(paths).load() < 0 && staged_fits(ctx(), d.light_park, paths)) ||
-           (camera_slot(npix).load() < 0 && staged_fits(ctx(), d.camera_park, npix));
+    return (near_shape(g_tune.light, paths, d.num_tris) < 0 && staged_fits(ctx(), d.light_park, paths)) ||
+           (near_shape(g_tune.camera, npix, d.num_tris) < 0 && staged_fits(ctx(), d.camera_park, npix));
 }
 
-// The launch shapes of replayed light and camera passes: the timed ones, or, where nothing
-// was timed, kUntunedPass.  Their scratch is reserved here, before any capture.
+// The launch shapes of replayed light and camera passes: the timed ones (near_shape), or,
+// where nothing was timed, kUntunedPass.  Their scratch is reserved here, before any capture.
 void async_pass_shapes(const HostScene& sc) {
     DeviceState& d = ctx().dev;
     const long long npix = (long long)sc.camera.width * sc.camera.height;
     const long long paths = cfg().photons_per_iter > 0 ? cfg().photons_per_iter : npix;
     auto timed = [](int v) { return !cfg().autotune ? 0 : v >= 0 ? v : kUntunedPass; };
     void* park = nullptr;
-    d.async_lvar = fitting_shape(ctx(), d.light_park, timed(light_slot(paths).load()), paths, &park);
-    d.async_cvar = fitting_shape(ctx(), d.camera_park, timed(camera_slot(npix).load()), npix, &park);
+    d.async_lvar = fitting_shape(ctx(), d.light_park, timed(near_shape(g_tune.light, paths, d.num_tris)), paths, &park);
+    d.async_cvar = fitting_shape(ctx(), d.camera_park, timed(near_shape(g_tune.camera, npix, d.num_tris)), npix, &park);
 }
 
 int async_setup(const HostScene& sc) {

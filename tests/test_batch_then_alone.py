@@ -22,8 +22,8 @@ def out(s):
 cs, rs = [Context(), Context()], []
 for k, c in enumerate(cs):
     with c:
-        rs.append(Renderer(scenes.water_pool(160, 90, grid=24), photons_per_iter=2600000, max_path_length=8, seed=4 + k,
-                           verbose=True))
+        rs.append(Renderer(scenes.water_pool(160, 90, grid=24), photons_per_iter=(2600000, {second})[k], max_path_length=8,
+                           seed=4 + k, verbose=True))
 batch_render(cs, 2)
 for c, r in zip(cs, rs):
     out("alone")
@@ -31,17 +31,20 @@ for c, r in zip(cs, rs):
         r.render(3)
         image = r.image()
 with cs[1]:
-    r = Renderer(scenes.water_pool(160, 90, grid=24), photons_per_iter=2600000, max_path_length=8, seed=5)
+    r = Renderer(scenes.water_pool(160, 90, grid=24), photons_per_iter={second}, max_path_length=8, seed=5)
     r.render(5)
     np.testing.assert_allclose(image, r.image(), rtol=1e-5, atol=1e-7)
 """
 
 
-def test_the_second_scene_of_a_class_replays_the_shapes_timed_for_the_first():
+@pytest.mark.parametrize("second", [2600000, 4500000, 1500000], ids=["the same class", "the next", "the one before"])
+def test_the_second_scene_of_a_class_replays_the_shapes_timed_for_the_first(second):
     """Both scenes get their capacities from the batch, in which nothing of their own was
-    timed.  The first one rendered alone times the class; the second one has nothing left to
-    time and must not stay with the shapes that it was given in the batch."""
-    out = subprocess.run([sys.executable, "-c", TWO.format(root=str(ROOT))], capture_output=True, text=True, timeout=300)
+    timed.  The first one rendered alone times its class; the second one, of that class of
+    paths or a neighbouring one, has nothing left to time and must not stay with the shapes
+    that it was given in the batch."""
+    out = subprocess.run([sys.executable, "-c", TWO.format(root=str(ROOT), second=second)], capture_output=True, text=True,
+                         timeout=300)
     assert out.returncode == 0, out.stderr
     first, second = [[json.loads(line) for line in part.splitlines() if line.startswith('{"autotune":') or
                       line.startswith('{"replayed_iterations":')] for part in out.stdout.split("alone\n")[1:3]]
