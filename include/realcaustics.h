@@ -126,8 +126,9 @@ typedef struct rc_config {
      * queries and differ only in their photons. */
     unsigned long long camera_seed;
     /* 1 (default): the first iteration of each size class times the launch shapes of
-     * the light pass, the camera pass (block size x register cap) and the gather
-     * (resident blocks per SM x queries per warp) and keeps the fastest for the process;
+     * the light pass, the camera pass (block size x register cap, or staged) and the gather
+     * (resident blocks per SM x queries per warp x levels per step, or parking) and keeps the
+     * fastest for the process; rendering calls of other threads wait meanwhile.
      * 0: the fixed default shapes. */
     int autotune;
     /* 1 (default): with the uniform sampler and no learned proposal, when an iteration
@@ -187,7 +188,8 @@ int rc_scene_dump(int which, unsigned* out, long long cap, long long* words);
  * the reference's single global scene, from any thread.  A thread that binds its own
  * context holds its own scene, configuration, last error and device buffers (and a CUDA
  * stream): scenes in different contexts render concurrently from different threads.
- * Autotuner choices are shared by all contexts.  rc_context_bind(NULL) returns the
+ * Autotuner choices are shared by all contexts (and timed while no other thread
+ * renders).  rc_context_bind(NULL) returns the
  * thread to the default context.  rc_context_destroy releases the context's scene and
  * device memory; it must not be bound or in use on another thread. */
 typedef struct rc_context rc_context;
